@@ -390,8 +390,17 @@ void Tracer::release_instanced() {
     two_level_ok_ = 0;
 }
 
+void Tracer::drop_graphs() {
+    for (cudaGraphExec_t& g : wf_exec_) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    wf_graph_key_.clear();
+}
+
 void Tracer::free_all() {
     release_instanced();
+    drop_graphs();
     for (int k = 0; k < kSceneBufs; ++k) {
         if (bufs_[k]) dev_free(bufs_[k]);
         bufs_[k] = nullptr;
@@ -455,7 +464,7 @@ void texture_tables(unsigned char perm512[512], const float** marble30) {
 Tracer::~Tracer() {
     free_all();
     if (wf_counts_host_) cudaFreeHost(wf_counts_host_);
-    if (wf_ctl_host_) cudaFreeHost(wf_ctl_host_);
+    drop_graphs();
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
     for (cudaEvent_t e : wf_ev_)
@@ -1110,6 +1119,16 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     const long chunk_total = batch_max;
     const bool cache = cache_mode != 0 && mlp != nullptr && mlp->ready();
     const long P = std::max<long>(1, std::min<long>(chunk_total, wf_pool > 0 ? wf_pool : auto_pool(cache)));
+    // the parameters the wavefront's kernels read; the sampler's are each view's own
+    RenderParams rpw{};
+    rpw.max_bounce = rp.max_bounce;
+    rpw.rr_start = rp.rr_start;
+    rpw.film = rp.film;
+    rpw.sample_L = rp.sample_L;
+    rpw.sample_sig = rp.sample_sig;
+    rpw.counters = rp.counters;
+    rpw.err = rp.err;
+    rpw.trace_sample = -1;
     WfState st{};
     if (wf_cap_ < P) {
         for (int k : {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26,
@@ -1119,10 +1138,11 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         }
         wf_cap_ = 0;
         const size_t n = (size_t)P;
+        // [31]: the counts, and the control block after them (one copy reads both back)
         const size_t sizes[] = {4 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n,                       // pix smp draw flags pend vis
                                 16 * n, 16 * n, 16 * n, 16 * n, 8 * n, 8 * n, 4 * n, 16 * n,  // ro rd beta L pf sig hprim huvi
                                 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n,  // sh_* mis_* ld nee
-                                8 * n, 8 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n, 256,  // ev mis_hit queues counts
+                                8 * n, 8 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n, kWfCountsBytes + sizeof(WfCtl),  // ev mis_hit queues counts
                                 4 * n};                                                           // wid
         for (size_t k = 0; k < sizeof sizes / sizeof sizes[0]; ++k) TRY(dev_alloc(&wf_bufs_[k], sizes[k]));
         TRY(dev_alloc(&wf_bufs_[35], 4 * (size_t)kShadeClasses * n));  // class-grouped shade lists
@@ -1138,7 +1158,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         TRY(dev_alloc(&wf_bufs_[34], 4 * (size_t)chunk_total));
         wf_fs_cap_ = chunk_total;
     }
-    if (!wf_counts_host_) TRY(cudaMallocHost((void**)&wf_counts_host_, 64));
+    if (!wf_counts_host_) TRY(cudaMallocHost((void**)&wf_counts_host_, kWfCountsBytes + sizeof(WfCtl)));
     void** b = wf_bufs_;
     st.pix = (int32_t*)b[0]; st.smp = (int32_t*)b[1]; st.draw = (uint32_t*)b[2]; st.flags = (uint32_t*)b[3];
     st.pend = (uint32_t*)b[4]; st.vis = (uint32_t*)b[5];
@@ -1231,47 +1251,42 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     const bool two_level = wide && sv.ninst > 0;
     unsigned tb = wf_trace_blocks_[two_level ? 2 : (wide ? 0 : 1)];
     if (trace_blocks_per_sm > 0) tb = std::min(tb, (unsigned)trace_blocks_per_sm * wf_sms_);
-    const unsigned cgrid = (unsigned)((P + kCompactTile - 1) / kCompactTile);
+    const unsigned cgrid = (unsigned)std::min<long>((P + kCompactTile - 1) / kCompactTile, wf_sms_ * kWfGridPerSm / 2);
     const dim3 gblock(32, 4);
-    // control block (device) and its host mirror
-    if (!wf_bufs_[47]) TRY(dev_alloc(&wf_bufs_[47], sizeof(WfCtl)));
-    WfCtl* d_ctl = (WfCtl*)wf_bufs_[47];
-    if (!wf_ctl_host_) TRY(cudaMallocHost((void**)&wf_ctl_host_, sizeof(WfCtl)));
-    WfCtl* h_ctl = (WfCtl*)wf_ctl_host_;
-    // graph mode: one iteration captured twice (path-ray list in q_a or in q_b), launched in groups
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-    auto free_graphs = [&]() {
-        for (cudaGraphExec_t& g : gexec)
-            if (g) cudaGraphExecDestroy(g);
-    };
+    // control block (device, after the counts) and its host mirror
+    WfCtl* d_ctl = (WfCtl*)((unsigned char*)st.counts + kWfCountsBytes);
+    WfCtl* h_ctl = (WfCtl*)((unsigned char*)wf_counts_host_ + kWfCountsBytes);
+    const unsigned list_grid = wf_sms_ * kWfGridPerSm;
     auto launch_iteration = [&](int32_t* q_ext, int32_t* q_fin, bool full, uint32_t take, uint32_t n_ext,
                                 uint32_t n_fin, uint32_t nray, uint32_t n_query) -> std::string {
         // full: grids for the largest lists (graph mode); else sized to the host's counts
         k_wf_control<<<1, 32, 0, s>>>(st, d_ctl);
         if (!full) TRY(cudaEventRecord(wf_ev_[0], s));
-        if (full || take) k_wf_generate<<<full ? blocks(P) : blocks(take), kWfBlock, 0, s>>>(sv, rp, st, q_ext, d_ctl);
+        if (full || take)
+            k_wf_generate<<<std::min(full ? blocks(P) : blocks(take), list_grid), kWfBlock, 0, s>>>(st, q_ext, d_ctl);
         if (!full) TRY(cudaEventRecord(wf_ev_[1], s));
         if (full || nray) {
-            const unsigned g = full ? tb : std::min(blocks(nray), tb);
-            if (two_level) k_wf_trace<true, true><<<g, kWfBlock, 0, s>>>(sv, rp, st, q_ext, d_ctl, st.counts + 8, bvh.n);
-            else if (wide) k_wf_trace<true><<<g, kWfBlock, 0, s>>>(sv, rp, st, q_ext, d_ctl, st.counts + 8, bvh.n);
-            else k_wf_trace<false><<<g, kWfBlock, 0, s>>>(sv, rp, st, q_ext, d_ctl, st.counts + 8, bvh.n);
+            const unsigned g = full ? tb : (unsigned)std::min<long>(nray, tb);
+            if (two_level) k_wf_trace<true, true><<<g, kWfBlock, 0, s>>>(sv, rpw, st, q_ext, d_ctl, st.counts + 8, bvh.n);
+            else if (wide) k_wf_trace<true><<<g, kWfBlock, 0, s>>>(sv, rpw, st, q_ext, d_ctl, st.counts + 8, bvh.n);
+            else k_wf_trace<false><<<g, kWfBlock, 0, s>>>(sv, rpw, st, q_ext, d_ctl, st.counts + 8, bvh.n);
         }
         if (st.cache && (full || n_query)) {  // the previous shade's cache queries, before finalize adds them
-            const std::string me = mlp->forward(st.feat, full ? (int)P : (int)n_query, (float*)st.cache_L, rp.err, s,
+            const std::string me = mlp->forward(st.feat, full ? (int)P : (int)n_query, (float*)st.cache_L, rpw.err, s,
                                                 st.q_cache, 4, &d_ctl->n_query);
             if (!me.empty()) return me;
         }
         if (!full) TRY(cudaEventRecord(wf_ev_[2], s));
         if (full || n_fin) {
-            const unsigned g = full ? blocks(P) : blocks(n_fin);
-            if (rec) k_wf_finalize<true><<<g, kWfBlock, 0, s>>>(sv, rp, st, q_fin, d_ctl);
-            else k_wf_finalize<false><<<g, kWfBlock, 0, s>>>(sv, rp, st, q_fin, d_ctl);
+            const unsigned g = std::min(full ? blocks(P) : blocks(n_fin), list_grid);
+            if (rec) k_wf_finalize<true><<<g, kWfBlock, 0, s>>>(sv, rpw, st, q_fin, d_ctl);
+            else k_wf_finalize<false><<<g, kWfBlock, 0, s>>>(sv, rpw, st, q_fin, d_ctl);
         }
         if (!full) TRY(cudaEventRecord(wf_ev_[3], s));
         if (full || n_ext) {
             const unsigned g = full ? blocks(P) : blocks(n_ext);
-            k_wf_classify<<<g, kWfBlock, 0, s>>>(sv, st, q_ext, d_ctl, (int)P);
+            const long tiles = ((full ? P : (long)n_ext) + kClassifyTile - 1) / kClassifyTile;
+            k_wf_classify<<<(unsigned)std::min<long>(tiles, list_grid), kWfBlock, 0, s>>>(st, q_ext, d_ctl, (int)P);
             const unsigned gs = std::min(g, shade_grid_);
             TRY(cudaEventRecord(shade_fork_, s));
             int nb = 0;
@@ -1279,7 +1294,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
                 if (!shade_used_[c]) continue;
                 cudaStream_t cs = shade_streams_[nb];
                 TRY(cudaStreamWaitEvent(cs, shade_fork_, 0));
-                const std::string le = launch_shade(rec, c, shade_lm_[c], shade_tex_[c], gs, sv, rp, st, (int)P, cs);
+                const std::string le = launch_shade(rec, c, shade_lm_[c], shade_tex_[c], gs, sv, rpw, st, (int)P, cs);
                 if (!le.empty()) return le;
                 TRY(cudaEventRecord(shade_join_[nb], cs));
                 ++nb;
@@ -1287,31 +1302,63 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
             for (int k = 0; k < nb; ++k) TRY(cudaStreamWaitEvent(s, shade_join_[k], 0));
         }
         if (!full) TRY(cudaEventRecord(wf_ev_[4], s));
-        k_wf_compact<<<cgrid, kCompactThreads, 0, s>>>(st, q_fin, (int)P);
+        k_wf_compact<<<cgrid, kCompactThreads, 0, s>>>(st, q_fin, d_ctl, (int)P);
         if (!full) TRY(cudaEventRecord(wf_ev_[5], s));
         TRY(cudaGetLastError());
         return "";
     };
+    // graph mode: one iteration captured twice (path-ray list in q_a or in q_b).  The pair is
+    // kept for the next render while everything the kernels were captured with -- their
+    // parameters by value, the grids and the launched variants -- is the same bytes: capture and
+    // instantiation cost 0.2 ms, a quarter of a thumbnail's render.
     const bool graph = wf_graph != 0;
     if (graph) {
-        for (int k = 0; k < 2; ++k) {
-            cudaGraph_t g = nullptr;
-            TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            const std::string ce = launch_iteration(k ? st.q_b : st.q_a, k ? st.q_a : st.q_b, true, 0, 0, 0, 0, 0);
-            cudaGraph_t gg = nullptr;
-            const cudaError_t ee = cudaStreamEndCapture(s, &gg);
-            g = gg;
-            if (!ce.empty() || ee != cudaSuccess) {
-                if (g) cudaGraphDestroy(g);
-                free_graphs();
-                return ce.empty() ? std::string("graph capture: ") + cudaGetErrorString(ee) : ce;
+        struct {
+            SceneView sv;
+            RenderParams rp;
+            WfState st;
+            long P;
+            const void* mlp;
+            int32_t nleaf, rec;
+            unsigned tb;
+            int32_t used[kShadeClasses], lm[kShadeClasses], tex[kShadeClasses];
+        } key;
+        memset(&key, 0, sizeof key);
+        key.sv = sv;
+        key.rp = rpw;
+        key.st = st;
+        key.P = P;
+        key.mlp = cache ? mlp : nullptr;
+        key.nleaf = bvh.n;
+        key.rec = rec;
+        key.tb = tb;
+        for (int c = 0; c < kShadeClasses; ++c) {
+            key.used[c] = shade_used_[c];
+            key.lm[c] = shade_lm_[c];
+            key.tex[c] = shade_tex_[c];
+        }
+        const std::string kb((const char*)&key, sizeof key);
+        if (kb != wf_graph_key_) {
+            drop_graphs();
+            for (int k = 0; k < 2; ++k) {
+                TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+                const std::string ce = launch_iteration(k ? st.q_b : st.q_a, k ? st.q_a : st.q_b, true, 0, 0, 0, 0, 0);
+                cudaGraph_t g = nullptr;
+                const cudaError_t ee = cudaStreamEndCapture(s, &g);
+                if (!ce.empty() || ee != cudaSuccess) {
+                    if (g) cudaGraphDestroy(g);
+                    drop_graphs();
+                    return ce.empty() ? std::string("graph capture: ") + cudaGetErrorString(ee) : ce;
+                }
+                const cudaError_t ie = cudaGraphInstantiate(&wf_exec_[k], g, 0);
+                cudaGraphDestroy(g);
+                if (ie != cudaSuccess) {
+                    wf_exec_[k] = nullptr;
+                    drop_graphs();
+                    return std::string("graph instantiate: ") + cudaGetErrorString(ie);
+                }
             }
-            const cudaError_t ie = cudaGraphInstantiate(&gexec[k], g, 0);
-            cudaGraphDestroy(g);
-            if (ie != cudaSuccess) {
-                free_graphs();
-                return std::string("graph instantiate: ") + cudaGetErrorString(ie);
-            }
+            wf_graph_key_ = kb;
         }
     }
     for (const auto& batch : batches) {
@@ -1329,22 +1376,25 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         TRY(cudaMemcpyAsync(d_ctl, h_ctl, sizeof(WfCtl), cudaMemcpyHostToDevice, s));
         uint32_t nfree = (uint32_t)P;
         if (graph) {
-            int par = 0, group = 4;
+            // A pool that holds the whole batch drains after max_bounce + 1 iterations (every path
+            // is at the same bounce; the last one only finalizes), so the host looks at the
+            // counts then; a smaller pool is refilled as paths end and is looked at in groups.
+            int par = 0, group = P >= ctot ? std::min(rp.max_bounce, 17) + 1 : 4;
             for (;;) {
-                for (int k = 0; k < group; ++k, par ^= 1) TRY(cudaGraphLaunch(gexec[par], s));
+                for (int k = 0; k < group; ++k, par ^= 1) TRY(cudaGraphLaunch(wf_exec_[par], s));
                 launches += group * (st.cache ? 8 : 7);
-                TRY(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(WfCtl), cudaMemcpyDeviceToHost, s));
+                TRY(cudaMemcpyAsync(wf_counts_host_, st.counts, kWfCountsBytes + sizeof(WfCtl), cudaMemcpyDeviceToHost, s));
                 TRY(cudaStreamSynchronize(s));
-                if (!h_ctl->active) break;
-                if (h_ctl->iters > 1000000) {
-                    free_graphs();
-                    return "wavefront did not converge";
-                }
-                group = std::min(group * 2, 16);
+                const uint32_t* c = wf_counts_host_;
+                const bool left = h_ctl->active && (h_ctl->n_ext | c[0] | c[2] | c[3] | c[12] ||
+                                                    h_ctl->generated < h_ctl->ctot);
+                if (!left) break;
+                if (h_ctl->iters > 1000000) return "wavefront did not converge";
+                group = P >= ctot ? 8 : 4;
             }
             iters += (int)h_ctl->iters;
             last_cache_queries += (double)h_ctl->queries;
-            nfree = h_ctl->nfree;
+            nfree = wf_counts_host_[4];
         } else {
             long generated = 0;
             uint32_t n_cont = 0, n_fin = 0, n_sh = 0, n_mis = 0, n_query = 0;
@@ -1377,10 +1427,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
             }
             // the last compaction left the counts of an empty pool; the control block follows them
         }
-        if (nfree != (uint32_t)P) {
-            free_graphs();
-            return "wavefront: path pool did not drain";
-        }
+        if (nfree != (uint32_t)P) return "wavefront: path pool did not drain";
         TRY(cudaEventRecord(wf_ev_[0], s));
         for (const WfView& v : vv) {
             const dim3 ggrid((unsigned)((std::min(v.x1 + 2, v.W) - v.x0 + 31) / 32),
@@ -1395,7 +1442,6 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         TRY(cudaEventElapsedTime(&ms, wf_ev_[0], wf_ev_[6]));
         last_stage_ms[5] += ms;
     }
-    free_graphs();
     if (cache) {  // train the cache on this render's unbiased suffixes
         const std::string te = train_cache(st.counts, st.tr_feat, st.tr_target, st.tr_cap, s, rp.err);
         if (!te.empty()) return te;

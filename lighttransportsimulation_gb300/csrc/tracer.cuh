@@ -285,8 +285,12 @@ class Tracer {
     std::string train_cache(uint32_t* d_counts, uint16_t* tr_feat, float* tr_target, uint32_t tr_cap, cudaStream_t s,
                             uint32_t* d_err);
     long wf_cap_ = 0, wf_fs_cap_ = 0;
-    uint32_t* wf_counts_host_ = nullptr;
-    void* wf_ctl_host_ = nullptr;  // pinned mirror of the wavefront control block
+    uint32_t* wf_counts_host_ = nullptr;  // pinned mirror of the counts and the control block
+    // the captured wavefront iteration (path rays in q_a, in q_b), kept between renders, and the
+    // parameters it was captured with
+    cudaGraphExec_t wf_exec_[2] = {nullptr, nullptr};
+    std::string wf_graph_key_;
+    void drop_graphs();
     cudaEvent_t wf_ev_[7] = {nullptr};
     unsigned wf_trace_blocks_[3] = {0, 0, 0};  // resident blocks of k_wf_trace: wide, binary, two-level
     unsigned wf_sms_ = 0;  // resident blocks of k_wf_trace (wide, binary) on this device

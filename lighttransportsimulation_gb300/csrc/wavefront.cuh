@@ -77,6 +77,9 @@ struct WfState {
     float* tr_target;       // [tr_cap][3] training targets
 };
 
+// Bytes of WfState::counts; the control block follows in the same buffer.
+constexpr size_t kWfCountsBytes = 256;
+
 // Per-iteration bookkeeping on the device (so an iteration can run as a CUDA graph): k_wf_control
 // turns the previous compaction's counts into this iteration's list sizes and new samples.
 struct WfCtl {
@@ -192,12 +195,16 @@ __device__ __forceinline__ void tile_pixel(long k, int cw, int ch, int& ci, int&
     }
 }
 
+// Blocks per SM of the list kernels' grids (generate, classify, finalize; compact half): a few
+// waves of resident blocks, and the kernels stride over their lists from there.  The grids of a
+// captured iteration cannot follow the lists' sizes, and one block per 128 pool slots (half a
+// million blocks per kernel on the 2^26-slot pool) cost 9 ms of a 153 ms render in blocks that
+// found nothing to do.
+constexpr unsigned kWfGridPerSm = 32;
+
 // generate: starts batch samples gen0 .. gen0 + take - 1 in the first `take` free slots,
 // appending them to the path-ray list after its `n_cont` continuing paths.
-__global__ __launch_bounds__(kWfBlock) void k_wf_generate(const SceneView sv, const RenderParams rp, WfState st,
-                                                          int32_t* q_ext, const WfCtl* __restrict__ ctl) {
-    const long t = (long)blockIdx.x * kWfBlock + threadIdx.x;
-    if (t >= (long)ctl->take) return;
+__device__ __forceinline__ void generate_one(const WfState& st, int32_t* q_ext, const WfCtl* __restrict__ ctl, long t) {
     const long w = ctl->gen0 + t;
     const uint32_t n_cont = ctl->n_cont;
     const int nviews = (int)ctl->nviews;
@@ -238,6 +245,11 @@ __global__ __launch_bounds__(kWfBlock) void k_wf_generate(const SceneView sv, co
     st.L[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
     st.sig[slot] = kSigBasis;
     q_ext[n_cont + t] = slot;
+}
+__global__ __launch_bounds__(kWfBlock) void k_wf_generate(WfState st, int32_t* q_ext, const WfCtl* __restrict__ ctl) {
+    const long take = (long)ctl->take;
+    for (long t = (long)blockIdx.x * kWfBlock + threadIdx.x; t < take; t += (long)gridDim.x * kWfBlock)
+        generate_one(st, q_ext, ctl, t);
 }
 
 // Work counters (RenderParams::counters): [0..2] all rays (rays, node visits, triangle tests),
@@ -352,14 +364,20 @@ __global__ __launch_bounds__(kWfBlock, kTraceMinBlocks) void k_wf_trace(const Sc
         if (!exhausted && __popc(idle) >= kRefillIdle) {
             // the list sizes, read at each refill rather than held through the traversal
             const uint32_t e1 = __ldg(&ctl->n_ext), e2 = e1 + __ldg(&ctl->n_sh), n = e2 + __ldg(&ctl->n_mis);
+            // Fewer rays than the grid has lanes: each warp takes one equal share and no more (the
+            // shares cover the lists), so that the rays spread over every warp of the chip instead
+            // of diverging 32 to a warp while most warps find nothing.
+            const uint32_t warps = gridDim.x * (kWfBlock / 32);
+            const bool spread = n < 32u * warps;
+            const uint32_t take = spread ? (n + warps - 1u) / warps : (uint32_t)__popc(idle);
             const int leader = __ffs(idle) - 1;
             uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(idle));
+            if ((int)lane == leader) base = atomicAdd(fetch, take);
             base = __shfl_sync(~0u, base, leader);
-            if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
+            if (spread || base + take >= n) exhausted = true;
             if (!active) {
-                const uint32_t idx = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (idx < n) {
+                const uint32_t pos = (uint32_t)__popc(idle & ((1u << lane) - 1u)), idx = base + pos;
+                if (pos < take && idx < n) {
                     kind = idx < e1 ? TR_EXTEND : (idx < e2 ? TR_SHADOW : TR_MIS);
                     p = kind == TR_EXTEND ? q_ext[idx] : (kind == TR_SHADOW ? st.q_shadow[idx - e1] : st.q_mis[idx - e2]);
                     active = wf_ray_begin(kind, t, sv, st, p, nleaf, cur, INST);
@@ -414,19 +432,46 @@ __global__ __launch_bounds__(kWfBlock, kTraceMinBlocks) void k_wf_trace(const Sc
 
 // shade: one bounce of PathTracingIntegrator::evaluate up to the next ray.
 // classify: groups this iteration's paths by the shade class of what they hit (0: left the
-// scene), so that shade runs warps over one material kind at a time.
-__global__ __launch_bounds__(kWfBlock) void k_wf_classify(const SceneView sv, WfState st, const int32_t* __restrict__ q,
+// scene), so that shade runs warps over one material kind at a time.  A block counts a tile of
+// kClassifyTile paths in shared memory and reserves its runs with one atomic per class (one per
+// warp and class before: two million warps on the same few words).
+constexpr int kClassifyItems = 8, kClassifyTile = kWfBlock * kClassifyItems;
+__global__ __launch_bounds__(kWfBlock) void k_wf_classify(WfState st, const int32_t* __restrict__ q,
                                                           const WfCtl* __restrict__ ctl, int pool) {
-    const int t = blockIdx.x * kWfBlock + threadIdx.x;
-    if (t >= (int)ctl->n_ext) return;
-    const int p = q[t];
-    const int c = hit_class(st.hprim[p]);  // 0: left the scene
-    const unsigned grp = __match_any_sync(__activemask(), c);
-    const int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(st.counts + 16 + c, (uint32_t)__popc(grp));
-    base = __shfl_sync(grp, base, leader);
-    st.q_cls[(size_t)c * pool + base + __popc(grp & ((1u << lane) - 1u))] = p;
+    __shared__ uint32_t s_count[kShadeClasses], s_base[kShadeClasses];
+    const uint32_t n = ctl->n_ext;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t first = blockIdx.x * kClassifyTile; first < n; first += gridDim.x * kClassifyTile) {
+        if (threadIdx.x < kShadeClasses) s_count[threadIdx.x] = 0u;
+        __syncthreads();
+        int p[kClassifyItems], c[kClassifyItems];
+        uint32_t pos[kClassifyItems];
+#pragma unroll
+        for (int k = 0; k < kClassifyItems; ++k) {
+            const uint32_t t = first + k * kWfBlock + threadIdx.x;
+            p[k] = t < n ? q[t] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < kClassifyItems; ++k) c[k] = p[k] >= 0 ? hit_class(st.hprim[p[k]]) : -1;
+#pragma unroll
+        for (int k = 0; k < kClassifyItems; ++k) {
+            const unsigned grp = __match_any_sync(~0u, c[k]);
+            const int leader = __ffs(grp) - 1;
+            uint32_t base = 0;
+            if (lane == leader && c[k] >= 0) base = atomicAdd(s_count + c[k], (uint32_t)__popc(grp));
+            pos[k] = __shfl_sync(~0u, base, leader) + __popc(grp & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        if (threadIdx.x < kShadeClasses) {
+            const uint32_t v = s_count[threadIdx.x];
+            s_base[threadIdx.x] = v ? atomicAdd(st.counts + 16 + threadIdx.x, v) : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kClassifyItems; ++k)
+            if (c[k] >= 0) st.q_cls[(size_t)c[k] * pool + s_base[c[k]] + pos[k]] = p[k];
+        __syncthreads();  // the next tile clears the counts
+    }
 }
 
 // Resident blocks per SM the shade kernel is compiled for (caps its registers).
@@ -662,11 +707,7 @@ __global__ __launch_bounds__(kWfBlock, LTS_SHADE_MIN_BLOCKS) void k_wf_shade(con
 // finalize: direct light of the bounce, deferred parity events; a finished path stores its
 // sample and frees its slot (pix = -1).
 template <bool RECORD>
-__global__ __launch_bounds__(kWfBlock) void k_wf_finalize(const SceneView sv, const RenderParams rp, WfState st,
-                                                          const int32_t* __restrict__ q, const WfCtl* __restrict__ ctl) {
-    const int t = blockIdx.x * kWfBlock + threadIdx.x;
-    if (t >= (int)ctl->n_fin) return;
-    const int p = q[t];
+__device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderParams& rp, const WfState& st, int p) {
     const uint32_t pend = st.pend[p];
     float4 l4 = st.L[p];
     Spec L{l4.x, l4.y, l4.z};
@@ -762,6 +803,13 @@ __global__ __launch_bounds__(kWfBlock) void k_wf_finalize(const SceneView sv, co
     }
     st.pix[p] = -1;
 }
+template <bool RECORD>
+__global__ __launch_bounds__(kWfBlock) void k_wf_finalize(const SceneView sv, const RenderParams rp, WfState st,
+                                                          const int32_t* __restrict__ q, const WfCtl* __restrict__ ctl) {
+    const uint32_t n = ctl->n_fin;
+    for (uint32_t t = blockIdx.x * kWfBlock + threadIdx.x; t < n; t += gridDim.x * kWfBlock)
+        finalize_one<RECORD>(sv, rp, st, q[t]);
+}
 
 // Every slot starts free (pix = -1, in the free list in slot order); the counts read as after a
 // compaction of an empty pool (counts zeroed by the host first).
@@ -776,10 +824,12 @@ __global__ void k_wf_init_free(int32_t* q_free, int32_t* pix, uint32_t* counts, 
 
 // control: one iteration's sizes from the previous compaction (path rays continuing, shadow and
 // MIS rays, free slots, cache queries) and the batch's remaining samples; then clears the
-// per-iteration counters (words 0..31).  `active` is 0 once nothing is left to do, and every
-// kernel of such an iteration finds empty lists.
+// per-iteration counters (words 0..31).  `active` is 0 once nothing is left to do: every kernel
+// of such an iteration finds empty lists, compact does nothing, and the counts of the last
+// compaction (an empty pool: every slot free) stay for the host and the next batch.
 __global__ void k_wf_control(WfState st, WfCtl* ctl) {
     __shared__ uint32_t c[16];
+    __shared__ uint32_t s_active;
     if (threadIdx.x < 16) c[threadIdx.x] = st.counts[threadIdx.x];
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -799,9 +849,10 @@ __global__ void k_wf_control(WfState st, WfCtl* ctl) {
         x.queries += x.n_query;
         if (x.active) ++x.iters;
         *ctl = x;
+        s_active = x.active;
     }
     __syncthreads();
-    if (threadIdx.x < 32) st.counts[threadIdx.x] = 0u;
+    if (threadIdx.x < 32 && (s_active || threadIdx.x >= 8)) st.counts[threadIdx.x] = 0u;
 }
 
 // compact: one pass over the pool after shade.  Every live slot (pix >= 0) was shaded in this
@@ -810,11 +861,11 @@ __global__ void k_wf_control(WfState st, WfCtl* ctl) {
 // kCompactTile slots and reserves its runs with one atomic per list, so every list is in slot
 // order within a tile.
 constexpr int kCompactThreads = 256, kCompactItems = 4, kCompactTile = kCompactThreads * kCompactItems;
-__global__ __launch_bounds__(kCompactThreads) void k_wf_compact(WfState st, int32_t* __restrict__ q_ext_next, int P) {
+__device__ __forceinline__ void compact_tile(const WfState& st, int32_t* __restrict__ q_ext_next, int P, int tile) {
     __shared__ uint32_t s_warp[4][kCompactThreads / 32];
     __shared__ uint32_t s_base[4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int first = blockIdx.x * kCompactTile + tid * kCompactItems;
+    const int first = tile * kCompactTile + tid * kCompactItems;
     uint32_t flags[kCompactItems];
     uint32_t cnt[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -868,6 +919,15 @@ __global__ __launch_bounds__(kCompactThreads) void k_wf_compact(WfState st, int3
 #pragma unroll
         for (int l = 0; l < 4; ++l)
             if ((f >> l) & 1u) dst[l][pos[l]++] = first + k;
+    }
+}
+__global__ __launch_bounds__(kCompactThreads) void k_wf_compact(WfState st, int32_t* __restrict__ q_ext_next,
+                                                                const WfCtl* __restrict__ ctl, int P) {
+    if (!ctl->active) return;
+    const int tiles = (P + kCompactTile - 1) / kCompactTile;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        __syncthreads();  // the previous tile's counts have been read
+        compact_tile(st, q_ext_next, P, tile);
     }
 }
 
