@@ -33,8 +33,6 @@
 namespace lts {
 namespace {
 
-constexpr int kBdptMaxBounce = 8;  // longest path the kernel's vertex arrays hold
-
 enum : int { BV_CAMERA = 0, BV_LIGHT = 1, BV_SURFACE = 2 };
 
 struct BVert {

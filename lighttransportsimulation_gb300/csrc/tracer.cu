@@ -1,19 +1,6 @@
-// Path-tracing megakernel (sm_103a): one thread per pixel, all samples and bounces, as the
-// reference's PathTracingKernel (intergrators/IntegratorKernels.cu:17-23) runs
-// PathTracingIntegrator::evaluate (intergrators/PathTracingIntegrator.cuh:26-109).
-//
-// Differences in mechanism, not in arithmetic:
-//  - scene tables are SoA arrays and materials/lights are `switch`-dispatched records, so the
-//    per-bounce device `new`/`free` of BSDFs and BxDFs (materials/Material.cuh:41-52) is gone;
-//  - traversal reads 64-byte two-child nodes and triangles in leaf order, visits the nearer
-//    child first and keeps its node stack in shared memory; the closest hit is the same as the
-//    reference's left-first visit (edges are excluded by the epsilon test, so exact-t ties
-//    between neighbouring triangles cannot occur);
-//  - the closest-hit SurfaceInteraction is built once from the winning triangle rather than on
-//    every closer hit (it is a pure function of the ray and the triangle);
-//  - the film accumulates each pixel's own 2x2 splat footprint in compensated FP32 (Kahan) in
-//    shared memory and flushes it once per pixel to FP64 sums; the rare wider splats go straight
-//    to FP64 atomics.  The resolve divides in FP64.
+// The renderer's host side and its set-up kernels (sm_103a): scene upload, traversal structures,
+// film resolve, ray queries and the wavefront path tracer (wavefront.cuh).  The one-launch
+// integrators are in mega.cu.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -29,15 +16,6 @@
 #include "tracer.cuh"
 #include "tracer_dev.cuh"
 #include "mlp.cuh"
-
-namespace lts {
-namespace {
-
-}  // namespace
-}  // namespace lts
-
-#include "megakernel.cuh"
-#include "bdpt.cuh"
 
 namespace lts {
 namespace {
@@ -356,7 +334,7 @@ std::string ensure_texture_tables() {
 std::string set_libm_double(int on) {
     const int v = on ? 1 : 0;
     TRY(cudaMemcpyToSymbol(c_libm_double, &v, sizeof v));
-    return "";
+    return mega_set_libm_double(on);
 }
 
 std::string kat_launch(int fn, const float* d_in, int n, float* d_out, cudaStream_t s) {
@@ -498,7 +476,8 @@ std::string Tracer::upload_scene(const HostScene& sc, cudaStream_t s) {
     last_upload_bytes = 0;
     view_ = SceneView{};
     {
-        const std::string te = ensure_texture_tables();
+        std::string te = ensure_texture_tables();
+        if (te.empty()) te = mega_init();
         if (!te.empty()) return te;
     }
     if (!ev0_) {
@@ -535,7 +514,7 @@ std::string Tracer::upload_scene(const HostScene& sc, cudaStream_t s) {
         shade_lm_[c] = 0;
         shade_tex_[c] = false;
     }
-    bdpt_matte_only_ = true;
+    matte_only_ = true;
     for (size_t m = 0; m < mats.size(); ++m) {
         const HostMaterial& h = sc.materials[m];
         const int c = mats[m].shade_class;
@@ -544,7 +523,7 @@ std::string Tracer::upload_scene(const HostScene& sc, cudaStream_t s) {
         shade_lm_[c] |= lm;
         const bool tex = h.tex[0].kind != TEX_CONSTANT || (h.kind == 2 && h.tex[1].kind != TEX_CONSTANT);
         shade_tex_[c] = shade_tex_[c] || tex;
-        if ((lm & ~LM_MATTE) || tex) bdpt_matte_only_ = false;
+        if ((lm & ~LM_MATTE) || tex) matte_only_ = false;
     }
     std::vector<DevLight> lights(sc.lights.size());
     for (size_t l = 0; l < lights.size(); ++l) {
@@ -995,28 +974,11 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     if (!e.empty()) return e;
     last_paths = (double)ns;
     if (d.integrator == LTS_INTEGRATOR_WAVEFRONT) return render_wavefront(sc, bvh, d, s, d_err, rp, sv, ns);
-    const dim3 block(kBX, kBY);
-    const dim3 grid((rp.x1 - rp.x0 + kBX - 1) / kBX, (rp.y1 - rp.y0 + kBY - 1) / kBY);
     TRY(cudaEventRecord(ev0_, s));
-    if (d.integrator == LTS_INTEGRATOR_FP64) {
-        e = render64_launch(sv, rp, bvh.n, d.record_samples != 0, s);
-        if (!e.empty()) return e;
-    } else if (d.integrator == LTS_INTEGRATOR_BDPT) {
-        // one thread per pixel and sample slice: enough blocks for every SM to hold its resident
-        // ones about four times over (a small film alone would leave most SMs idle)
-        int dev = 0, sms = 0;
-        TRY(cudaGetDevice(&dev));
-        TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const long want = 4L * LTS_BDPT_MIN_BLOCKS * sms, have = (long)grid.x * grid.y;
-        const dim3 gridz(grid.x, grid.y, (unsigned)std::max(1L, std::min<long>(rp.spp, (want + have - 1) / have)));
-        // compiled for the lobes the scene has: Lambertian / Oren-Nayar alone, or every lobe
-        if (bdpt_matte_only_) k_bdpt<LM_MATTE, false><<<gridz, block, 0, s>>>(sv, rp, bvh.n, splat_, bdpt_strategy);
-        else k_bdpt<LM_ALL, true><<<gridz, block, 0, s>>>(sv, rp, bvh.n, splat_, bdpt_strategy);
-    } else if (d.record_samples) {
-        k_pathtrace<true><<<grid, block, 0, s>>>(sv, rp, bvh.n);
-    } else {
-        k_pathtrace<false><<<grid, block, 0, s>>>(sv, rp, bvh.n);
-    }
+    if (d.integrator == LTS_INTEGRATOR_FP64) e = render64_launch(sv, rp, bvh.n, d.record_samples != 0, s);
+    else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, s);
+    else e = mega_launch(sv, rp, bvh.n, d.record_samples != 0, matte_only_, s);
+    if (!e.empty()) return e;
     TRY(cudaEventRecord(ev1_, s));
     TRY(cudaGetLastError());
     last_launches = 1;

@@ -128,6 +128,17 @@ std::string set_libm_double(int on);
 // Known-answer check of single float device functions (lts_debug_kat): n records of 16 floats.
 std::string kat_launch(int fn, const float* d_in, int n, float* d_out, cudaStream_t s);
 
+// The float one-launch integrators (mega.cu): the path-tracing megakernel and the bidirectional
+// integrator; set_libm_double of that translation unit.  matte_only: every material is Lambertian
+// or Oren-Nayar with constant textures.
+std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool record, bool matte_only,
+                        cudaStream_t s);
+std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
+                        bool matte_only, cudaStream_t s);
+std::string mega_set_libm_double(int on);
+std::string mega_init();  // that translation unit's texture tables (once per process)
+constexpr int kBdptMaxBounce = 8;  // longest path of the bidirectional integrator
+
 // FP64 oracle renderer (render64.cu): the megakernel integrator in double on the binary LBVH.
 std::string render64_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool record, cudaStream_t s);
 
@@ -253,7 +264,7 @@ class Tracer {
     // shade classes of the loaded scene: used, lobe mask and textured (the shade kernel variant)
     bool shade_used_[kShadeClasses] = {false};
     int shade_lm_[kShadeClasses] = {0};
-    bool bdpt_matte_only_ = false;  // every material Lambertian / Oren-Nayar with constant textures
+    bool matte_only_ = false;  // every material Lambertian / Oren-Nayar with constant textures
     bool shade_tex_[kShadeClasses] = {false};
     unsigned shade_grid_ = 0;  // resident blocks of the shade kernel on this device
     // side streams and fork / join events: the classes' shade launches run concurrently (as

@@ -24,6 +24,8 @@
 // execution.  Included by tracer.cu (one translation unit shares the constant tables).
 #pragma once
 
+#include "shade.cuh"
+
 namespace lts {
 namespace {
 
@@ -137,21 +139,6 @@ __device__ void write_features(const WfState& st, const SI& si, const Bsdf& f, u
     o[23] = make_uint2(0u, 0u);
 }
 
-// Resume a (pixel, sample) stream at draw `draw` (regenerates the current Philox block).
-__device__ __forceinline__ void rng_resume(Rng& r) {
-    const uint32_t k = r.draw & 3u;
-    if (k == 0u) return;
-    const uint32_t d = r.draw;
-    r.draw = d & ~3u;
-    philox_block(r);
-    r.draw = d;
-    for (uint32_t q = 0; q < k; ++q) {
-        r.w0 = r.w1;
-        r.w1 = r.w2;
-        r.w2 = r.w3;
-    }
-}
-
 __device__ __forceinline__ void camera_ray(const WfView& vw, float pfx, float pfy, V3& rd, V3& rxd, V3& ryd) {
     const float* cam = vw.cam;
     const float spp_scale = vw.spp_scale;
@@ -163,36 +150,6 @@ __device__ __forceinline__ void camera_ray(const WfView& vw, float pfx, float pf
     const V3 dy0 = normalize(cllc + cright * (pfx / rx) + cup * ((pfy + 1) / ry) - co);
     rxd = rd + (dx0 - rd) * spp_scale;
     ryd = rd + (dy0 - rd) * spp_scale;
-}
-
-// Order in which a slice's samples of one sample index visit the crop's pixels: 8 x 4 tiles
-// (one warp each) left to right in bands of four rows, so the rays a warp traces start from a
-// compact patch of the image instead of a 32 x 1 strip (partial tiles at the right and bottom
-// edges are row-major).  Position k in 0 .. cw * ch - 1 -> crop pixel (ci, cj).
-#ifndef LTS_PIXEL_TILES
-#define LTS_PIXEL_TILES 1  // 0: row-major pixel order
-#endif
-constexpr int kTileW = 8, kTileH = 4;
-__device__ __forceinline__ void tile_pixel(long k, int cw, int ch, int& ci, int& cj) {
-    if (!LTS_PIXEL_TILES) {
-        ci = (int)(k % cw);
-        cj = (int)(k / cw);
-        return;
-    }
-    const long band_px = (long)kTileH * cw;
-    const int band = (int)(k / band_px);
-    const int rows = min(kTileH, ch - band * kTileH);
-    const int o = (int)(k - band * band_px);
-    const int full = cw / kTileW, tile_px = kTileW * rows;
-    if (o < full * tile_px) {
-        const int tx = o / tile_px, r = o - tx * tile_px;
-        ci = tx * kTileW + r % kTileW;
-        cj = band * kTileH + r / kTileW;
-    } else {  // the narrower last tile of the band
-        const int rem = cw - full * kTileW, r = o - full * tile_px;
-        ci = full * kTileW + r % rem;
-        cj = band * kTileH + r / rem;
-    }
 }
 
 // Blocks per SM of the list kernels' grids (generate, classify, finalize; compact half): a few
@@ -478,6 +435,33 @@ __global__ __launch_bounds__(kWfBlock) void k_wf_classify(WfState st, const int3
 #ifndef LTS_SHADE_MIN_BLOCKS
 #define LTS_SHADE_MIN_BLOCKS 5  // 6 and 4 measured 2 % and 5 % slower on the stress scene
 #endif
+// Where shade_scatter's rays and their weights go: the path state.
+struct WfScatter {
+    WfState& st;
+    int p;
+    uint32_t pend;
+    __device__ __forceinline__ void nee(Spec beta, float lpdf) {
+        pend |= WF_NEE;
+        st.nee_beta[p] = make_float4(beta.r, beta.g, beta.b, lpdf);
+    }
+    __device__ __forceinline__ void shadow(V3 o, V3 d, Spec c, bool on) {
+        st.sh_o[p] = make_float4(o.x, o.y, o.z, 0.f);
+        st.sh_d[p] = make_float4(d.x, d.y, d.z, 1 - kShadowEps);
+        st.sh_c[p] = make_float4(c.r, c.g, c.b, on ? 1.f : 0.f);
+        pend |= WF_VIS;
+    }
+    __device__ __forceinline__ void mis(V3 o, V3 d, Spec fv, float wgt, float spdf, int light) {
+        st.mis_o[p] = make_float4(o.x, o.y, o.z, 0.f);
+        st.mis_d[p] = make_float4(d.x, d.y, d.z, 0.f);
+        st.mis_fv[p] = make_float4(fv.r, fv.g, fv.b, wgt);
+        st.mis_x[p] = make_float4(spdf, __int_as_float(light), 0.f, 0.f);
+        pend |= WF_MIS;
+    }
+    __device__ __forceinline__ void ray(V3 o, V3 d) {
+        st.ro[p] = make_float4(o.x, o.y, o.z, 0.f);
+        st.rd[p] = make_float4(d.x, d.y, d.z, 0.f);
+    }
+};
 // One path's bounce; LM / TEX: the lobes and textures its material can have (shade_variant).
 template <bool RECORD, int LM, bool TEX>
 __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParams& rp, WfState& st, int p) {
@@ -572,112 +556,10 @@ __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParam
     if (!done && bsdf_roughness(f) > kCacheRough) rough_seen = true;
     uint64_t ev_mis = 0, ev_main = 0;
     if (!done) {
-        if (sv.nlight > 0) {
-            pend |= WF_NEE;
-            const float ul = rng_1d(rng);
-            int off = 0;
-            {
-                const int size = sv.nlight;
-                if (size != 1) {
-                    int first = 0, len = size;
-                    while (len > 0) {
-                        const int half = len >> 1, middle = first + half;
-                        if (__ldg(sv.light_cdf + middle) <= ul) {
-                            first = middle + 1;
-                            len -= half + 1;
-                        } else {
-                            len = half;
-                        }
-                    }
-                    off = (int)clampf((float)(first - 1), 0.0f, (float)(size - 2));
-                }
-            }
-            const float lpdf_sel = __ldg(sv.light_func + off) / (sv.light_func_int * sv.nlight);
-            st.nee_beta[p] = make_float4(beta.r, beta.g, beta.b, lpdf_sel);
-            const F2 ulight = rng_2d(rng);
-            const F2 uscat = rng_2d(rng);
-            const DevLight& Lt = sv.lights[off];
-            const uint32_t fl = specular ? BSDF_ALL : (BSDF_ALL & ~BSDF_SPECULAR);
-            LightSample ls;
-            const bool delta = sample_li(sv, Lt, si, ulight, ls);
-            if (ls.pdf > 0 && !is_black(ls.Li)) {
-                const Spec fv = bsdf_f<LM>(f, si.wo, ls.wi, fl, RECORD ? &evs : nullptr) * absdot(ls.wi, si.sn);
-                const float spdf = bsdf_pdf<LM>(f, si.wo, ls.wi, fl, RECORD ? &evs : nullptr);
-                if (!is_black(fv)) {
-                    const V3 org = offset_origin(si.p, si.perr, si.n, ls.p1 - si.p);
-                    const V3 tgt = offset_origin(ls.p1, ls.perr1, ls.n1, org - ls.p1);
-                    Spec c;
-                    if (delta) {
-                        c = fv * ls.Li / ls.pdf;
-                    } else {
-                        const float fp = 1 * ls.pdf, gp = 1 * spdf;
-                        const float wgt = (fp * fp) / (fp * fp + gp * gp);
-                        c = fv * ls.Li * wgt / ls.pdf;
-                    }
-                    const V3 dir = tgt - org;
-                    st.sh_o[p] = make_float4(org.x, org.y, org.z, 0.f);
-                    st.sh_d[p] = make_float4(dir.x, dir.y, dir.z, 1 - kShadowEps);
-                    st.sh_c[p] = make_float4(c.r, c.g, c.b, is_black(ls.Li) ? 0.f : 1.f);
-                    pend |= WF_VIS;
-                }
-            }
-            if (!delta) {
-                V3 wi = ls.wi;
-                float spdf = 0;
-                uint32_t stype = 0;
-                EvSink cap{nullptr, 0};
-                Spec fv = bsdf_sample<LM>(f, si.wo, wi, uscat, spdf, fl, stype, RECORD ? &cap : nullptr);
-                ev_mis = cap.cap;
-                fv = fv * absdot(wi, si.sn);
-                const bool sampled_spec = (stype & BSDF_SPECULAR) != 0;
-                if (!is_black(fv) && spdf > 0) {
-                    float wgt = 1;
-                    bool skip = false;
-                    if (!sampled_spec) {
-                        float lp;
-                        if (Lt.kind == 0) lp = area_pdf(sv, Lt, si.p, si.perr, si.n, wi);
-                        else if (Lt.kind == 1) lp = sph_pdf_infinite(wi);
-                        else lp = 0.0f;
-                        if (lp == 0) skip = true;
-                        else {
-                            const float fp = 1 * spdf, gp = 1 * lp;
-                            wgt = (fp * fp) / (fp * fp + gp * gp);
-                        }
-                    }
-                    if (!skip) {
-                        const V3 org = offset_origin(si.p, si.perr, si.n, wi);
-                        st.mis_o[p] = make_float4(org.x, org.y, org.z, 0.f);
-                        st.mis_d[p] = make_float4(wi.x, wi.y, wi.z, 0.f);
-                        st.mis_fv[p] = make_float4(fv.r, fv.g, fv.b, wgt);
-                        st.mis_x[p] = make_float4(spdf, __int_as_float(off), 0.f, 0.f);
-                        pend |= WF_MIS;
-                    }
-                }
-            }
-        }
-        // path BSDF sample, throughput, spawn, Russian roulette (PathTracingIntegrator.cuh:80-103)
-        V3 wi = v3(0, 0, 0);
-        float pdf = 0;
-        uint32_t stype = 0;
-        const F2 ub = rng_2d(rng);
-        EvSink cap{nullptr, 0};
-        const Spec fv = bsdf_sample<LM>(f, si.wo, wi, ub, pdf, BSDF_ALL, stype, RECORD ? &cap : nullptr);
-        ev_main = cap.cap;
-        if (is_black(fv) || pdf == 0) {
-            done = true;
-        } else {
-            specular = (stype & BSDF_SPECULAR) != 0;
-            beta = beta * (fv * absdot(wi, si.sn) / pdf);
-            const V3 no = offset_origin(si.p, si.perr, si.n, wi);
-            st.ro[p] = make_float4(no.x, no.y, no.z, 0.f);
-            st.rd[p] = make_float4(wi.x, wi.y, wi.z, 0.f);
-            if (bounce >= rp.rr_start) {
-                const float qq = fmaxf(0.05f, 1 - lum(beta));
-                if (rng_1d(rng) < qq) done = true;
-                else beta = beta / (1 - qq);
-            }
-            if (bounce + 1 >= rp.max_bounce) done = true;
-        }
+        WfScatter out{st, p, pend};
+        done = shade_scatter<RECORD, LM>(sv, rp, si, f, bounce, beta, specular, rng, out, RECORD ? &evs : nullptr, ev_mis,
+                                         ev_main);
+        pend = out.pend;
     }
     st.pend[p] = pend | (done ? WF_DONE : 0u);
     st.draw[p] = rng.draw;
