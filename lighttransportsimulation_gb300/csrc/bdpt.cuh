@@ -1,8 +1,20 @@
-// Bidirectional path tracing (sm_103a megakernel): one thread per pixel, every sample builds a
-// camera subpath and a light subpath and combines every connection strategy (s light vertices,
-// t camera vertices) with multiple-importance weights -- the algorithm of Veach's thesis as PBRT
-// v3 states it (ch. 16.3: random walks with forward / reverse area densities, ConnectBDPT,
-// MISWeight's ratio chain).
+// Bidirectional path tracing (sm_103a): every sample builds a camera subpath and a light subpath
+// and combines every connection strategy (s light vertices, t camera vertices) with
+// multiple-importance weights -- the algorithm of Veach's thesis as PBRT v3 states it (ch. 16.3:
+// random walks with forward / reverse area densities, ConnectBDPT, MISWeight's ratio chain).
+//
+// Three kernels over a chunk of samples:
+//   k_bdpt_walk     one thread per sample: both random walks in one loop, the vertices written to
+//                   a structure of arrays in device memory
+//   k_bdpt_connect  one thread per (strategy, sample), the strategy uniform over a block: the
+//                   connection, its shadow ray and its MIS weight
+//   k_bdpt_film     one thread per sample: the contributions summed in strategy order and filtered
+//                   into the film
+// As one kernel (a thread per pixel with its vertices in local memory) the same work ran at 4.7
+// of 32 lanes and waited on instruction fetch (39.5 stall cycles per issue): lanes were at
+// different strategies of different samples and the body is far larger than the instruction
+// caches.  Here a warp is at one strategy, and a kernel's body is one stage: the box lit by one
+// triangle, 256 x 256, 16 spp, 5 bounces, 81.2 -> 12.0 ms with the same contributions bit for bit.
 //
 // The reference ships this integrator disabled and unfinished (intergrators/
 // BidirectionalPathIntegrator.cuh:285-660, LightTransportSimulation.cu:116-121): its light walk
@@ -28,6 +40,7 @@
 // scaled by 1 / spp at resolve.
 #pragma once
 
+#include "shade.cuh"
 #include "tracer_dev.cuh"
 
 namespace lts {
@@ -192,126 +205,341 @@ __device__ __forceinline__ real bv_pdf(const SceneView& sv, const BCam& cam, con
     return bv_convert(pdf, v, next);
 }
 
-// VisibilityTester::unoccluded between two vertices (offset origins as spawnRayTo).
-__device__ __forceinline__ bool bdpt_visible(const SceneView& sv, int nleaf, const BVert& a, const BVert& b,
-                                             uint32_t* stack, uint32_t* err, Work& wk) {
-    const V3 org = offset_origin(a.p, a.perr, a.n, b.p - a.p);
-    const V3 tgt = offset_origin(b.p, b.perr, b.n, org - b.p);
-    return !scene_occluded(sv, nleaf, org, tgt - org, 1 - kShadowEps, stack, err, wk);
+// The chunk's buffers.  A vertex is kBvWords 16-byte words, word w of vertex slot v of sample k at
+// vert[(v * words + w) * cap + k] (lanes of a warp read neighbouring samples); slots: camera
+// vertices 1 .. maxb + 1, then light vertices 0 .. maxb.  Matte scenes leave out the last words.
+constexpr int kBvWordsMatte = 8, kBvWordsAll = 11;
+struct BdptBuf {
+    uint4* vert;
+    float2* pdf;    // (pdf_fwd, pdf_rev) of vertex slot v of sample k at [v * cap + k]
+    uint4* head;    // per sample: film x, y bits; draw after both walks; n_cam | n_light << 4 |
+                    // connectible camera vertices << 8 (bit 8 + c: vertex c)
+    uint32_t* delta;  // per sample: delta camera vertices (bit c), delta light vertices (bit 16 + l)
+    float4* contrib;  // [strategy * cap + k]
+    int cap;
+};
+// The strategies rendered, in the order their contributions are summed (t outer, s inner).
+constexpr int kBdptMaxStrategies = 64;
+struct BdptStrategies {
+    int n;
+    unsigned char s[kBdptMaxStrategies], t[kBdptMaxStrategies];
+};
+
+template <int LM>
+__device__ __forceinline__ int bv_words() {
+    return (LM & ~LM_MATTE) ? kBvWordsAll : kBvWordsMatte;
+}
+template <int LM>
+__device__ __forceinline__ void bv_store(const BdptBuf& b, int slot, int k, const BVert& v) {
+    uint4* o = b.vert + (size_t)slot * bv_words<LM>() * b.cap + k;
+    auto put = [&](int w, V3 a, uint32_t x) {
+        o[(size_t)w * b.cap] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), x);
+    };
+    put(0, v.p, (uint32_t)v.type | ((uint32_t)v.f.lobe << 4) | (v.f.type << 8));
+    put(1, v.n, (uint32_t)v.light);
+    put(2, v.perr, __float_as_uint(v.f.a));
+    put(3, v.wo, __float_as_uint(v.f.b));
+    put(4, v3(v.beta.r, v.beta.g, v.beta.b), __float_as_uint(v.f.R.r));
+    put(5, v.f.ns, __float_as_uint(v.f.R.g));
+    put(6, v.f.ss, __float_as_uint(v.f.R.b));
+    put(7, v.f.ts, __float_as_uint(v.f.eta));
+    if (LM & ~LM_MATTE) {
+        put(8, v3(v.f.T.r, v.f.T.g, v.f.T.b), __float_as_uint(v.f.alpha));
+        put(9, v3(v.f.k.r, v.f.k.g, v.f.k.b), 0u);
+        put(10, v3(v.f.eta3.r, v.f.eta3.g, v.f.eta3.b), 0u);
+    }
+}
+// The stored vertex (the words of fields the caller does not use are not read).
+template <int LM>
+__device__ __forceinline__ void bv_load(const BdptBuf& b, int slot, int k, BVert& v) {
+    const uint4* o = b.vert + (size_t)slot * bv_words<LM>() * b.cap + k;
+    auto get = [&](int w, V3& a) -> uint32_t {
+        const uint4 q = __ldg(o + (size_t)w * b.cap);
+        a = v3(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z));
+        return q.w;
+    };
+    V3 c;
+    const uint32_t m = get(0, v.p);
+    v.type = (int)(m & 15u);
+    v.f.lobe = (int)((m >> 4) & 15u);
+    v.f.type = m >> 8;
+    v.light = (int)get(1, v.n);
+    v.f.ng = v.n;
+    v.f.a = __uint_as_float(get(2, v.perr));
+    v.f.b = __uint_as_float(get(3, v.wo));
+    v.f.R.r = __uint_as_float(get(4, c));
+    v.beta = Spec{c.x, c.y, c.z};
+    v.f.R.g = __uint_as_float(get(5, v.f.ns));
+    v.f.R.b = __uint_as_float(get(6, v.f.ss));
+    v.f.eta = __uint_as_float(get(7, v.f.ts));
+    if (LM & ~LM_MATTE) {
+        v.f.alpha = __uint_as_float(get(8, c));
+        v.f.T = Spec{c.x, c.y, c.z};
+        get(9, c);
+        v.f.k = Spec{c.x, c.y, c.z};
+        get(10, c);
+        v.f.eta3 = Spec{c.x, c.y, c.z};
+    }
+}
+__device__ __forceinline__ BVert bv_camera(const BCam& cam) {
+    BVert v;
+    v.type = BV_CAMERA;
+    v.delta = 0;
+    v.light = -1;
+    v.p = cam.o;
+    v.n = v3(0, 0, 0);
+    v.perr = v3(0, 0, 0);
+    v.beta = spec(1.0f);
+    v.pdf_fwd = v.pdf_rev = 0;
+    v.f.lobe = LOBE_NONE;
+    v.f.type = 0;
+    return v;
 }
 
-// RandomWalk: extends `path` (path[0] is the walk's start, already filled) by up to max_depth
-// surface vertices; returns the vertices added.
-template <int LM, bool TEX>
-__device__ int bdpt_walk(const SceneView& sv, int nleaf, BVert* path, V3 ro, V3 rd, Spec beta, real pdf_fwd,
-                         int max_depth, bool importance, Rng& rng, bool diff0, V3 rxo, V3 rxd, V3 ryd,
-                         uint32_t* stack, uint32_t* err, Work& wk, unsigned long long& rays) {
-    int bounces = 0;
-    real pdf_rev = 0;
-    while (bounces < max_depth) {
-        SI si;
-        ++rays;
-        if (!scene_intersect(sv, nleaf, ro, rd, INFINITY, si, stack, err, wk)) break;
-        if (is_black(beta)) break;
-        BVert& v = path[bounces + 1];
-        BVert& prev = path[bounces];
-        if (diff0 && bounces == 0) {  // camera-ray differentials for the first hit's textures
-            const V3 n = si.n;
-            const real d = -dot(n, si.p);
-            const real tx = (-dot(n, rxo) - d) / dot(n, rxd);
-            const real ty = (-dot(n, rxo) - d) / dot(n, ryd);
-            si.dpdx = (rxo + rxd * tx) - si.p;
-            si.dpdy = (rxo + ryd * ty) - si.p;
-        } else {
-            si.dpdx = v3(0, 0, 0);
-            si.dpdy = v3(0, 0, 0);
-        }
-        v.type = BV_SURFACE;
-        v.delta = 0;
-        v.light = si.light;
-        v.p = si.p;
-        v.n = si.n;
-        v.perr = si.perr;
-        v.wo = -rd;
-        v.beta = beta;
-        v.pdf_rev = 0;
-        v.pdf_fwd = bv_convert(pdf_fwd, prev, v);
-        if (!make_bsdf<LM, TEX>(sv, si, v.f, nullptr)) v.f.lobe = LOBE_NONE;
-        ++bounces;
-        if (bounces >= max_depth || v.f.lobe == LOBE_NONE) break;
-        V3 wi;
-        uint32_t stype = 0;
-        real pdf = 0;
-        const Spec fv = bsdf_sample<LM>(v.f, v.wo, wi, rng_2d(rng), pdf, BSDF_ALL, stype, nullptr);
-        if (is_black(fv) || pdf == 0) break;
-        beta = beta * (fv * absdot(wi, v.f.ns) / pdf);
-        pdf_fwd = pdf;
-        pdf_rev = bsdf_pdf<LM>(v.f, wi, v.wo, BSDF_ALL, nullptr);
-        if (stype & BSDF_SPECULAR) {
-            v.delta = 1;
-            pdf_fwd = pdf_rev = 0;
-        }
-        if (importance) {
-            beta = beta * bdpt_shading_fix(v.f, v.wo, wi);
-            // specular transmission scales radiance by (eta_i / eta_t)^2 (the BSDF applies it);
-            // importance is not scaled (PBRT's TransportMode), so light paths undo it
-            if (v.f.lobe == LOBE_FRESNEL_SPECULAR && (stype & BSDF_TRANSMISSION)) {
-                const bool entering = dot(v.wo, v.f.ns) > 0;
-                const real ei = entering ? 1.0f : v.f.eta, et = entering ? v.f.eta : 1.0f;
-                beta = beta * ((et * et) / (ei * ei));
+// The pixel of batch sample `idx` (all pixels of sample 0, then of sample 1, ...; pixels in 8 x 4
+// tiles) and its sample number.
+__device__ __forceinline__ void bdpt_pixel(const RenderParams& rp, long idx, int& i, int& j, int& s) {
+    const int cw = rp.x1 - rp.x0, ch = rp.y1 - rp.y0;
+    const long npix = (long)cw * ch;
+    s = (int)(idx / npix);
+    int ci, cj;
+    tile_pixel(idx - s * npix, cw, ch, ci, cj);
+    i = rp.x0 + ci;
+    j = rp.y0 + cj;
+}
+
+// GenerateCameraSubpath and GenerateLightSubpath (the random walks of RandomWalk) of samples
+// first .. first + n - 1.  One loop: a lane whose camera walk has ended starts its light walk in the
+// next turn; the block's warps trace and extend together (barriers), as in the path tracer's
+// megakernel.
+constexpr int kBdptWalkThreads = 256;
+#ifndef LTS_BDPT_WALK_BLOCKS
+#define LTS_BDPT_WALK_BLOCKS 2
+#endif
+template <int LM, bool TEX, bool WIDE>
+__global__ __launch_bounds__(kBdptWalkThreads, LTS_BDPT_WALK_BLOCKS) void k_bdpt_walk(const SceneView sv, const RenderParams rp,
+                                                                                      int nleaf, BdptBuf buf, long first, int n) {
+    __shared__ uint32_t s_stack[kStack * kBdptWalkThreads / 2 * 2];
+    uint32_t* stack = s_stack + (threadIdx.x / kThreads) * (kStack * kThreads) + threadIdx.x % kThreads;
+    const int k = blockIdx.x * kBdptWalkThreads + threadIdx.x;
+    const bool in = k < n;
+    const BCam cam = bdpt_camera(sv);
+    const int maxb = min(rp.max_bounce, kBdptMaxBounce);
+    unsigned rays = 0;
+    Work wk{0u, 0u};
+    int i = 0, j = 0, s_ix = 0;
+    if (in) bdpt_pixel(rp, first + k, i, j, s_ix);
+    Rng rng;
+    rng.key = rp.seed + wang_hash((uint32_t)(j * sv.width + i));
+    rng.sample = (uint32_t)s_ix;
+    rng.draw = 0;
+    const real rx = (real)(cam.W - 1), ry = (real)(cam.H - 1);
+    // camera subpath: the path tracer's primary ray
+    const F2 fs = rng_2d(rng);
+    (void)rng_2d(rng);
+    const real pfx = (real)(i + fs.x), pfy = (real)(j + fs.y);
+    V3 ro = cam.o, rd = normalize(cam.llc + cam.right * (pfx / rx) + cam.up * (pfy / ry) - cam.o);
+    Spec beta = spec(1.0f);
+    real cpx, cpy, cos_t;
+    bdpt_raster(cam, rd, cpx, cpy, cos_t);
+    real pdf_fwd = bdpt_pdf_dir(cam, cos_t);
+    V3 prev_p = cam.o, prev_n = v3(0, 0, 0);
+    int phase = in ? 0 : 2, bounces = 0, max_depth = maxb + 1;  // phase 0: camera walk, 1: light walk, 2: done
+    int n_cam = 1, n_light = 0;
+    uint32_t conn = 0, delta = 0;
+    while (__syncthreads_or(phase < 2)) {
+        const bool on = phase < 2 && bounces < max_depth;
+        Trav t;
+        warp_rays<false, WIDE>(on, t, sv, nleaf, ro, rd, INFINITY, stack, rp.err, wk);
+        __syncthreads();
+        bool end = phase < 2;
+        if (on) {
+            ++rays;
+            if (t.best >= 0 && !is_black(beta)) {
+                SI si;
+                make_si(sv, t.best, rd, t.bu, t.bv, t.binv, si, &ro);
+                if (phase == 0 && bounces == 0) {  // camera-ray differentials for the first hit's textures
+                    const V3 dx0 = normalize(cam.llc + cam.right * ((pfx + 1) / rx) + cam.up * (pfy / ry) - cam.o);
+                    const V3 dy0 = normalize(cam.llc + cam.right * (pfx / rx) + cam.up * ((pfy + 1) / ry) - cam.o);
+                    const V3 rxd = rd + (dx0 - rd) * rp.spp_scale, ryd = rd + (dy0 - rd) * rp.spp_scale;
+                    const V3 nn = si.n;
+                    const real d = -dot(nn, si.p);
+                    const real tx = (-dot(nn, ro) - d) / dot(nn, rxd);
+                    const real ty = (-dot(nn, ro) - d) / dot(nn, ryd);
+                    si.dpdx = (ro + rxd * tx) - si.p;
+                    si.dpdy = (ro + ryd * ty) - si.p;
+                } else {
+                    si.dpdx = v3(0, 0, 0);
+                    si.dpdy = v3(0, 0, 0);
+                }
+                BVert v, prev;
+                v.type = BV_SURFACE;
+                v.light = si.light;
+                v.p = si.p;
+                v.n = si.n;
+                v.perr = si.perr;
+                v.wo = -rd;
+                v.beta = beta;
+                v.f = Bsdf{};
+                prev.p = prev_p;
+                prev.n = prev_n;
+                if (!make_bsdf<LM, TEX>(sv, si, v.f, nullptr)) v.f.lobe = LOBE_NONE;
+                v.f.ng = si.n;
+                const int slot = phase == 0 ? bounces : maxb + 2 + bounces;  // camera vertex bounces + 1, light bounces + 1
+                buf.pdf[(size_t)slot * buf.cap + k] = make_float2(bv_convert(pdf_fwd, prev, v), 0.f);
+                bv_store<LM>(buf, slot, k, v);
+                if (phase == 0 && bv_connectible(v)) conn |= 1u << (bounces + 1);
+                ++bounces;
+                if (bounces < max_depth && v.f.lobe != LOBE_NONE) {
+                    V3 wi;
+                    uint32_t stype = 0;
+                    real pdf = 0;
+                    const Spec fv = bsdf_sample<LM>(v.f, v.wo, wi, rng_2d(rng), pdf, BSDF_ALL, stype, nullptr);
+                    if (!is_black(fv) && pdf != 0) {
+                        end = false;
+                        beta = beta * (fv * absdot(wi, v.f.ns) / pdf);
+                        pdf_fwd = pdf;
+                        real pdf_rev = bsdf_pdf<LM>(v.f, wi, v.wo, BSDF_ALL, nullptr);
+                        if (stype & BSDF_SPECULAR) {
+                            delta |= phase == 0 ? 1u << bounces : 0x10000u << bounces;
+                            pdf_fwd = pdf_rev = 0;
+                        }
+                        if (phase == 1) {  // importance
+                            beta = beta * bdpt_shading_fix(v.f, v.wo, wi);
+                            // specular transmission scales radiance by (eta_i / eta_t)^2 (the BSDF applies
+                            // it); importance is not scaled (PBRT's TransportMode), so light paths undo it
+                            if (v.f.lobe == LOBE_FRESNEL_SPECULAR && (stype & BSDF_TRANSMISSION)) {
+                                const bool entering = dot(v.wo, v.f.ns) > 0;
+                                const real ei = entering ? 1.0f : v.f.eta, et = entering ? v.f.eta : 1.0f;
+                                beta = beta * ((et * et) / (ei * ei));
+                            }
+                        }
+                        // the vertex before: camera vertex 0 has no slot
+                        if (slot > 0) buf.pdf[(size_t)(slot - 1) * buf.cap + k].y = bv_convert(pdf_rev, v, prev);
+                        ro = offset_origin(si.p, si.perr, si.n, wi);
+                        rd = wi;
+                        prev_p = v.p;
+                        prev_n = v.n;
+                    }
+                }
             }
         }
-        prev.pdf_rev = bv_convert(pdf_rev, v, prev);
-        ro = offset_origin(si.p, si.perr, si.n, wi);
-        rd = wi;
+        if (end && phase == 1) {
+            n_light = 1 + bounces;
+            phase = 2;
+        } else if (end) {  // the camera walk is over: the light walk's start
+            n_cam = 1 + bounces;
+            phase = 2;
+            bounces = 0;
+            max_depth = maxb;
+            real lpick;
+            const int li = bdpt_pick_light(sv, rng_1d(rng), lpick);
+            const F2 u1 = rng_2d(rng), u2 = rng_2d(rng);
+            const DevLight& L = sv.lights[li];
+            BVert l0 = bv_camera(cam);
+            l0.type = BV_LIGHT;
+            l0.light = li;
+            l0.f = Bsdf{};
+            l0.wo = v3(0, 0, 0);
+            V3 dir, nl;
+            real pdf_pos = 0, pdf_dir = 0;
+            const Spec Le = Spec{L.L[0], L.L[1], L.L[2]};
+            if (L.kind == 0) {  // point on the triangle (Triangle::sample), cosine-weighted direction
+                // weights of p0, p1, p2 as Triangle::sample draws them (Triangle.cu:232-259); the
+                // emitting side is the surface normal make_si gives a hit there
+                const real su = xsqrt(u1.x);
+                const real w0 = 1 - su, w1 = u1.y * su, w2 = 1 - w0 - w1;
+                V3 p0, p1, p2;
+                prim_tri(sv, L.prim, p0, p1, p2);
+                SI ls;
+                make_si(sv, L.prim, v3(0, 0, 1), w1, w2, 1.0f, ls);
+                nl = ls.n;
+                l0.p = p0 * w0 + p1 * w1 + p2 * w2;
+                l0.perr = (vabs(p0 * w0) + vabs(p1 * w1) + vabs(p2 * w2)) * gamma_n(6);
+                l0.n = nl;
+                const real r = xsqrt(u2.x), th = mul_dc(u2.y, LTS_2PI);
+                const real lx = r * xcos(th), ly = r * xsin(th), lz = xsqrt(xmax(0.0f, 1 - lx * lx - ly * ly));
+                V3 a, b;
+                coordinate_system(nl, a, b);
+                dir = normalize(a * lx + b * ly + nl * lz);
+                pdf_pos = 1 / L.area;
+                pdf_dir = lz * LTS_INV_PI_F;
+            } else {  // point light: uniform sphere of directions
+                const real z = 1 - 2 * u1.x, r = xsqrt(xmax(0.0f, 1 - z * z)), ph = mul_dc(u1.y, LTS_2PI);
+                dir = v3(r * xcos(ph), r * xsin(ph), z);
+                nl = dir;
+                l0.p = v3(L.p[0], L.p[1], L.p[2]);
+                pdf_pos = 1;
+                pdf_dir = (real)(0.25 * LTS_INV_PI_F);
+            }
+            if (pdf_pos > 0 && pdf_dir > 0 && !is_black(Le)) {
+                l0.beta = Le;
+                buf.pdf[(size_t)(maxb + 1) * buf.cap + k] = make_float2(pdf_pos * lpick, 0.f);
+                bv_store<LM>(buf, maxb + 1, k, l0);
+                beta = Le * (absdot(nl, dir) / (lpick * pdf_pos * pdf_dir));
+                pdf_fwd = pdf_dir;
+                ro = offset_origin(l0.p, l0.perr, l0.n, dir);
+                rd = dir;
+                prev_p = l0.p;
+                prev_n = l0.n;
+                phase = 1;  // a walk of no surface vertices (max_bounce 0) ends in the next turn
+            }
+        }
     }
-    return bounces;
+    if (in) {
+        buf.head[k] = make_uint4(__float_as_uint(pfx), __float_as_uint(pfy), rng.draw,
+                                 (uint32_t)n_cam | ((uint32_t)n_light << 4) | (conn << 8));
+        buf.delta[k] = delta;
+    }
+    const unsigned tot = __reduce_add_sync(~0u, rays);
+    if ((threadIdx.x & 31) == 0 && rp.counters) atomicAdd(rp.counters, (unsigned long long)tot);
 }
 
 // MISWeight: the balance heuristic over every strategy that could have made the same path, from
 // the ratio chain of forward and reverse densities; the connection endpoints' densities (and the
-// resampled endpoint of s = 1 or t = 1) replace the stored ones for the evaluation.
+// resampled endpoint of s = 1 or t = 1) replace the stored ones for the evaluation.  qs / pt: the
+// connected light and camera vertices (s, t > 0), qsm / ptm the ones before them (s, t > 1).
 template <int LM>
-__device__ real bdpt_mis(const SceneView& sv, const BCam& cam, const BVert* lp, const BVert* cp, const BVert& sampled,
-                         int s, int t) {
+__device__ real bdpt_mis(const SceneView& sv, const BCam& cam, const BdptBuf& buf, int k, int maxb, int s, int t,
+                         const BVert& qs, const BVert& pt, const BVert& qsm, const BVert& ptm) {
     if (s + t == 2) return 1;
-    const BVert* qs = s > 0 ? (s == 1 ? &sampled : &lp[s - 1]) : nullptr;
-    const BVert* pt = t > 0 ? (t == 1 ? &sampled : &cp[t - 1]) : nullptr;
-    const BVert* qsm = s > 1 ? &lp[s - 2] : nullptr;
-    const BVert* ptm = t > 1 ? &cp[t - 2] : nullptr;
     // overridden reverse densities of the four vertices around the connection
     real pt_rev = 0, ptm_rev = 0, qs_rev = 0, qsm_rev = 0;
-    if (pt) {
-        if (s > 0) pt_rev = bv_pdf<LM>(sv, cam, *qs, qsm, *pt);
-        else pt_rev = bv_pdf_light_origin(sv, *pt);  // pt is an emitting surface
+    if (s > 0) pt_rev = bv_pdf<LM>(sv, cam, qs, s > 1 ? &qsm : nullptr, pt);
+    else pt_rev = bv_pdf_light_origin(sv, pt);  // pt is an emitting surface
+    if (t > 1) {
+        if (s > 0) ptm_rev = bv_pdf<LM>(sv, cam, pt, &qs, ptm);
+        else ptm_rev = bv_pdf_light(sv, pt, ptm);  // PdfLight of the emitting surface pt toward ptm
     }
-    if (ptm) {
-        if (s > 0) ptm_rev = bv_pdf<LM>(sv, cam, *pt, qs, *ptm);
-        else {  // PdfLight of the emitting surface pt toward ptm
-            BVert lv = *pt;
-            lv.type = BV_LIGHT;
-            ptm_rev = bv_pdf_light(sv, lv, *ptm);
-        }
-    }
-    if (qs) qs_rev = bv_pdf<LM>(sv, cam, *pt, ptm, *qs);
-    if (qsm) qsm_rev = bv_pdf<LM>(sv, cam, *qs, pt, *qsm);
+    if (s > 0) qs_rev = bv_pdf<LM>(sv, cam, pt, t > 1 ? &ptm : nullptr, qs);
+    if (s > 1) qsm_rev = bv_pdf<LM>(sv, cam, qs, &pt, qsm);
+    const uint32_t delta = buf.delta[k];
     auto remap0 = [](real f) -> real { return f != 0 ? f : 1; };
     real sum = 0, ri = 1;
     for (int i = t - 1; i > 0; --i) {
-        const BVert& v = i == t - 1 ? *pt : cp[i];
-        const real rev = i == t - 1 ? pt_rev : (i == t - 2 ? ptm_rev : cp[i].pdf_rev);
-        ri *= remap0(rev) / remap0(v.pdf_fwd);
-        const bool d_i = i == t - 1 ? false : cp[i].delta != 0;
-        const bool d_im = (i - 1 == t - 1) ? false : cp[i - 1].delta != 0;
+        const float2 w = __ldg(buf.pdf + (size_t)(i - 1) * buf.cap + k);
+        const real rev = i == t - 1 ? pt_rev : (i == t - 2 ? ptm_rev : w.y);
+        ri *= remap0(rev) / remap0(w.x);
+        const bool d_i = i == t - 1 ? false : ((delta >> i) & 1u) != 0;
+        const bool d_im = ((delta >> (i - 1)) & 1u) != 0;
         if (!d_i && !d_im) sum += ri;
     }
     ri = 1;
     for (int i = s - 1; i >= 0; --i) {
-        const BVert& v = i == s - 1 ? *qs : lp[i];
-        const real rev = i == s - 1 ? qs_rev : (i == s - 2 ? qsm_rev : lp[i].pdf_rev);
-        ri *= remap0(rev) / remap0(v.pdf_fwd);
-        const bool d_i = i == s - 1 ? false : lp[i].delta != 0;
-        const bool d_light = i > 0 ? lp[i - 1].delta != 0 : bv_delta_light(sv, s == 1 ? sampled : lp[0]);
+        const float2 w = __ldg(buf.pdf + (size_t)(maxb + 1 + i) * buf.cap + k);
+        const real fwd = s == 1 ? qs.pdf_fwd : w.x;  // s = 1: the resampled light point
+        const real rev = i == s - 1 ? qs_rev : (i == s - 2 ? qsm_rev : w.y);
+        ri *= remap0(rev) / remap0(fwd);
+        const bool d_i = i == s - 1 ? false : ((delta >> (16 + i)) & 1u) != 0;
+        bool d_light;
+        if (i > 0) {
+            d_light = ((delta >> (16 + i - 1)) & 1u) != 0;
+        } else if (s == 1) {
+            d_light = bv_delta_light(sv, qs);
+        } else {
+            const uint32_t li = __ldg(buf.vert + ((size_t)(maxb + 1) * bv_words<LM>() + 1) * buf.cap + k).w;
+            d_light = sv.lights[li].kind == 2;
+        }
         if (!d_i && !d_light) sum += ri;
     }
     return 1 / (1 + sum);
@@ -359,221 +587,130 @@ __device__ __forceinline__ void bdpt_add_splat(const SceneView& sv, real rx, rea
         }
 }
 
-#ifndef LTS_BDPT_MIN_BLOCKS
-// Resident blocks per SM the register budget is cut for: the kernel is bound by latency, and more
-// warps pay even with spills (Msamples/s on the bench's box: 2 blocks 5.44, 3 (168 registers, no
-// spills) 5.84, 4 6.27, 5 6.60, 6 7.14, 8 (64 registers) 8.19; the traversal stacks' shared
-// memory allows 9).
-#define LTS_BDPT_MIN_BLOCKS 8
-#endif
-template <int LM, bool TEX>
-__global__ __launch_bounds__(kThreads, LTS_BDPT_MIN_BLOCKS) void k_bdpt(const SceneView sv, const RenderParams rp, int nleaf,
-                                                      double* __restrict__ splat, int only) {
+// ConnectBDPT of strategy (s, t) = strategies[blockIdx.y] for samples first .. first + n - 1.
+constexpr int kBdptConnectBlocks = 4;  // resident blocks per SM the register budget is cut for
+template <int LM, bool WIDE>
+__global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(const SceneView sv, const RenderParams rp, int nleaf,
+                                                                               BdptBuf buf, const BdptStrategies st, long first,
+                                                                               int n, int only, double* __restrict__ splat) {
     __shared__ uint32_t s_stack[kStack * kThreads];
-    const int tid = threadIdx.y * kBX + threadIdx.x;
-    uint32_t* stack = s_stack + tid;
-    const int i = rp.x0 + blockIdx.x * kBX + threadIdx.x;
-    const int j = rp.y0 + blockIdx.y * kBY + threadIdx.y;
-    if (i >= rp.x1 || j >= rp.y1) return;
-    const BCam cam = bdpt_camera(sv);
-    const int W = sv.width, H = sv.height;
-    const real rx = (real)(W - 1), ry = (real)(H - 1);
-    Rng rng;
-    rng.key = rp.seed + wang_hash((uint32_t)(j * W + i));
-    unsigned long long rays = 0;
-    Work wk{0u, 0u};
+    const int k = blockIdx.x * kThreads + threadIdx.x;
+    const int s = st.s[blockIdx.y], t = st.t[blockIdx.y];
     const int maxb = min(rp.max_bounce, kBdptMaxBounce);
-    BVert cp[kBdptMaxBounce + 2], lp[kBdptMaxBounce + 1];
-    // the pixel's samples are split over gridDim.z slices of the grid (sample s_ix draws the same
-    // numbers whatever the split; the film and splat sums are atomic)
-    for (int s_ix = (int)blockIdx.z; s_ix < rp.spp; s_ix += (int)gridDim.z) {
-        rng.sample = (uint32_t)s_ix;
-        rng.draw = 0;
-        // camera subpath (GenerateCameraSubpath): the path tracer's primary ray and differentials
-        const F2 fs = rng_2d(rng);
-        (void)rng_2d(rng);
-        const real pfx = (real)(i + fs.x), pfy = (real)(j + fs.y);
-        const V3 rd = normalize(cam.llc + cam.right * (pfx / rx) + cam.up * (pfy / ry) - cam.o);
-        const V3 dx0 = normalize(cam.llc + cam.right * ((pfx + 1) / rx) + cam.up * (pfy / ry) - cam.o);
-        const V3 dy0 = normalize(cam.llc + cam.right * (pfx / rx) + cam.up * ((pfy + 1) / ry) - cam.o);
-        const V3 rxd = rd + (dx0 - rd) * rp.spp_scale, ryd = rd + (dy0 - rd) * rp.spp_scale;
-        BVert& c0 = cp[0];
-        c0.type = BV_CAMERA;
-        c0.delta = 0;
-        c0.light = -1;
-        c0.p = cam.o;
-        c0.n = v3(0, 0, 0);
-        c0.perr = v3(0, 0, 0);
-        c0.beta = spec(1.0f);
-        c0.pdf_fwd = c0.pdf_rev = 0;
-        c0.f.lobe = LOBE_NONE;
-        real cpx, cpy, cos_t;
-        bdpt_raster(cam, rd, cpx, cpy, cos_t);
-        const int n_cam = 1 + bdpt_walk<LM, TEX>(sv, nleaf, cp, cam.o, rd, spec(1.0f), bdpt_pdf_dir(cam, cos_t), maxb + 1,
-                                        false, rng, true, cam.o, rxd, ryd, stack, rp.err, wk, rays);
-        // light subpath (GenerateLightSubpath)
-        int n_light = 0;
-        {
-            real lpick;
-            const int li = bdpt_pick_light(sv, rng_1d(rng), lpick);
-            const F2 u1 = rng_2d(rng), u2 = rng_2d(rng);
-            const DevLight& L = sv.lights[li];
-            BVert& l0 = lp[0];
-            l0.type = BV_LIGHT;
-            l0.light = li;
-            l0.pdf_rev = 0;
-            l0.f.lobe = LOBE_NONE;
-            V3 dir, nl;
-            real pdf_pos = 0, pdf_dir = 0;
-            Spec Le = spec(0.0f);
-            if (L.kind == 0) {  // point on the triangle (Triangle::sample), cosine-weighted direction
-                // weights of p0, p1, p2 as Triangle::sample draws them (Triangle.cu:232-259); the
-                // emitting side is the surface normal make_si gives a hit there
-                const real su = xsqrt(u1.x);
-                const real w0 = 1 - su, w1 = u1.y * su, w2 = 1 - w0 - w1;
-                V3 p0, p1, p2;
-                prim_tri(sv, L.prim, p0, p1, p2);
-                SI ls;
-                make_si(sv, L.prim, v3(0, 0, 1), w1, w2, 1.0f, ls);
-                nl = ls.n;
-                l0.p = p0 * w0 + p1 * w1 + p2 * w2;
-                l0.perr = (vabs(p0 * w0) + vabs(p1 * w1) + vabs(p2 * w2)) * gamma_n(6);
-                l0.n = nl;
-                l0.delta = 0;
-                const real r = xsqrt(u2.x), th = mul_dc(u2.y, LTS_2PI);
-                const real lx = r * xcos(th), ly = r * xsin(th), lz = xsqrt(xmax(0.0f, 1 - lx * lx - ly * ly));
-                V3 a, b;
-                coordinate_system(nl, a, b);
-                dir = normalize(a * lx + b * ly + nl * lz);
-                pdf_pos = 1 / L.area;
-                pdf_dir = lz * LTS_INV_PI_F;
-                Le = Spec{L.L[0], L.L[1], L.L[2]};
-            } else {  // point light: uniform sphere of directions
-                const real z = 1 - 2 * u1.x, r = xsqrt(xmax(0.0f, 1 - z * z)), ph = mul_dc(u1.y, LTS_2PI);
-                dir = v3(r * xcos(ph), r * xsin(ph), z);
-                nl = dir;
-                l0.p = v3(L.p[0], L.p[1], L.p[2]);
-                l0.perr = v3(0, 0, 0);
-                l0.n = v3(0, 0, 0);
-                l0.delta = 0;
-                pdf_pos = 1;
-                pdf_dir = (real)(0.25 * LTS_INV_PI_F);
-                Le = Spec{L.L[0], L.L[1], L.L[2]};
-            }
-            if (pdf_pos > 0 && pdf_dir > 0 && !is_black(Le)) {
-                l0.beta = Le;
-                l0.pdf_fwd = pdf_pos * lpick;
-                const Spec beta = Le * (absdot(nl, dir) / (lpick * pdf_pos * pdf_dir));
-                const V3 org = offset_origin(l0.p, l0.perr, l0.n, dir);
-                n_light = 1 + bdpt_walk<LM, TEX>(sv, nleaf, lp, org, dir, beta, pdf_dir, maxb, true, rng, false, org, dir, dir,
-                                        stack, rp.err, wk, rays);
-            }
-        }
-        // every strategy
-        Spec L = spec(0.0f);
-        for (int t = 1; t <= n_cam; ++t) {
-            for (int s = 0; s <= n_light; ++s) {
-                const int depth = t + s - 2;
-                if ((s == 1 && t == 1) || depth < 0 || depth > maxb) continue;
-                if (only >= 0 && (s != only / 100 || t != only % 100)) continue;
-                Spec c = spec(0.0f);
-                BVert sampled;
-                sampled.type = BV_CAMERA;
-                sampled.delta = 0;
-                sampled.light = -1;
-                bool splat_it = false;
-                real spx = 0, spy = 0;
-                if (t > 1 && s != 0 && cp[t - 1].type == BV_LIGHT) continue;
-                if (s == 0) {  // the camera path's end is on a light
-                    const BVert& pt = cp[t - 1];
-                    if (bv_is_light(pt)) c = bv_le(sv, pt, normalize(cp[t - 2].p - pt.p)) * pt.beta;
-                } else if (t == 1) {  // connect the light path's end to the camera
-                    const BVert& qs = lp[s - 1];
-                    if (bv_connectible(qs)) {
-                        const V3 d = cam.o - qs.p;
-                        const real l2 = len2(d);
-                        const V3 wi = d * xsqrt(1 / l2);
-                        real cos_c;
-                        if (l2 > 0 && bdpt_raster(cam, -wi, spx, spy, cos_c)) {
-                            const real pdf = l2 / cos_c;  // solid angle at qs (lens area 1)
-                            sampled.type = BV_CAMERA;
-                            sampled.p = cam.o;
-                            sampled.n = v3(0, 0, 0);
-                            sampled.perr = v3(0, 0, 0);
-                            sampled.beta = spec(bdpt_we(cam, cos_c) / pdf);
-                            sampled.pdf_fwd = sampled.pdf_rev = 0;
-                            sampled.f.lobe = LOBE_NONE;
-                            // qs is a surface vertex: s >= 2 whenever t = 1
-                            c = qs.beta * bv_f<LM>(qs, sampled, true) * sampled.beta * absdot(wi, qs.f.ns);
-                            if (!is_black(c)) {
-                                ++rays;
-                                if (!bdpt_visible(sv, nleaf, qs, sampled, stack, rp.err, wk)) c = spec(0.0f);
-                            }
-                            splat_it = true;
-                        }
-                    }
-                } else if (s == 1) {  // connect the camera path's end to a sampled light point
-                    const BVert& pt = cp[t - 1];
-                    if (bv_connectible(pt)) {
-                        real lpick;
-                        const int li = bdpt_pick_light(sv, rng_1d(rng), lpick);
-                        const F2 ul = rng_2d(rng);
-                        const DevLight& Lt = sv.lights[li];
-                        SI psi;
-                        psi.p = pt.p;
-                        psi.perr = pt.perr;
-                        psi.n = pt.n;
-                        LightSample ls;
-                        const bool delta = sample_li(sv, Lt, psi, ul, ls);
-                        if (ls.pdf > 0 && !is_black(ls.Li)) {
-                            sampled.type = BV_LIGHT;
-                            sampled.light = li;
-                            sampled.delta = 0;
-                            sampled.p = ls.p1;
-                            sampled.n = delta ? v3(0, 0, 0) : ls.n1;
-                            sampled.perr = ls.perr1;
-                            sampled.beta = ls.Li / (ls.pdf * lpick);
-                            sampled.pdf_rev = 0;
-                            sampled.f.lobe = LOBE_NONE;
-                            sampled.pdf_fwd = bv_pdf_light_origin(sv, sampled);
-                            c = pt.beta * bv_f<LM>(pt, sampled, false) * sampled.beta;
-                            c = c * absdot(ls.wi, pt.f.ns);
-                            if (!is_black(c)) {
-                                ++rays;
-                                if (!bdpt_visible(sv, nleaf, pt, sampled, stack, rp.err, wk)) c = spec(0.0f);
-                            }
-                        }
-                    }
-                } else {  // connect two surface vertices (s >= 2, t >= 2)
-                    const BVert& qs = lp[s - 1];
-                    const BVert& pt = cp[t - 1];
-                    if (bv_connectible(qs) && bv_connectible(pt)) {
-                        c = qs.beta * bv_f<LM>(qs, pt, true) * bv_f<LM>(pt, qs, false) * pt.beta;
-                        if (!is_black(c)) {  // generalized geometry term G with visibility
-                            V3 d = qs.p - pt.p;
-                            real g = 1 / len2(d);
-                            d = d * xsqrt(g);
-                            g *= absdot(qs.f.ns, d) * absdot(pt.f.ns, d);
-                            ++rays;
-                            c = bdpt_visible(sv, nleaf, qs, pt, stack, rp.err, wk) ? c * g : spec(0.0f);
-                        }
-                    }
-                }
-                if (is_black(c)) continue;
-                if (only < 0) c = c * bdpt_mis<LM>(sv, cam, lp, cp, sampled, s, t);
-                if (splat_it) {
-                    bdpt_add_splat(sv, spx, spy, c, splat);
-                } else {
-                    L = L + c;
+    const bool in = k < n;
+    const uint4 h = in ? __ldg(buf.head + k) : make_uint4(0u, 0u, 0u, 0u);
+    const int n_cam = (int)(h.w & 15u), n_light = (int)((h.w >> 4) & 15u);
+    const bool have = in && t <= n_cam && s <= n_light;
+    const BCam cam = bdpt_camera(sv);
+    Spec c = spec(0.0f);
+    BVert qs, pt, qsm, ptm;
+    real spx = 0, spy = 0, geo = 1;
+    bool vis = false;  // the connection needs its shadow ray
+    if (have) {
+        if (t == 1) pt = bv_camera(cam);
+        else bv_load<LM>(buf, t - 2, k, pt);
+        if (t == 2) ptm = bv_camera(cam);
+        else if (t > 2) bv_load<LM>(buf, t - 3, k, ptm);
+        if (s == 1) qs = bv_camera(cam);  // resampled below
+        else if (s > 1) bv_load<LM>(buf, maxb + s, k, qs);
+        if (s > 1) bv_load<LM>(buf, maxb + s - 1, k, qsm);
+        if (s == 0) {  // the camera path's end is on a light
+            if (bv_is_light(pt)) c = bv_le(sv, pt, normalize(ptm.p - pt.p)) * pt.beta;
+        } else if (t == 1) {  // connect the light path's end to the camera
+            if (bv_connectible(qs)) {
+                const V3 d = cam.o - qs.p;
+                const real l2 = len2(d);
+                const V3 wi = d * xsqrt(1 / l2);
+                real cos_c;
+                if (l2 > 0 && bdpt_raster(cam, -wi, spx, spy, cos_c)) {
+                    const real pdf = l2 / cos_c;  // solid angle at qs (lens area 1)
+                    pt.beta = spec(bdpt_we(cam, cos_c) / pdf);
+                    // qs is a surface vertex: s >= 2 whenever t = 1
+                    c = qs.beta * bv_f<LM>(qs, pt, true) * pt.beta * absdot(wi, qs.f.ns);
+                    vis = !is_black(c);
                 }
             }
+        } else if (s == 1) {  // connect the camera path's end to a sampled light point
+            if (bv_connectible(pt)) {
+                // three draws for each connectible camera vertex before this one
+                int i, j, s_ix;
+                bdpt_pixel(rp, first + k, i, j, s_ix);
+                Rng rng;
+                rng.key = rp.seed + wang_hash((uint32_t)(j * sv.width + i));
+                rng.sample = (uint32_t)s_ix;
+                rng.draw = h.z;
+                if (only < 0) rng.draw += 3u * (uint32_t)__popc((h.w >> 8) & ((1u << (t - 1)) - 1u));
+                rng_resume(rng);
+                real lpick;
+                const int li = bdpt_pick_light(sv, rng_1d(rng), lpick);
+                const F2 ul = rng_2d(rng);
+                const DevLight& Lt = sv.lights[li];
+                SI psi;
+                psi.p = pt.p;
+                psi.perr = pt.perr;
+                psi.n = pt.n;
+                LightSample ls;
+                const bool dl = sample_li(sv, Lt, psi, ul, ls);
+                if (ls.pdf > 0 && !is_black(ls.Li)) {
+                    qs.type = BV_LIGHT;
+                    qs.light = li;
+                    qs.p = ls.p1;
+                    qs.n = dl ? v3(0, 0, 0) : ls.n1;
+                    qs.perr = ls.perr1;
+                    qs.beta = ls.Li / (ls.pdf * lpick);
+                    qs.pdf_fwd = bv_pdf_light_origin(sv, qs);
+                    c = pt.beta * bv_f<LM>(pt, qs, false) * qs.beta;
+                    c = c * absdot(ls.wi, pt.f.ns);
+                    vis = !is_black(c);
+                }
+            }
+        } else if (bv_connectible(qs) && bv_connectible(pt)) {  // connect two surface vertices (s >= 2, t >= 2)
+            c = qs.beta * bv_f<LM>(qs, pt, true) * bv_f<LM>(pt, qs, false) * pt.beta;
+            if (!is_black(c)) {  // generalized geometry term G with visibility
+                V3 d = qs.p - pt.p;
+                real g = 1 / len2(d);
+                d = d * xsqrt(g);
+                g *= absdot(qs.f.ns, d) * absdot(pt.f.ns, d);
+                geo = g;
+                vis = true;
+            }
         }
-        bdpt_add_sample(sv, rp, pfx, pfy, L);
     }
-    const unsigned mask = __activemask();
-    const unsigned tot = __reduce_add_sync(mask, (unsigned)rays);
-    const unsigned lane = (unsigned)tid & 31u;
-    if ((mask & ((1u << lane) - 1u)) == 0u && rp.counters) atomicAdd(rp.counters, (unsigned long long)tot);
+    // VisibilityTester::unoccluded between the vertices (offset origins as spawnRayTo), from the
+    // camera path's end (t = 1: from the light path's)
+    if (__any_sync(~0u, vis)) {
+        V3 org = v3(0, 0, 0), dir = v3(0, 0, 1);
+        if (vis) {
+            const BVert &a = t == 1 || s >= 2 ? qs : pt, &b = t == 1 || s >= 2 ? pt : qs;
+            org = offset_origin(a.p, a.perr, a.n, b.p - a.p);
+            dir = offset_origin(b.p, b.perr, b.n, org - b.p) - org;
+        }
+        Trav tr;
+        Work wk{0u, 0u};
+        warp_rays<true, WIDE>(vis, tr, sv, nleaf, org, dir, 1 - kShadowEps, s_stack + threadIdx.x, rp.err, wk);
+        if (vis) c = tr.best == 1 ? spec(0.0f) : (s >= 2 && t >= 2 ? c * geo : c);
+    }
+    if (have && !is_black(c)) {
+        if (only < 0) c = c * bdpt_mis<LM>(sv, cam, buf, k, maxb, s, t, qs, pt, qsm, ptm);
+        if (t == 1) bdpt_add_splat(sv, spx, spy, c, splat);
+    }
+    if (in && t > 1) buf.contrib[(size_t)blockIdx.y * buf.cap + k] = make_float4(c.r, c.g, c.b, 0.f);
+    const unsigned tot = __popc(__ballot_sync(~0u, vis));
+    if ((threadIdx.x & 31) == 0 && tot && rp.counters) atomicAdd(rp.counters, (unsigned long long)tot);
+}
+
+__global__ __launch_bounds__(kThreads) void k_bdpt_film(const SceneView sv, const RenderParams rp, BdptBuf buf,
+                                                        const BdptStrategies st, int n) {
+    const int k = blockIdx.x * kThreads + threadIdx.x;
+    if (k >= n) return;
+    Spec L = spec(0.0f);
+    for (int q = 0; q < st.n; ++q) {
+        if (st.t[q] == 1) continue;
+        const float4 c = __ldg(buf.contrib + (size_t)q * buf.cap + k);
+        L = L + Spec{c.x, c.y, c.z};
+    }
+    const uint4 h = __ldg(buf.head + k);
+    bdpt_add_sample(sv, rp, __uint_as_float(h.x), __uint_as_float(h.y), L);
 }
 
 }  // namespace

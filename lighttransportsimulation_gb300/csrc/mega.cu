@@ -332,20 +332,58 @@ std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, 
     return "";
 }
 
+namespace {
+// The strategies (s, t) of a path of at most maxb + 2 vertices (only >= 0: the one s = only / 100,
+// t = only % 100), camera vertices outer, light vertices inner.
+BdptStrategies bdpt_strategies(int maxb, int only) {
+    BdptStrategies st;
+    st.n = 0;
+    for (int t = 1; t <= maxb + 2; ++t)
+        for (int s = 0; s <= maxb + 1; ++s) {
+            const int depth = t + s - 2;
+            if ((s == 1 && t == 1) || depth < 0 || depth > maxb) continue;
+            if (only >= 0 && (s != only / 100 || t != only % 100)) continue;
+            if (st.n < kBdptMaxStrategies) {
+                st.s[st.n] = (unsigned char)s;
+                st.t[st.n] = (unsigned char)t;
+                ++st.n;
+            }
+        }
+    return st;
+}
+static_assert((kBdptMaxBounce + 2) * (kBdptMaxBounce + 3) / 2 + kBdptMaxBounce <= kBdptMaxStrategies,
+              "every strategy of the longest path fits the list");
+}  // namespace
+
+size_t bdpt_sample_bytes(int max_bounce, int strategy) {
+    const int maxb = std::min(max_bounce, kBdptMaxBounce);
+    return (size_t)(2 * maxb + 2) * (16 * kBvWordsAll + 8) + 16 * (size_t)bdpt_strategies(maxb, strategy).n + 20;
+}
+
 std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
-                        bool matte_only, cudaStream_t s) {
-    // one thread per pixel and sample slice: enough blocks for every SM to hold its resident
-    // ones about four times over (a small film alone would leave most SMs idle)
-    const dim3 block(kBX, kBY);
-    dim3 grid((rp.x1 - rp.x0 + kBX - 1) / kBX, (rp.y1 - rp.y0 + kBY - 1) / kBY);
-    int dev = 0, sms = 0;
-    TRY(cudaGetDevice(&dev));
-    TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const long want = 4L * LTS_BDPT_MIN_BLOCKS * sms, have = (long)grid.x * grid.y;
-    grid.z = (unsigned)std::max(1L, std::min<long>(rp.spp, (want + have - 1) / have));
-    if (matte_only) k_bdpt<LM_MATTE, false><<<grid, block, 0, s>>>(sv, rp, nleaf, splat, strategy);
-    else k_bdpt<LM_ALL, true><<<grid, block, 0, s>>>(sv, rp, nleaf, splat, strategy);
-    TRY(cudaGetLastError());
+                        bool matte_only, void* ws, long cap, cudaStream_t s) {
+    const int maxb = std::min(rp.max_bounce, kBdptMaxBounce);
+    const BdptStrategies st = bdpt_strategies(maxb, strategy);
+    const bool wide = sv.wnodes != nullptr && sv.ninst == 0;
+    const size_t slots = 2 * (size_t)maxb + 2, words = matte_only && wide ? kBvWordsMatte : kBvWordsAll;
+    BdptBuf buf;
+    buf.cap = (int)cap;
+    buf.vert = static_cast<uint4*>(ws);
+    buf.head = buf.vert + slots * words * cap;
+    buf.contrib = reinterpret_cast<float4*>(buf.head + cap);
+    buf.pdf = reinterpret_cast<float2*>(buf.contrib + (size_t)st.n * cap);
+    buf.delta = reinterpret_cast<uint32_t*>(buf.pdf + slots * cap);
+    const long total = (long)(rp.x1 - rp.x0) * (rp.y1 - rp.y0) * rp.spp;
+    for (long first = 0; first < total; first += cap) {
+        const int n = (int)std::min(cap, total - first);
+        const unsigned gw = (unsigned)((n + kBdptWalkThreads - 1) / kBdptWalkThreads), gs = (unsigned)((n + kThreads - 1) / kThreads);
+        auto kw = !wide ? k_bdpt_walk<LM_ALL, true, false> : matte_only ? k_bdpt_walk<LM_MATTE, false, true> : k_bdpt_walk<LM_ALL, true, true>;
+        auto kc = !wide ? k_bdpt_connect<LM_ALL, false> : matte_only ? k_bdpt_connect<LM_MATTE, true> : k_bdpt_connect<LM_ALL, true>;
+        kw<<<gw, kBdptWalkThreads, 0, s>>>(sv, rp, nleaf, buf, first, n);
+        if (st.n > 0) kc<<<dim3(gs, (unsigned)st.n), kThreads, 0, s>>>(sv, rp, nleaf, buf, st, first, n, strategy, splat);
+        k_bdpt_film<<<gs, kThreads, 0, s>>>(sv, rp, buf, st, n);
+        TRY(cudaGetLastError());
+    }
     return "";
 }
 

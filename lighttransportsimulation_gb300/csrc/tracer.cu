@@ -400,6 +400,9 @@ void Tracer::free_all() {
     splat_ = nullptr;
     splat_cap_ = 0;
     splat_spp_ = 0;
+    dev_free(bdpt_ws_);
+    bdpt_ws_ = nullptr;
+    bdpt_ws_cap_ = 0;
     dev_free(trace_);
     trace_ = nullptr;
     dev_free(views_film_);
@@ -974,9 +977,29 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     if (!e.empty()) return e;
     last_paths = (double)ns;
     if (d.integrator == LTS_INTEGRATOR_WAVEFRONT) return render_wavefront(sc, bvh, d, s, d_err, rp, sv, ns);
+    long bdpt_cap = 0;
+    if (d.integrator == LTS_INTEGRATOR_BDPT) {
+        // one chunk's workspace, kept: 2^18 samples keep every SM busy over the chunk's launches
+        // (0.5 GB at five bounces); fewer when that much cannot be allocated
+        const size_t per = bdpt_sample_bytes(d.max_bounce, bdpt_strategy);
+        bdpt_cap = std::min<long>((ns + 31) / 32 * 32, 1l << 18);
+        while (bdpt_ws_cap_ < per * bdpt_cap) {
+            dev_free(bdpt_ws_);
+            bdpt_ws_ = nullptr;
+            bdpt_ws_cap_ = 0;
+            const cudaError_t ae = dev_alloc(&bdpt_ws_, per * bdpt_cap);
+            if (ae == cudaSuccess) {
+                bdpt_ws_cap_ = per * bdpt_cap;
+            } else {
+                cudaGetLastError();
+                if (ae != cudaErrorMemoryAllocation || bdpt_cap <= 1024) TRY(ae);
+                bdpt_cap /= 2;
+            }
+        }
+    }
     TRY(cudaEventRecord(ev0_, s));
     if (d.integrator == LTS_INTEGRATOR_FP64) e = render64_launch(sv, rp, bvh.n, d.record_samples != 0, s);
-    else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, s);
+    else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, bdpt_ws_, bdpt_cap, s);
     else e = mega_launch(sv, rp, bvh.n, d.record_samples != 0, matte_only_, s);
     if (!e.empty()) return e;
     TRY(cudaEventRecord(ev1_, s));

@@ -133,8 +133,11 @@ std::string kat_launch(int fn, const float* d_in, int n, float* d_out, cudaStrea
 // or Oren-Nayar with constant textures.
 std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool record, bool matte_only,
                         cudaStream_t s);
+// The bidirectional integrator works on chunks of at most `cap` samples, whose vertices and
+// contributions lie in `ws` (bdpt_sample_bytes per sample; cap a multiple of 32).
+size_t bdpt_sample_bytes(int max_bounce, int strategy);
 std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
-                        bool matte_only, cudaStream_t s);
+                        bool matte_only, void* ws, long cap, cudaStream_t s);
 std::string mega_set_libm_double(int on);
 std::string mega_init();  // that translation unit's texture tables (once per process)
 constexpr int kBdptMaxBounce = 8;  // longest path of the bidirectional integrator
@@ -273,6 +276,8 @@ class Tracer {
     cudaEvent_t shade_fork_ = nullptr, shade_join_[kShadeClasses] = {nullptr};
     double* splat_ = nullptr;  // bidirectional integrator: light-to-camera splats, RGB per pixel
     size_t splat_cap_ = 0;
+    void* bdpt_ws_ = nullptr;  // bidirectional integrator: one chunk's vertices and contributions
+    size_t bdpt_ws_cap_ = 0;
     long splat_spp_ = 0;       // samples per pixel the splats hold
     uint64_t ikey_ = 0;              // key of the scene upload and render-tree choice built from
     uint64_t upload_serial_ = 0;
