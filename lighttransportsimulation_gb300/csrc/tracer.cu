@@ -1068,23 +1068,23 @@ long Tracer::auto_pool(bool cache) const {
 static std::string launch_shade(bool record, int cls, int lm, bool tex, unsigned grid, const SceneView& sv,
                                 const RenderParams& rp, const WfState& st, int pool, cudaStream_t s) {
     if (record) {
-        k_wf_shade<true, LM_ALL, true><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        k_wf_shade<true, LM_ALL, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     } else if (cls == 0) {
-        k_wf_shade<false, 0, false><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        k_wf_shade<false, 0, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_MATTE) {
-        if (tex) k_wf_shade<false, LM_MATTE, true><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_MATTE, false><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_MATTE, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_MATTE, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_GLASS) {
-        if (tex) k_wf_shade<false, LM_GLASS, true><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_GLASS, false><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_GLASS, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_GLASS, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_MIRROR) {
-        if (tex) k_wf_shade<false, LM_MIRROR, true><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_MIRROR, false><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_MIRROR, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_MIRROR, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_METAL) {
-        if (tex) k_wf_shade<false, LM_METAL, true><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_METAL, false><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_METAL, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_METAL, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     } else {
-        k_wf_shade<false, LM_ALL, true><<<grid, kWfBlock, 0, s>>>(sv, rp, st, pool, cls);
+        k_wf_shade<false, LM_ALL, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
     }
     TRY(cudaGetLastError());
     return "";
@@ -1225,7 +1225,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         wf_trace_blocks_[2] = (unsigned)std::max(1, per_i * sms);
         wf_sms_ = (unsigned)sms;
         int per_s = 0;
-        TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_s, k_wf_shade<false, LM_ALL, true>, kWfBlock, 0));
+        TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_s, k_wf_shade<false, LM_ALL, true>, kShadeBlock, 0));
         shade_grid_ = (unsigned)std::max(1, per_s * sms * 2);
         for (int k = 0; k < kShadeClasses; ++k) {
             TRY(cudaStreamCreateWithFlags(&shade_streams_[k], cudaStreamNonBlocking));
@@ -1269,10 +1269,9 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         }
         if (!full) TRY(cudaEventRecord(wf_ev_[3], s));
         if (full || n_ext) {
-            const unsigned g = full ? blocks(P) : blocks(n_ext);
             const long tiles = ((full ? P : (long)n_ext) + kClassifyTile - 1) / kClassifyTile;
             k_wf_classify<<<(unsigned)std::min<long>(tiles, list_grid), kWfBlock, 0, s>>>(st, q_ext, d_ctl, (int)P);
-            const unsigned gs = std::min(g, shade_grid_);
+            const unsigned gs = (unsigned)std::min<long>(((full ? P : (long)n_ext) + kShadeBlock - 1) / kShadeBlock, shade_grid_);
             TRY(cudaEventRecord(shade_fork_, s));
             int nb = 0;
             for (int c = 0; c < kShadeClasses; ++c) {

@@ -431,10 +431,13 @@ __global__ __launch_bounds__(kWfBlock) void k_wf_classify(WfState st, const int3
     }
 }
 
-// Resident blocks per SM the shade kernel is compiled for (caps its registers).
-#ifndef LTS_SHADE_MIN_BLOCKS
-#define LTS_SHADE_MIN_BLOCKS 5  // 6 and 4 measured 2 % and 5 % slower on the stress scene
-#endif
+// One block of 640 threads per SM (96 registers a thread), its warps in step: shade's body is
+// larger than the instruction caches and several classes' kernels share an SM, so warps running
+// free waited on instruction fetch.  Stress scene, 1920 x 1080 x 64: shade 86.5 ms per render with
+// five free blocks of 128, 79.0 with a barrier per path in those, 75.4 as two blocks of 320, 74.4
+// as one of 640; more barriers inside the body (before the material, the light sample, the MIS
+// sample, the path sample) 82.2, prefetching the next path's state and shading record 87.
+constexpr int kShadeBlock = 640;
 // Where shade_scatter's rays and their weights go: the path state.
 struct WfScatter {
     WfState& st;
@@ -577,12 +580,15 @@ __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParam
 // shade over one class's list (k_wf_classify), grid-stride: one launch per shade class present in
 // the scene, each compiled for its material kind (fewer registers, no spills, a smaller kernel).
 template <bool RECORD, int LM, bool TEX>
-__global__ __launch_bounds__(kWfBlock, LTS_SHADE_MIN_BLOCKS) void k_wf_shade(const SceneView sv, const RenderParams rp,
-                                                                              WfState st, int pool, int cls) {
+__global__ __launch_bounds__(kShadeBlock, 1) void k_wf_shade(const SceneView sv, const RenderParams rp,
+                                                                                 WfState st, int pool, int cls) {
     const uint32_t n = st.counts[16 + cls];
     const int32_t* __restrict__ q = st.q_cls + (size_t)cls * pool;
-    for (uint32_t i = blockIdx.x * kWfBlock + threadIdx.x; i < n; i += gridDim.x * kWfBlock)
-        shade_one<RECORD, LM, TEX>(sv, rp, st, q[i]);
+    for (uint32_t first = blockIdx.x * kShadeBlock; first < n; first += gridDim.x * kShadeBlock) {
+        __syncthreads();
+        const uint32_t i = first + threadIdx.x;
+        if (i < n) shade_one<RECORD, LM, TEX>(sv, rp, st, q[i]);
+    }
 }
 
 
