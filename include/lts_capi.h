@@ -283,7 +283,7 @@ int lts_autotune_views(lts_ctx* ctx, const lts_view* views, int32_t n, const lts
  *                             render_bvh 1 or 2; the closest hits are the same up to rounding
  *   "wavefront_pool"          path-state pool capacity in paths (0: automatic -- every path of
  *                             a batch at once, up to 2^26 slots and a quarter of the free
- *                             device memory, ~400 B per slot, ~650 B with the radiance cache)
+ *                             device memory, ~350 B per slot, ~600 B with the radiance cache)
  *   "wavefront_sample_chunk"  finished-sample buffer capacity in samples (0: automatic, 2^27);
  *                             samples per pixel are rendered in chunks that fit it
  *   "watertight"              0 (default): the reference's triangle tests (Moller-Trumbore with

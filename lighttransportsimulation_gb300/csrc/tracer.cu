@@ -1115,23 +1115,32 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     rpw.err = rp.err;
     rpw.trace_sample = -1;
     WfState st{};
+    // the pool's arrays (bytes per slot), then the counts with the control block after them (one
+    // copy reads both back)
+    struct PoolArray {
+        void** at;
+        size_t bytes;
+    } const arrays[] = {
+        {(void**)&st.ray, 32}, {(void**)&st.path, 32}, {(void**)&st.hit, 16}, {(void**)&st.sh, 32}, {(void**)&st.nee, 32},
+        {(void**)&st.mis, 32}, {(void**)&st.mis_fv, 16}, {(void**)&st.ld_mis, 16}, {(void**)&st.pf, 8}, {(void**)&st.sig, 8},
+        {(void**)&st.ev_mis, 8}, {(void**)&st.ev_main, 8}, {(void**)&st.pend, 4}, {(void**)&st.vis, 4}, {(void**)&st.hprim, 4},
+        {(void**)&st.wid, 4}, {(void**)&st.view, 4}, {(void**)&st.mis_hit, 4}, {(void**)&st.q_a, 4}, {(void**)&st.q_b, 4},
+        {(void**)&st.q_shadow, 4}, {(void**)&st.q_mis, 4}, {(void**)&st.q_free, 4}, {(void**)&st.q_cls, 4 * kShadeClasses}};
+    constexpr int kArrays = sizeof arrays / sizeof arrays[0], kCountsBuf = 31;
+    static_assert(kArrays <= kCountsBuf, "the pool's arrays come before the other buffers");
     if (wf_cap_ < P) {
-        for (int k : {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26,
-                      27, 28, 29, 30, 31, 32, 35, 45}) {
-            if (wf_bufs_[k]) dev_free(wf_bufs_[k]);
+        for (int k = 0; k <= kCountsBuf; ++k) {
+            dev_free(wf_bufs_[k]);
             wf_bufs_[k] = nullptr;
         }
         wf_cap_ = 0;
-        const size_t n = (size_t)P;
-        // [31]: the counts, and the control block after them (one copy reads both back)
-        const size_t sizes[] = {4 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n,                       // pix smp draw flags pend vis
-                                16 * n, 16 * n, 16 * n, 16 * n, 8 * n, 8 * n, 4 * n, 16 * n,  // ro rd beta L pf sig hprim huvi
-                                16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n, 16 * n,  // sh_* mis_* ld nee
-                                8 * n, 8 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n, 4 * n, kWfCountsBytes + sizeof(WfCtl),  // ev mis_hit queues counts
-                                4 * n};                                                           // wid
-        for (size_t k = 0; k < sizeof sizes / sizeof sizes[0]; ++k) TRY(dev_alloc(&wf_bufs_[k], sizes[k]));
-        TRY(dev_alloc(&wf_bufs_[35], 4 * (size_t)kShadeClasses * n));  // class-grouped shade lists
-        TRY(dev_alloc(&wf_bufs_[45], 4 * n));                             // view slice of each path
+        size_t per = 0;
+        for (int k = 0; k < kArrays; ++k) {
+            TRY(dev_alloc(&wf_bufs_[k], arrays[k].bytes * (size_t)P));
+            per += arrays[k].bytes;
+        }
+        if (per != kPoolSlotBytes) return "wavefront: pool bytes per slot";
+        TRY(dev_alloc(&wf_bufs_[kCountsBuf], kWfCountsBytes + sizeof(WfCtl)));
         wf_cap_ = P;
     }
     if (wf_fs_cap_ < chunk_total) {
@@ -1145,19 +1154,10 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     }
     if (!wf_counts_host_) TRY(cudaMallocHost((void**)&wf_counts_host_, kWfCountsBytes + sizeof(WfCtl)));
     void** b = wf_bufs_;
-    st.pix = (int32_t*)b[0]; st.smp = (int32_t*)b[1]; st.draw = (uint32_t*)b[2]; st.flags = (uint32_t*)b[3];
-    st.pend = (uint32_t*)b[4]; st.vis = (uint32_t*)b[5];
-    st.ro = (float4*)b[6]; st.rd = (float4*)b[7]; st.beta = (float4*)b[8]; st.L = (float4*)b[9];
-    st.pf = (float2*)b[10]; st.sig = (uint64_t*)b[11]; st.hprim = (int32_t*)b[12]; st.huvi = (float4*)b[13];
-    st.sh_o = (float4*)b[14]; st.sh_d = (float4*)b[15]; st.sh_c = (float4*)b[16];
-    st.mis_o = (float4*)b[17]; st.mis_d = (float4*)b[18]; st.mis_fv = (float4*)b[19]; st.mis_x = (float4*)b[20];
-    st.ld_mis = (float4*)b[21]; st.nee_beta = (float4*)b[22];
-    st.ev_mis = (uint64_t*)b[23]; st.ev_main = (uint64_t*)b[24]; st.mis_hit = (int32_t*)b[25];
-    st.q_a = (int32_t*)b[26]; st.q_b = (int32_t*)b[27]; st.q_shadow = (int32_t*)b[28]; st.q_mis = (int32_t*)b[29];
-    st.q_free = (int32_t*)b[30]; st.counts = (uint32_t*)b[31]; st.wid = (int32_t*)b[32];
+    for (int k = 0; k < kArrays; ++k) *arrays[k].at = b[k];
+    st.counts = (uint32_t*)b[kCountsBuf];
     st.fs_L = (float4*)b[33]; st.fs_y = (float*)b[34];
-    st.q_cls = (int32_t*)b[35];
-    st.view = (int32_t*)b[45];
+    for (const auto& bt : batches) st.many_views |= bt.size() > 1;
     if (!wf_bufs_[46]) TRY(dev_alloc(&wf_bufs_[46], sizeof(WfView) * kMaxViews));
     st.views = (const WfView*)b[46];
     // radiance cache buffers (allocated on first use with the cache on)
@@ -1204,7 +1204,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     auto blocks = [](long n) { return (unsigned)((n + kWfBlock - 1) / kWfBlock); };
     TRY(cudaEventRecord(ev0_, s));
     TRY(cudaMemsetAsync(st.counts, 0, 128, s));
-    k_wf_init_free<<<blocks(P), kWfBlock, 0, s>>>(st.q_free, st.pix, st.counts, (int)P);  // every slot free
+    k_wf_init_free<<<blocks(P), kWfBlock, 0, s>>>(st.q_free, st.pend, st.counts, (int)P);  // every slot free
     TRY(cudaMemsetAsync(st.counts + 32, 0, 8, s));  // training records and eligible vertices of this render
     const bool rec = rp.sample_sig != nullptr;
     const bool wide = sv.wnodes != nullptr;

@@ -292,7 +292,7 @@ class Tracer {
     void* wf_bufs_[48] = {nullptr};
     // Device bytes per pool slot: the path state and lists, and the radiance cache's features,
     // prediction, query list and training-record links.
-    static constexpr size_t kPoolSlotBytes = 392, kCacheSlotBytes = 248;
+    static constexpr size_t kPoolSlotBytes = 348, kCacheSlotBytes = 248;
     long auto_pool(bool cache) const;
     long wf_cache_cap_ = 0, wf_train_cap_ = 0;
     // eligible training vertices per path of the last cached render (-1: none yet) and the

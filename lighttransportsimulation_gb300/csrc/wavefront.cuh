@@ -29,7 +29,7 @@
 namespace lts {
 namespace {
 
-enum : uint32_t { WF_VIS = 1u, WF_MIS = 2u, WF_NEE = 4u, WF_DONE = 8u, WF_CACHE = 16u };
+enum : uint32_t { WF_VIS = 1u, WF_MIS = 2u, WF_NEE = 4u, WF_DONE = 8u, WF_CACHE = 16u, WF_FREE = 32u };
 // path flags (low byte; the bounce count sits above bit 8)
 // FL_RECORDED: the path holds a training record; FL_OFFERED: its one chance of a record (at its
 // first vertex after a rough one) has been taken, whether or not the coin accepted it.
@@ -37,23 +37,29 @@ enum : uint32_t { FL_SPECULAR = 1u, FL_ROUGH = 2u, FL_UNBIASED = 4u, FL_RECORDED
 constexpr int kWfBlock = 128;
 constexpr uint64_t kSigBasis = 0xcbf29ce484222325ull;
 
+// A path's state.  What a stage reads together lies together in 32-byte groups (one sector): a
+// stage's list is one shade class or one ray kind, whose paths are scattered among the others', so
+// a lane's 4- and 16-byte words of separate arrays each cost a sector of their own (stress scene,
+// 1920 x 1080 x 64: shade 74.4 ms per render from arrays of words, 52.5 from these groups).
 struct WfState {
-    int32_t *pix, *smp, *wid;  // pixel (within its view's film), sample, the sample's batch index
-                               // in row-major pixel order (where finalize stores it)
-    int32_t* view;             // slice of the batch the path belongs to
-    const WfView* views;       // the batch's slices (count in WfCtl::nviews)
-    uint32_t *draw, *flags, *pend, *vis;
-    float4 *ro, *rd, *beta, *L;
+    float4* ray;         // [2 pool] origin, flags | direction, sampler draw
+    float4* path;        // [2 pool] throughput, pixel (within its view's film) | radiance, sample
+    int32_t* wid;        // the sample's batch index in row-major pixel order (where finalize stores it)
+    int32_t* view;       // slice of the batch the path belongs to
+    const WfView* views; // the batch's slices (count in WfCtl::nviews)
+    uint32_t *pend, *vis;  // pend: WF_* of the last vertex (WF_FREE: the slot holds no path)
     float2* pf;
     uint64_t* sig;
-    int32_t* hprim;
-    float4* huvi;
-    float4 *sh_o, *sh_d, *sh_c;
-    float4 *mis_o, *mis_d, *mis_fv, *mis_x, *ld_mis;
-    float4* nee_beta;
+    int32_t* hprim;      // the path ray's hit, for classify
+    float4* hit;         // barycentrics, 1 / det, the hit (hit_prim / hit_class)
+    float4* sh;          // [2 pool] shadow ray: origin, - | direction, -
+    float4* nee;         // [2 pool] throughput at the light sample, its selection pdf | contribution, on
+    float4* mis;         // [2 pool] MIS ray: origin, BSDF pdf | direction, light
+    float4 *mis_fv, *ld_mis;
     uint64_t *ev_mis, *ev_main;
     int32_t* mis_hit;
     int32_t *q_a, *q_b, *q_shadow, *q_mis, *q_free;
+    int many_views;    // the batches have more than one slice (st.view is read)
     uint32_t* counts;  // written by compact: [0] next path rays, [2] shadow, [3] mis, [4] free;
                        // [8] trace fetch counter; [16 + c] paths of shade class c (classify)
     int32_t* q_cls;    // [kShadeClasses][pool] this iteration's paths grouped by shade class
@@ -78,6 +84,29 @@ struct WfState {
     uint16_t* tr_feat;      // [tr_cap][96] training features (count in counts[32])
     float* tr_target;       // [tr_cap][3] training targets
 };
+
+// A 32-byte group of the path state, moved by one 256-bit access.
+struct F4x2 {
+    float4 a, b;
+};
+__device__ __forceinline__ F4x2 ld_group(const float4* g, int p) {
+    F4x2 v;
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.a.w), "=f"(v.b.x), "=f"(v.b.y), "=f"(v.b.z), "=f"(v.b.w)
+                 : "l"(g + 2 * (size_t)p)
+                 : "memory");
+    return v;
+}
+// The same for a ray, which trace reads once: as two streaming loads, so that the state does not
+// push the tree out of L1 (stress scene: trace 104.4 ms per render, 106.6 with ld_group).
+__device__ __forceinline__ F4x2 ld_ray(const float4* g, int p) {
+    return F4x2{__ldcs(g + 2 * (size_t)p), __ldcs(g + 2 * (size_t)p + 1)};
+}
+__device__ __forceinline__ void st_group(float4* g, int p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(g + 2 * (size_t)p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
 
 // Bytes of WfState::counts; the control block follows in the same buffer.
 constexpr size_t kWfCountsBytes = 256;
@@ -187,19 +216,15 @@ __device__ __forceinline__ void generate_one(const WfState& st, int32_t* q_ext, 
     V3 rd, rxd, ryd;
     camera_ray(vw, pfx, pfy, rd, rxd, ryd);
     st.view[slot] = v;
-    st.pix[slot] = id;
-    st.smp[slot] = s;
     st.wid[slot] = (int32_t)(w - pc + (long)cj * cw + ci);  // the sample's place in row-major order
-    st.draw[slot] = rng.draw;
-    st.flags[slot] =
+    const uint32_t flags =
         (st.cache && wang_hash((uint32_t)id ^ ((uint32_t)s * 0x9E3779B9u) ^ (vw.seed * 0x85EBCA6Bu)) % 1000u < st.unb_permille)
             ? FL_UNBIASED : 0u;
     st.pend[slot] = 0u;
     st.pf[slot] = make_float2(pfx, pfy);
-    st.ro[slot] = make_float4(vw.cam[0], vw.cam[1], vw.cam[2], 0.f);
-    st.rd[slot] = make_float4(rd.x, rd.y, rd.z, 0.f);
-    st.beta[slot] = make_float4(1.f, 1.f, 1.f, 0.f);
-    st.L[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+    st_group(st.ray, slot, make_float4(vw.cam[0], vw.cam[1], vw.cam[2], __uint_as_float(flags)),
+             make_float4(rd.x, rd.y, rd.z, __uint_as_float(rng.draw)));
+    st_group(st.path, slot, make_float4(1.f, 1.f, 1.f, __int_as_float(id)), make_float4(0.f, 0.f, 0.f, __int_as_float(s)));
     st.sig[slot] = kSigBasis;
     q_ext[n_cont + t] = slot;
 }
@@ -217,24 +242,18 @@ enum : int { TR_EXTEND = 0, TR_SHADOW = 1, TR_MIS = 2 };
 // The ray of path slot p for each traversal kind.
 __device__ __forceinline__ bool wf_ray_begin(int kind, Trav& t, const SceneView& sv, const WfState& st, int p,
                                              int nleaf, Work& wk, const bool inst = false) {
-    if (kind == TR_EXTEND) {  // path ray, closest hit (BVH::intersect, BVH.cuh:365-398)
-        const float4 o = st.ro[p], d = st.rd[p];
-        return trav_begin(false, t, sv, nleaf, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), INFINITY, wk, inst);
-    } else if (kind == TR_SHADOW) {  // VisibilityTester::unoccluded (VisibilityTester.cu:9-12), any hit
-        const float4 o = st.sh_o[p], d = st.sh_d[p];
-        return trav_begin(true, t, sv, nleaf, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), d.w, wk, inst);
-    } else {  // MIS BSDF ray, closest hit
-        const float4 o = st.mis_o[p], d = st.mis_d[p];
-        return trav_begin(false, t, sv, nleaf, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), INFINITY, wk, inst);
-    }
+    // path ray, closest hit (BVH::intersect, BVH.cuh:365-398); shadow ray, any hit
+    // (VisibilityTester::unoccluded, VisibilityTester.cu:9-12); MIS BSDF ray, closest hit
+    const F4x2 r = ld_ray(kind == TR_EXTEND ? st.ray : (kind == TR_SHADOW ? st.sh : st.mis), p);
+    return trav_begin(kind == TR_SHADOW, t, sv, nleaf, v3(r.a.x, r.a.y, r.a.z), v3(r.b.x, r.b.y, r.b.z),
+                      kind == TR_SHADOW ? 1 - kShadowEps : INFINITY, wk, inst);
 }
 // Two-level BVH: the world ray of a ray in flight, re-read from the path state (the traversal
 // holds the current instance's object-space ray) to enter the next instance.
 __device__ __forceinline__ bool wf_ray_next_instance(int kind, Trav& t, const SceneView& sv, const WfState& st,
                                                      int p) {
-    const float4 o = kind == TR_EXTEND ? st.ro[p] : (kind == TR_SHADOW ? st.sh_o[p] : st.mis_o[p]);
-    const float4 d = kind == TR_EXTEND ? st.rd[p] : (kind == TR_SHADOW ? st.sh_d[p] : st.mis_d[p]);
-    return inst_next(kind == TR_SHADOW, t, sv, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z));
+    const F4x2 r = ld_ray(kind == TR_EXTEND ? st.ray : (kind == TR_SHADOW ? st.sh : st.mis), p);
+    return inst_next(kind == TR_SHADOW, t, sv, v3(r.a.x, r.a.y, r.a.z), v3(r.b.x, r.b.y, r.b.z));
 }
 
 // Results of a finished traversal.  MIS: radiance of the sampled light where the BSDF ray lands
@@ -242,15 +261,14 @@ __device__ __forceinline__ bool wf_ray_next_instance(int kind, Trav& t, const Sc
 __device__ __forceinline__ void wf_ray_end(int kind, const Trav& t, const SceneView& sv, WfState& st, int p) {
     if (kind == TR_EXTEND) {
         st.hprim[p] = t.best;  // with its shade class (hit_prim / hit_class)
-        st.huvi[p] = make_float4(t.bu, t.bv, t.binv, t.tmax);
+        st.hit[p] = make_float4(t.bu, t.bv, t.binv, __int_as_float(t.best));
     } else if (kind == TR_SHADOW) {
         st.vis[p] = t.best == 1 ? 0u : 1u;
     } else {
         // Landing on the sampled area light needs the surface at the hit (its normal faces the
         // ray?): that evaluation is left to finalize (ld_mis.w = 2, xyz = barycentrics and inv),
         // which has the registers for it; here only the light index of the hit is read.
-        const float4 x = st.mis_x[p];
-        const int off = __float_as_int(x.y);
+        const int off = __float_as_int(st.mis[2 * (size_t)p + 1].w);
         const DevLight& Lt = sv.lights[off];
         const int hp = hit_prim(t.best);
         const bool found = hp >= 0;
@@ -262,7 +280,7 @@ __device__ __forceinline__ void wf_ray_end(int kind, const Trav& t, const SceneV
             const Spec Li = Lt.kind == 1 ? Spec{Lt.L[0], Lt.L[1], Lt.L[2]} : spec(0.0f);
             Spec c = spec(0.0f);
             const bool add = !is_black(Li);
-            if (add) c = Spec{fv.x, fv.y, fv.z} * Li * spec(1.0f) * fv.w / x.x;
+            if (add) c = Spec{fv.x, fv.y, fv.z} * Li * spec(1.0f) * fv.w / st.mis[2 * (size_t)p].w;
             st.ld_mis[p] = make_float4(c.r, c.g, c.b, add ? 1.f : 0.f);
         }
         st.mis_hit[p] = found ? hp + 1 : 0;
@@ -443,47 +461,45 @@ struct WfScatter {
     WfState& st;
     int p;
     uint32_t pend;
+    V3 ro, rd;  // the next ray, stored with the path's flags and draw
     __device__ __forceinline__ void nee(Spec beta, float lpdf) {
         pend |= WF_NEE;
-        st.nee_beta[p] = make_float4(beta.r, beta.g, beta.b, lpdf);
+        st.nee[2 * (size_t)p] = make_float4(beta.r, beta.g, beta.b, lpdf);
     }
     __device__ __forceinline__ void shadow(V3 o, V3 d, Spec c, bool on) {
-        st.sh_o[p] = make_float4(o.x, o.y, o.z, 0.f);
-        st.sh_d[p] = make_float4(d.x, d.y, d.z, 1 - kShadowEps);
-        st.sh_c[p] = make_float4(c.r, c.g, c.b, on ? 1.f : 0.f);
+        st_group(st.sh, p, make_float4(o.x, o.y, o.z, 0.f), make_float4(d.x, d.y, d.z, 0.f));
+        st.nee[2 * (size_t)p + 1] = make_float4(c.r, c.g, c.b, on ? 1.f : 0.f);
         pend |= WF_VIS;
     }
     __device__ __forceinline__ void mis(V3 o, V3 d, Spec fv, float wgt, float spdf, int light) {
-        st.mis_o[p] = make_float4(o.x, o.y, o.z, 0.f);
-        st.mis_d[p] = make_float4(d.x, d.y, d.z, 0.f);
+        st_group(st.mis, p, make_float4(o.x, o.y, o.z, spdf), make_float4(d.x, d.y, d.z, __int_as_float(light)));
         st.mis_fv[p] = make_float4(fv.r, fv.g, fv.b, wgt);
-        st.mis_x[p] = make_float4(spdf, __int_as_float(light), 0.f, 0.f);
         pend |= WF_MIS;
     }
     __device__ __forceinline__ void ray(V3 o, V3 d) {
-        st.ro[p] = make_float4(o.x, o.y, o.z, 0.f);
-        st.rd[p] = make_float4(d.x, d.y, d.z, 0.f);
+        ro = o;
+        rd = d;
     }
 };
 // One path's bounce; LM / TEX: the lobes and textures its material can have (shade_variant).
 template <bool RECORD, int LM, bool TEX>
 __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParams& rp, WfState& st, int p) {
-    const uint32_t flags = st.flags[p];
+    const F4x2 g0 = ld_group(st.ray, p), g1 = ld_group(st.path, p);
+    const float4 h = st.hit[p];
+    const uint32_t flags = __float_as_uint(g0.a.w);
     const int bounce = (int)(flags >> 8);
     bool specular = (flags & 1u) != 0;
-    const float4 o4 = st.ro[p], d4 = st.rd[p];
-    const V3 ro = v3(o4.x, o4.y, o4.z), rd = v3(d4.x, d4.y, d4.z);
-    const float4 b4 = st.beta[p], l4 = st.L[p];
-    Spec beta{b4.x, b4.y, b4.z}, L{l4.x, l4.y, l4.z};
+    const V3 ro = v3(g0.a.x, g0.a.y, g0.a.z), rd = v3(g0.b.x, g0.b.y, g0.b.z);
+    Spec beta{g1.a.x, g1.a.y, g1.a.z}, L{g1.b.x, g1.b.y, g1.b.z};
+    const uint32_t pix = __float_as_uint(g1.a.w), smp = __float_as_uint(g1.b.w);
     uint64_t sig = RECORD ? st.sig[p] : 0ull;
     EvSink evs{&sig, 0};
-    const int prim = hit_prim(st.hprim[p]);
+    const int prim = hit_prim(__float_as_int(h.w));
     const bool hit = prim >= 0;
     uint32_t pend = 0;
     if (RECORD) fnv_mix(sig, 0x100000000ull + (uint64_t)(prim + 1));
     SI si;
     if (hit) {
-        const float4 h = st.huvi[p];
         make_si(sv, prim, rd, h.x, h.y, h.z, si, &ro);
     }
     if (bounce == 0 || specular) {
@@ -504,10 +520,10 @@ __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParam
         }
     }
     Rng rng;
-    const WfView& vw = st.views[st.view[p]];
-    rng.key = vw.seed + wang_hash((uint32_t)st.pix[p]);
-    rng.sample = (uint32_t)st.smp[p];
-    rng.draw = st.draw[p];
+    const WfView& vw = st.views[st.many_views ? st.view[p] : 0];
+    rng.key = vw.seed + wang_hash(pix);
+    rng.sample = smp;
+    rng.draw = __float_as_uint(g0.b.w);
     rng_resume(rng);
     bool done = !hit;
     Bsdf f;
@@ -544,7 +560,7 @@ __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParam
         } else if (!offered) {
             offered = true;
             atomicAdd(&st.counts[33], 1u);
-            const uint32_t coin = wang_hash((uint32_t)st.pix[p] * 0x9E3779B9u ^ (uint32_t)st.smp[p] * 0x85EBCA6Bu ^
+            const uint32_t coin = wang_hash(pix * 0x9E3779B9u ^ smp * 0x85EBCA6Bu ^
                                             vw.seed * 0xC2B2AE35u ^ 0x27D4EB2Fu);
             const uint32_t r = coin <= st.tr_accept ? atomicAdd(&st.counts[32], 1u) : 0xFFFFFFFFu;
             if (r < st.tr_cap) {
@@ -558,18 +574,21 @@ __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParam
     }
     if (!done && bsdf_roughness(f) > kCacheRough) rough_seen = true;
     uint64_t ev_mis = 0, ev_main = 0;
+    WfScatter out{st, p, pend, ro, rd};
     if (!done) {
-        WfScatter out{st, p, pend};
         done = shade_scatter<RECORD, LM>(sv, rp, si, f, bounce, beta, specular, rng, out, RECORD ? &evs : nullptr, ev_mis,
                                          ev_main);
         pend = out.pend;
     }
     st.pend[p] = pend | (done ? WF_DONE : 0u);
-    st.draw[p] = rng.draw;
-    st.flags[p] = ((uint32_t)(bounce + 1) << 8) | (specular ? FL_SPECULAR : 0u) | (rough_seen ? FL_ROUGH : 0u) |
-                  (flags & FL_UNBIASED) | (recorded ? FL_RECORDED : 0u) | (offered ? FL_OFFERED : 0u);
-    st.beta[p] = make_float4(beta.r, beta.g, beta.b, 0.f);
-    st.L[p] = make_float4(L.r, L.g, L.b, 0.f);
+    if (!done || st.cache) {  // a path that has ended is only finalized (with the cache: its flags are read)
+        const uint32_t f2 = ((uint32_t)(bounce + 1) << 8) | (specular ? FL_SPECULAR : 0u) | (rough_seen ? FL_ROUGH : 0u) |
+                            (flags & FL_UNBIASED) | (recorded ? FL_RECORDED : 0u) | (offered ? FL_OFFERED : 0u);
+        st_group(st.ray, p, make_float4(out.ro.x, out.ro.y, out.ro.z, __uint_as_float(f2)),
+                 make_float4(out.rd.x, out.rd.y, out.rd.z, __uint_as_float(rng.draw)));
+    }
+    st_group(st.path, p, make_float4(beta.r, beta.g, beta.b, __uint_as_float(pix)),
+             make_float4(L.r, L.g, L.b, __uint_as_float(smp)));
     if (RECORD) {
         st.sig[p] = sig;
         st.ev_mis[p] = ev_mis;
@@ -593,19 +612,20 @@ __global__ __launch_bounds__(kShadeBlock, 1) void k_wf_shade(const SceneView sv,
 
 
 // finalize: direct light of the bounce, deferred parity events; a finished path stores its
-// sample and frees its slot (pix = -1).
+// sample and frees its slot (WF_FREE).
 template <bool RECORD>
 __device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderParams& rp, const WfState& st, int p) {
     const uint32_t pend = st.pend[p];
-    float4 l4 = st.L[p];
+    const float4 l4 = st.path[2 * (size_t)p + 1];
     Spec L{l4.x, l4.y, l4.z};
     uint64_t sig = RECORD ? st.sig[p] : 0ull;
     if (pend & WF_NEE) {
+        const float4 nb = st.nee[2 * (size_t)p];
         Spec Ld = spec(0.0f);
         if (pend & WF_VIS) {
             const uint32_t vis = st.vis[p];
             if (RECORD) fnv_mix(sig, 0x300000000ull + vis);
-            const float4 c = st.sh_c[p];
+            const float4 c = st.nee[2 * (size_t)p + 1];
             if (vis && c.w != 0.f) Ld = Ld + Spec{c.x, c.y, c.z};
         }
         if (RECORD && st.ev_mis[p]) fnv_mix(sig, st.ev_mis[p]);
@@ -613,25 +633,25 @@ __device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderPa
             if (RECORD) fnv_mix(sig, 0x200000000ull + (uint64_t)st.mis_hit[p]);
             float4 c = st.ld_mis[p];
             if (c.w == 2.f) {  // the BSDF ray landed on the sampled area light (IntegratorHelper.cuh:225-243)
-                const float4 d = st.mis_d[p], fv = st.mis_fv[p], x = st.mis_x[p], mo = st.mis_o[p];
-                const V3 wi = v3(d.x, d.y, d.z);
-                const DevLight& Lt = sv.lights[__float_as_int(x.y)];
+                const float4 fv = st.mis_fv[p];
+                const F4x2 m = ld_group(st.mis, p);
+                const V3 wi = v3(m.b.x, m.b.y, m.b.z);
+                const DevLight& Lt = sv.lights[__float_as_int(m.b.w)];
                 SI lit;
-                const V3 mro = v3(mo.x, mo.y, mo.z);
+                const V3 mro = v3(m.a.x, m.a.y, m.a.z);
                 make_si(sv, st.mis_hit[p] - 1, wi, c.x, c.y, c.z, lit, &mro);
                 const Spec Li = dot(lit.n, -wi) > 0.f ? Spec{Lt.L[0], Lt.L[1], Lt.L[2]} : spec(0.0f);
                 Spec cs = spec(0.0f);
                 const bool add = !is_black(Li);
-                if (add) cs = Spec{fv.x, fv.y, fv.z} * Li * spec(1.0f) * fv.w / x.x;
+                if (add) cs = Spec{fv.x, fv.y, fv.z} * Li * spec(1.0f) * fv.w / m.a.w;
                 c = make_float4(cs.r, cs.g, cs.b, add ? 1.f : 0.f);
             }
             if (c.w != 0.f) Ld = Ld + Spec{c.x, c.y, c.z};
         }
-        const float4 nb = st.nee_beta[p];
         L = L + Spec{nb.x, nb.y, nb.z} * (Ld / nb.w);
     }
     if (pend & WF_CACHE) {  // the path ends in the cache: beta * cached radiance of the vertex
-        const float4 c = st.cache_L[p], b = st.beta[p];
+        const float4 c = st.cache_L[p], b = st.path[2 * (size_t)p];
         L = L + Spec{b.x, b.y, b.z} * Spec{c.x, c.y, c.z};
     }
     if (RECORD && st.ev_main[p]) fnv_mix(sig, st.ev_main[p]);
@@ -641,10 +661,10 @@ __device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderPa
         st.ev_main[p] = 0;
     }
     if (!(pend & WF_DONE)) {
-        st.L[p] = make_float4(L.r, L.g, L.b, 0.f);
+        st.path[2 * (size_t)p + 1] = make_float4(L.r, L.g, L.b, l4.w);
         return;
     }
-    if (st.cache && (st.flags[p] & FL_RECORDED)) {  // training target: radiance after the vertex / beta there
+    if (st.cache && (__float_as_uint(st.ray[2 * (size_t)p].w) & FL_RECORDED)) {  // training target: radiance after the vertex / beta there
         const int r = st.tr_idx[p];
         const float4 tb = st.tr_beta[p], l0 = st.tr_L0[p];
         float* tg = st.tr_target + 3 * (size_t)r;
@@ -656,8 +676,8 @@ __device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderPa
     // floor(pf + 1)] per axis.  With pf in [i, i + 1] that is i .. i + 2, gathered later, plus
     // the column i - 1 (row j - 1) when pf rounds to exactly i (j), added here.
     const float2 pf = st.pf[p];
-    const int id = st.pix[p];
-    const WfView& vw = st.views[st.view[p]];
+    const int id = __float_as_int(st.path[2 * (size_t)p].w);
+    const WfView& vw = st.views[st.many_views ? st.view[p] : 0];
     const int W = vw.W, H = vw.H;
     const int i = id % W, j = id / W;
     double* const film = rp.film + 4 * (size_t)vw.film_off;
@@ -683,13 +703,13 @@ __device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderPa
     st.fs_L[w] = make_float4(L.r, L.g, L.b, pf.x);
     st.fs_y[w] = pf.y;
     if (RECORD) {
-        const size_t k = ((size_t)(j - vw.y0) * (vw.x1 - vw.x0) + (i - vw.x0)) * vw.spp + st.smp[p];
+        const size_t k = ((size_t)(j - vw.y0) * (vw.x1 - vw.x0) + (i - vw.x0)) * vw.spp + __float_as_int(l4.w);
         rp.sample_L[3 * k + 0] = L.r;
         rp.sample_L[3 * k + 1] = L.g;
         rp.sample_L[3 * k + 2] = L.b;
         rp.sample_sig[k] = sig;
     }
-    st.pix[p] = -1;
+    st.pend[p] = WF_FREE;
 }
 template <bool RECORD>
 __global__ __launch_bounds__(kWfBlock) void k_wf_finalize(const SceneView sv, const RenderParams rp, WfState st,
@@ -699,13 +719,13 @@ __global__ __launch_bounds__(kWfBlock) void k_wf_finalize(const SceneView sv, co
         finalize_one<RECORD>(sv, rp, st, q[t]);
 }
 
-// Every slot starts free (pix = -1, in the free list in slot order); the counts read as after a
+// Every slot starts free (WF_FREE, in the free list in slot order); the counts read as after a
 // compaction of an empty pool (counts zeroed by the host first).
-__global__ void k_wf_init_free(int32_t* q_free, int32_t* pix, uint32_t* counts, int n) {
+__global__ void k_wf_init_free(int32_t* q_free, uint32_t* pend, uint32_t* counts, int n) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) {
         q_free[t] = t;
-        pix[t] = -1;
+        pend[t] = WF_FREE;
     }
     if (t == 0) counts[4] = (uint32_t)n;
 }
@@ -743,9 +763,9 @@ __global__ void k_wf_control(WfState st, WfCtl* ctl) {
     if (threadIdx.x < 32 && (s_active || threadIdx.x >= 8)) st.counts[threadIdx.x] = 0u;
 }
 
-// compact: one pass over the pool after shade.  Every live slot (pix >= 0) was shaded in this
-// iteration, so its pend flags say which lists it joins: path rays (not finished), shadow rays
-// (WF_VIS), MIS rays (WF_MIS); a slot with pix < 0 is free.  Each block scans its tile of
+// compact: one pass over the pool after shade.  Every live slot was shaded in this iteration, so
+// its pend flags say which lists it joins: path rays (not finished), shadow rays (WF_VIS), MIS
+// rays (WF_MIS), or the free slots (WF_FREE).  Each block scans its tile of
 // kCompactTile slots and reserves its runs with one atomic per list, so every list is in slot
 // order within a tile.
 constexpr int kCompactThreads = 256, kCompactItems = 4, kCompactTile = kCompactThreads * kCompactItems;
@@ -761,12 +781,9 @@ __device__ __forceinline__ void compact_tile(const WfState& st, int32_t* __restr
         const int slot = first + k;
         uint32_t f = 0;
         if (slot < P) {
-            if (st.pix[slot] >= 0) {
-                const uint32_t pend = st.pend[slot];
-                f = ((pend & WF_DONE) ? 0u : 1u) | ((pend & WF_VIS) ? 2u : 0u) | ((pend & WF_MIS) ? 4u : 0u);
-            } else {
-                f = 8u;
-            }
+            const uint32_t pend = st.pend[slot];
+            f = (pend & WF_FREE) ? 8u
+                                 : ((pend & WF_DONE) ? 0u : 1u) | ((pend & WF_VIS) ? 2u : 0u) | ((pend & WF_MIS) ? 4u : 0u);
         }
         flags[k] = f;
 #pragma unroll
