@@ -146,8 +146,7 @@ __global__ __launch_bounds__(kBlock) void k_scene_bounds(const float* __restrict
         uint32_t v = s_red[0][threadIdx.x];
         for (int w = 1; w < kBlock / 32; ++w)
             v = threadIdx.x < 3 ? min(v, s_red[w][threadIdx.x]) : max(v, s_red[w][threadIdx.x]);
-        if (threadIdx.x < 3) atomicMin(gb + threadIdx.x, v);
-        else atomicMax(gb + threadIdx.x, v);
+        atomicMax(gb + threadIdx.x, threadIdx.x < 3 ? ~v : v);  // gb starts zeroed: minima as their complements
     }
 }
 
@@ -162,6 +161,19 @@ __device__ __forceinline__ uint32_t left_shift3(uint32_t x) {
     return x;
 }
 
+__device__ __forceinline__ uint32_t morton_code(const float mn[3], const float mx[3], const float gmn[3], const float gmx[3]) {
+    uint32_t q[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float c = mn[k] * 0.5f + mx[k] * 0.5f;        // BVH.cuh:95
+        float o = c - gmn[k];                                // Bound.cuh:169-175
+        if (gmx[k] > gmn[k]) o = __fdiv_rn(o, gmx[k] - gmn[k]);
+        const float s = __fmul_rn((float)(1 << 10), o);     // * mortonScale (BVH.cuh:136)
+        q[k] = (uint32_t)s;                                  // float -> uint32_t truncation
+    }
+    return left_shift3(q[0]) | (left_shift3(q[1]) << 1) | (left_shift3(q[2]) << 2);
+}
+
 __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ tri, int n, const uint32_t* __restrict__ gb,
                                                    int code_limit, uint32_t* __restrict__ codes,
                                                    int32_t* __restrict__ ids, uint32_t* __restrict__ hist) {
@@ -171,7 +183,7 @@ __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ tri
     float gmn[3], gmx[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        gmn[k] = key_float(gb[k]);
+        gmn[k] = key_float(~gb[k]);
         gmx[k] = key_float(gb[3 + k]);
     }
     for (long first = (long)blockIdx.x * kBlock; first < n; first += (long)gridDim.x * kBlock) {
@@ -186,16 +198,7 @@ __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ tri
             if (code_limit < 0 || i < code_limit) {
                 float mn[3], mx[3];
                 tri_bounds(s_tri + 9 * threadIdx.x, mn, mx);
-                uint32_t q[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float c = mn[k] * 0.5f + mx[k] * 0.5f;        // BVH.cuh:95
-                    float o = c - gmn[k];                                // Bound.cuh:169-175
-                    if (gmx[k] > gmn[k]) o = __fdiv_rn(o, gmx[k] - gmn[k]);
-                    const float s = __fmul_rn((float)(1 << 10), o);     // * mortonScale (BVH.cuh:136)
-                    q[k] = (uint32_t)s;                                  // float -> uint32_t truncation
-                }
-                code = left_shift3(q[0]) | (left_shift3(q[1]) << 1) | (left_shift3(q[2]) << 2);
+                code = morton_code(mn, mx, gmn, gmx);
                 id = (int32_t)i;
             }
             codes[i] = code;
@@ -226,19 +229,9 @@ __device__ __forceinline__ uint32_t block_excl_scan256(uint32_t v, uint32_t* s_w
     return wsum + x - v;
 }
 
-__global__ void k_digit_prefix(const uint32_t* __restrict__ hist, uint32_t* __restrict__ prefix) {
-    __shared__ uint32_t s_warp[8];
-    const uint32_t v = hist[blockIdx.x * 256 + threadIdx.x];
-    prefix[blockIdx.x * 256 + threadIdx.x] = block_excl_scan256(v, s_warp);
-}
-
 #ifndef LTS_SORT_MIN_BLOCKS
 #define LTS_SORT_MIN_BLOCKS 4  // resident sort tiles per SM the register budget is cut for
 #endif
-#ifndef LTS_SORT_LOOKBACK
-#define LTS_SORT_LOOKBACK 4  // predecessor tiles read per look-back round trip
-#endif
-constexpr int kLookback = LTS_SORT_LOOKBACK;
 #ifndef LTS_SORT_BALLOT_MATCH
 #define LTS_SORT_BALLOT_MATCH 1  // 0: __match_any_sync
 #endif
@@ -260,14 +253,23 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool valid) {
 #endif
 }
 
-// vin null: every value is its key's position (the identity ids of the first pass).
+__global__ void k_digit_prefix(const uint32_t* __restrict__ hist, uint32_t* __restrict__ prefix) {
+    __shared__ uint32_t s_warp[8];
+    const uint32_t v = hist[blockIdx.x * 256 + threadIdx.x];
+    prefix[blockIdx.x * 256 + threadIdx.x] = block_excl_scan256(v, s_warp);
+}
+
+// vin null: every value is its key's position (the identity ids of the first pass).  ITEMS keys per
+// thread; LOOKBACK predecessor tiles read per look-back round trip.
+template <int ITEMS, int LOOKBACK, bool SCAN>
 __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                                                            uint32_t* __restrict__ kout, int32_t* __restrict__ vout,
-                                                           int n, int shift, const uint32_t* __restrict__ gprefix,
+                                                           int n, int shift, const uint32_t* __restrict__ prefix,
                                                            uint32_t* __restrict__ status, uint32_t* __restrict__ tile_counter,
                                                            uint32_t* __restrict__ err) {
-    __shared__ uint32_t s_keys[kSortTile];
-    __shared__ int32_t s_vals[kSortTile];
+    constexpr int kTile = kSortThreads * ITEMS;
+    __shared__ uint32_t s_keys[kTile];
+    __shared__ int32_t s_vals[kTile];
     __shared__ uint32_t s_whist[kSortThreads / 32][256];
     __shared__ uint32_t s_tile_start[256];
     __shared__ uint32_t s_dst[256];
@@ -279,14 +281,14 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
     for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += kSortThreads) (&s_whist[0][0])[i] = 0;
     __syncthreads();
     const int tile = s_tile;
-    const long base = (long)tile * kSortTile;
-    const long wbase = base + (long)warp * 32 * kSortItems;
+    const long base = (long)tile * kTile;
+    const long wbase = base + (long)warp * 32 * ITEMS;
 
-    uint32_t key[kSortItems];
-    int32_t val[kSortItems];
-    uint32_t rank[kSortItems];
+    uint32_t key[ITEMS];
+    int32_t val[ITEMS];
+    uint32_t rank[ITEMS];
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const long idx = wbase + i * 32 + lane;
         if (idx < n) {
             key[i] = __ldg(kin + idx);
@@ -296,9 +298,12 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
             val[i] = 0;
         }
     }
+    // the digits' first output positions: an exclusive scan of the pass' histogram, by every tile
+    // (SCAN) or made before the passes
+    const uint32_t gprefix = SCAN ? block_excl_scan256(__ldg(prefix + threadIdx.x), s_warp) : __ldg(prefix + threadIdx.x);
     const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const long idx = wbase + i * 32 + lane;
         const bool valid = idx < n;
         const uint32_t d = (key[i] >> shift) & 255u;
@@ -327,20 +332,20 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
     s_tile_start[dig] = start;
     uint32_t excl = 0;
     if (tile > 0) {
-        // look back kLookback predecessors per round trip (each status word carries its flag and
+        // look back LOOKBACK predecessors per round trip (each status word carries its flag and
         // count together), consumed newest first until an inclusive prefix; a predecessor that
         // has published nothing yet is re-read (bounded wait)
         int k = tile - 1, spins = 0;
         while (k >= 0) {
-            uint32_t v[kLookback];
+            uint32_t v[LOOKBACK];
 #pragma unroll
-            for (int j = 0; j < kLookback; ++j)
+            for (int j = 0; j < LOOKBACK; ++j)
                 v[j] = k - j >= 0 ? ld_relaxed(status + (size_t)(k - j) * 256 + dig) : kFlagPrefix;
-            int used = kLookback;
+            int used = LOOKBACK;
             bool done = false;
 #pragma unroll
-            for (int j = 0; j < kLookback; ++j) {
-                if (done || used < kLookback) continue;
+            for (int j = 0; j < LOOKBACK; ++j) {
+                if (done || used < LOOKBACK) continue;
                 const uint32_t f = v[j] & ~kCountMask;
                 if (f == 0) {
                     used = j;
@@ -351,14 +356,14 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
             }
             if (done) break;
             k -= used;
-            if (used < kLookback && !spin_or_give_up(spins, err)) break;
+            if (used < LOOKBACK && !spin_or_give_up(spins, err)) break;
         }
         st_relaxed(st + dig, kFlagPrefix | (excl + tot));
     }
-    s_dst[dig] = gprefix[dig] + excl;
+    s_dst[dig] = gprefix + excl;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const long idx = wbase + i * 32 + lane;
         if (idx < n) {
             const uint32_t d = (key[i] >> shift) & 255u;
@@ -368,13 +373,94 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
         }
     }
     __syncthreads();
-    const int tile_n = (int)min((long)kSortTile, n - base);
+    const int tile_n = (int)min((long)kTile, n - base);
     for (int j = threadIdx.x; j < tile_n; j += kSortThreads) {
         const uint32_t k = s_keys[j];
         const uint32_t d = (k >> shift) & 255u;
         const uint32_t dst = s_dst[d] + (uint32_t)j - s_tile_start[d];
         kout[dst] = k;
         vout[dst] = s_vals[j];
+    }
+}
+
+// ------------------------------------------------------------------ 1-3 in one block
+// Scene bounds, Morton codes and the stable sort of up to kSmallSort primitives by one block: a
+// bitonic sort of (code, position) words in shared memory.  For so few primitives the six
+// launches, six clears and the sort tiles' latencies were all there is to the time (a build of 1,280
+// triangles, launch to finish: 107 us, 4 x 8 us of it in sort passes over one tile; 38 now).
+constexpr int kSmallThreads = 1024, kSmallSort = 4096;
+__global__ __launch_bounds__(kSmallThreads) void k_small_sort(const float* __restrict__ tri, int n, int code_limit,
+                                                              uint32_t* __restrict__ codes, int32_t* __restrict__ ids,
+                                                              uint32_t* __restrict__ group_done, int ngroups) {
+    __shared__ uint64_t s_key[kSmallSort];
+    __shared__ uint32_t s_red[kSmallThreads / 32][6];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < ngroups; i += kSmallThreads) group_done[i] = 0u;  // the tree's counters
+    uint32_t key[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // complements of the minima, maxima
+    for (int i = tid; i < n; i += kSmallThreads) {
+        float t[9], mn[3], mx[3];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) t[k] = __ldg(tri + 9L * i + k);
+        tri_bounds(t, mn, mx);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            key[k] = max(key[k], ~float_key(mn[k]));
+            key[3 + k] = max(key[3 + k], float_key(mx[k]));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        key[k] = __reduce_max_sync(~0u, key[k]);
+        if (lane == 0) s_red[warp][k] = key[k];
+    }
+    __syncthreads();
+    float gmn[3], gmx[3];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const uint32_t v = __reduce_max_sync(~0u, s_red[lane][k]);
+        if (k < 3) gmn[k] = key_float(~v);
+        else gmx[k - 3] = key_float(v);
+    }
+    int p2 = 64;
+    while (p2 < n) p2 <<= 1;
+    for (int i = tid; i < p2; i += kSmallThreads) {
+        uint64_t w = ~0ull;
+        if (i < n) {
+            uint32_t code = 0;
+            if (code_limit < 0 || i < code_limit) {
+                float t[9], mn[3], mx[3];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) t[k] = __ldg(tri + 9L * i + k);
+                tri_bounds(t, mn, mx);
+                code = morton_code(mn, mx, gmn, gmx);
+            }
+            w = ((uint64_t)code << 32) | (uint32_t)i;
+        }
+        s_key[i] = w;
+    }
+    __syncthreads();
+    // pair p of a stage of stride j joins elements e and e + j, e = 2 j (p / j) + p % j; strides up to
+    // 32 stay within the 64 elements of a warp's pairs, so those stages need no block barrier
+    for (int k = 2; k <= p2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int p = tid; p < p2 / 2; p += kSmallThreads) {
+                const int e = 2 * (p & ~(j - 1)) + (p & (j - 1));
+                const uint64_t a = s_key[e], b = s_key[e + j];
+                if ((a > b) == ((e & k) == 0)) {
+                    s_key[e] = b;
+                    s_key[e + j] = a;
+                }
+            }
+            const bool next_in_warp = j > 1 ? (j >> 1) <= 32 : k <= 32;  // the next stage's stride (k itself after j = 1)
+            if (j <= 32 && next_in_warp) __syncwarp();
+            else __syncthreads();
+        }
+    __syncthreads();
+    for (int i = tid; i < n; i += kSmallThreads) {
+        const uint64_t w = s_key[i];
+        const int pos = (int)(uint32_t)w;
+        codes[i] = (uint32_t)(w >> 32);
+        ids[i] = code_limit < 0 || pos < code_limit ? pos : 0;
     }
 }
 
@@ -411,26 +497,36 @@ __device__ __forceinline__ int delta(const uint32_t* __restrict__ c, int n, int 
 //  * a block of kTreeBlock threads owns kTreeBlock consecutive leaves; when g and g+1 both lie in
 //    the block the children meet in a shared-memory slot of g (box, child reference, far range
 //    end; a block-scope fence and a shared arrival bitmask), without barriers;
-//  * otherwise they meet in device memory, in a second kernel (k_tree_top), so that no block of
-//    k_tree waits on another: k_tree lists such a child (its reference; its record is written),
-//    and also a child left alone in a shared slot after the block's climbs (its sibling reaches
-//    into another block).  k_tree_top climbs from every listed child: both children of a parent
-//    swap the build's epoch into the arrival word of g with acq_rel order, and the second reads
-//    its sibling back -- the sibling's node record, or its triangle for a leaf.  Only the
-//    ~log2(n / kTreeBlock) ancestors of each block edge meet there.
-constexpr int kTreeBlock = 512;
-#ifndef LTS_TREE_MIN_BLOCKS
-#define LTS_TREE_MIN_BLOCKS 4  // resident blocks per SM the register budget is cut for
-#endif
+//  * what is left of the block is its forest, the subtrees whose parents reach into another block:
+//    at most kForestCap - 1 of them (each side's deltas rise strictly outwards, and a delta takes
+//    54 values: 2..31 for distinct codes, 40 + 8..31 for equal ones), consecutive and covering the
+//    block.  The block writes them, in order, to device memory; the last block of a group of
+//    kTreeGroup to finish takes the group's forests as its items (subtrees instead of leaves) and
+//    climbs again, the last group of a group of groups likewise, up to the root.  No block waits:
+//    the others of a group just end.  (The ancestors of the block edges used to meet in a second
+//    kernel through arrival words in device memory, one dependent chain of exchanges per edge:
+//    24 us for 1,280 triangles, 47 for 200,000, 94 for 16M.)
+// Leaves (threads) per block: 512, or 256 above kTreeLarge leaves, where shorter longest climbs beat
+// the levels of merging they add (16M, sorted: 0.96 ms against 1.04; 1M: 0.097 against 0.094).
+constexpr int kTreeLarge = 4000000;
+__host__ __device__ constexpr int tree_block(long n) { return n > kTreeLarge ? 256 : 512; }
+constexpr int kTreeGroup = 24;  // forests merged by one block: 24 x ~18 subtrees fill its threads
+constexpr int kForestCap = 128;  // entries of 32 bytes per block: up to 127 subtrees, the last word their count
 
-__device__ __forceinline__ void put_node(BvhNode* __restrict__ nodes, int idx, const float* cb, int lref, int rref, int lo,
-                                         int hi) {
-    float4* P = reinterpret_cast<float4*>(nodes + idx);
-    P[0] = make_float4(cb[0], cb[1], cb[2], cb[3]);
-    P[1] = make_float4(cb[4], cb[5], cb[6], cb[7]);
-    P[2] = make_float4(cb[8], cb[9], cb[10], cb[11]);
-    reinterpret_cast<int4*>(P)[3] = make_int4(lref, rref, lo, hi);
+// One subtree of a forest: box, reference, last leaf (it begins after its predecessor's).
+struct alignas(16) ForestEntry {
+    float4 a;  // min.xyz, max.x
+    float4 b;  // max.yz, reference bits, last leaf bits
+};
+__host__ __device__ constexpr long tree_blocks(long n) { return (n + tree_block(n) - 1) / tree_block(n); }
+constexpr size_t forest_bytes(long n) { return (size_t)tree_blocks(n) * kForestCap * sizeof(ForestEntry); }
+// Completion counters: one per group of every level.
+constexpr long tree_counters(long n) {
+    long c = 0;
+    for (long m = tree_blocks(n); m > 1; m = (m + kTreeGroup - 1) / kTreeGroup) c += (m + kTreeGroup - 1) / kTreeGroup;
+    return c;
 }
+
 __device__ __forceinline__ void put_root(float* __restrict__ root_bounds, const float* mn, const float* mx) {
     for (int k = 0; k < 3; ++k) {
         root_bounds[k] = mn[k];
@@ -438,231 +534,310 @@ __device__ __forceinline__ void put_root(float* __restrict__ root_bounds, const 
     }
 }
 
-// Children (own box / ref, sibling box / ref) of the parent in left-right order, and the union.
-__device__ __forceinline__ void pair_up(bool left, float* mn, float* mx, const float* smn, const float* smx, float* cb) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        cb[k] = left ? mn[k] : smn[k];
-        cb[3 + k] = left ? mx[k] : smx[k];
-        cb[6 + k] = left ? smn[k] : mn[k];
-        cb[9 + k] = left ? smx[k] : mx[k];
-        mn[k] = fminf(cb[k], cb[6 + k]);  // bUnion(left, right)
-        mx[k] = fmaxf(cb[3 + k], cb[9 + k]);
-    }
-}
+// Slot k of the boundary between items k and k + 1 holds what the record of the node split there
+// needs: both child boxes, both child references, the far items of the node's range and, once
+// both children arrived, the node's index.  The climbs touch only shared memory (so the
+// block-scope fences wait on nothing in flight to device memory); the records go out after the
+// block's barrier, one 64-byte line per thread.
+//   slot[k][2 side + 0] = (min.x, min.y, min.z, max.x)      side 0: left child, 1: right
+//   slot[k][2 side + 1] = (max.y, max.z, reference, far item)
+//   slot[k][4]          = (node index, arrival bits: 1 left, 2 right, -, -)
+// Five 16-byte words per slot put eight consecutive slots in distinct bank groups.
+template <int kTreeBlock>
+struct TreeShared {
+    float4 slot[kTreeBlock][5];
+    int delta[kTreeBlock + 1];    // delta across the boundary before item k (-1 outside the array)
+    int pos[kTreeBlock + 1];      // first leaf of item k (item count: one past the last leaf)
+    int root[kTreeBlock];         // forest: 0, or where the subtree beginning at item k is: slot * 2 + side + 1,
+                                  // or -1 / -2: edge[0] / edge[1]
+    float4 edge[2][2];            // the subtrees whose parent lies beyond the first / last boundary
+    int warp[kTreeBlock / 32];
+    int list[kTreeGroup + 1];     // a group's forests: entries before forest j
+    int last;
+};
 
-// Arrival word of a split: the build's epoch (kEpochBits) above a leaf flag and the far range end
-// of the child that arrived (its first leaf for a left child, its last for a right child), so
-// that the second arrival learns its sibling's shape from the exchange itself.
-constexpr int kEpochBits = 7;
-constexpr uint32_t kEpochMax = (1u << kEpochBits) - 1u;
-constexpr uint32_t kArrivalLeaf = 1u << 24, kArrivalEnd = kArrivalLeaf - 1u;
-static_assert(32 - kEpochBits == 25, "epoch above the leaf flag and a 24-bit position");
-
-// The climb through device memory from node [L, R] (reference ref, box mn/mx, its record already
-// written), the `left` child of the parent split at g.
-__device__ void climb_global(const float* __restrict__ tri, int n, int mode, const int32_t* __restrict__ ids,
-                             const uint32_t* __restrict__ codes, BvhNode* __restrict__ nodes,
-                             uint32_t* __restrict__ arrivals, uint32_t epoch, float* __restrict__ root_bounds, int L,
-                             int R, int ref, int g, bool left, float* mn, float* mx) {
-    for (;;) {
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> arrival(arrivals[g]);
-        const uint32_t mine = (epoch << 25) | (L == R ? kArrivalLeaf : 0u) | (uint32_t)(left ? L : R);
-        const uint32_t other = arrival.exchange(mine, cuda::memory_order_acq_rel);
-        if ((other >> 25) != epoch) return;  // first arrival stops
-        const int sp = left ? g + 1 : g;     // the sibling's position next to the split
-        const int send = (int)(other & kArrivalEnd);
-        if (left) R = send;
-        else L = send;
-        const bool root = (L == 0 && R == n - 1);
-        // the parent's side, read alongside the sibling's box
-        const bool pleft = !root && delta(codes, n, R, R + 1) > delta(codes, n, L, L - 1);
-        float smn[3], smx[3];
-        int sref;
-        if (other & kArrivalLeaf) {
-            const int prim = (mode == BVH_MODE_REFERENCE) ? sp : __ldg(ids + sp);
-            float t[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) t[k] = __ldg(tri + 9L * prim + k);
-            tri_bounds(t, smn, smx);
-            sref = ~sp;
-        } else {
-            const float4 a = __ldcg(&nodes[sp].a), b = __ldcg(&nodes[sp].b), c = __ldcg(&nodes[sp].c);
-            smn[0] = fminf(a.x, b.z); smn[1] = fminf(a.y, b.w); smn[2] = fminf(a.z, c.x);
-            smx[0] = fmaxf(a.w, c.y); smx[1] = fmaxf(b.x, c.z); smx[2] = fmaxf(b.y, c.w);
-            sref = sp;
-        }
-        float cb[12];
-        pair_up(left, mn, mx, smn, smx, cb);
-        const int lref = left ? ref : sref, rref = left ? sref : ref;
-        if (root) {
-            put_node(nodes, 0, cb, lref, rref, L, R);
-            put_root(root_bounds, mn, mx);
-            return;
-        }
-        left = pleft;
-        ref = left ? R : L;
-        put_node(nodes, ref, cb, lref, rref, L, R);
-        g = left ? R : L - 1;
-    }
-}
-
-__global__ __launch_bounds__(kTreeBlock, LTS_TREE_MIN_BLOCKS) void k_tree(const float* __restrict__ tri, int n, int mode,
-                                                     const int32_t* __restrict__ ids, const uint32_t* __restrict__ codes,
-                                                     BvhNode* __restrict__ nodes, int32_t* __restrict__ pending,
-                                                     uint32_t* __restrict__ pending_count, int32_t* __restrict__ leaf_prim,
-                                                     float* __restrict__ root_bounds) {
-    // Slot g - b0 of a split g inside the block holds what its parent's record needs: both child
-    // boxes, both child references, the parent's range [far end of the left child, far end of the
-    // right child] and, once both children arrived, the parent's node index.  The climbs touch
-    // only shared memory (so the block-scope fences wait on nothing in flight to device memory);
-    // the records go out after the block's barrier, one 64-byte line per thread.
-    //   s_slot[slot][2 side + 0] = (min.x, min.y, min.z, max.x)      side 0: left child, 1: right
-    //   s_slot[slot][2 side + 1] = (max.y, max.z, reference, far end)
-    //   s_slot[slot][4]          = (parent index, arrival bits: 1 left, 2 right, -, -)
-    // Five 16-byte words per slot put eight consecutive slots in distinct bank groups.
-    // Children that meet across blocks are listed in shared memory first and appended to the
-    // device list with one atomic per block (a same-address atomic per child serialises): the
-    // climbs list at most two (the one node ending at the block's last leaf whose parent lies
-    // beyond, and the one starting at its first), the lone slots at most one each.
-    __shared__ uint32_t s_code[kTreeBlock + 2];      // codes of positions b0-1 .. b0+kTreeBlock
-    __shared__ float4 s_slot[kTreeBlock][5];
-    constexpr uint32_t kPendCap = kTreeBlock + 2;
-    __shared__ int32_t s_pend[kPendCap];
-    __shared__ uint32_t s_npend, s_pbase;
-    auto push = [&](int32_t r) {  // past the bound above (never, by the count) straight to the device list
-        const uint32_t i = atomicAdd(&s_npend, 1u);
-        if (i < kPendCap) s_pend[i] = r;
-        else pending[atomicAdd(pending_count, 1u)] = r;
-    };
-    const int b0 = blockIdx.x * kTreeBlock, b1 = min(b0 + kTreeBlock, n) - 1;
-    for (int k = threadIdx.x; k < kTreeBlock + 2; k += kTreeBlock) {
-        const int pos = b0 - 1 + k;
-        s_code[k] = (pos >= 0 && pos < n) ? __ldg(codes + pos) : 0u;
-    }
-    s_slot[threadIdx.x][4] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (threadIdx.x == 0) s_npend = 0u;
+// The climb over the block's `cnt` items (thread i < cnt holds item i: reference, box), the node
+// records, and the forest into `out` (entries in order, then their count).  Returns the count;
+// the whole tree (no forest) gives 0.  Every thread of the block calls it.
+template <int kTreeBlock>
+__device__ int tree_climb(TreeShared<kTreeBlock>& sh, int cnt, int n, int ref, float* mn, float* mx, BvhNode* __restrict__ nodes,
+                          float* __restrict__ root_bounds, ForestEntry* __restrict__ out) {
+    const int i = threadIdx.x;
+    auto have_of = [&](int slot) -> uint32_t* { return reinterpret_cast<uint32_t*>(&sh.slot[slot][4]) + 1; };
+    sh.slot[i][4] = make_float4(0.f, 0.f, 0.f, 0.f);
+    sh.root[i] = 0;
     __syncthreads();
-    auto sdelta = [&](int a, int b) -> int {  // delta of positions within [b0-1, b1+1]
-        if (b < 0 || b >= n) return -1;
-        return delta_codes(s_code[a - b0 + 1], s_code[b - b0 + 1], a, b);
-    };
-    auto have_of = [&](int slot) -> uint32_t* { return reinterpret_cast<uint32_t*>(&s_slot[slot][4]) + 1; };
-
-    const int l = b0 + threadIdx.x;
-    int prim = 0;
-    if (l <= b1) {
-        prim = (mode == BVH_MODE_REFERENCE) ? l : __ldg(ids + l);
-        float mn[3], mx[3];
-        gather_tri_bounds(tri, n, (reinterpret_cast<uintptr_t>(tri) & 15u) == 0, prim, mn, mx);
-        if (n == 1) {
-            put_root(root_bounds, mn, mx);
-        } else {
-            int L = l, R = l, ref = ~l;
-            bool left = sdelta(l, l + 1) > sdelta(l, l - 1);
-            int g = left ? l : l - 1;
-            // block-local climb
-            for (;;) {
-                if (g < b0 || g + 1 > b1) {  // the parent reaches into another block
-                    push(ref);
-                    break;
-                }
-                const int side = left ? 0 : 1, slot = g - b0;
-                s_slot[slot][2 * side] = make_float4(mn[0], mn[1], mn[2], mx[0]);
-                s_slot[slot][2 * side + 1] = make_float4(mx[1], mx[2], __int_as_float(ref), __int_as_float(left ? L : R));
-                __threadfence_block();
-                if (!(atomicOr(have_of(slot), 1u << side) & (2u >> side))) break;  // first arrival stops
-                __threadfence_block();
-                const float4 e0 = s_slot[slot][2 * (side ^ 1)], e1 = s_slot[slot][2 * (side ^ 1) + 1];
-                const float smn[3] = {e0.x, e0.y, e0.z}, smx[3] = {e0.w, e1.x, e1.y};
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {  // bUnion(left, right), operands in that order
-                    mn[k] = left ? fminf(mn[k], smn[k]) : fminf(smn[k], mn[k]);
-                    mx[k] = left ? fmaxf(mx[k], smx[k]) : fmaxf(smx[k], mx[k]);
-                }
-                if (left) R = __float_as_int(e1.w);
-                else L = __float_as_int(e1.w);
-                int* idx = reinterpret_cast<int*>(&s_slot[slot][4]);
-                if (L == 0 && R == n - 1) {
-                    *idx = 0;
-                    put_root(root_bounds, mn, mx);
-                    break;
-                }
-                left = sdelta(R, R + 1) > sdelta(L, L - 1);
-                ref = left ? R : L;
-                *idx = ref;
-                g = left ? R : L - 1;
+    if (i < cnt) {
+        int li = i, ri = i;
+        for (;;) {
+            const bool left = sh.delta[ri + 1] > sh.delta[li];
+            const int bound = left ? ri + 1 : li;  // the boundary its parent is split at
+            if (bound == 0 || bound == cnt) {      // the parent reaches out of the block
+                const int e = bound == 0 ? 0 : 1;
+                sh.edge[e][0] = make_float4(mn[0], mn[1], mn[2], mx[0]);
+                sh.edge[e][1] = make_float4(mx[1], mx[2], __int_as_float(ref), __int_as_float(sh.pos[ri + 1] - 1));
+                sh.root[li] = -1 - e;
+                break;
             }
+            const int side = left ? 0 : 1, slot = bound - 1;
+            sh.slot[slot][2 * side] = make_float4(mn[0], mn[1], mn[2], mx[0]);
+            sh.slot[slot][2 * side + 1] = make_float4(mx[1], mx[2], __int_as_float(ref), __int_as_float(left ? li : ri));
+            __threadfence_block();
+            if (!(atomicOr(have_of(slot), 1u << side) & (2u >> side))) break;  // first arrival stops
+            __threadfence_block();
+            const float4 e0 = sh.slot[slot][2 * (side ^ 1)], e1 = sh.slot[slot][2 * (side ^ 1) + 1];
+            const float smn[3] = {e0.x, e0.y, e0.z}, smx[3] = {e0.w, e1.x, e1.y};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {  // bUnion(left, right), operands in that order
+                mn[k] = left ? fminf(mn[k], smn[k]) : fminf(smn[k], mn[k]);
+                mx[k] = left ? fmaxf(mx[k], smx[k]) : fmaxf(smx[k], mx[k]);
+            }
+            if (left) ri = __float_as_int(e1.w);
+            else li = __float_as_int(e1.w);
+            const int L = sh.pos[li], R = sh.pos[ri + 1] - 1;
+            int* idx = reinterpret_cast<int*>(&sh.slot[slot][4]);
+            if (L == 0 && R == n - 1) {
+                *idx = 0;
+                put_root(root_bounds, mn, mx);
+                break;
+            }
+            ref = sh.delta[ri + 1] > sh.delta[li] ? R : L;
+            *idx = ref;
         }
     }
     __syncthreads();
-    if (l <= b1) leaf_prim[l] = prim;
-    const int slot = threadIdx.x;
-    if (b0 + slot + 1 <= b1) {
-        const float4 w = s_slot[slot][4];
+    if (i + 1 < cnt) {
+        const float4 w = sh.slot[i][4];
         const uint32_t have = __float_as_uint(w.y);
-        if (have == 3u) {  // the record of the parent formed here
-            const float4 a0 = s_slot[slot][0], a1 = s_slot[slot][1], c0 = s_slot[slot][2], c1 = s_slot[slot][3];
+        if (have == 3u) {  // the record of the node formed here
+            const float4 a0 = sh.slot[i][0], a1 = sh.slot[i][1], c0 = sh.slot[i][2], c1 = sh.slot[i][3];
             float4* P = reinterpret_cast<float4*>(nodes + __float_as_int(w.x));
             P[0] = a0;
             P[1] = make_float4(a1.x, a1.y, c0.x, c0.y);
             P[2] = make_float4(c0.z, c0.w, c1.x, c1.y);
-            reinterpret_cast<int4*>(P)[3] = make_int4(__float_as_int(a1.z), __float_as_int(c1.z), __float_as_int(a1.w),
-                                                      __float_as_int(c1.w));  // (left ref, right ref, lo, hi)
-        } else if (have != 0u) {  // a child alone: its sibling reaches into another block
-            push(__float_as_int(s_slot[slot][have == 1u ? 1 : 3].z));
+            reinterpret_cast<int4*>(P)[3] = make_int4(__float_as_int(a1.z), __float_as_int(c1.z), sh.pos[__float_as_int(a1.w)],
+                                                      sh.pos[__float_as_int(c1.w) + 1] - 1);  // (left ref, right ref, lo, hi)
+        } else if (have == 1u) {  // a left child alone: its sibling reaches out of the block
+            sh.root[__float_as_int(sh.slot[i][1].w)] = 2 * i + 1;
+        } else if (have == 2u) {  // a right child alone
+            sh.root[i + 1] = 2 * i + 2;
         }
     }
     __syncthreads();
-    const uint32_t np = min(s_npend, kPendCap);
-    if (np == 0u) return;
-    if (threadIdx.x == 0) s_pbase = atomicAdd(pending_count, np);
+    const int r = i < cnt ? sh.root[i] : 0, lane = i & 31, warp = i >> 5;
+    const unsigned m = __ballot_sync(~0u, r != 0);
+    if (lane == 0) sh.warp[warp] = __popc(m);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < np; i += kTreeBlock) pending[s_pbase + i] = s_pend[i];
+    int before = 0, total = 0;
+    for (int w = 0; w < kTreeBlock / 32; ++w) {
+        const int c = sh.warp[w];
+        before += w < warp ? c : 0;
+        total += c;
+    }
+    if (r != 0) {
+        const int at = before + __popc(m & ((1u << lane) - 1u));
+        float4 a, b;
+        if (r < 0) {
+            a = sh.edge[-1 - r][0];
+            b = sh.edge[-1 - r][1];
+        } else {  // a lone child: its far item becomes its last leaf
+            const int slot = (r - 1) >> 1, side = (r - 1) & 1;
+            a = sh.slot[slot][2 * side];
+            b = sh.slot[slot][2 * side + 1];
+            b.w = __int_as_float(sh.pos[(side == 0 ? slot : __float_as_int(b.w)) + 1] - 1);
+        }
+        if (at < kForestCap - 1) {
+            out[at].a = a;
+            out[at].b = b;
+        }
+    }
+    if (i == 0) out[kForestCap - 1].a.x = __int_as_float(total);
+    __syncthreads();
+    return total;
 }
 
-// Climbs from every child k_tree listed (at most 2n - 2 of them), grid-stride.
-__global__ __launch_bounds__(kBlock) void k_tree_top(const float* __restrict__ tri, int n, int mode,
+template <int kTreeBlock>
+__global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const float* __restrict__ tri, int n, int mode,
                                                      const int32_t* __restrict__ ids, const uint32_t* __restrict__ codes,
-                                                     BvhNode* __restrict__ nodes, uint32_t* __restrict__ arrivals,
-                                                     uint32_t epoch, const int32_t* __restrict__ pending,
-                                                     const uint32_t* __restrict__ pending_count,
+                                                     BvhNode* __restrict__ nodes, ForestEntry* __restrict__ forest,
+                                                     uint32_t* __restrict__ group_done, int32_t* __restrict__ leaf_prim,
                                                      float* __restrict__ root_bounds) {
-    const int count = (int)*pending_count;
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < count; i += gridDim.x * kBlock) {
-        const int ref = pending[i];
-        int L, R;
-        float mn[3], mx[3];
-        if (ref < 0) {  // leaf ~ref
-            L = R = ~ref;
-            const int prim = (mode == BVH_MODE_REFERENCE) ? L : __ldg(ids + L);
-            float t[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) t[k] = __ldg(tri + 9L * prim + k);
-            tri_bounds(t, mn, mx);
-        } else {        // interior node: its record holds both child boxes and its range
-            const float4 a = __ldcg(&nodes[ref].a), b = __ldcg(&nodes[ref].b), c = __ldcg(&nodes[ref].c);
-            const int4 d = __ldcg(&nodes[ref].d);
-            mn[0] = fminf(a.x, b.z); mn[1] = fminf(a.y, b.w); mn[2] = fminf(a.z, c.x);
-            mx[0] = fmaxf(a.w, c.y); mx[1] = fmaxf(b.x, c.z); mx[2] = fmaxf(b.y, c.w);
-            L = d.z;
-            R = d.w;
-        }
-        const bool left = delta(codes, n, R, R + 1) > delta(codes, n, L, L - 1);
-        climb_global(tri, n, mode, ids, codes, nodes, arrivals, epoch, root_bounds, L, R, ref, left ? R : L - 1, left,
-                     mn, mx);
+    __shared__ TreeShared<kTreeBlock> sh;
+    const int b0 = blockIdx.x * kTreeBlock, cnt = min(kTreeBlock, n - b0);
+    const int i = threadIdx.x, l = b0 + i;
+    // deltas across the block's boundaries b0 .. b0 + cnt, each thread's from its own two codes
+    if (i <= cnt) {
+        sh.delta[i] = l == 0 || l >= n ? -1 : delta_codes(__ldg(codes + l - 1), __ldg(codes + l), l - 1, l);
+        sh.pos[i] = l;
     }
+    if (i == 0 && cnt == kTreeBlock) {
+        sh.delta[cnt] = delta(codes, n, b0 + cnt - 1, b0 + cnt);
+        sh.pos[cnt] = b0 + cnt;
+    }
+    float mn[3], mx[3];
+    if (i < cnt) {
+        const int prim = (mode == BVH_MODE_REFERENCE) ? l : __ldg(ids + l);
+        leaf_prim[l] = prim;
+        gather_tri_bounds(tri, n, (reinterpret_cast<uintptr_t>(tri) & 15u) == 0, prim, mn, mx);
+        if (n == 1) put_root(root_bounds, mn, mx);
+    }
+    if (n == 1) return;
+    long first = blockIdx.x;  // the first block of the forest this block has written
+    int roots = tree_climb(sh, cnt, n, ~l, mn, mx, nodes, root_bounds, forest + first * kForestCap);
+    long span = 1;            // blocks per forest of this level
+    for (long count = gridDim.x; count > 1;) {
+        // publish the forest; the last of its group goes on with the group's
+        const long groups = (count + kTreeGroup - 1) / kTreeGroup, group = first / span / kTreeGroup;
+        const int nlists0 = (int)min((long)kTreeGroup, count - group * kTreeGroup);
+        if (i == 0) {
+            __threadfence();
+            sh.last = (int)atomicAdd(group_done + group, 1u) == nlists0 - 1;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!sh.last) return;
+        group_done += groups;
+        first = group * kTreeGroup * span;
+        // the group's subtrees as items, kTreeBlock at a time; the forests of several chunks (more
+        // subtrees than threads) are written over the lists read before, and merged again
+        int nlists = nlists0;
+        long step = span;
+        for (;;) {
+            if (i < nlists) sh.list[i + 1] = __float_as_int(__ldcg(&forest[(first + i * step) * kForestCap + kForestCap - 1].a.x));
+            __syncthreads();
+            if (i == 0) {
+                sh.list[0] = 0;
+                for (int j = 0; j < nlists; ++j) sh.list[j + 1] += sh.list[j];
+            }
+            __syncthreads();
+            const int total = sh.list[nlists], chunks = (total + kTreeBlock - 1) / kTreeBlock;
+            for (int c = 0; c < chunks; ++c) {
+                const int c0 = c * kTreeBlock, m = min(kTreeBlock, total - c0);
+                auto entry = [&](int k) -> const ForestEntry* {
+                    int j = 0;
+                    while (k >= sh.list[j + 1]) ++j;
+                    return forest + (first + j * step) * kForestCap + (k - sh.list[j]);
+                };
+                int ref = 0;
+                if (i < m) {
+                    const ForestEntry* e = entry(c0 + i);
+                    const float4 a = __ldcg(&e->a), b = __ldcg(&e->b);
+                    mn[0] = a.x; mn[1] = a.y; mn[2] = a.z;
+                    mx[0] = a.w; mx[1] = b.x; mx[2] = b.y;
+                    ref = __float_as_int(b.z);
+                    const int end = __float_as_int(b.w) + 1;
+                    sh.pos[i + 1] = end;
+                    sh.delta[i + 1] = end >= n ? -1 : delta_codes(__ldg(codes + end - 1), __ldg(codes + end), end - 1, end);
+                }
+                if (i == 0) {
+                    const int p = c0 == 0 ? (int)(first * kTreeBlock) : __float_as_int(__ldcg(&entry(c0 - 1)->b).w) + 1;
+                    sh.pos[0] = p;
+                    sh.delta[0] = p == 0 ? -1 : delta_codes(__ldg(codes + p - 1), __ldg(codes + p), p - 1, p);
+                }
+                __syncthreads();
+                // chunk c's forest over list c: at most 127 entries a list, so the chunks up to c
+                // have read every list up to c
+                roots = tree_climb(sh, m, n, ref, mn, mx, nodes, root_bounds, forest + (first + c * step) * kForestCap);
+            }
+            if (chunks <= 1) break;
+            nlists = chunks;
+            __threadfence_block();
+            __syncthreads();
+        }
+        span *= kTreeGroup;
+        count = groups;
+    }
+    (void)roots;
 }
 
 inline int grid_for(long items, int per_block) { return (int)((items + per_block - 1) / per_block); }
-#ifndef LTS_TREE_TOP_BLOCKS_PER_SM
-#define LTS_TREE_TOP_BLOCKS_PER_SM 32
-#endif
-// k_tree_top's grid: close to one listed child per thread (the list holds at most 2n - 2;
-// each climb is a chain of dependent device-memory round trips, so a thread should start its
-// climbs at once rather than one after another), capped at LTS_TREE_TOP_BLOCKS_PER_SM per SM.
-inline int tree_top_grid(long n, int sms) {
-    return (int)std::max<long>(1, std::min<long>(grid_for(2 * n, kBlock), (long)sms * LTS_TREE_TOP_BLOCKS_PER_SM));
+
+// The build in the reference's flattened order (BVH.cuh:311-329: interior 0 .. n - 2, leaves
+// n - 1 .. 2n - 2): each interior node writes its children's indices and, at their indices, their
+// boxes.
+__global__ __launch_bounds__(kBlock) void k_dump(const BvhNode* __restrict__ nodes, int n, const float* __restrict__ root_bounds,
+                                                 int32_t* __restrict__ left, int32_t* __restrict__ right,
+                                                 float* __restrict__ bounds) {
+    const long i = (long)blockIdx.x * kBlock + threadIdx.x;
+    if (i < n) left[n - 1 + i] = right[n - 1 + i] = -1;
+    if (i < 6) bounds[i] = root_bounds[i];
+    if (i >= n - 1) return;
+    const float4 a = nodes[i].a, b = nodes[i].b, c = nodes[i].c;
+    const int4 d = nodes[i].d;
+    const int lc = d.x < 0 ? n - 1 + ~d.x : d.x, rc = d.y < 0 ? n - 1 + ~d.y : d.y;
+    left[i] = lc;
+    right[i] = rc;
+    float2* const lb = reinterpret_cast<float2*>(bounds + 6 * (size_t)lc);
+    float2* const rb = reinterpret_cast<float2*>(bounds + 6 * (size_t)rc);
+    lb[0] = make_float2(a.x, a.y);
+    lb[1] = make_float2(a.z, a.w);
+    lb[2] = make_float2(b.x, b.y);
+    rb[0] = make_float2(b.z, b.w);
+    rb[1] = make_float2(c.x, c.y);
+    rb[2] = make_float2(c.z, c.w);
+}
+
+// Sort tiles: kSortItems keys per thread once the tiles fill the SMs' resident blocks; smaller tiles
+// below that, whose passes are a tile's latency (a chain of ranking steps) and the look-back over
+// all tiles at once (400,000 keys, ms of the four passes: 15 keys and 4 tiles a round trip 0.055, 4
+// and 16 0.059, 8 and 16 0.051, 8 and 32 0.066, 10 and 16 0.051; at 700,000 15 keys are faster).
+constexpr int kSortSmallMax = 500000, kSortSmallItems = 8, kSortSmallLookback = 16, kSortLookback = 4;
+// Triangles per thread of the two streaming kernels before every SM has its eight blocks: each block
+// ends with atomics on the same words (400,000 triangles: Morton codes 12.2 us, 18.4 at one).
+constexpr int kStreamItems = 4;
+constexpr long sort_tile(long n) { return kSortThreads * (n <= kSortSmallMax ? kSortSmallItems : kSortItems); }
+constexpr long sort_tiles(long n) { return (n + sort_tile(n) - 1) / sort_tile(n); }
+
+// The words every build starts from zero, in one buffer: scene box (8), sort tile counters (8),
+// histograms (4 x 256), the tree's group counters, then the sort's look-back table.
+constexpr size_t kZeroHist = 16, kZeroGroups = kZeroHist + 4 * 256;
+constexpr size_t zero_status(long n) { return kZeroGroups + ((size_t)tree_counters(n) + 7) / 8 * 8; }
+constexpr size_t zero_words(long n) { return zero_status(n) + 4 * 256 * (size_t)sort_tiles(n); }
+
+// The build's launches, shared by Lbvh and the allocation-free entry point.  kalt / valt: the sort's
+// second key and value buffers; `zero`: zero_words(n) words; `forest`: forest_bytes(n).  mark(k) is
+// called before stage k (bounds, Morton codes, sort, clear, tree) and after the last.
+template <class Mark>
+cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, uint32_t* codes, int32_t* ids, uint32_t* kalt,
+                           int32_t* valt, uint32_t* zero, ForestEntry* forest, BvhNode* nodes, int32_t* leaf_prim,
+                           float* root_bounds, uint32_t* err, int sms, cudaStream_t s, int* launches, Mark mark) {
+    uint32_t* const groups = zero + kZeroGroups;
+    mark(0);
+    if (n <= kSmallSort) {
+        mark(1);
+        mark(2);
+        k_small_sort<<<1, kSmallThreads, 0, s>>>(tri, n, code_limit, codes, ids, groups, (int)tree_counters(n));
+        *launches = 2;
+    } else {
+        cudaError_t e = cudaMemsetAsync(zero, 0, 4 * zero_words(n), s);
+        if (e != cudaSuccess) return e;
+        const int stream_grid = std::min(grid_for(n, kBlock * kStreamItems), sms * 8);
+        k_scene_bounds<<<stream_grid, kBlock, 0, s>>>(tri, n, zero);
+        mark(1);
+        const bool identity = code_limit < 0 || code_limit >= n;  // every id is its position
+        uint32_t* const hist = zero + kZeroHist;
+        k_morton<<<stream_grid, kBlock, 0, s>>>(tri, n, zero, code_limit, codes, identity ? nullptr : ids, hist);
+        mark(2);
+        uint32_t* const status = zero + zero_status(n);
+        const size_t tiles = (size_t)sort_tiles(n);
+        if (n > kSortSmallMax) k_digit_prefix<<<4, 256, 0, s>>>(hist, hist);
+        uint32_t *kin = codes, *kout = kalt;
+        int32_t *vin = ids, *vout = valt;
+        for (int p = 0; p < 4; ++p) {
+            auto k = n <= kSortSmallMax ? k_onesweep<kSortSmallItems, kSortSmallLookback, true> : k_onesweep<kSortItems, kSortLookback, false>;
+            k<<<(int)tiles, kSortThreads, 0, s>>>(kin, (p == 0 && identity) ? nullptr : vin, kout, vout, n, 8 * p, hist + 256 * p,
+                                                  status + (size_t)p * 256 * tiles, zero + 8 + p, err);
+            std::swap(kin, kout);
+            std::swap(vin, vout);
+        }
+        *launches = n > kSortSmallMax ? 8 : 7;
+    }
+    mark(3);
+    mark(4);
+    auto tree = tree_block(n) == 512 ? k_tree<512> : k_tree<256>;
+    tree<<<(int)tree_blocks(n), tree_block(n), 0, s>>>(tri, n, mode, ids, codes, nodes, forest, groups, leaf_prim, root_bounds);
+    mark(5);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -674,7 +849,7 @@ inline int tree_top_grid(long n, int sms) {
     } while (0)
 
 Lbvh::~Lbvh() {
-    void* ptrs[] = {nodes, root_bounds, leaf_prim, codes, ids, codes_alt_, hist_, status_, counters_, gbounds_, flags_};
+    void* ptrs[] = {nodes, root_bounds, leaf_prim, codes, ids, codes_alt_, zero_};
     for (void* p : ptrs)
         if (p) dev_free(p);
     for (auto& e : ev_)
@@ -685,10 +860,10 @@ std::string Lbvh::reserve(int nn) {
     if (!ev_[0])
         for (auto& e : ev_) LTS_TRY(cudaEventCreate(&e));
     if (nn <= cap_) return "";
-    void* ptrs[] = {nodes, root_bounds, leaf_prim, codes, ids, codes_alt_, hist_, status_, counters_, gbounds_, flags_};
+    void* ptrs[] = {nodes, root_bounds, leaf_prim, codes, ids, codes_alt_, zero_};
     for (void* p : ptrs)
         if (p) dev_free(p);
-    const size_t N = (size_t)nn, tiles = (N + kSortTile - 1) / kSortTile;
+    const size_t N = (size_t)nn;
     bytes_ = 0;
     auto al = [&](void** p, size_t b) -> cudaError_t {
         bytes_ += b;
@@ -699,16 +874,11 @@ std::string Lbvh::reserve(int nn) {
     LTS_TRY(al((void**)&leaf_prim, 4 * N));
     LTS_TRY(al((void**)&codes, 4 * N));
     LTS_TRY(al((void**)&ids, 4 * N));
-    // the sort's ping-pong keys and ids, one allocation: after the sort it holds the tree's list
-    // of up to 2n - 2 children that meet across blocks
-    LTS_TRY(al((void**)&codes_alt_, 8 * N));
+    // the sort's ping-pong keys and ids, one allocation: after the sort it holds the tree's forests
+    LTS_TRY(al((void**)&codes_alt_, std::max({8 * N, forest_bytes(nn), forest_bytes(std::min(nn, kTreeLarge))})));
     ids_alt_ = reinterpret_cast<int32_t*>(codes_alt_ + N);
-    LTS_TRY(al((void**)&hist_, 4 * 2 * 4 * 256));  // histograms then prefixes
-    LTS_TRY(al((void**)&status_, 4 * 4 * 256 * tiles));
-    LTS_TRY(al((void**)&counters_, 4 * 8));
-    LTS_TRY(al((void**)&gbounds_, 4 * 6));
-    LTS_TRY(al((void**)&flags_, 4 * (N > 1 ? N - 1 : 1)));
-    clear_arrivals_ = true;  // arrival words of fresh memory are zeroed before the first build
+    // a smaller build may take smaller sort tiles, hence more of them than a larger one
+    LTS_TRY(al((void**)&zero_, 4 * std::max(zero_words(nn), zero_words(std::min(nn, kSortSmallMax)))));
     cap_ = nn;
     return "";
 }
@@ -722,61 +892,22 @@ std::string Lbvh::build(const float* d_tri, int nn, int md, int code_limit, cuda
     mode = md;
     launches = 0;
     ++serial;
-    const size_t N = (size_t)nn, tiles = (N + kSortTile - 1) / kSortTile;
     int dev = 0, sms = 0;
     LTS_TRY(cudaGetDevice(&dev));
     LTS_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int stream_grid = std::min(grid_for((long)N, kBlock), sms * 8);
+    cudaError_t me = cudaSuccess;
+    LTS_TRY(build_launches(d_tri, nn, md, code_limit, codes, ids, codes_alt_, ids_alt_, zero_,
+                           reinterpret_cast<ForestEntry*>(codes_alt_), nodes, leaf_prim, root_bounds, d_error, sms, s, &launches,
+                           [&](int k) {
+                               const cudaError_t e = cudaEventRecord(ev_[k], s);
+                               if (e != cudaSuccess) me = e;
+                           }));
+    LTS_TRY(me);
+    return "";
+}
 
-    LTS_TRY(cudaEventRecord(ev_[0], s));
-    LTS_TRY(cudaMemsetAsync(gbounds_, 0xff, 12, s));
-    LTS_TRY(cudaMemsetAsync(gbounds_ + 3, 0x00, 12, s));
-    k_scene_bounds<<<stream_grid, kBlock, 0, s>>>(d_tri, nn, gbounds_);
-    ++launches;
-    LTS_TRY(cudaEventRecord(ev_[1], s));
-    LTS_TRY(cudaMemsetAsync(hist_, 0, 4 * 4 * 256, s));
-    const bool identity = code_limit < 0 || code_limit >= nn;  // every id is its position
-    k_morton<<<stream_grid, kBlock, 0, s>>>(d_tri, nn, gbounds_, code_limit, codes, identity ? nullptr : ids, hist_);
-    ++launches;
-    LTS_TRY(cudaEventRecord(ev_[2], s));
-    LTS_TRY(cudaMemsetAsync(status_, 0, 4 * 4 * 256 * tiles, s));
-    LTS_TRY(cudaMemsetAsync(counters_, 0, 4 * 8, s));
-    k_digit_prefix<<<4, 256, 0, s>>>(hist_, hist_ + 4 * 256);
-    ++launches;
-    uint32_t* kin = codes;
-    int32_t* vin = ids;
-    uint32_t* kout = codes_alt_;
-    int32_t* vout = ids_alt_;
-    for (int p = 0; p < 4; ++p) {
-        k_onesweep<<<(int)tiles, kSortThreads, 0, s>>>(kin, (p == 0 && identity) ? nullptr : vin, kout, vout, nn, 8 * p,
-                                                        hist_ + 4 * 256 + 256 * p, status_ + (size_t)p * 256 * tiles,
-                                                        counters_ + p, d_error);
-        ++launches;
-        std::swap(kin, kout);
-        std::swap(vin, vout);
-    }
-    LTS_TRY(cudaEventRecord(ev_[3], s));
-    // the arrival words keep the epoch of the build that last touched them, so a new epoch per
-    // build replaces clearing them; they are cleared only when fresh or when the epoch wraps
-    if (++epoch_ > kEpochMax) {
-        clear_arrivals_ = true;
-        epoch_ = 1u;
-    }
-    if (clear_arrivals_) {  // every word of the allocation: a later, larger build reads past n - 1
-        LTS_TRY(cudaMemsetAsync(flags_, 0, 4 * (size_t)(cap_ > 1 ? cap_ - 1 : 1), s));
-        clear_arrivals_ = false;
-    }
-    LTS_TRY(cudaEventRecord(ev_[4], s));  // topology and refit run as one kernel, timed as the refit stage
-    int32_t* pending = reinterpret_cast<int32_t*>(codes_alt_);
-    k_tree<<<grid_for((long)N, kTreeBlock), kTreeBlock, 0, s>>>(d_tri, nn, md, ids, codes, nodes, pending, counters_ + 4,
-                                                                leaf_prim, root_bounds);
-    ++launches;
-    if (nn > 1) {
-        k_tree_top<<<tree_top_grid(nn, sms), kBlock, 0, s>>>(d_tri, nn, md, ids, codes, nodes, flags_, epoch_, pending,
-                                                             counters_ + 4, root_bounds);
-        ++launches;
-    }
-    LTS_TRY(cudaEventRecord(ev_[5], s));
+std::string Lbvh::flatten(int32_t* d_left, int32_t* d_right, float* d_bounds, cudaStream_t s) const {
+    k_dump<<<grid_for(n, kBlock), kBlock, 0, s>>>(nodes, n, root_bounds, d_left, d_right, d_bounds);
     LTS_TRY(cudaGetLastError());
     return "";
 }
@@ -823,7 +954,7 @@ void Lbvh::stage_ms(float out[5]) const {
 // one file-scope device array of fixed size, so a call allocates nothing; the caller supplies the
 // triangles and every output buffer.
 //
-// Limits and sharing: at most kNoAllocMaxPrims primitives (about 3.3 MiB of device memory that
+// Limits and sharing: at most kNoAllocMaxPrims primitives (about 2.5 MiB of device memory that
 // every GPU which loads the library keeps until process exit).  All calls share the one array and
 // it keeps the previous call's contents, so everything that must start at zero is cleared at the
 // start of each call, and two calls that overlap on the GPU (different streams, or different host
@@ -838,18 +969,14 @@ namespace lts {
 namespace {
 
 constexpr int kNoAllocMaxPrims = 1 << 18;
-constexpr size_t kNoAllocTiles = (kNoAllocMaxPrims + kSortTile - 1) / kSortTile;
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kOffCodes = 0;
-constexpr size_t kOffIds = kOffCodes + align256(4ull * kNoAllocMaxPrims);
-constexpr size_t kOffHist = kOffIds + align256(4ull * kNoAllocMaxPrims);
-static_assert(kOffIds == kOffCodes + 4ull * kNoAllocMaxPrims, "the tree's list of 2n ints spans both sort buffers");
-constexpr size_t kOffStatus = kOffHist + align256(4ull * 2 * 4 * 256);
-constexpr size_t kOffCounters = kOffStatus + align256(4ull * 4 * 256 * kNoAllocTiles);
-constexpr size_t kOffBounds = kOffCounters + 256;
-constexpr size_t kOffError = kOffBounds + 256;
-constexpr size_t kOffFlags = kOffError + 256;
-constexpr size_t kNoAllocBytes = kOffFlags + align256(4ull * kNoAllocMaxPrims);
+constexpr size_t kOffIds = kOffCodes + 4ull * kNoAllocMaxPrims;
+static_assert(kOffIds + 4ull * kNoAllocMaxPrims >= forest_bytes(kNoAllocMaxPrims), "the tree's forests lie in both sort buffers");
+constexpr size_t kOffZero = align256(kOffIds + 4ull * kNoAllocMaxPrims);
+constexpr size_t kOffError = kOffZero + align256(4 * zero_words(kNoAllocMaxPrims));
+constexpr size_t kNoAllocBytes = kOffError + 256;
+static_assert(kNoAllocMaxPrims <= kSortSmallMax, "one tile size, so the largest build has the most tiles");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -891,49 +1018,18 @@ extern "C" int lts_bvh_build_noalloc(const float* d_tri, int32_t n, int32_t mode
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint32_t* codes_alt = reinterpret_cast<uint32_t*>(base + kOffCodes);
     int32_t* ids_alt = reinterpret_cast<int32_t*>(base + kOffIds);
-    uint32_t* hist = reinterpret_cast<uint32_t*>(base + kOffHist);
-    uint32_t* status = reinterpret_cast<uint32_t*>(base + kOffStatus);
-    uint32_t* counters = reinterpret_cast<uint32_t*>(base + kOffCounters);
-    uint32_t* gbounds = reinterpret_cast<uint32_t*>(base + kOffBounds);
+    uint32_t* zero = reinterpret_cast<uint32_t*>(base + kOffZero);
     uint32_t* err = reinterpret_cast<uint32_t*>(base + kOffError);
-    uint32_t* flags = reinterpret_cast<uint32_t*>(base + kOffFlags);
-    BvhNode* nodes = static_cast<BvhNode*>(d_nodes);
-    const size_t N = (size_t)n, tiles = (N + kSortTile - 1) / kSortTile;
-    int sms = 0;
+    int sms = 0, launches = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return LTS_ERR_CUDA;
-    const int stream_grid = std::min(grid_for((long)N, kBlock), sms * 8);
-    // clear everything the kernels expect to start zeroed (or all-ones)
-    if (cudaMemsetAsync(err, 0, 4, s) != cudaSuccess || cudaMemsetAsync(gbounds, 0xff, 12, s) != cudaSuccess ||
-        cudaMemsetAsync(gbounds + 3, 0x00, 12, s) != cudaSuccess ||
-        cudaMemsetAsync(hist, 0, 4 * 4 * 256, s) != cudaSuccess ||
-        cudaMemsetAsync(status, 0, 4 * 4 * 256 * tiles, s) != cudaSuccess ||
-        cudaMemsetAsync(counters, 0, 4 * 8, s) != cudaSuccess)
+    const bool waits = n > kSmallSort;  // the sort's look-back: the only wait that can run out
+    if (waits && cudaMemsetAsync(err, 0, 4, s) != cudaSuccess) return LTS_ERR_CUDA;
+    if (build_launches(d_tri, n, mode, code_limit, d_codes, d_ids, codes_alt, ids_alt, zero,
+                       reinterpret_cast<ForestEntry*>(codes_alt), static_cast<BvhNode*>(d_nodes), d_leaf_prim, d_root_bounds, err,
+                       sms, s, &launches, [](int) {}) != cudaSuccess)
         return LTS_ERR_CUDA;
-    k_scene_bounds<<<stream_grid, kBlock, 0, s>>>(d_tri, n, gbounds);
-    const bool identity = code_limit < 0 || code_limit >= n;  // every id is its position
-    k_morton<<<stream_grid, kBlock, 0, s>>>(d_tri, n, gbounds, code_limit, d_codes, identity ? nullptr : d_ids, hist);
-    k_digit_prefix<<<4, 256, 0, s>>>(hist, hist + 4 * 256);
-    uint32_t* kin = d_codes;
-    int32_t* vin = d_ids;
-    uint32_t* kout = codes_alt;
-    int32_t* vout = ids_alt;
-    for (int p = 0; p < 4; ++p) {
-        k_onesweep<<<(int)tiles, kSortThreads, 0, s>>>(kin, (p == 0 && identity) ? nullptr : vin, kout, vout, n, 8 * p,
-                                                        hist + 4 * 256 + 256 * p, status + (size_t)p * 256 * tiles,
-                                                        counters + p, err);
-        std::swap(kin, kout);
-        std::swap(vin, vout);
-    }
-    if (n > 1 && cudaMemsetAsync(flags, 0, 4 * (N - 1), s) != cudaSuccess) return LTS_ERR_CUDA;  // arrival words, epoch 1
-    int32_t* pending = reinterpret_cast<int32_t*>(codes_alt);  // codes_alt and ids_alt: 2n ints
-    k_tree<<<grid_for((long)N, kTreeBlock), kTreeBlock, 0, s>>>(d_tri, n, mode, d_ids, d_codes, nodes, pending,
-                                                                counters + 4, d_leaf_prim, d_root_bounds);
-    if (n > 1)
-        k_tree_top<<<tree_top_grid(n, sms), kBlock, 0, s>>>(d_tri, n, mode, d_ids, d_codes, nodes, flags, 1u, pending,
-                                                            counters + 4, d_root_bounds);
-    if (cudaGetLastError() != cudaSuccess) return LTS_ERR_CUDA;
     uint32_t h_err = 0;
-    if (cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return LTS_ERR_CUDA;
+    if (waits && cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return LTS_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return LTS_ERR_CUDA;
     return h_err ? LTS_ERR_DEVICE : LTS_OK;
 }

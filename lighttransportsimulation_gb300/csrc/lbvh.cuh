@@ -37,6 +37,10 @@ class Lbvh {
     // topology and refit run as one kernel, reported as the refit stage (topology ~0).
     void stage_ms(float out[5]) const;
 
+    // The tree in the reference's flattened order: child indices [2n - 1] each (-1 for leaves) and
+    // boxes [2n - 1][6], device pointers (d_bounds 8-byte aligned).
+    std::string flatten(int32_t* d_left, int32_t* d_right, float* d_bounds, cudaStream_t s) const;
+
     int n = 0;
     int mode = BVH_MODE_SORTED;
     // Outputs (device).
@@ -53,11 +57,8 @@ class Lbvh {
     std::string reserve(int n);
     int cap_ = 0;
     size_t bytes_ = 0;
-    uint32_t *codes_alt_ = nullptr, *hist_ = nullptr, *status_ = nullptr, *counters_ = nullptr,
-             *gbounds_ = nullptr, *flags_ = nullptr;
+    uint32_t *codes_alt_ = nullptr, *zero_ = nullptr;  // sort buffers, then the tree's forests; words zeroed per build
     int32_t* ids_alt_ = nullptr;  // second half of codes_alt_'s allocation
-    uint32_t epoch_ = 0;            // tree-build epoch written into the arrival words (flags_)
-    bool clear_arrivals_ = false;   // flags_ is fresh memory and must be zeroed once
     cudaEvent_t ev_[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
 };
 
