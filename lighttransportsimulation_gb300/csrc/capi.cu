@@ -81,6 +81,9 @@ struct lts_ctx {
     bool loaded = false;
     float* d_tri = nullptr;  // scene triangle soup, 9 floats per triangle (scene order)
     size_t d_tri_cap = 0;
+    // kept between calls: the input of lts_bvh_build_triangles, the flattened tree of a dump
+    void *soup_ws = nullptr, *dump_ws = nullptr;
+    size_t soup_ws_cap = 0, dump_ws_cap = 0;
     std::unique_ptr<Lbvh> bvh;
     std::unique_ptr<Mlp> mlp;
     int bvh_mode = -1;        // mode of the BVH currently held (-1: none)
@@ -90,6 +93,8 @@ struct lts_ctx {
 };
 
 namespace {
+
+constexpr size_t kDumpKeep = 256ull << 20;
 
 int fail(lts_ctx* c, int code, const std::string& msg) {
     if (c) c->err = msg;
@@ -153,33 +158,46 @@ int dump_bvh(lts_ctx* ctx, lts_bvh_dump* d) {
         ctx->metrics.bvh_build_ms += st[i];
     }
     if (!d) return LTS_OK;
-    const int n = b.n, nodes = 2 * n - 1;
-    if (d->sorted_codes) CK(cudaMemcpy(d->sorted_codes, b.codes, 4 * (size_t)n, cudaMemcpyDeviceToHost));
-    if (d->sorted_ids) CK(cudaMemcpy(d->sorted_ids, b.ids, 4 * (size_t)n, cudaMemcpyDeviceToHost));
-    if (!d->node_key && !d->node_left && !d->node_right && !d->node_bounds) return LTS_OK;
-    std::vector<BvhNode> h((size_t)(n > 1 ? n - 1 : 0));
-    if (n > 1) CK(cudaMemcpy(h.data(), b.nodes, sizeof(BvhNode) * (n - 1), cudaMemcpyDeviceToHost));
-    float root[6];
-    CK(cudaMemcpy(root, b.root_bounds, 24, cudaMemcpyDeviceToHost));
-    // Reference flattened order: interior 0..n-2, leaves n-1..2n-2 (BVH.cuh:311-329).
-    std::vector<int32_t> key(nodes, -1), left(nodes, -1), right(nodes, -1);
-    std::vector<float> bnd((size_t)nodes * 6, 0.f);
-    for (int l = 0; l < n; ++l) key[n - 1 + l] = l;
-    auto flat = [n](int c) { return c < 0 ? (n - 1) + ~c : c; };
-    memcpy(&bnd[0], root, 24);
-    if (n == 1) memcpy(&bnd[0], root, 24);
-    for (int i = 0; i < n - 1; ++i) {
-        const float* f = reinterpret_cast<const float*>(&h[i]);
-        const int lc = flat(h[i].d.x), rc = flat(h[i].d.y);
-        left[i] = lc;
-        right[i] = rc;
-        memcpy(&bnd[(size_t)lc * 6], f, 24);
-        memcpy(&bnd[(size_t)rc * 6], f + 6, 24);
+    const int n = b.n;
+    const size_t nodes = 2 * (size_t)n - 1;
+    if (d->node_left || d->node_right || d->node_bounds) {
+        // flattened on the device and copied straight into the caller's arrays; a workspace of up to
+        // kDumpKeep bytes stays with the context
+        const size_t bytes = 8 * ((nodes + 1) / 2 * 2) + 24 * nodes;
+        void* ws = ctx->dump_ws;
+        if (ctx->dump_ws_cap < bytes) {
+            dev_free(ctx->dump_ws);
+            ctx->dump_ws = nullptr;
+            ctx->dump_ws_cap = 0;
+            CK(dev_alloc(&ws, bytes));
+            if (bytes <= kDumpKeep) {
+                ctx->dump_ws = ws;
+                ctx->dump_ws_cap = bytes;
+            }
+        }
+        int32_t* left = static_cast<int32_t*>(ws);
+        int32_t* right = left + (nodes + 1) / 2 * 2;
+        float* bounds = reinterpret_cast<float*>(right + (nodes + 1) / 2 * 2);
+        const std::string e = b.flatten(left, right, bounds, ctx->stream);
+        cudaError_t ce = e.empty() ? cudaSuccess : cudaErrorUnknown;
+        auto get = [&](void* to, const void* from, size_t bytes) {
+            if (to && ce == cudaSuccess) ce = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+        };
+        get(d->node_left, left, 4 * nodes);
+        get(d->node_right, right, 4 * nodes);
+        get(d->node_bounds, bounds, 24 * nodes);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
+        if (ws != ctx->dump_ws) dev_free(ws);
+        if (!e.empty()) return fail(ctx, LTS_ERR_CUDA, e);
+        if (ce != cudaSuccess) return cuda_fail(ctx, ce, "copy the tree");
     }
-    if (d->node_key) memcpy(d->node_key, key.data(), 4 * (size_t)nodes);
-    if (d->node_left) memcpy(d->node_left, left.data(), 4 * (size_t)nodes);
-    if (d->node_right) memcpy(d->node_right, right.data(), 4 * (size_t)nodes);
-    if (d->node_bounds) memcpy(d->node_bounds, bnd.data(), 24 * (size_t)nodes);
+    if (d->sorted_codes) CK(cudaMemcpyAsync(d->sorted_codes, b.codes, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+    if (d->sorted_ids) CK(cudaMemcpyAsync(d->sorted_ids, b.ids, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+    if (d->node_key) {
+        for (int i = 0; i < n - 1; ++i) d->node_key[i] = -1;
+        for (int l = 0; l < n; ++l) d->node_key[n - 1 + l] = l;
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
     return LTS_OK;
 }
 
@@ -226,6 +244,8 @@ void lts_destroy(lts_ctx* ctx) {
     ctx->tracer.reset();
     ctx->bvh.reset();
     dev_free(ctx->d_tri);
+    dev_free(ctx->soup_ws);
+    dev_free(ctx->dump_ws);
     dev_free(ctx->d_error);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -364,18 +384,24 @@ int lts_bvh_build_triangles(lts_ctx* ctx, const float* tri, int32_t n, int32_t m
     if (!ctx || !tri || n < 1) return fail(ctx, LTS_ERR_ARG, "bad triangle input");
     if (ctx->device == -1) return fail(ctx, LTS_ERR_STATE, "host-only context (device -1) cannot run kernels");
     CK(cudaSetDevice(ctx->device));
-    float* d = nullptr;
-    CK(dev_alloc((void**)&d, 36 * (size_t)n));
-    cudaError_t e = cudaMemcpyAsync(d, tri, 36 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
-    if (e != cudaSuccess) {
-        dev_free(d);
-        return cuda_fail(ctx, e, "copy triangles");
+    const size_t bytes = 36 * (size_t)n;
+    float* d = static_cast<float*>(ctx->soup_ws);
+    if (ctx->soup_ws_cap < bytes) {
+        dev_free(ctx->soup_ws);
+        ctx->soup_ws = nullptr;
+        ctx->soup_ws_cap = 0;
+        CK(dev_alloc((void**)&d, bytes));
+        if (bytes <= kDumpKeep) {
+            ctx->soup_ws = d;
+            ctx->soup_ws_cap = bytes;
+        }
     }
-    int rc = do_build(ctx, d, n, mode, code_limit);
+    cudaError_t e = cudaMemcpyAsync(d, tri, bytes, cudaMemcpyHostToDevice, ctx->stream);
+    int rc = e == cudaSuccess ? do_build(ctx, d, n, mode, code_limit) : cuda_fail(ctx, e, "copy triangles");
     if (rc == LTS_OK) rc = dump_bvh(ctx, dump);
     cudaStreamSynchronize(ctx->stream);
-    dev_free(d);
-    ctx->bvh_is_scene = false;
+    if (d != ctx->soup_ws) dev_free(d);
+    if (e == cudaSuccess) ctx->bvh_is_scene = false;
     return rc;
 }
 
