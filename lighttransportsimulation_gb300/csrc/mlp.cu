@@ -10,6 +10,7 @@
 #include "mlp.cuh"
 #include "umma.cuh"
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cmath>
 
@@ -96,20 +97,18 @@ constexpr uint32_t kSGa = kSGz + 4096;
 constexpr uint32_t kTrainBar = kSGa + 16384;
 constexpr uint32_t kTrainSmem = kTrainBar + 64;
 // Inference keeps kFwdGroups tiles in flight per CTA (one CTA per SM), one warpgroup of 128
-// threads per tile, sharing the weights: each tile has one 24 KB operand buffer at
-// fwd_buf(g) -- its features X (128 x 96), then each hidden layer's activations (128 x 64),
-// written over the buffer once the layer's products have completed -- an mbarrier and 64 TMEM
-// columns.
-#ifndef LTS_MLP_FWD_GROUPS
-#define LTS_MLP_FWD_GROUPS 6
-#endif
-constexpr int kFwdGroups = LTS_MLP_FWD_GROUPS;
+// threads per tile, sharing the weights: each tile has a 24 KB buffer at fwd_buf(g) for its features
+// X (128 x 96), an mbarrier and 96 TMEM columns -- the product D (128 x 64 FP32) and, as the next
+// product's A operand, the activations (128 x 64 bf16, two to a column).
+constexpr int kFwdGroups = 5;
 constexpr uint32_t kFwdTileBytes = 24576;
 __host__ __device__ constexpr uint32_t fwd_buf(int g) { return kSX + kFwdTileBytes * (uint32_t)g; }
-constexpr uint32_t kFwdBar = kSX + kFwdTileBytes * kFwdGroups;  // kFwdGroups mbarriers, then the TMEM slot
-constexpr uint32_t kFwdSmem = kFwdBar + 8 * kFwdGroups + 16;
-constexpr uint32_t kFwdCols = 64 * kFwdGroups <= 128 ? 128 : (64 * kFwdGroups <= 256 ? 256 : 512);
-static_assert(64 * kFwdGroups <= 512 && kFwdSmem <= 232448, "inference tiles exceed TMEM or shared memory");
+// then two mbarriers per tile (products, feature copies) and the TMEM slot
+constexpr uint32_t kFwdBar = kSX + kFwdTileBytes * kFwdGroups;
+constexpr uint32_t kFwdSmem = kFwdBar + 16 * kFwdGroups + 16;
+static_assert(kSX % 1024 == 0 && kFwdTileBytes % 1024 == 0, "swizzled copies need 1024-byte aligned buffers");
+constexpr uint32_t kFwdCols = 512, kFwdTileCols = 96, kFwdACol = 64;
+static_assert(kFwdTileCols * kFwdGroups <= kFwdCols && kFwdSmem <= 232448, "inference tiles exceed TMEM or shared memory");
 // TMEM columns: 0..63 the working product; dW_k^T accumulators (training) at kDwCol(k)
 __host__ __device__ constexpr uint32_t kDwCol(int L) { return 64u * (uint32_t)(L + 1); }
 
@@ -233,70 +232,152 @@ __device__ __forceinline__ void wg_publish(int id) {
     tc_fence_after();
 }
 
+// Two FP32 columns to one word of two bf16 (a in the low half), ReLU: rounded first, then clamped
+// (the same values; NaN becomes 0 as by fmaxf).
+__device__ __forceinline__ uint32_t relu_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
+    asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+    return r;
+}
+
 // Inference: out[r * stride + c] = exp(z_c), c < 3, for the feature rows r = rows[i] (rows null:
 // r = i), i < n.  Persistent CTAs of kFwdGroups warpgroups; warpgroup g runs tiles
-// blockIdx.x * kFwdGroups + g, + gridDim.x * kFwdGroups, ..., one row per thread, and
-// synchronises with named barrier 1 + g only, so the tiles of a CTA overlap each other's
-// epilogues and waits.
+// g * gridDim.x + blockIdx.x, + gridDim.x * kFwdGroups, ..., and synchronises with named barrier 1 + g
+// only, so the tiles of a CTA overlap each other's epilogues and waits.  A tile is a chain of six
+// dependent products, so what bounds the kernel is that chain's latency over the tiles in flight.
+// It is kept short: the hidden activations never leave TMEM (the epilogue loads D, rounds and
+// clamps, stores the next product's A operand; no shared-memory stores, no proxy fence, and the
+// product reads only the weights from shared memory), one barrier per layer, and the next tile's
+// features load while the current tile's hidden layers run.  Features in row order (MAP) come by
+// TMA, two swizzled boxes a tile that the first product reads as they are; listed rows (the
+// renderer's queries) by cp.async, 64 contiguous bytes per row.  2,073,600 rows, us a call: 235
+// through shared memory with the loads in the chain; 140 with the activations in TMEM and cp.async
+// for every tile (its address work and L1 traffic slow the chain: 95 without it); 97 with
+// TMA.  HBM floor 62, the products alone 64.
+template <bool MAP>
 __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t* __restrict__ w16,
                                                                  const uint16_t* __restrict__ feat,
                                                                  const int32_t* __restrict__ rows, int n,
                                                                  const uint32_t* d_n, float* __restrict__ out,
-                                                                 int stride, uint32_t* err) {
+                                                                 int stride, uint32_t* err,
+                                                                 const __grid_constant__ CUtensorMap map_a,
+                                                                 const __grid_constant__ CUtensorMap map_b) {
     if (d_n) n = min(n, (int)*d_n);  // a count produced on the device (at most n)
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int g = threadIdx.x >> 7, row = threadIdx.x & 127, bar_id = 1 + g;
-    uint64_t* mbar = (uint64_t*)(smem + kFwdBar) + g;
-    uint32_t* tslot = (uint32_t*)(smem + kFwdBar + 8 * kFwdGroups);
+    const int g = threadIdx.x >> 7, row = threadIdx.x & 127, lane = threadIdx.x & 31, bar_id = 1 + g;
+    uint64_t* mbar = (uint64_t*)(smem + kFwdBar) + 2 * g;
+    uint64_t* xbar = mbar + 1;  // MAP: the tile's features have arrived
+    uint32_t* tslot = (uint32_t*)(smem + kFwdBar + 16 * kFwdGroups);
+    const uint32_t sbase = smem_u32(smem), buf = fwd_buf(g);
+    const int ntiles = (n + 127) / 128, step = gridDim.x * kFwdGroups;
+    // The features of tile t into the buffer, a warp its 32 rows: each access 8 rows x 64 bytes.
+    // Returns this thread's feature row of the tile (-1: none).
+    auto load_tile = [&](int t) -> long {
+        const long i = (long)t * 128 + row;
+        const bool valid = t < ntiles && i < n;
+        if (MAP) {
+            if (row == 0 && t < ntiles) {
+                mbar_expect(xbar, kFwdTileBytes);  // rows past n arrive as zeros
+                tma_load_2d(sbase + buf, &map_a, 0, t * 128, xbar);
+                tma_load_2d(sbase + buf + 16384, &map_b, 64, t * 128, xbar);
+            }
+            return valid ? i : -1;
+        }
+        const int mine = valid ? (rows ? __ldg(rows + i) : (int)i) : -1;
+        if (t < ntiles) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int sub = 8 * q + (lane & 7), r = __shfl_sync(~0u, mine, sub);
+                const uint32_t dst = sbase + buf + rc_offset((row & ~31) + sub, 0, kMlpIn);
+#pragma unroll
+                for (int j4 = 0; j4 < 3; ++j4) {
+                    const int j = 4 * j4 + (lane >> 3);
+                    cp_async16(dst + 128u * j, feat + (size_t)max(r, 0) * kMlpIn + 8 * j, r >= 0);
+                }
+            }
+        }
+        return mine;
+    };
+    int tile = g * gridDim.x + blockIdx.x;
+    long r = -1;
+    if (row == 0) {
+        mbar_init(mbar, 1);
+        mbar_init(xbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    r = load_tile(tile);
     load_weights(smem, w16);
-    if (row == 0) mbar_init(mbar, 1);
     if ((threadIdx.x >> 5) == 0) tmem_alloc(tslot, kFwdCols);
     publish_smem();
-    const uint32_t tmem = *tslot + 64u * (uint32_t)g;
-    const uint32_t lane_base = (uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16;  // warp w: lanes 32 (w % 4) ..
-    const uint32_t sbase = smem_u32(smem), buf = fwd_buf(g);
-    uint32_t phase = 0;
-    const int ntiles = (n + 127) / 128;
-    for (int tile = blockIdx.x * kFwdGroups + g; tile < ntiles; tile += gridDim.x * kFwdGroups) {
-        const long i = (long)tile * 128 + row;
-        const bool valid = i < n;
-        const long r = valid ? (rows ? (long)__ldg(rows + i) : i) : 0;
-        const uint4* src = (const uint4*)(feat + r * kMlpIn);
-        for (int j = 0; j < kMlpIn / 8; ++j) {
-            const uint4 q = valid ? __ldg(src + j) : make_uint4(0, 0, 0, 0);
-            *(uint4*)(smem + buf + rc_offset(row, 8 * j, kMlpIn)) = q;
-        }
-        wg_publish(bar_id);
-        bool ok = true;
-        for (int L = 0; L < kMlpLayers; ++L) {
-            const int K = mlp_in(L), N = mlp_out(L);
-            if (row == 0) {
-                issue_fwd(tmem, sbase, buf, K, kSW(L), N, K);
-                umma_commit(mbar);
-            }
-            ok = wg_sync_and(bar_id, mbar_wait(mbar, phase, err));  // every thread of the warpgroup agrees
-            phase ^= 1u;
-            tc_fence_after();
-            if (!ok) break;
-            if (L < kMlpLayers - 1) {
-                float v[64];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) tmem_ld16(tmem + lane_base + 16 * q, v + 16 * q);
-#pragma unroll
-                for (int k = 0; k < 64; ++k) v[k] = fmaxf(v[k], 0.0f);
-                rc_store_row(smem + buf, row, 64, v);  // the layer's products have read the buffer
-                wg_publish(bar_id);
+    const uint32_t tmem = *tslot + kFwdTileCols * (uint32_t)g;
+    const uint32_t mine = tmem + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16);  // warp w: lanes 32 (w % 4) ..
+    uint32_t phase = 0, xphase = 0;
+    bool ok = true;  // a wait that runs out sets the error flag and is not repeated; the tile runs through
+    auto product = [&](int L) {  // issue layer L's product and wait for it
+        if (row == 0) {
+            if (L == 0 && MAP) {
+                if (ok) ok = mbar_wait(xbar, xphase, err);
+                const uint32_t idesc = umma_idesc_bf16(128, 64, false, false);
+                for (int s = 0; s < 6; ++s)
+                    umma_bf16(tmem, s < 4 ? umma_desc_swizzled(sbase + buf + 32 * s, 128)
+                                          : umma_desc_swizzled(sbase + buf + 16384 + 32 * (s - 4), 64),
+                              umma_desc(sbase + kSW(0) + s * 256, 128, 16 * kMlpIn), idesc, s > 0);
+            } else if (L == 0) {
+                issue_fwd(tmem, sbase, buf, kMlpIn, kSW(0), 64, kMlpIn);
             } else {
-                float z[16];
-                tmem_ld16(tmem + lane_base, z);
-                if (valid)
-                    for (int c = 0; c < kMlpOut; ++c) out[r * stride + c] = expf(z[c]);
+                const uint32_t idesc = umma_idesc_bf16(128, mlp_out(L), false, false);
+                for (int s = 0; s < 4; ++s)
+                    umma_bf16_ta(tmem, tmem + kFwdACol + 8 * s, umma_desc(sbase + kSW(L) + s * 256, 128, 16 * 64), idesc, s > 0);
             }
+            umma_commit(mbar);
         }
-        if (!ok) break;
-        tc_fence_before();
-        wg_sync(bar_id);  // every row read the output before the next tile's products
+        if (ok) ok = mbar_wait(mbar, phase, err);
+        phase ^= 1u;
+        __syncwarp();  // the lanes leave the wait one by one; the TMEM accesses are warp-wide
         tc_fence_after();
+    };
+    for (; tile < ntiles; tile += step) {
+        // the features are in (cp.async: published here), and every row of the tile before has read its
+        // outputs from TMEM
+        if (!MAP) {
+            cp_async_wait();
+            fence_async_smem();
+        }
+        tc_fence_before();
+        if (!wg_sync_and(bar_id, ok)) {  // a wait ran out: let what is in flight end, as far as it does
+            if (row == 0) {
+                mbar_wait(mbar, phase ^ 1u, err);
+                if (MAP) mbar_wait(xbar, xphase, err);
+            }
+            break;
+        }
+        tc_fence_after();
+        product(0);
+        xphase ^= 1u;
+        const long next = load_tile(tile + step);
+        for (int L = 1; L < kMlpLayers; ++L) {
+            uint32_t v[32], a[32];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                tmem_ld32(mine + 32 * h, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int k = 0; k < 16; ++k) a[16 * h + k] = relu_bf16x2(v[2 * k], v[2 * k + 1]);
+            }
+            tmem_st32(mine + kFwdACol, a);
+            tmem_wait_st();
+            tc_fence_before();
+            wg_sync(bar_id);
+            tc_fence_after();
+            product(L);
+        }
+        float z[16];
+        tmem_ld16(mine, z);
+        if (r >= 0)
+            for (int c = 0; c < kMlpOut; ++c) out[r * stride + c] = expf(z[c]);
+        r = next;
     }
     tc_fence_before();
     __syncthreads();
@@ -517,7 +598,8 @@ std::string Mlp::init(uint32_t seed, cudaStream_t s) {
         TRY(cudaGetDevice(&dev));
         TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         TRY(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
-        TRY(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
+        TRY(cudaFuncSetAttribute(k_mlp_forward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
+        TRY(cudaFuncSetAttribute(k_mlp_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
         blocks_train_ = sms;
         blocks_fwd_ = sms;  // one CTA of kFwdGroups tiles per SM
     }
@@ -572,14 +654,42 @@ std::string Mlp::get_grad(float* host, cudaStream_t s) {
     return "";
 }
 
+namespace {
+// A tensor map of n feature rows in boxes of 128 rows x `cols` columns (false: none could be made,
+// and the kernel copies the rows itself).
+bool feature_map(const uint16_t* d_feat, int n, int cols, CUtensorMapSwizzle swizzle, CUtensorMap* map) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Encode>(f);
+    }();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)kMlpIn, (cuuint64_t)n}, strides[1] = {2 * (cuuint64_t)kMlpIn};
+    const cuuint32_t box[2] = {(cuuint32_t)cols, 128}, one[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(d_feat), dims, strides, box, one,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+}  // namespace
+
 std::string Mlp::forward(const uint16_t* d_feat, int n, float* d_out, uint32_t* d_err, cudaStream_t s,
                          const int32_t* d_rows, int out_stride, const uint32_t* d_n) {
     if (!w32_) return "MLP not initialised";
     if (n <= 0) return "";
     const int tiles = (n + 127) / 128;
-    const int groups = (tiles + kFwdGroups - 1) / kFwdGroups;
-    k_mlp_forward<<<std::min(groups, blocks_fwd_), 128 * kFwdGroups, kFwdSmem, s>>>(e16_, d_feat, d_rows, n, d_n, d_out,
-                                                                                   out_stride, d_err);
+    // features in row order come through tensor maps of this call's buffer (96 columns as 64 + 32)
+    CUtensorMap map_a{}, map_b{};
+    const bool map = !d_rows && feature_map(d_feat, n, 64, CU_TENSOR_MAP_SWIZZLE_128B, &map_a) &&
+                     feature_map(d_feat, n, 32, CU_TENSOR_MAP_SWIZZLE_64B, &map_b);
+    auto k = map ? k_mlp_forward<true> : k_mlp_forward<false>;
+    k<<<std::min(tiles, blocks_fwd_), 128 * kFwdGroups, kFwdSmem, s>>>(e16_, d_feat, d_rows, n, d_n, d_out, out_stride, d_err,
+                                                                      map_a, map_b);
     TRY(cudaGetLastError());
     return "";
 }

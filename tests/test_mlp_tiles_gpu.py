@@ -1,0 +1,46 @@
+"""Radiance-cache inference over tiles, groups and partial tiles, through both feature paths (row
+order by TMA, listed rows by cp.async are the renderer's), against the oracle."""
+import numpy as np
+import pytest
+
+from oracle import mlp_np
+
+pytestmark = pytest.mark.gpu
+
+
+# one row; around a 128-row tile; around one tile on each of 152 SMs; around five tiles in flight per
+# SM (97,280 rows), which makes a warpgroup take a second tile
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 19455, 19457, 97280, 97281, 100003])
+def test_rows(built_lib, n):
+    import lighttransportsimulation_gb300 as lts
+    ctx = lts.Context(0)
+    net = lts.RadianceCacheMLP(ctx, seed=3)
+    rng = np.random.default_rng(n)
+    params = mlp_np.he_init(n)
+    net.set_params(params)
+    feat = mlp_np.bf16_bits(rng.uniform(-1, 1, (n, 96)).astype(np.float32))
+    out = net.forward(feat)
+    ref = mlp_np.forward(params, feat)
+    # the oracle rounds to bf16 where the kernel does; FP32 sums in another order can move an
+    # activation to its other bf16 neighbour (2^-8 relative), a few of 64 inputs of later layers
+    assert np.allclose(out, ref, rtol=2e-2, atol=1e-4)
+    assert np.sqrt(np.mean((out - ref) ** 2)) <= 2e-3 * np.sqrt(np.mean(ref ** 2))
+    ctx.close()
+
+
+def test_nan_and_infinite_features(built_lib):
+    """A NaN pre-activation leaves ReLU as 0, as fmaxf gives; rows beside it are not touched."""
+    import lighttransportsimulation_gb300 as lts
+    ctx = lts.Context(0)
+    net = lts.RadianceCacheMLP(ctx, seed=3)
+    rng = np.random.default_rng(0)
+    feat = mlp_np.bf16_bits(rng.uniform(-1, 1, (256, 96)).astype(np.float32))
+    clean = net.forward(feat)
+    feat[130, 5] = 0x7FC0
+    feat[200, 7] = 0x7F80
+    out = net.forward(feat)
+    keep = np.ones(256, bool)
+    keep[[130, 200]] = False
+    assert np.array_equal(out[keep], clean[keep])
+    assert np.array_equal(out[130], np.ones(3, np.float32))  # every hidden unit 0: exp(0)
+    ctx.close()
