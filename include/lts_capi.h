@@ -310,6 +310,10 @@ int lts_set_option(lts_ctx* ctx, const char* key, int64_t value);
  * distance (INFINITY for none; t may be NULL).  Uses the render BVH of the last render, else
  * builds a sorted-leaf LBVH of the scene. */
 int lts_intersect(lts_ctx* ctx, const float* rays, int32_t n, int32_t any, int32_t* prim, float* t);
+/* The same queries from separate arrays: o, d n x 3 floats (host), tmax one float (tmax_count 1) or
+ * n. */
+int lts_intersect_arrays(lts_ctx* ctx, const float* o, const float* d, const float* tmax, int32_t tmax_count, int32_t n,
+                         int32_t any, int32_t* prim, float* t);
 
 /* Known-answer check of single device functions (no counterpart in the reference: it runs the
  * renderer's float device code on the GPU for values a test compares with the reference's own

@@ -40,7 +40,7 @@ EXPORTS = ["lts_create", "lts_destroy", "lts_last_error", "lts_stream", "lts_rea
            "lts_debug_trace_get", "lts_set_option", "lts_debug_umma_probe", "lts_mlp_init", "lts_mlp_set_params",
            "lts_mlp_get_params", "lts_mlp_forward", "lts_mlp_train_step", "lts_mlp_forward_device_async",
            "lts_mlp_train_step_device_async", "lts_render_views", "lts_autotune_views", "lts_obj_to_bin",
-           "lts_debug_wait_timeout", "lts_debug_kat", "lts_intersect", "lts_scene_get_image",
+           "lts_debug_wait_timeout", "lts_debug_kat", "lts_intersect", "lts_intersect_arrays", "lts_scene_get_image",
            "lts_debug_image_lookup"]
 
 
@@ -141,6 +141,7 @@ def library():
             "lts_debug_wait_timeout": (I, [P, I]),
             "lts_debug_kat": (I, [P, I, P, I, P]),
             "lts_intersect": (I, [P, P, I, I, P, P]),
+            "lts_intersect_arrays": (I, [P, P, P, P, I, I, I, P, P]),
             "lts_scene_get_image": (I, [P, I, I, P, P]),
             "lts_debug_image_lookup": (I, [P, I, P, I, P]),
         }
@@ -251,15 +252,16 @@ class Scene:
         return func[:n], cdf
 
     def _query(self, o, d, tmax, any_hit):
-        o = np.asarray(o, np.float32).reshape(-1, 3)
-        d = np.asarray(d, np.float32).reshape(-1, 3)
+        o = np.ascontiguousarray(o, np.float32).reshape(-1, 3)
         n = len(o)
-        rays = np.zeros((n, 8), np.float32)
-        rays[:, 0:3], rays[:, 4:7] = o, d
-        rays[:, 3] = np.broadcast_to(np.asarray(tmax, np.float32), (n,))
+        d = np.ascontiguousarray(np.broadcast_to(np.asarray(d, np.float32).reshape(-1, 3), (n, 3)))
+        tmax = np.asarray(tmax, np.float32)
+        every = np.broadcast_to(tmax, (n,))
+        tmax = np.ascontiguousarray(tmax if tmax.size == 1 else every)
         prim = np.empty(n, np.int32)
-        t = np.empty(n, np.float32)
-        self.ctx.check(self.ctx.lib.lts_intersect(self.ctx.h, _ptr(rays), n, 1 if any_hit else 0, _ptr(prim), _ptr(t)))
+        t = None if any_hit else np.empty(n, np.float32)
+        self.ctx.check(self.ctx.lib.lts_intersect_arrays(self.ctx.h, _ptr(o), _ptr(d), _ptr(tmax), tmax.size if n else 1, n,
+                                                         1 if any_hit else 0, _ptr(prim), _ptr(t)))
         return prim, t
 
     def intersect(self, o, d, tmax=np.inf):

@@ -82,8 +82,9 @@ struct lts_ctx {
     float* d_tri = nullptr;  // scene triangle soup, 9 floats per triangle (scene order)
     size_t d_tri_cap = 0;
     // kept between calls: the input of lts_bvh_build_triangles, the flattened tree of a dump
-    void *soup_ws = nullptr, *dump_ws = nullptr;
-    size_t soup_ws_cap = 0, dump_ws_cap = 0;
+    // and a batch of ray queries
+    void *soup_ws = nullptr, *dump_ws = nullptr, *ray_ws = nullptr;
+    size_t soup_ws_cap = 0, dump_ws_cap = 0, ray_ws_cap = 0;
     std::unique_ptr<Lbvh> bvh;
     std::unique_ptr<Mlp> mlp;
     int bvh_mode = -1;        // mode of the BVH currently held (-1: none)
@@ -94,7 +95,7 @@ struct lts_ctx {
 
 namespace {
 
-constexpr size_t kDumpKeep = 256ull << 20;
+constexpr size_t kDumpKeep = 256ull << 20;  // most bytes of each workspace kept between calls
 
 int fail(lts_ctx* c, int code, const std::string& msg) {
     if (c) c->err = msg;
@@ -246,6 +247,7 @@ void lts_destroy(lts_ctx* ctx) {
     dev_free(ctx->d_tri);
     dev_free(ctx->soup_ws);
     dev_free(ctx->dump_ws);
+    dev_free(ctx->ray_ws);
     dev_free(ctx->d_error);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -706,9 +708,10 @@ int lts_set_option(lts_ctx* ctx, const char* key, int64_t value) {
     return LTS_OK;
 }
 
-int lts_intersect(lts_ctx* ctx, const float* rays, int32_t n, int32_t any, int32_t* prim, float* t) {
-    if (!ctx || n < 0 || (n > 0 && (!rays || !prim)) || (any != 0 && any != 1) || n > (1 << 28))
-        return fail(ctx, LTS_ERR_ARG, "bad ray query");
+namespace {
+// The two forms of a batch of ray queries: `o` alone (interleaved records), or o, d and tmax.
+int ray_queries(lts_ctx* ctx, const float* o, const float* d, const float* tmax, bool one_tmax, int32_t n, int32_t any,
+                int32_t* prim, float* t) {
     if (ctx->device == -1) return fail(ctx, LTS_ERR_STATE, "host-only context (device -1) cannot run kernels");
     if (!ctx->loaded) return fail(ctx, LTS_ERR_STATE, "no scene loaded");
     CK(cudaSetDevice(ctx->device));
@@ -717,24 +720,53 @@ int lts_intersect(lts_ctx* ctx, const float* rays, int32_t n, int32_t any, int32
         if (rc) return rc;
     }
     if (n == 0) return LTS_OK;
-    unsigned char* d = nullptr;
-    CK(dev_alloc((void**)&d, 32 * (size_t)n + 8 * (size_t)n));
-    float4* d_rays = reinterpret_cast<float4*>(d);
-    int32_t* d_prim = reinterpret_cast<int32_t*>(d + 32 * (size_t)n);
-    float* d_t = reinterpret_cast<float*>(d + 36 * (size_t)n);
-    cudaError_t e = cudaMemcpyAsync(d_rays, rays, 32 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
-    std::string msg = e == cudaSuccess ? ctx->tracer->intersect(*ctx->bvh, d_rays, n, any, d_prim, d_t, ctx->stream,
-                                                                 ctx->d_error)
-                                       : "";
-    if (e == cudaSuccess && msg.empty())
-        e = cudaMemcpyAsync(prim, d_prim, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && msg.empty() && t)
-        e = cudaMemcpyAsync(t, d_t, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && msg.empty()) e = cudaStreamSynchronize(ctx->stream);
-    dev_free(d);
+    // rays, then results; up to kDumpKeep bytes stay with the context
+    const size_t N = (size_t)n, rays = d ? 24 * N + 4 * (one_tmax ? 4 : N) : 32 * N, bytes = rays + 8 * N;
+    unsigned char* ws = static_cast<unsigned char*>(ctx->ray_ws);
+    if (ctx->ray_ws_cap < bytes) {
+        dev_free(ctx->ray_ws);
+        ctx->ray_ws = nullptr;
+        ctx->ray_ws_cap = 0;
+        CK(dev_alloc((void**)&ws, bytes));
+        if (bytes <= kDumpKeep) {
+            ctx->ray_ws = ws;
+            ctx->ray_ws_cap = bytes;
+        }
+    }
+    float* d_o = reinterpret_cast<float*>(ws);
+    float* d_d = d ? d_o + 3 * N : nullptr;
+    float* d_tmax = d ? d_d + 3 * N : nullptr;
+    int32_t* d_prim = reinterpret_cast<int32_t*>(ws + rays);
+    float* d_t = t ? reinterpret_cast<float*>(d_prim + N) : nullptr;
+    cudaError_t e = cudaMemcpyAsync(d_o, o, (d ? 12 : 32) * N, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess && d) e = cudaMemcpyAsync(d_d, d, 12 * N, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess && d) e = cudaMemcpyAsync(d_tmax, tmax, 4 * (one_tmax ? 1 : N), cudaMemcpyHostToDevice, ctx->stream);
+    std::string msg;
+    if (e == cudaSuccess)
+        msg = ctx->tracer->intersect(*ctx->bvh, d_o, d_d, d_tmax, one_tmax, n, any, d_prim, d_t, ctx->stream, ctx->d_error);
+    if (e == cudaSuccess && msg.empty()) e = cudaMemcpyAsync(prim, d_prim, 4 * N, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess && msg.empty() && t) e = cudaMemcpyAsync(t, d_t, 4 * N, cudaMemcpyDeviceToHost, ctx->stream);
+    const cudaError_t se = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess && msg.empty()) e = se;
+    if (ws != ctx->ray_ws) dev_free(ws);
     if (!msg.empty()) return fail(ctx, LTS_ERR_CUDA, msg);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "ray query");
     return check_device_error(ctx);
+}
+}  // namespace
+
+int lts_intersect(lts_ctx* ctx, const float* rays, int32_t n, int32_t any, int32_t* prim, float* t) {
+    if (!ctx || n < 0 || (n > 0 && (!rays || !prim)) || (any != 0 && any != 1) || n > (1 << 28))
+        return fail(ctx, LTS_ERR_ARG, "bad ray query");
+    return ray_queries(ctx, rays, nullptr, nullptr, false, n, any, prim, t);
+}
+
+int lts_intersect_arrays(lts_ctx* ctx, const float* o, const float* d, const float* tmax, int32_t tmax_count, int32_t n,
+                         int32_t any, int32_t* prim, float* t) {
+    if (!ctx || n < 0 || (n > 0 && (!o || !d || !tmax || !prim)) || (any != 0 && any != 1) || n > (1 << 28) ||
+        (n > 0 && tmax_count != 1 && tmax_count != n))
+        return fail(ctx, LTS_ERR_ARG, "bad ray query");
+    return ray_queries(ctx, o, d, tmax, tmax_count == 1, n, any, prim, t);
 }
 
 int lts_debug_kat(lts_ctx* ctx, int32_t fn, const float* in, int32_t n, float* out) {

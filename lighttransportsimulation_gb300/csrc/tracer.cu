@@ -256,26 +256,6 @@ __global__ void k_debug_kat(int fn, const float* __restrict__ in, int n, float* 
     for (int k = 0; k < 16; ++k) out[16 * (size_t)r + k] = o[k];
 }
 
-// Batch ray queries: Scene::intersect (closest hit) or Scene::simpleIntersect (any hit within
-// tMax), one ray per thread, through the renderer's own traversal and triangle tests.
-template <bool ANY>
-__global__ __launch_bounds__(kThreads) void k_intersect(const SceneView sv, int nleaf, const float4* __restrict__ rays,
-                                                        int n, int32_t* __restrict__ prim, float* __restrict__ tout,
-                                                        uint32_t* err) {
-    __shared__ uint32_t s_stack[kStack * kThreads];
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
-    const TraceRay r = make_trace_ray(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z));
-    real tmax = a.w, bu = 0, bv = 0, binv = 0;
-    Work wk{0u, 0u};
-    const int h = sv.ninst ? traverse<ANY, true>(sv, nleaf, r, tmax, bu, bv, binv, s_stack + threadIdx.x, err, wk)
-                           : traverse<ANY>(sv, nleaf, r, tmax, bu, bv, binv, s_stack + threadIdx.x, err, wk);
-    if (!ANY && h >= 0) hit_exact(sv, h, r.o, r.d, tmax, bu, bv, binv);
-    prim[i] = ANY ? (h > 0 ? 1 : 0) : h;
-    if (tout) tout[i] = (!ANY && h >= 0) ? (float)tmax : INFINITY;
-}
-
 }  // namespace
 }  // namespace lts
 
@@ -283,6 +263,119 @@ __global__ __launch_bounds__(kThreads) void k_intersect(const SceneView sv, int 
 
 namespace lts {
 namespace {
+
+// A batch of rays: interleaved {o, tmax, d, -} (tmax null), or arrays of origins, directions and
+// tmax (one, or one per ray).
+struct RayBatch {
+    const float* o;
+    const float* d;
+    const float* tmax;
+    int tmax_stride;  // 0: one tmax for all
+};
+__device__ __forceinline__ void load_ray(const RayBatch& b, int i, V3& o, V3& d, real& tmax) {
+    if (b.tmax) {
+        o = v3(__ldg(b.o + 3 * (size_t)i), __ldg(b.o + 3 * (size_t)i + 1), __ldg(b.o + 3 * (size_t)i + 2));
+        d = v3(__ldg(b.d + 3 * (size_t)i), __ldg(b.d + 3 * (size_t)i + 1), __ldg(b.d + 3 * (size_t)i + 2));
+        tmax = __ldg(b.tmax + (size_t)i * b.tmax_stride);
+    } else {
+        const float4* r = reinterpret_cast<const float4*>(b.o) + 2 * (size_t)i;
+        const float4 p = __ldg(r), q = __ldg(r + 1);
+        o = v3(p.x, p.y, p.z);
+        d = v3(q.x, q.y, q.z);
+        tmax = p.w;
+    }
+}
+// Batch ray queries: Scene::intersect (closest hit) or Scene::simpleIntersect (any hit within
+// tMax), through the renderer's own traversal and triangle tests.
+// k_intersect_wide, the 8-wide flat tree: persistent warps that fetch new rays for lanes whose ray has
+// finished, node visits and triangle tests apart, as the wavefront's trace kernel (1M scattered rays
+// against the 1.3M-triangle displaced sphere: 666 us; a ray per thread, a warp's rays in step,
+// 737).  k_intersect: any other tree, one ray per thread.
+template <bool ANY>
+__global__ __launch_bounds__(kThreads, kTraceMinBlocks) void k_intersect_wide(const SceneView sv, int nleaf, const RayBatch b,
+                                                                              uint32_t n, uint32_t* fetch,
+                                                                              int32_t* __restrict__ prim,
+                                                                              float* __restrict__ tout, uint32_t* err) {
+    __shared__ uint32_t s_stack[kStack * kThreads];
+    uint32_t* stack = s_stack + threadIdx.x;
+    const unsigned lane = threadIdx.x & 31u;
+    Trav t;
+    Work wk{0u, 0u};
+    uint32_t i = 0;
+    bool active = false, exhausted = false;
+    auto finish = [&]() {
+        if (ANY) {
+            prim[i] = t.best == 1 ? 1 : 0;
+            if (tout) tout[i] = INFINITY;
+            return;
+        }
+        const int h = hit_prim(t.best);
+        if (h >= 0) {
+            V3 o, d;
+            real tmax;
+            load_ray(b, (int)i, o, d, tmax);
+            hit_exact(sv, h, o, d, t.tmax, t.bu, t.bv, t.binv);
+        }
+        prim[i] = h;
+        if (tout) tout[i] = h >= 0 ? (float)t.tmax : INFINITY;
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(~0u, !active);
+        if (!exhausted && __popc(idle) >= kRefillIdle) {
+            const uint32_t warps = gridDim.x * (kThreads / 32);
+            const bool spread = n < 32u * warps;  // one equal share per warp (see k_wf_trace)
+            const uint32_t take = spread ? (n + warps - 1u) / warps : (uint32_t)__popc(idle);
+            const int leader = __ffs(idle) - 1;
+            uint32_t base = 0;
+            if ((int)lane == leader) base = atomicAdd(fetch, take);
+            base = __shfl_sync(~0u, base, leader);
+            if (spread || base + take >= n) exhausted = true;
+            const uint32_t pos = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!active && pos < take && base + pos < n) {
+                i = base + pos;
+                V3 o, d;
+                real tmax;
+                load_ray(b, (int)i, o, d, tmax);
+                active = trav_begin(ANY, t, sv, nleaf, o, d, tmax, wk);
+                if (!active) finish();
+            }
+        }
+        if (__ballot_sync(~0u, active) == 0u) {
+            if (exhausted) break;
+            continue;
+        }
+        for (;;) {
+            const bool has_leaf = active && t.lbits != 0u;
+            const bool want_node = active && !has_leaf;
+            const unsigned lm = __ballot_sync(~0u, has_leaf), nm = __ballot_sync(~0u, want_node);
+            const bool leaf_mode = lm != 0u && __popc(lm) * 4 >= __popc(nm) * kLeafBias;
+            if (leaf_mode ? has_leaf : want_node) {
+                const bool fin = leaf_mode ? wide_leaf_step(ANY, t, sv, err, wk) : wide_node_step(ANY, t, sv, stack, err, wk);
+                if (fin) {
+                    finish();
+                    active = false;
+                }
+            }
+            const unsigned act = __ballot_sync(~0u, active);
+            if (act == 0u || (!exhausted && 32 - __popc(act) >= kRefillIdle)) break;
+        }
+    }
+}
+template <bool ANY>
+__global__ __launch_bounds__(kThreads) void k_intersect(const SceneView sv, int nleaf, const RayBatch b, int n,
+                                                        int32_t* __restrict__ prim, float* __restrict__ tout, uint32_t* err) {
+    __shared__ uint32_t s_stack[kStack * kThreads];
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= n) return;
+    V3 o, d;
+    real tmax, bu = 0, bv = 0, binv = 0;
+    load_ray(b, i, o, d, tmax);
+    Work wk{0u, 0u};
+    const int h = traverse<ANY, true>(sv, nleaf, make_trace_ray(o, d), tmax, bu, bv, binv, s_stack + threadIdx.x, err, wk);
+    if (!ANY && h >= 0) hit_exact(sv, h, o, d, tmax, bu, bv, binv);
+    prim[i] = ANY ? (h > 0 ? 1 : 0) : h;
+    if (tout) tout[i] = (!ANY && h >= 0) ? (float)tmax : INFINITY;
+}
 
 static_assert(kWfBlock == kThreads, "wavefront stages share the traversal stack layout");
 
@@ -860,18 +953,32 @@ std::string Tracer::traversal_view(const Lbvh& bvh, cudaStream_t s, uint32_t* d_
     return "";
 }
 
-std::string Tracer::intersect(const Lbvh& bvh, const float4* d_rays, int n, int any, int32_t* d_prim, float* d_t,
-                              cudaStream_t s, uint32_t* d_err) {
+std::string Tracer::intersect(const Lbvh& bvh, const float* d_o, const float* d_d, const float* d_tmax, bool one_tmax, int n,
+                              int any, int32_t* d_prim, float* d_t, cudaStream_t s, uint32_t* d_err) {
     if (bvh.n != view_.ntri) return "bad argument: BVH does not match the scene";
     SceneView sv;
     const std::string e = traversal_view(bvh, s, d_err, &sv);
     if (!e.empty()) return e;
     if (n <= 0) return "";
-    const unsigned grid = (unsigned)((n + kThreads - 1) / kThreads);
-    if (any)
-        k_intersect<true><<<grid, kThreads, 0, s>>>(sv, bvh.n, d_rays, n, d_prim, d_t, d_err);
-    else
-        k_intersect<false><<<grid, kThreads, 0, s>>>(sv, bvh.n, d_rays, n, d_prim, d_t, d_err);
+    const RayBatch batch{d_o, d_d, d_tmax, one_tmax ? 0 : 1};
+    if (sv.wnodes && sv.ninst == 0) {
+        if (isect_grid_ == 0) {
+            int dev = 0, sms = 0, per = 0;
+            TRY(cudaGetDevice(&dev));
+            TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_intersect_wide<false>, kThreads, 0));
+            isect_grid_ = (unsigned)std::max(1, per * sms);
+        }
+        uint32_t* fetch = reinterpret_cast<uint32_t*>(counters_ + 15);  // renders use the words before it
+        TRY(cudaMemsetAsync(fetch, 0, 4, s));
+        const unsigned grid = std::min(isect_grid_, (unsigned)n);
+        auto k = any ? k_intersect_wide<true> : k_intersect_wide<false>;
+        k<<<grid, kThreads, 0, s>>>(sv, bvh.n, batch, (uint32_t)n, fetch, d_prim, d_t, d_err);
+    } else {
+        const unsigned grid = (unsigned)((n + kThreads - 1) / kThreads);
+        auto k = any ? k_intersect<true> : k_intersect<false>;
+        k<<<grid, kThreads, 0, s>>>(sv, bvh.n, batch, n, d_prim, d_t, d_err);
+    }
     TRY(cudaGetLastError());
     return "";
 }

@@ -219,10 +219,11 @@ class Tracer {
     double last_stage_ms[6] = {0, 0, 0, 0, 0, 0};
     double last_kind_work[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 
-    // Batch ray queries (lts_intersect): rays as n x {o.xyz, tmax, d.xyz, 0} on the device; any = 0
-    // closest hit -> prim (-1: none) and t; any = 1 -> prim 1 (occluded) or 0.
-    std::string intersect(const Lbvh& bvh, const float4* d_rays, int n, int any, int32_t* d_prim, float* d_t,
-                          cudaStream_t s, uint32_t* d_err);
+    // Batch ray queries (lts_intersect, lts_intersect_arrays) over device arrays: d_tmax null, d_o
+    // holds n x {o.xyz, tmax, d.xyz, 0}; else d_o, d_d n x 3 and d_tmax one value or n.  any = 0
+    // closest hit -> prim (-1: none) and t; any = 1 -> prim 1 (occluded) or 0.  d_t may be null.
+    std::string intersect(const Lbvh& bvh, const float* d_o, const float* d_d, const float* d_tmax, bool one_tmax, int n,
+                          int any, int32_t* d_prim, float* d_t, cudaStream_t s, uint32_t* d_err);
 
     // n image-texture lookups (Mipmap::lookUp) of image `idx` at d_st[2n] into d_rgb[3n].
     std::string image_lookup(int idx, const float* d_st, int n, float* d_rgb, cudaStream_t s);
@@ -269,6 +270,7 @@ class Tracer {
     int shade_lm_[kShadeClasses] = {0};
     bool matte_only_ = false;  // every material Lambertian / Oren-Nayar with constant textures
     bool shade_tex_[kShadeClasses] = {false};
+    unsigned isect_grid_ = 0;  // resident blocks of the persistent ray-query kernel
     unsigned shade_grid_ = 0;  // resident blocks of the shade kernel on this device
     // side streams and fork / join events: the classes' shade launches run concurrently (as
     // parallel branches of the captured iteration graph)
