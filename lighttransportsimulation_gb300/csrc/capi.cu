@@ -431,7 +431,7 @@ int lts_render(lts_ctx* ctx, const lts_render_desc* desc, lts_render_out* out) {
     }
     std::string e = ctx->tracer->render(ctx->scene, *ctx->bvh, *desc, out, ctx->stream, ctx->d_error);
     if (!e.empty()) return fail(ctx, e.find("argument") != std::string::npos ? LTS_ERR_ARG : LTS_ERR_CUDA, e);
-    int rc = check_device_error(ctx);
+    const int rc = ctx->tracer->last_err ? check_device_error(ctx) : LTS_OK;
     if (rc) return rc;
     ctx->metrics.render_ms = ctx->tracer->last_ms;
     ctx->metrics.paths = ctx->tracer->last_paths;

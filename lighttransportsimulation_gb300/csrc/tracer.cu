@@ -537,7 +537,7 @@ void texture_tables(unsigned char perm512[512], const float** marble30) {
 
 Tracer::~Tracer() {
     free_all();
-    if (wf_counts_host_) cudaFreeHost(wf_counts_host_);
+    if (host_words_) cudaFreeHost(host_words_);
     drop_graphs();
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
@@ -1155,7 +1155,7 @@ std::string Tracer::render_wavefront(const HostScene& sc, const Lbvh& bvh, const
 // render, 2^24 398, all 2^26 paths 421), up to kPoolMax slots and a quarter of the device memory
 // that is free or already held by the pool.
 long Tracer::auto_pool(bool cache) const {
-    constexpr long kPoolMax = 1l << 26, kPoolMin = 1l << 21;
+    constexpr long kPoolMax = 1l << 26;
     const size_t per_slot = kPoolSlotBytes + (cache ? kCacheSlotBytes : 0);
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
@@ -1172,26 +1172,26 @@ long Tracer::auto_pool(bool cache) const {
 // until it drains, then every slice is gathered into its view's film.
 // The shade launch of one class: the kernel variant compiled for its lobes and textures
 // (record mode, the parity runs, uses the general one).
-static std::string launch_shade(bool record, int cls, int lm, bool tex, unsigned grid, const SceneView& sv,
+static std::string launch_shade(bool record, int cls, int lm, bool tex, unsigned grid, unsigned block, const SceneView& sv,
                                 const RenderParams& rp, const WfState& st, int pool, cudaStream_t s) {
     if (record) {
-        k_wf_shade<true, LM_ALL, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        k_wf_shade<true, LM_ALL, true><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     } else if (cls == 0) {
-        k_wf_shade<false, 0, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        k_wf_shade<false, 0, false><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_MATTE) {
-        if (tex) k_wf_shade<false, LM_MATTE, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_MATTE, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_MATTE, true><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_MATTE, false><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_GLASS) {
-        if (tex) k_wf_shade<false, LM_GLASS, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_GLASS, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_GLASS, true><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_GLASS, false><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_MIRROR) {
-        if (tex) k_wf_shade<false, LM_MIRROR, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_MIRROR, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_MIRROR, true><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_MIRROR, false><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     } else if (lm == LM_METAL) {
-        if (tex) k_wf_shade<false, LM_METAL, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
-        else k_wf_shade<false, LM_METAL, false><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        if (tex) k_wf_shade<false, LM_METAL, true><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
+        else k_wf_shade<false, LM_METAL, false><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     } else {
-        k_wf_shade<false, LM_ALL, true><<<grid, kShadeBlock, 0, s>>>(sv, rp, st, pool, cls);
+        k_wf_shade<false, LM_ALL, true><<<grid, block, 0, s>>>(sv, rp, st, pool, cls);
     }
     TRY(cudaGetLastError());
     return "";
@@ -1210,7 +1210,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     if (batch_max >= (1l << 31)) return "wavefront: batch too large";
     const long chunk_total = batch_max;
     const bool cache = cache_mode != 0 && mlp != nullptr && mlp->ready();
-    const long P = std::max<long>(1, std::min<long>(chunk_total, wf_pool > 0 ? wf_pool : auto_pool(cache)));
+    const long P = std::max<long>(1, std::min<long>(chunk_total, wf_pool > 0 ? wf_pool : chunk_total <= kPoolMin ? kPoolMin : auto_pool(cache)));
     // the parameters the wavefront's kernels read; the sampler's are each view's own
     RenderParams rpw{};
     rpw.max_bounce = rp.max_bounce;
@@ -1259,7 +1259,11 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         TRY(dev_alloc(&wf_bufs_[34], 4 * (size_t)chunk_total));
         wf_fs_cap_ = chunk_total;
     }
-    if (!wf_counts_host_) TRY(cudaMallocHost((void**)&wf_counts_host_, kWfCountsBytes + sizeof(WfCtl)));
+    static_assert(sizeof(HostWords::wf) >= kWfCountsBytes + sizeof(WfCtl), "the counts and the control block fit");
+    HostWords* words = nullptr;
+    const std::string pe = pinned(&words);
+    if (!pe.empty()) return pe;
+    uint32_t* const counts_host = reinterpret_cast<uint32_t*>(words->wf);
     void** b = wf_bufs_;
     for (int k = 0; k < kArrays; ++k) *arrays[k].at = b[k];
     st.counts = (uint32_t*)b[kCountsBuf];
@@ -1310,9 +1314,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     }
     auto blocks = [](long n) { return (unsigned)((n + kWfBlock - 1) / kWfBlock); };
     TRY(cudaEventRecord(ev0_, s));
-    TRY(cudaMemsetAsync(st.counts, 0, 128, s));
-    k_wf_init_free<<<blocks(P), kWfBlock, 0, s>>>(st.q_free, st.pend, st.counts, (int)P);  // every slot free
-    TRY(cudaMemsetAsync(st.counts + 32, 0, 8, s));  // training records and eligible vertices of this render
+    k_wf_init_free<<<blocks(P), kWfBlock, 0, s>>>(st.q_free, st.pend, st.counts, (int)P);  // every slot free, counts
     const bool rec = rp.sample_sig != nullptr;
     const bool wide = sv.wnodes != nullptr;
     int iters = 0, launches = 1;
@@ -1347,7 +1349,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     const dim3 gblock(32, 4);
     // control block (device, after the counts) and its host mirror
     WfCtl* d_ctl = (WfCtl*)((unsigned char*)st.counts + kWfCountsBytes);
-    WfCtl* h_ctl = (WfCtl*)((unsigned char*)wf_counts_host_ + kWfCountsBytes);
+    WfCtl* h_ctl = (WfCtl*)((unsigned char*)counts_host + kWfCountsBytes);
     const unsigned list_grid = wf_sms_ * kWfGridPerSm;
     auto launch_iteration = [&](int32_t* q_ext, int32_t* q_fin, bool full, uint32_t take, uint32_t n_ext,
                                 uint32_t n_fin, uint32_t nray, uint32_t n_query) -> std::string {
@@ -1378,14 +1380,17 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         if (full || n_ext) {
             const long tiles = ((full ? P : (long)n_ext) + kClassifyTile - 1) / kClassifyTile;
             k_wf_classify<<<(unsigned)std::min<long>(tiles, list_grid), kWfBlock, 0, s>>>(st, q_ext, d_ctl, (int)P);
-            const unsigned gs = (unsigned)std::min<long>(((full ? P : (long)n_ext) + kShadeBlock - 1) / kShadeBlock, shade_grid_);
+            // a pool too small to give every SM a shade block is shaded in blocks of 128, spread over the
+            // chip
+            const unsigned sb = P < (long)wf_sms_ * kShadeBlock ? 128 : kShadeBlock;
+            const unsigned gs = (unsigned)std::min<long>(((full ? P : (long)n_ext) + sb - 1) / sb, shade_grid_);
             TRY(cudaEventRecord(shade_fork_, s));
             int nb = 0;
             for (int c = 0; c < kShadeClasses; ++c) {
                 if (!shade_used_[c]) continue;
                 cudaStream_t cs = shade_streams_[nb];
                 TRY(cudaStreamWaitEvent(cs, shade_fork_, 0));
-                const std::string le = launch_shade(rec, c, shade_lm_[c], shade_tex_[c], gs, sv, rpw, st, (int)P, cs);
+                const std::string le = launch_shade(rec, c, shade_lm_[c], shade_tex_[c], gs, sb, sv, rpw, st, (int)P, cs);
                 if (!le.empty()) return le;
                 TRY(cudaEventRecord(shade_join_[nb], cs));
                 ++nb;
@@ -1474,9 +1479,9 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
             for (;;) {
                 for (int k = 0; k < group; ++k, par ^= 1) TRY(cudaGraphLaunch(wf_exec_[par], s));
                 launches += group * (st.cache ? 8 : 7);
-                TRY(cudaMemcpyAsync(wf_counts_host_, st.counts, kWfCountsBytes + sizeof(WfCtl), cudaMemcpyDeviceToHost, s));
+                TRY(cudaMemcpyAsync(counts_host, st.counts, kWfCountsBytes + sizeof(WfCtl), cudaMemcpyDeviceToHost, s));
                 TRY(cudaStreamSynchronize(s));
-                const uint32_t* c = wf_counts_host_;
+                const uint32_t* c = counts_host;
                 const bool left = h_ctl->active && (h_ctl->n_ext | c[0] | c[2] | c[3] | c[12] ||
                                                     h_ctl->generated < h_ctl->ctot);
                 if (!left) break;
@@ -1485,7 +1490,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
             }
             iters += (int)h_ctl->iters;
             last_cache_queries += (double)h_ctl->queries;
-            nfree = wf_counts_host_[4];
+            nfree = counts_host[4];
         } else {
             long generated = 0;
             uint32_t n_cont = 0, n_fin = 0, n_sh = 0, n_mis = 0, n_query = 0;
@@ -1500,7 +1505,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
                 if (!ie.empty()) return ie;
                 launches += 7 + (n_query ? 1 : 0);
                 last_cache_queries += n_query;
-                TRY(cudaMemcpyAsync(wf_counts_host_, st.counts, 64, cudaMemcpyDeviceToHost, s));
+                TRY(cudaMemcpyAsync(counts_host, st.counts, 64, cudaMemcpyDeviceToHost, s));
                 TRY(cudaStreamSynchronize(s));
                 for (int k = 0; k < 5; ++k) {
                     float ms = 0;
@@ -1509,11 +1514,11 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
                 }
                 generated += take;
                 n_fin = n_ext;
-                n_cont = wf_counts_host_[0];
-                n_sh = wf_counts_host_[2];
-                n_mis = wf_counts_host_[3];
-                nfree = wf_counts_host_[4];
-                n_query = wf_counts_host_[12];
+                n_cont = counts_host[0];
+                n_sh = counts_host[2];
+                n_mis = counts_host[3];
+                nfree = counts_host[4];
+                n_query = counts_host[12];
                 std::swap(q_ext, q_fin);
             }
             // the last compaction left the counts of an empty pool; the control block follows them
@@ -1528,10 +1533,8 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         }
         TRY(cudaEventRecord(wf_ev_[6], s));
         TRY(cudaGetLastError());
-        TRY(cudaEventSynchronize(wf_ev_[6]));
-        float ms = 0;
-        TRY(cudaEventElapsedTime(&ms, wf_ev_[0], wf_ev_[6]));
-        last_stage_ms[5] += ms;
+        gather_timed_ = true;  // read when the stream has been waited for anyway
+        if (&batch != &batches.back()) settle_gather(true);
     }
     if (cache) {  // train the cache on this render's unbiased suffixes
         const std::string te = train_cache(st.counts, st.tr_feat, st.tr_target, st.tr_cap, s, rp.err);
@@ -1595,16 +1598,41 @@ std::string Tracer::train_cache(uint32_t* d_counts, uint16_t* tr_feat, float* tr
     return "";
 }
 
+void Tracer::settle_gather(bool wait) {
+    float ms = 0;
+    if (gather_timed_ && (!wait || cudaEventSynchronize(wf_ev_[6]) == cudaSuccess) &&
+        cudaEventElapsedTime(&ms, wf_ev_[0], wf_ev_[6]) == cudaSuccess)
+        last_stage_ms[5] += ms;
+    gather_timed_ = false;
+}
+
+std::string Tracer::pinned(HostWords** w) {
+    if (!host_words_) TRY(cudaMallocHost((void**)&host_words_, sizeof(HostWords)));
+    *w = host_words_;
+    return "";
+}
+
 std::string Tracer::render(const HostScene& sc, const Lbvh& bvh, const lts_render_desc& d, lts_render_out* out,
                            cudaStream_t s, uint32_t* d_err) {
     std::string e = render_async(sc, bvh, d, s, d_err);
     if (!e.empty()) return e;
-    TRY(cudaStreamSynchronize(s));
+    // the counters, the error word and the film in one wait
+    HostWords* w = nullptr;
+    if (!(e = pinned(&w)).empty()) return e;
+    TRY(cudaMemcpyAsync(w->counters, counters_, sizeof w->counters, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(&w->err, d_err, 4, cudaMemcpyDeviceToHost, s));
+    if (out && (out->film_rgb || out->film_sums)) {
+        e = film_get(sc, out->film_rgb, out->film_sums, s);
+        if (!e.empty()) return e;
+    } else {
+        TRY(cudaStreamSynchronize(s));
+        settle_gather(false);
+    }
+    last_err = w->err;
     float ms = 0;
     TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
     last_ms = ms;
-    unsigned long long cnt[12] = {0};
-    TRY(cudaMemcpy(cnt, counters_, sizeof cnt, cudaMemcpyDeviceToHost));
+    const unsigned long long* cnt = w->counters;
     for (int k = 0; k < 9; ++k) last_kind_work[k] = (double)cnt[3 + k];
     last_rays = (double)cnt[0];
     last_node_visits = (double)cnt[1];
@@ -1615,10 +1643,6 @@ std::string Tracer::render(const HostScene& sc, const Lbvh& bvh, const lts_rende
         out->rays = rays;
         out->node_visits = last_node_visits;
         out->tri_tests = last_tri_tests;
-        if (out->film_rgb || out->film_sums) {
-            e = film_get(sc, out->film_rgb, out->film_sums, s);
-            if (!e.empty()) return e;
-        }
         if (d.record_samples) {
             const size_t ns = (size_t)last_paths;
             if (out->sample_L) TRY(cudaMemcpy(out->sample_L, rec_L_, 12 * ns, cudaMemcpyDeviceToHost));
@@ -1639,6 +1663,7 @@ std::string Tracer::film_get(const HostScene& sc, float* rgb, double* sums, cuda
     }
     if (sums) TRY(cudaMemcpyAsync(sums, film_, 32 * (size_t)W * H, cudaMemcpyDeviceToHost, s));
     TRY(cudaStreamSynchronize(s));
+    settle_gather(false);
     return "";
 }
 
@@ -1718,6 +1743,7 @@ std::string Tracer::render_views(const HostScene& sc, const Lbvh& bvh, const lts
     if (!e.empty()) return e;
     TRY(cudaStreamSynchronize(s));
     float ms = 0;
+    settle_gather(false);
     TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
     last_ms = ms;
     unsigned long long cnt[12] = {0};

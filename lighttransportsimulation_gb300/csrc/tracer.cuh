@@ -171,6 +171,7 @@ class Tracer {
                              const lts_render_desc& d, float* const* films, lts_render_out* out, cudaStream_t s,
                              uint32_t* d_err);
 
+    uint32_t last_err = 0;  // the device error word as the last render found it
     double last_ms = 0, last_paths = 0, last_rays = 0, last_node_visits = 0, last_tri_tests = 0;
     // Path-pool capacity of the wavefront integrator (0: automatic, see auto_pool).
     long wf_pool = 0;
@@ -303,7 +304,19 @@ class Tracer {
     std::string train_cache(uint32_t* d_counts, uint16_t* tr_feat, float* tr_target, uint32_t tr_cap, cudaStream_t s,
                             uint32_t* d_err);
     long wf_cap_ = 0, wf_fs_cap_ = 0;
-    uint32_t* wf_counts_host_ = nullptr;  // pinned mirror of the counts and the control block
+    // pinned words read back with one wait: the wavefront's counts and control block, a render's
+    // counters and the device error word
+    struct HostWords {
+        alignas(8) unsigned char wf[512];
+        unsigned long long counters[12];
+        uint32_t err;
+    };
+    HostWords* host_words_ = nullptr;
+    std::string pinned(HostWords** w);
+    bool gather_timed_ = false;  // wf_ev_[0] and [6] hold a film gather's time not yet in last_stage_ms[5]
+    void settle_gather(bool wait);
+    // pools of up to this many paths are made whatever memory is free
+    static constexpr long kPoolMin = 1l << 21;
     // the captured wavefront iteration (path rays in q_a, in q_b), kept between renders, and the
     // parameters it was captured with
     cudaGraphExec_t wf_exec_[2] = {nullptr, nullptr};

@@ -603,7 +603,7 @@ __global__ __launch_bounds__(kShadeBlock, 1) void k_wf_shade(const SceneView sv,
                                                                                  WfState st, int pool, int cls) {
     const uint32_t n = st.counts[16 + cls];
     const int32_t* __restrict__ q = st.q_cls + (size_t)cls * pool;
-    for (uint32_t first = blockIdx.x * kShadeBlock; first < n; first += gridDim.x * kShadeBlock) {
+    for (uint32_t first = blockIdx.x * blockDim.x; first < n; first += gridDim.x * blockDim.x) {
         __syncthreads();
         const uint32_t i = first + threadIdx.x;
         if (i < n) shade_one<RECORD, LM, TEX>(sv, rp, st, q[i]);
@@ -720,14 +720,14 @@ __global__ __launch_bounds__(kWfBlock) void k_wf_finalize(const SceneView sv, co
 }
 
 // Every slot starts free (WF_FREE, in the free list in slot order); the counts read as after a
-// compaction of an empty pool (counts zeroed by the host first).
+// compaction of an empty pool.
 __global__ void k_wf_init_free(int32_t* q_free, uint32_t* pend, uint32_t* counts, int n) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) {
         q_free[t] = t;
         pend[t] = WF_FREE;
     }
-    if (t == 0) counts[4] = (uint32_t)n;
+    if (t < kWfCountsBytes / 4) counts[t] = t == 4 ? (uint32_t)n : 0u;
 }
 
 // control: one iteration's sizes from the previous compaction (path rays continuing, shadow and
