@@ -3,18 +3,24 @@
 // multiple-importance weights -- the algorithm of Veach's thesis as PBRT v3 states it (ch. 16.3:
 // random walks with forward / reverse area densities, ConnectBDPT, MISWeight's ratio chain).
 //
-// Three kernels over a chunk of samples:
+// Five kernels over a chunk of samples:
 //   k_bdpt_walk     one thread per sample: both random walks in one loop, the vertices written to
 //                   a structure of arrays in device memory
 //   k_bdpt_connect  one thread per (strategy, sample), the strategy uniform over a block: the
-//                   connection, its shadow ray and its MIS weight
+//                   connection's unweighted contribution and its shadow ray, listed
+//   k_bdpt_shadow   persistent warps over the listed rays (k_bdpt_shadow_any: trees other than the
+//                   8-wide flat one)
+//   k_bdpt_weight   one thread per listed connection: the MIS weight of those that see each other
 //   k_bdpt_film     one thread per sample: the contributions summed in strategy order and filtered
 //                   into the film
 // As one kernel (a thread per pixel with its vertices in local memory) the same work ran at 4.7
 // of 32 lanes and waited on instruction fetch (39.5 stall cycles per issue): lanes were at
 // different strategies of different samples and the body is far larger than the instruction
 // caches.  Here a warp is at one strategy, and a kernel's body is one stage: the box lit by one
-// triangle, 256 x 256, 16 spp, 5 bounces, 81.2 -> 12.0 ms with the same contributions bit for bit.
+// triangle, 256 x 256, 16 spp, 5 bounces, 81.2 -> 12.0 ms with the same contributions bit for bit
+// while the connection still traced its ray and weighted its result (10.5 of 32 lanes, waiting for
+// a warp's longest ray: 1.78 ms a chunk), 8.5 ms with the rays listed
+// (0.41 ms a chunk connecting, 0.25 the rays, 0.31 the weights, beside 1.11 for the walks).
 //
 // The reference ships this integrator disabled and unfinished (intergrators/
 // BidirectionalPathIntegrator.cuh:285-660, LightTransportSimulation.cu:116-121): its light walk
@@ -216,8 +222,14 @@ struct BdptBuf {
                     // connectible camera vertices << 8 (bit 8 + c: vertex c)
     uint32_t* delta;  // per sample: delta camera vertices (bit c), delta light vertices (bit 16 + l)
     float4* contrib;  // [strategy * cap + k]
+    // the connections with a contribution, in list order (count[0] of them): the ray's origin and its
+    // sample, its direction and its strategy | kConnFree (no ray to trace), 1 when it sees
+    float4 *ray_o, *ray_d;
+    uint32_t* sees;
+    uint32_t* count;  // [0] listed, [1] trace fetch
     int cap;
 };
+constexpr uint32_t kConnFree = 256u;
 // The strategies rendered, in the order their contributions are summed (t outer, s inner).
 constexpr int kBdptMaxStrategies = 64;
 struct BdptStrategies {
@@ -587,13 +599,53 @@ __device__ __forceinline__ void bdpt_add_splat(const SceneView& sv, real rx, rea
         }
 }
 
-// ConnectBDPT of strategy (s, t) = strategies[blockIdx.y] for samples first .. first + n - 1.
-constexpr int kBdptConnectBlocks = 4;  // resident blocks per SM the register budget is cut for
-template <int LM, bool WIDE>
-__global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(const SceneView sv, const RenderParams rp, int nleaf,
+// s = 1: the light point sampled from camera vertex pt of strategy (1, t), into qs; false: no light
+// reaches pt from it.
+template <int LM>
+__device__ __forceinline__ bool bdpt_light_point(const SceneView& sv, const RenderParams& rp, const BdptBuf& buf, long first, int k,
+                                                 int t, int only, const BVert& pt, BVert& qs, V3* wi = nullptr) {
+    const uint4 h = __ldg(buf.head + k);
+    // three draws for each connectible camera vertex before this one
+    int i, j, s_ix;
+    bdpt_pixel(rp, first + k, i, j, s_ix);
+    Rng rng;
+    rng.key = rp.seed + wang_hash((uint32_t)(j * sv.width + i));
+    rng.sample = (uint32_t)s_ix;
+    rng.draw = h.z;
+    if (only < 0) rng.draw += 3u * (uint32_t)__popc((h.w >> 8) & ((1u << (t - 1)) - 1u));
+    rng_resume(rng);
+    real lpick;
+    const int li = bdpt_pick_light(sv, rng_1d(rng), lpick);
+    const F2 ul = rng_2d(rng);
+    const DevLight& Lt = sv.lights[li];
+    SI psi;
+    psi.p = pt.p;
+    psi.perr = pt.perr;
+    psi.n = pt.n;
+    LightSample ls;
+    const bool dl = sample_li(sv, Lt, psi, ul, ls);
+    if (!(ls.pdf > 0) || is_black(ls.Li)) return false;
+    qs.type = BV_LIGHT;
+    qs.light = li;
+    qs.p = ls.p1;
+    qs.n = dl ? v3(0, 0, 0) : ls.n1;
+    qs.perr = ls.perr1;
+    qs.beta = ls.Li / (ls.pdf * lpick);
+    qs.pdf_fwd = bv_pdf_light_origin(sv, qs);
+    if (wi) *wi = ls.wi;
+    return true;
+}
+
+// The part of ConnectBDPT before visibility, for strategy (s, t) = strategies[blockIdx.y] and samples
+// first .. first + n - 1.
+// Resident blocks per SM the register budgets are cut for.  The box above: 3, 4 and 5 blocks of the
+// connection and of the weight are within 2 % of each other, 6 and 10 of the rays 1 and 3 % slower
+// than 8; fetching at 8 or 16 idle lanes costs the same as at 12.
+constexpr int kBdptConnectBlocks = 4, kBdptShadowBlocks = 8;
+template <int LM>
+__global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(const SceneView sv, const RenderParams rp,
                                                                                BdptBuf buf, const BdptStrategies st, long first,
-                                                                               int n, int only, double* __restrict__ splat) {
-    __shared__ uint32_t s_stack[kStack * kThreads];
+                                                                               int n, int only) {
     const int k = blockIdx.x * kThreads + threadIdx.x;
     const int s = st.s[blockIdx.y], t = st.t[blockIdx.y];
     const int maxb = min(rp.max_bounce, kBdptMaxBounce);
@@ -603,7 +655,7 @@ __global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(c
     const bool have = in && t <= n_cam && s <= n_light;
     const BCam cam = bdpt_camera(sv);
     Spec c = spec(0.0f);
-    BVert qs, pt, qsm, ptm;
+    BVert qs, pt, ptm;
     real spx = 0, spy = 0, geo = 1;
     bool vis = false;  // the connection needs its shadow ray
     if (have) {
@@ -613,7 +665,6 @@ __global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(c
         else if (t > 2) bv_load<LM>(buf, t - 3, k, ptm);
         if (s == 1) qs = bv_camera(cam);  // resampled below
         else if (s > 1) bv_load<LM>(buf, maxb + s, k, qs);
-        if (s > 1) bv_load<LM>(buf, maxb + s - 1, k, qsm);
         if (s == 0) {  // the camera path's end is on a light
             if (bv_is_light(pt)) c = bv_le(sv, pt, normalize(ptm.p - pt.p)) * pt.beta;
         } else if (t == 1) {  // connect the light path's end to the camera
@@ -632,35 +683,10 @@ __global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(c
             }
         } else if (s == 1) {  // connect the camera path's end to a sampled light point
             if (bv_connectible(pt)) {
-                // three draws for each connectible camera vertex before this one
-                int i, j, s_ix;
-                bdpt_pixel(rp, first + k, i, j, s_ix);
-                Rng rng;
-                rng.key = rp.seed + wang_hash((uint32_t)(j * sv.width + i));
-                rng.sample = (uint32_t)s_ix;
-                rng.draw = h.z;
-                if (only < 0) rng.draw += 3u * (uint32_t)__popc((h.w >> 8) & ((1u << (t - 1)) - 1u));
-                rng_resume(rng);
-                real lpick;
-                const int li = bdpt_pick_light(sv, rng_1d(rng), lpick);
-                const F2 ul = rng_2d(rng);
-                const DevLight& Lt = sv.lights[li];
-                SI psi;
-                psi.p = pt.p;
-                psi.perr = pt.perr;
-                psi.n = pt.n;
-                LightSample ls;
-                const bool dl = sample_li(sv, Lt, psi, ul, ls);
-                if (ls.pdf > 0 && !is_black(ls.Li)) {
-                    qs.type = BV_LIGHT;
-                    qs.light = li;
-                    qs.p = ls.p1;
-                    qs.n = dl ? v3(0, 0, 0) : ls.n1;
-                    qs.perr = ls.perr1;
-                    qs.beta = ls.Li / (ls.pdf * lpick);
-                    qs.pdf_fwd = bv_pdf_light_origin(sv, qs);
+                V3 wi;
+                if (bdpt_light_point<LM>(sv, rp, buf, first, k, t, only, pt, qs, &wi)) {
                     c = pt.beta * bv_f<LM>(pt, qs, false) * qs.beta;
-                    c = c * absdot(ls.wi, pt.f.ns);
+                    c = c * absdot(wi, pt.f.ns);
                     vis = !is_black(c);
                 }
             }
@@ -677,26 +703,141 @@ __global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_connect(c
         }
     }
     // VisibilityTester::unoccluded between the vertices (offset origins as spawnRayTo), from the
-    // camera path's end (t = 1: from the light path's)
-    if (__any_sync(~0u, vis)) {
-        V3 org = v3(0, 0, 0), dir = v3(0, 0, 1);
-        if (vis) {
-            const BVert &a = t == 1 || s >= 2 ? qs : pt, &b = t == 1 || s >= 2 ? pt : qs;
-            org = offset_origin(a.p, a.perr, a.n, b.p - a.p);
-            dir = offset_origin(b.p, b.perr, b.n, org - b.p) - org;
+    // camera path's end (t = 1 and surface connections: from the light path's)
+    const bool keep = have && !is_black(c);
+    const unsigned m = __ballot_sync(~0u, keep);
+    if (m) {
+        const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(buf.count, (uint32_t)__popc(m));
+        base = __shfl_sync(~0u, base, leader);
+        if (keep) {
+            const uint32_t at = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
+            V3 org = v3(0, 0, 0), dir = v3(0, 0, 1);
+            if (vis) {
+                const BVert &a = t == 1 || s >= 2 ? qs : pt, &b = t == 1 || s >= 2 ? pt : qs;
+                org = offset_origin(a.p, a.perr, a.n, b.p - a.p);
+                dir = offset_origin(b.p, b.perr, b.n, org - b.p) - org;
+            }
+            buf.ray_o[at] = make_float4(org.x, org.y, org.z, __int_as_float(k));
+            buf.ray_d[at] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(blockIdx.y | (vis ? 0u : kConnFree)));
+            if (!vis) buf.sees[at] = 1u;
         }
-        Trav tr;
-        Work wk{0u, 0u};
-        warp_rays<true, WIDE>(vis, tr, sv, nleaf, org, dir, 1 - kShadowEps, s_stack + threadIdx.x, rp.err, wk);
-        if (vis) c = tr.best == 1 ? spec(0.0f) : (s >= 2 && t >= 2 ? c * geo : c);
     }
-    if (have && !is_black(c)) {
-        if (only < 0) c = c * bdpt_mis<LM>(sv, cam, buf, k, maxb, s, t, qs, pt, qsm, ptm);
-        if (t == 1) bdpt_add_splat(sv, spx, spy, c, splat);
-    }
-    if (in && t > 1) buf.contrib[(size_t)blockIdx.y * buf.cap + k] = make_float4(c.r, c.g, c.b, 0.f);
+    // geo: what a surface connection that sees is multiplied with
+    if (in) buf.contrib[(size_t)blockIdx.y * buf.cap + k] = keep ? make_float4(c.r, c.g, c.b, geo) : make_float4(0, 0, 0, 0);
     const unsigned tot = __popc(__ballot_sync(~0u, vis));
     if ((threadIdx.x & 31) == 0 && tot && rp.counters) atomicAdd(rp.counters, (unsigned long long)tot);
+}
+
+// The listed rays through the 8-wide flat tree: persistent warps that fetch new rays for lanes whose
+// ray has finished (as the wavefront's trace kernel).
+__global__ __launch_bounds__(kThreads, kBdptShadowBlocks) void k_bdpt_shadow(const SceneView sv, const RenderParams rp, int nleaf, BdptBuf buf) {
+    __shared__ uint32_t s_stack[kStack * kThreads];
+    uint32_t* stack = s_stack + threadIdx.x;
+    const unsigned lane = threadIdx.x & 31u;
+    const uint32_t n = *buf.count;
+    Trav t;
+    Work wk{0u, 0u};
+    uint32_t i = 0;
+    bool active = false, exhausted = false;
+    constexpr int kIdle = 12;  // lanes without a ray that make the warp fetch
+    for (;;) {
+        const unsigned idle = __ballot_sync(~0u, !active);
+        if (!exhausted && __popc(idle) >= kIdle) {
+            const uint32_t take = (uint32_t)__popc(idle);
+            const int leader = __ffs(idle) - 1;
+            uint32_t base = 0;
+            if ((int)lane == leader) base = atomicAdd(buf.count + 1, take);
+            base = __shfl_sync(~0u, base, leader);
+            if (base + take >= n) exhausted = true;
+            i = active ? i : base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!active && i < n) {
+                const float4 d = __ldcs(buf.ray_d + i);
+                if (!(__float_as_uint(d.w) & kConnFree)) {
+                    const float4 o = __ldcs(buf.ray_o + i);
+                    active = trav_begin(true, t, sv, nleaf, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1 - kShadowEps, wk);
+                    if (!active) buf.sees[i] = t.best == 1 ? 0u : 1u;
+                }
+            }
+        }
+        if (__ballot_sync(~0u, active) == 0u) {
+            if (exhausted) break;
+            continue;
+        }
+        for (;;) {
+            const bool has_leaf = active && t.lbits != 0u;
+            const bool want_node = active && !has_leaf;
+            const unsigned lm = __ballot_sync(~0u, has_leaf), nm = __ballot_sync(~0u, want_node);
+            const bool leaf_mode = lm != 0u && __popc(lm) * 4 >= __popc(nm);
+            if (leaf_mode ? has_leaf : want_node) {
+                const bool fin = leaf_mode ? wide_leaf_step(true, t, sv, rp.err, wk) : wide_node_step(true, t, sv, stack, rp.err, wk);
+                if (fin) {
+                    buf.sees[i] = t.best == 1 ? 0u : 1u;
+                    active = false;
+                }
+            }
+            const unsigned act = __ballot_sync(~0u, active);
+            if (act == 0u || (!exhausted && 32 - __popc(act) >= kIdle)) break;
+        }
+    }
+}
+__global__ __launch_bounds__(kThreads) void k_bdpt_shadow_any(const SceneView sv, const RenderParams rp, int nleaf, BdptBuf buf) {
+    __shared__ uint32_t s_stack[kStack * kThreads];
+    const uint32_t n = *buf.count;
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+        const float4 o = buf.ray_o[i], d = buf.ray_d[i];
+        if (__float_as_uint(d.w) & kConnFree) continue;
+        Work wk{0u, 0u};
+        buf.sees[i] = scene_occluded(sv, nleaf, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1 - kShadowEps, s_stack + threadIdx.x, rp.err,
+                                     wk) ? 0u : 1u;
+    }
+}
+
+// The part of ConnectBDPT after visibility: the listed connections that see each other, weighted; t = 1
+// goes to the film where it lands, the others stay for k_bdpt_film.
+template <int LM>
+__global__ __launch_bounds__(kThreads, kBdptConnectBlocks) void k_bdpt_weight(const SceneView sv, const RenderParams rp, BdptBuf buf,
+                                                                              const BdptStrategies st, long first, int only,
+                                                                              double* __restrict__ splat) {
+    const uint32_t n = *buf.count;
+    const int maxb = min(rp.max_bounce, kBdptMaxBounce);
+    const BCam cam = bdpt_camera(sv);
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+        const int k = __float_as_int(buf.ray_o[i].w);
+        const uint32_t q = __float_as_uint(buf.ray_d[i].w) & (kConnFree - 1u);
+        float4* const slot = buf.contrib + (size_t)q * buf.cap + k;
+        if (!buf.sees[i]) {
+            *slot = make_float4(0, 0, 0, 0);
+            continue;
+        }
+        const int s = st.s[q], t = st.t[q];
+        const float4 c4 = *slot;
+        Spec c{c4.x, c4.y, c4.z};
+        if (s >= 2 && t >= 2) c = c * c4.w;
+        BVert qs, pt, qsm, ptm;
+        real spx = 0, spy = 0;
+        if (t == 1) pt = bv_camera(cam);
+        else bv_load<LM>(buf, t - 2, k, pt);
+        if (t == 2) ptm = bv_camera(cam);
+        else if (t > 2) bv_load<LM>(buf, t - 3, k, ptm);
+        if (s == 1) {
+            qs = bv_camera(cam);
+            bdpt_light_point<LM>(sv, rp, buf, first, k, t, only, pt, qs);
+        }
+        if (s > 1) bv_load<LM>(buf, maxb + s, k, qs);
+        if (s > 1) bv_load<LM>(buf, maxb + s - 1, k, qsm);
+        if (!is_black(c) && only < 0) c = c * bdpt_mis<LM>(sv, cam, buf, k, maxb, s, t, qs, pt, qsm, ptm);
+        if (t == 1) {
+            real cos_c;
+            const V3 d = cam.o - qs.p;
+            const V3 wi = d * xsqrt(1 / len2(d));
+            bdpt_raster(cam, -wi, spx, spy, cos_c);
+            if (!is_black(c)) bdpt_add_splat(sv, spx, spy, c, splat);
+        } else {
+            *slot = make_float4(c.r, c.g, c.b, 0.f);
+        }
+    }
 }
 
 __global__ __launch_bounds__(kThreads) void k_bdpt_film(const SceneView sv, const RenderParams rp, BdptBuf buf,

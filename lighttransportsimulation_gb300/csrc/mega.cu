@@ -357,11 +357,11 @@ static_assert((kBdptMaxBounce + 2) * (kBdptMaxBounce + 3) / 2 + kBdptMaxBounce <
 
 size_t bdpt_sample_bytes(int max_bounce, int strategy) {
     const int maxb = std::min(max_bounce, kBdptMaxBounce);
-    return (size_t)(2 * maxb + 2) * (16 * kBvWordsAll + 8) + 16 * (size_t)bdpt_strategies(maxb, strategy).n + 20;
+    return (size_t)(2 * maxb + 2) * (16 * kBvWordsAll + 8) + (16 + 36) * (size_t)bdpt_strategies(maxb, strategy).n + 20;
 }
 
 std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
-                        bool matte_only, void* ws, long cap, cudaStream_t s) {
+                        bool matte_only, void* ws, long cap, uint32_t* d_count, cudaStream_t s) {
     const int maxb = std::min(rp.max_bounce, kBdptMaxBounce);
     const BdptStrategies st = bdpt_strategies(maxb, strategy);
     const bool wide = sv.wnodes != nullptr && sv.ninst == 0;
@@ -371,16 +371,31 @@ std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, 
     buf.vert = static_cast<uint4*>(ws);
     buf.head = buf.vert + slots * words * cap;
     buf.contrib = reinterpret_cast<float4*>(buf.head + cap);
-    buf.pdf = reinterpret_cast<float2*>(buf.contrib + (size_t)st.n * cap);
+    buf.ray_o = buf.contrib + (size_t)st.n * cap;
+    buf.ray_d = buf.ray_o + (size_t)st.n * cap;
+    buf.pdf = reinterpret_cast<float2*>(buf.ray_d + (size_t)st.n * cap);
     buf.delta = reinterpret_cast<uint32_t*>(buf.pdf + slots * cap);
+    buf.sees = buf.delta + cap;
+    buf.count = d_count;
     const long total = (long)(rp.x1 - rp.x0) * (rp.y1 - rp.y0) * rp.spp;
+    int dev = 0, sms = 0;
+    TRY(cudaGetDevice(&dev));
+    TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     for (long first = 0; first < total; first += cap) {
         const int n = (int)std::min(cap, total - first);
         const unsigned gw = (unsigned)((n + kBdptWalkThreads - 1) / kBdptWalkThreads), gs = (unsigned)((n + kThreads - 1) / kThreads);
         auto kw = !wide ? k_bdpt_walk<LM_ALL, true, false> : matte_only ? k_bdpt_walk<LM_MATTE, false, true> : k_bdpt_walk<LM_ALL, true, true>;
-        auto kc = !wide ? k_bdpt_connect<LM_ALL, false> : matte_only ? k_bdpt_connect<LM_MATTE, true> : k_bdpt_connect<LM_ALL, true>;
+        const bool matte = wide && matte_only;
         kw<<<gw, kBdptWalkThreads, 0, s>>>(sv, rp, nleaf, buf, first, n);
-        if (st.n > 0) kc<<<dim3(gs, (unsigned)st.n), kThreads, 0, s>>>(sv, rp, nleaf, buf, st, first, n, strategy, splat);
+        if (st.n > 0) {
+            TRY(cudaMemsetAsync(buf.count, 0, 8, s));
+            auto kc = matte ? k_bdpt_connect<LM_MATTE> : k_bdpt_connect<LM_ALL>;
+            kc<<<dim3(gs, (unsigned)st.n), kThreads, 0, s>>>(sv, rp, buf, st, first, n, strategy);
+            auto ks = wide ? k_bdpt_shadow : k_bdpt_shadow_any;
+            ks<<<kBdptShadowBlocks * sms, kThreads, 0, s>>>(sv, rp, nleaf, buf);
+            auto kt = matte ? k_bdpt_weight<LM_MATTE> : k_bdpt_weight<LM_ALL>;
+            kt<<<kBdptConnectBlocks * 4 * sms, kThreads, 0, s>>>(sv, rp, buf, st, first, strategy, splat);
+        }
         k_bdpt_film<<<gs, kThreads, 0, s>>>(sv, rp, buf, st, n);
         TRY(cudaGetLastError());
     }

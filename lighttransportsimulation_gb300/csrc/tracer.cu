@@ -1087,7 +1087,7 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     long bdpt_cap = 0;
     if (d.integrator == LTS_INTEGRATOR_BDPT) {
         // one chunk's workspace, kept: 2^18 samples keep every SM busy over the chunk's launches
-        // (0.5 GB at five bounces); fewer when that much cannot be allocated
+        // (0.9 GB at five bounces); fewer when that much cannot be allocated
         const size_t per = bdpt_sample_bytes(d.max_bounce, bdpt_strategy);
         bdpt_cap = std::min<long>((ns + 31) / 32 * 32, 1l << 18);
         while (bdpt_ws_cap_ < per * bdpt_cap) {
@@ -1106,7 +1106,8 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     }
     TRY(cudaEventRecord(ev0_, s));
     if (d.integrator == LTS_INTEGRATOR_FP64) e = render64_launch(sv, rp, bvh.n, d.record_samples != 0, s);
-    else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, bdpt_ws_, bdpt_cap, s);
+    else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, bdpt_ws_, bdpt_cap,
+                                                                   reinterpret_cast<uint32_t*>(counters_ + 13), s);
     else e = mega_launch(sv, rp, bvh.n, d.record_samples != 0, matte_only_, s);
     if (!e.empty()) return e;
     TRY(cudaEventRecord(ev1_, s));

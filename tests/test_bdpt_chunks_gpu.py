@@ -54,3 +54,21 @@ def test_strategies_one_by_one(tmp_path):
     b = film(s, 8, 1, strategy=2)["film_sums"]
     assert np.array_equal(a, b) and a[..., :3].max() > 0
     ctx.close()
+
+
+@pytest.mark.parametrize("level,spp", [(0, 1), (2, 5)])
+def test_shadow_rays_by_either_tree(tmp_path, level, spp):
+    """The listed shadow rays through the 8-wide tree (fetched by persistent warps) and through the binary one (a
+    stride loop) see the same, so the films are equal up to the splats' summation order."""
+    sc, sub = scenes.write_tri_light_box(str(tmp_path), level=level)
+    films = []
+    for width in (8, 2):
+        ctx = lts.Context(0)
+        s = lts.Scene.parse(ctx, str(tmp_path), sc, sub, 37, 23)
+        ctx.set_option("bvh_width", width)
+        r = film(s, spp, 4)
+        films.append((r["film_sums"], ctx.metrics().rays))
+        ctx.close()
+    (a, na), (b, nb) = films
+    assert na == nb > 37 * 23 * spp and a[..., :3].max() > 0
+    assert np.all(np.abs(a - b) <= 1e-12 * max(1.0, np.abs(a).max()))
