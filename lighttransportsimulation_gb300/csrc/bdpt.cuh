@@ -766,16 +766,9 @@ __global__ __launch_bounds__(kThreads, kBdptShadowBlocks) void k_bdpt_shadow(con
             continue;
         }
         for (;;) {
-            const bool has_leaf = active && t.lbits != 0u;
-            const bool want_node = active && !has_leaf;
-            const unsigned lm = __ballot_sync(~0u, has_leaf), nm = __ballot_sync(~0u, want_node);
-            const bool leaf_mode = lm != 0u && __popc(lm) * 4 >= __popc(nm);
-            if (leaf_mode ? has_leaf : want_node) {
-                const bool fin = leaf_mode ? wide_leaf_step(true, t, sv, rp.err, wk) : wide_node_step(true, t, sv, stack, rp.err, wk);
-                if (fin) {
-                    buf.sees[i] = t.best == 1 ? 0u : 1u;
-                    active = false;
-                }
+            if (wide_warp_step(true, active, t, sv, stack, rp.err, wk)) {
+                buf.sees[i] = t.best == 1 ? 0u : 1u;
+                active = false;
             }
             const unsigned act = __ballot_sync(~0u, active);
             if (act == 0u || (!exhausted && 32 - __popc(act) >= kIdle)) break;

@@ -171,15 +171,8 @@ __device__ __forceinline__ bool shade_scatter(const SceneView& sv, const RenderP
 __device__ __forceinline__ void trace_warp(const bool any, bool active, Trav& t, const SceneView& sv, uint32_t* stack,
                                            uint32_t* err, Work& wk) {
     for (;;) {
-        const bool has_leaf = active && t.lbits != 0u;
-        const bool want_node = active && !has_leaf;
-        const unsigned lm = __ballot_sync(~0u, has_leaf), nm = __ballot_sync(~0u, want_node);
-        if ((lm | nm) == 0u) return;
-        const bool leaf_mode = lm != 0u && __popc(lm) * 4 >= __popc(nm);
-        if (leaf_mode ? has_leaf : want_node) {
-            const bool fin = leaf_mode ? wide_leaf_step(any, t, sv, err, wk) : wide_node_step(any, t, sv, stack, err, wk);
-            if (fin) active = false;
-        }
+        if (__ballot_sync(~0u, active) == 0u) return;
+        if (wide_warp_step(any, active, t, sv, stack, err, wk)) active = false;
     }
 }
 

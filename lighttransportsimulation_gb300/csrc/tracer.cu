@@ -345,16 +345,9 @@ __global__ __launch_bounds__(kThreads, kTraceMinBlocks) void k_intersect_wide(co
             continue;
         }
         for (;;) {
-            const bool has_leaf = active && t.lbits != 0u;
-            const bool want_node = active && !has_leaf;
-            const unsigned lm = __ballot_sync(~0u, has_leaf), nm = __ballot_sync(~0u, want_node);
-            const bool leaf_mode = lm != 0u && __popc(lm) * 4 >= __popc(nm) * kLeafBias;
-            if (leaf_mode ? has_leaf : want_node) {
-                const bool fin = leaf_mode ? wide_leaf_step(ANY, t, sv, err, wk) : wide_node_step(ANY, t, sv, stack, err, wk);
-                if (fin) {
-                    finish();
-                    active = false;
-                }
+            if (wide_warp_step(ANY, active, t, sv, stack, err, wk)) {
+                finish();
+                active = false;
             }
             const unsigned act = __ballot_sync(~0u, active);
             if (act == 0u || (!exhausted && 32 - __popc(act) >= kRefillIdle)) break;

@@ -487,7 +487,8 @@ struct Trav {
     int best;  // closest: primitive (-1 none); any: 1 on a hit
     int node, sp;
     uint32_t gbase, gbits;
-    uint32_t lbits, lbase;  // split steps: the last node's pending triangles (bit k: triangle lbase + k)
+    uint32_t lbits, lbase;  // split steps: a node's pending triangles (bit k: triangle lbase + k)
+    uint32_t lbits2, lbase2;  // and those of a node visited ahead of them
     // two-level BVH: the instance being traversed (-1: the top-level tree, whose ray is the world
     // ray) and the instances whose world boxes the ray enters, still to visit
     int inst;
@@ -506,8 +507,8 @@ __device__ __forceinline__ bool trav_begin(const bool any, Trav& t, const SceneV
     t.sp = 0;
     t.gbase = 0;
     t.gbits = 0;
-    t.lbits = 0;
-    t.lbase = 0;
+    t.lbits = t.lbits2 = 0;
+    t.lbase = t.lbase2 = 0;
     t.inst = -1;
     t.imask = 0;
     real te;
@@ -688,12 +689,13 @@ __device__ __forceinline__ bool trav_step_wide(const bool any, Trav& t, const Sc
     return false;
 }
 
-// The same node visit split in two (the wavefront trace kernel): wide_node_step tests the child
-// boxes and leaves the node's hit leaves pending in t.lbits instead of testing them; then
-// wide_leaf_step tests them one triangle per call before the next node step.  Per ray the order
-// of box and triangle tests is trav_step_wide's, so the hits are the same; a warp can run the
-// triangle tests of all its lanes together instead of inside divergent node steps.  Both
-// return true when the traversal has finished.
+// The same node visit split in two (the kernels whose warps step together): wide_node_step tests
+// the child boxes and leaves the node's hit leaves pending in t.lbits instead of testing them;
+// wide_leaf_step tests them one triangle per call.  A warp can run the triangle tests of all its
+// lanes together instead of inside divergent node steps.  One node may be visited ahead of pending
+// triangles; its own wait behind them (t.lbits2).  So per ray the triangles come in
+// trav_step_wide's order, and those it would not have tested lie behind the closest hit: the hits
+// are the same.  Both return true when the traversal has finished.
 __device__ __forceinline__ bool wide_node_step(const bool any, Trav& t, const SceneView& sv, uint32_t* stack,
                                                uint32_t* err, Work& wk, const bool inst = false) {
     if ((unsigned)t.node >= (unsigned)sv.wcount) {
@@ -749,8 +751,14 @@ __device__ __forceinline__ bool wide_node_step(const bool any, Trav& t, const Sc
         }
     }
     if (leaves) {
-        t.lbits = leaf_tri_bits(leaves, m.w);
-        t.lbase = m.y;
+        const uint32_t tb = leaf_tri_bits(leaves, m.w);
+        if (!inst && t.lbits) {
+            t.lbits2 = tb;
+            t.lbase2 = m.y;
+        } else {
+            t.lbits = tb;
+            t.lbase = m.y;
+        }
     }
     if (hits) {
         if (t.gbits & 0xffu) {
@@ -796,7 +804,32 @@ __device__ __forceinline__ bool wide_leaf_step(const bool any, Trav& t, const Sc
         t.best = 1;
         return true;
     }
+    if (!inst && t.lbits == 0u) {
+        t.lbits = t.lbits2;
+        t.lbase = t.lbase2;
+        t.lbits2 = 0u;
+    }
     return t.lbits == 0u && t.node < 0;
+}
+
+// One step of a warp (all lanes call): the step that more of its lanes can take -- a triangle of
+// those with pending triangles, a node of those that have one to visit and not yet visited one
+// ahead.  True for a lane whose ray has finished.  Without the node ahead a lane waited for the
+// other kind of step as soon as it hit a leaf, and the triangles had to be run at a quarter of the
+// lanes that wanted a node: trace stages of the stress scene (2.4M triangles, 1920 x 1080, 64 spp)
+// 104.2 -> 99.4 ms and the displaced sphere (1.3M, 1024 x 1024, 64 spp) 78.1 -> 73.6; in ms for the
+// first, the other rules tried: triangles already at half or a
+// quarter of the node lanes: 100.2 and 102.6; only at one and a half times or twice: 105.4 and
+// 111.2; two nodes ahead spill (147); shadow rays without the node ahead: 101.9.  Rays through
+// instances visit no node ahead and run triangles from a quarter of the lanes on: their state fills
+// the registers, and the pair more made the stress frame of instances 202 -> 264 ms.
+__device__ __forceinline__ bool wide_warp_step(const bool any, const bool active, Trav& t, const SceneView& sv,
+                                               uint32_t* stack, uint32_t* err, Work& wk, const bool inst = false) {
+    const bool leaf = active && t.lbits != 0u, node = active && (inst ? !leaf : t.node >= 0 && t.lbits2 == 0u);
+    const int nl = __popc(__ballot_sync(~0u, leaf)), nn = __popc(__ballot_sync(~0u, node));
+    const bool leaf_mode = inst ? nl != 0 && 4 * nl >= nn : nl >= nn;
+    if (!(leaf_mode ? leaf : node)) return false;
+    return leaf_mode ? wide_leaf_step(any, t, sv, err, wk, inst) : wide_node_step(any, t, sv, stack, err, wk, inst);
 }
 
 #endif  // !LTS_FP64

@@ -292,10 +292,6 @@ __device__ __forceinline__ void wf_ray_end(int kind, const Trav& t, const SceneV
 #define LTS_REFILL_IDLE 12 // idle lanes of a warp that trigger fetching new rays
 #endif
 constexpr int kRefillIdle = LTS_REFILL_IDLE;
-#ifndef LTS_LEAF_BIAS
-#define LTS_LEAF_BIAS 1  // leaf steps when lanes with pending leaves x 4 >= lanes due a node x this
-#endif
-constexpr int kLeafBias = LTS_LEAF_BIAS;
 // Resident blocks per SM the trace kernel is compiled for (caps its registers): 8 blocks = 32
 // warps at 64 registers without spills; the kernel waits on node and triangle loads, and the
 // extra warps hide them (stress scene: trace 420 ms per render at 8, 444 at 7, 484 at 6; 9 and
@@ -371,18 +367,8 @@ __global__ __launch_bounds__(kWfBlock, kTraceMinBlocks) void k_wf_trace(const Sc
         for (;;) {
             bool fin = false;
             if (WIDE) {
-                // lanes with pending leaf triangles and lanes due a node visit: the warp runs
-                // whichever step more of its lanes wait for
-                const bool has_leaf = active && t.lbits != 0u;
-                const bool want_node = active && !has_leaf;
-                const unsigned lm = __ballot_sync(~0u, has_leaf), nm = __ballot_sync(~0u, want_node);
-                const bool leaf_mode = lm != 0u && __popc(lm) * 4 >= __popc(nm) * kLeafBias;
-                if (leaf_mode ? has_leaf : want_node) {
-                    const bool any = kind == TR_SHADOW;
-                    fin = leaf_mode ? wide_leaf_step(any, t, sv, rp.err, cur, INST)
-                                    : wide_node_step(any, t, sv, stack, rp.err, cur, INST);
-                    if (INST && fin && wf_ray_next_instance(kind, t, sv, st, p)) fin = false;
-                }
+                fin = wide_warp_step(kind == TR_SHADOW, active, t, sv, stack, rp.err, cur, INST);
+                if (INST && fin && wf_ray_next_instance(kind, t, sv, st, p)) fin = false;
             } else if (active) {
                 fin = trav_step_binary(kind == TR_SHADOW, t, sv, stack, rp.err, cur);
             }
