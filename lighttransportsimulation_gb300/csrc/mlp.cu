@@ -13,6 +13,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cmath>
+#include <cstring>
 
 namespace lts {
 namespace {
@@ -84,18 +85,21 @@ __global__ __launch_bounds__(128) void k_umma_probe(const uint16_t* __restrict__
 
 
 // ------------------------------------------------------------------ the radiance-cache MLP
-// Shared memory (bytes).  Weights in RC layout: W0 64x96, W1..W4 64x64, W5 16x64; the input
-// tile X (128 x 96), hidden activations H1..H5 (128 x 64 each),
-// the output-gradient tile Gz (128 x 16) and one hidden-gradient tile Ga (128 x 64).  MN-major
+// Shared memory (bytes).  Weights in RC layout: W0 64x96, W1..W4 64x64, W5 16x64; two input
+// tiles X (128 x 96: this tile's and the next one's), hidden activations H1..H5 (128 x 64 each),
+// the output-gradient tile Gz (128 x 16) and two hidden-gradient tiles Ga (128 x 64).  MN-major
 // reads of a 64- or 96-column buffer with M = 128 run past its end into the next buffer; those
 // product rows are never used.
 __host__ __device__ constexpr uint32_t kSW(int L) { return L == 0 ? 0u : 12288u + 8192u * (uint32_t)(L - 1); }
 constexpr uint32_t kSX = 47104;
-constexpr uint32_t kSH = kSX + 24576;
+constexpr uint32_t kSH = kSX + 2 * 24576;
 constexpr uint32_t kSGz = kSH + 5 * 16384;
 constexpr uint32_t kSGa = kSGz + 4096;
-constexpr uint32_t kTrainBar = kSGa + 16384;
+constexpr uint32_t kTrainBar = kSGa + 2 * 16384;
 constexpr uint32_t kTrainSmem = kTrainBar + 64;
+// Eight warps, two per 32 rows (columns 0..31 and 32..63), and one warp that issues the products.
+constexpr int kTrainThreads = 288;
+static_assert(kTrainSmem <= 232448, "training tile exceeds shared memory");
 // Inference keeps kFwdGroups tiles in flight per CTA (one CTA per SM), one warpgroup of 128
 // threads per tile, sharing the weights: each tile has a 24 KB buffer at fwd_buf(g) for its features
 // X (128 x 96), an mbarrier and 96 TMEM columns -- the product D (128 x 64 FP32) and, as the next
@@ -112,41 +116,51 @@ static_assert(kFwdTileCols * kFwdGroups <= kFwdCols && kFwdSmem <= 232448, "infe
 // TMEM columns: 0..63 the working product; dW_k^T accumulators (training) at kDwCol(k)
 __host__ __device__ constexpr uint32_t kDwCol(int L) { return 64u * (uint32_t)(L + 1); }
 
+// Two floats to one word of two bf16, a in the low half.
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) |
-           ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
 }
-__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-
-// Row `row` of an R x C RC-layout buffer, C a multiple of 8: store / load n = C values.
-__device__ __forceinline__ void rc_store_row(unsigned char* buf, int row, int C, const float* v) {
-    for (int j = 0; j < C / 8; ++j) {
-        const uint4 q = make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]),
-                                   pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
-        *(uint4*)(buf + rc_offset(row, 8 * j, C)) = q;
-    }
+// And ReLU: rounded first, then clamped (the same values; NaN becomes 0 as by fmaxf).
+__device__ __forceinline__ uint32_t relu_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r = pack_bf16x2(__uint_as_float(a), __uint_as_float(b));
+    asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+    return r;
 }
-__device__ __forceinline__ void rc_load_row(const unsigned char* buf, int row, int C, float* v) {
-    for (int j = 0; j < C / 8; ++j) {
-        const uint4 q = *(const uint4*)(buf + rc_offset(row, 8 * j, C));
-        v[8 * j] = bf16_lo(q.x); v[8 * j + 1] = bf16_hi(q.x);
-        v[8 * j + 2] = bf16_lo(q.y); v[8 * j + 3] = bf16_hi(q.y);
-        v[8 * j + 4] = bf16_lo(q.z); v[8 * j + 5] = bf16_hi(q.z);
-        v[8 * j + 6] = bf16_lo(q.w); v[8 * j + 7] = bf16_hi(q.w);
-    }
+// All ones in the halves of w that are > 0.
+__device__ __forceinline__ uint32_t positive_bf16x2(uint32_t w) {
+    __nv_bfloat162 v;
+    memcpy(&v, &w, 4);
+    return __hgt2_mask(v, __floats2bfloat162_rn(0.f, 0.f));
 }
 
-// Weights (global, bf16 row-major [out][in]) into their RC slots.
-__device__ void load_weights(unsigned char* smem, const uint16_t* __restrict__ w16) {
-    for (int L = 0; L < kMlpLayers; ++L) {
-        const int R = mlp_out(L), C = mlp_in(L);
-        const uint4* src = (const uint4*)(w16 + mlp_offset(L));
-        for (int e = threadIdx.x; e < R * C / 8; e += blockDim.x) {
-            const int r = e / (C / 8), j = e % (C / 8);
-            *(uint4*)(smem + kSW(L) + rc_offset(r, 8 * j, C)) = __ldg(src + e);
-        }
+// Row `row` of an R x C RC-layout buffer: store / load the 8 NJ values (two to a word) from column c0 on.
+template <int NJ>
+__device__ __forceinline__ void rc_store_row(unsigned char* buf, int row, int C, int c0, const uint32_t* v) {
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+        *(uint4*)(buf + rc_offset(row, c0 + 8 * j, C)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+template <int NJ>
+__device__ __forceinline__ void rc_load_row(const unsigned char* buf, int row, int C, int c0, uint32_t* v) {
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        const uint4 q = *(const uint4*)(buf + rc_offset(row, c0 + 8 * j, C));
+        v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
     }
+}
+
+// Weights (global, bf16 row-major [out][in]) into their RC slots: every copy of a thread in flight
+// at once (a loop per layer paid the latency per layer), landed on return.
+__device__ void load_weights(uint32_t sbase, const uint16_t* __restrict__ w16) {
+    for (int e = threadIdx.x; e < kMlpParams / 8; e += blockDim.x) {
+        int L = 0, f = e;
+        if (e >= 768) L = 1 + (e - 768) / 512, f = (e - 768) % 512;  // W0 64 x 96, the others 64 (16) x 64
+        const int C = mlp_in(L), r = f / (C / 8), j = f % (C / 8);
+        cp_async16(sbase + kSW(L) + rc_offset(r, 8 * j, C), w16 + 8 * e, true);
+    }
+    cp_async_wait();
 }
 
 // All threads: makes the shared-memory operands written so far visible to the tensor cores.
@@ -167,52 +181,6 @@ __device__ __forceinline__ void issue_fwd(uint32_t tmem_d, uint32_t sbase, uint3
                   umma_desc(sbase + w_off + s * 256, 128, 16 * K), idesc, s > 0);
 }
 
-// 64 columns of this thread's TMEM lane starting at column c0.
-__device__ __forceinline__ void tmem_row64(uint32_t tmem, int c0, float* v) {
-    const uint32_t lane_base = (uint32_t)(32 * (threadIdx.x >> 5)) << 16;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) tmem_ld16(tmem + lane_base + c0 + 16 * q, v + 16 * q);
-}
-
-// Forward pass of one 128-row training tile whose features are already in X; leaves the hidden
-// activations H1..H5 in their slots (the backward pass reads them) and returns z (16 values).
-__device__ bool mlp_forward_tile(unsigned char* smem, uint32_t tmem, uint64_t* mbar, uint32_t& phase, uint32_t* err,
-                                 float* z) {
-    const uint32_t sbase = smem_u32(smem);
-    const int row = threadIdx.x;
-    float v[64];
-    for (int L = 0; L < kMlpLayers; ++L) {
-        const uint32_t a_off = L == 0 ? kSX : kSH + (L - 1) * 16384;
-        const int K = mlp_in(L), N = mlp_out(L);
-        if (threadIdx.x == 0) {
-            issue_fwd(tmem, sbase, a_off, K, kSW(L), N, K);
-            umma_commit(mbar);
-        }
-        if (!__syncthreads_and(mbar_wait(mbar, phase, err))) return false;  // every thread agrees
-        phase ^= 1u;
-        tc_fence_after();
-        if (L < kMlpLayers - 1) {
-            tmem_row64(tmem, 0, v);
-#pragma unroll
-            for (int k = 0; k < 64; ++k) v[k] = fmaxf(v[k], 0.0f);
-            rc_store_row(smem + kSH + L * 16384, row, 64, v);
-            publish_smem();
-        } else {
-            tmem_ld16(tmem + ((uint32_t)(32 * (threadIdx.x >> 5)) << 16), z);
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ void load_feature_row(unsigned char* smem, const uint16_t* __restrict__ feat, long grow,
-                                                 bool valid) {
-    const uint4* src = (const uint4*)(feat + grow * kMlpIn);
-    for (int j = 0; j < kMlpIn / 8; ++j) {
-        const uint4 q = valid ? __ldg(src + j) : make_uint4(0, 0, 0, 0);
-        *(uint4*)(smem + kSX + rc_offset(threadIdx.x, 8 * j, kMlpIn)) = q;
-    }
-}
-
 // Named barrier over the 128 threads of warpgroup `id - 1` (barrier 0 is __syncthreads).
 __device__ __forceinline__ void wg_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 __device__ __forceinline__ bool wg_sync_and(int id, bool v) {
@@ -224,23 +192,6 @@ __device__ __forceinline__ bool wg_sync_and(int id, bool v) {
         : "memory");
     return r != 0;
 }
-// The warpgroup's shared-memory operands written so far, visible to the tensor cores.
-__device__ __forceinline__ void wg_publish(int id) {
-    fence_async_smem();
-    tc_fence_before();
-    wg_sync(id);
-    tc_fence_after();
-}
-
-// Two FP32 columns to one word of two bf16 (a in the low half), ReLU: rounded first, then clamped
-// (the same values; NaN becomes 0 as by fmaxf).
-__device__ __forceinline__ uint32_t relu_bf16x2(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(b)), "f"(__uint_as_float(a)));
-    asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
-    return r;
-}
-
 // Inference: out[r * stride + c] = exp(z_c), c < 3, for the feature rows r = rows[i] (rows null:
 // r = i), i < n.  Persistent CTAs of kFwdGroups warpgroups; warpgroup g runs tiles
 // g * gridDim.x + blockIdx.x, + gridDim.x * kFwdGroups, ..., and synchronises with named barrier 1 + g
@@ -308,7 +259,7 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
     }
     __syncwarp();
     r = load_tile(tile);
-    load_weights(smem, w16);
+    load_weights(smem_u32(smem), w16);
     if ((threadIdx.x >> 5) == 0) tmem_alloc(tslot, kFwdCols);
     publish_smem();
     const uint32_t tmem = *tslot + kFwdTileCols * (uint32_t)g;
@@ -387,106 +338,190 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
 // Training: gradient of mean over samples and channels of (pred - t)^2 / (pred^2 + 0.01)
 // (relative L2; the denominator is not differentiated) for every weight, accumulated per CTA in
 // TMEM (dW_k^T = H_k^T G_k) and added to grad[] once per CTA.
-__global__ __launch_bounds__(128) void k_mlp_train(const uint16_t* __restrict__ w16, const uint16_t* __restrict__ feat,
-                                                   const float* __restrict__ target, int n, float* __restrict__ grad,
-                                                   float* __restrict__ loss, uint32_t* err) {
+// A tile of 128 rows is a chain of eleven dependent products, so the chain's latency bounds the
+// kernel: TMEM holds one tile's accumulators (448 columns) and shared memory one tile's
+// activations.  What is not in the chain is kept off it: a warp of its own issues the products (the
+// rows' warps wait only for what they read), two warps share 32 rows, the weight gradients' products
+// run behind the epilogue that follows them (two Ga buffers, no commit of their own: the next
+// commit covers them), features of the next tile and targets of this one load ahead, and a layer
+// costs one barrier; an epilogue works on two values at a time (conversion, ReLU, mask).  65,536
+// rows (four rounds of tiles over 152 SMs), us for a step and the parameters' readback: 88.6 with 128
+// threads that issued, waited and converted one by one; about 83 with the products taken off the
+// chain, 76 with two values at a time, 71.1 with every weight copy in flight at once.
+__global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* __restrict__ w16,
+                                                                const uint16_t* __restrict__ feat,
+                                                                const float* __restrict__ target, int n,
+                                                                float* __restrict__ grad, float* __restrict__ loss,
+                                                                uint32_t* err) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* mbar = (uint64_t*)(smem + kTrainBar);
     uint32_t* tslot = (uint32_t*)(smem + kTrainBar + 16);
     const uint32_t sbase = smem_u32(smem);
-    load_weights(smem, w16);
-    if (threadIdx.x == 0) mbar_init(mbar, 1);
-    if ((threadIdx.x >> 5) == 0) tmem_alloc(tslot, 512);
-    publish_smem();
-    const uint32_t tmem = *tslot;
-    const uint32_t lane_base = (uint32_t)(32 * (threadIdx.x >> 5)) << 16;
+    const int warp = threadIdx.x >> 5;
+    const bool worker = warp < 8, issuer = threadIdx.x == kTrainThreads - 32;
+    const int row = threadIdx.x & 127, c0 = 32 * ((threadIdx.x >> 7) & 1);  // a worker's row and first column
+    const int ntiles = (n + 127) / 128;
+    if (issuer) mbar_init(mbar, 1);
+    if (warp == 0) tmem_alloc(tslot, 512);
+    // the features of `tile` into X buffer b, half a row per worker
+    auto fetch = [&](int tile, int b) {
+        const long r = (long)tile * 128 + row;
+        if (!worker || tile >= ntiles) return;
+        const bool in = r < n;
+        const uint16_t* src = feat + (in ? r : 0) * kMlpIn;
+        for (int j = c0 ? 6 : 0, e = j + 6; j < e; ++j)
+            cp_async16(sbase + kSX + 24576 * b + rc_offset(row, 8 * j, kMlpIn), src + 8 * j, in);
+    };
+    fetch(blockIdx.x, 0);
+    load_weights(sbase, w16);
     uint32_t phase = 0;
-    bool first = true, ok = true;
+    bool any = false, ok = true;
+    // Shared-memory operands to the tensor cores, TMEM reads done; false when a wait ran out in any thread.
+    auto publish = [&]() {
+        fence_async_smem();
+        tc_fence_before();
+        ok = __syncthreads_and(ok);
+        tc_fence_after();
+        return ok;
+    };
+    auto wait = [&]() {
+        ok = mbar_wait(mbar, phase, err) && ok;
+        phase ^= 1u;
+        __syncwarp();
+        tc_fence_after();
+    };
+    publish();
+    const uint32_t tmem = *tslot, mine = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + c0;
+    // D = activations . W_L^T
+    auto forward = [&](int L, int b) {
+        if (!issuer) return;
+        issue_fwd(tmem, sbase, L == 0 ? kSX + 24576 * b : kSH + (L - 1) * 16384, mlp_in(L), kSW(L), mlp_out(L), mlp_in(L));
+        umma_commit(mbar);
+    };
     float loss_acc = 0.0f;
     const float inv_count = 1.0f / (3.0f * (float)n);
-    const int ntiles = (n + 127) / 128;
-    const int row = threadIdx.x;
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    int b = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, b ^= 1) {
         const long grow = (long)tile * 128 + row;
         const bool valid = grow < n;
-        load_feature_row(smem, feat, grow, valid);
-        publish_smem();
-        float z[16];
-        if (!(ok = mlp_forward_tile(smem, tmem, mbar, phase, err, z))) break;
-        // output gradient
-        float g[64];
+        float t[kMlpOut] = {};
+        if (worker && c0 == 0 && valid)
+            for (int c = 0; c < kMlpOut; ++c) t[c] = __ldg(target + grow * 3 + c);
+        uint32_t d[32], a[16];
+        cp_async_wait();
+        if (!publish()) break;
+        forward(0, b);
+        for (int L = 0; L < kMlpLayers - 1; ++L) {
+            if (worker) {
+                wait();
+                // the tile before has now left its X buffer and everything else to this one
+                if (L == 0) fetch(tile + gridDim.x, b ^ 1);
+                tmem_ld32(mine, d);
+                tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 16; ++c) g[c] = 0.0f;
-        if (valid) {
-            for (int c = 0; c < kMlpOut; ++c) {
-                const float pred = expf(z[c]), t = target[grow * 3 + c];
-                const float d = pred - t, den = pred * pred + 0.01f;
-                loss_acc += d * d / den;
-                g[c] = 2.0f * d / den * pred * inv_count;  // d/dz through exp
+                for (int k = 0; k < 16; ++k) a[k] = relu_bf16x2(d[2 * k], d[2 * k + 1]);
+                rc_store_row<4>(smem + kSH + L * 16384, row, 64, c0, a);
+            }
+            if (!publish()) break;
+            forward(L + 1, b);
+        }
+        if (!ok) break;
+        if (worker) {
+            wait();
+            if (c0 == 0) {  // output gradient
+                float z[16], g[kMlpOut] = {};
+                tmem_ld16(mine, z);
+                if (valid) {
+                    for (int c = 0; c < kMlpOut; ++c) {
+                        const float pred = expf(z[c]);
+                        const float dif = pred - t[c], den = pred * pred + 0.01f;
+                        loss_acc += dif * dif / den;
+                        g[c] = 2.0f * dif / den * pred * inv_count;  // d/dz through exp
+                    }
+                }
+                a[0] = pack_bf16x2(g[0], g[1]);
+                a[1] = pack_bf16x2(g[2], 0.0f);
+#pragma unroll
+                for (int k = 2; k < 8; ++k) a[k] = 0u;
+                rc_store_row<2>(smem + kSGz, row, 16, 0, a);
             }
         }
-        rc_store_row(smem + kSGz, row, 16, g);
-        publish_smem();
+        if (!publish()) break;
         // layer 5: G_h5 = Gz . W5 ; dW5^T += H5^T . Gz
-        if (threadIdx.x == 0) {
+        if (issuer) {
             umma_bf16(tmem, umma_desc(sbase + kSGz, 128, 16 * 16), umma_desc(sbase + kSW(5), 16 * 64, 128),
                       umma_idesc_bf16(128, 64, false, true), false);
+            umma_commit(mbar);
             const uint32_t h5 = kSH + 4 * 16384;
             for (int s = 0; s < 8; ++s)
                 umma_bf16(tmem + kDwCol(5), umma_desc(sbase + h5 + s * 2 * 16 * 64, 16 * 64, 128),
                           umma_desc(sbase + kSGz + s * 2 * 16 * 16, 16 * 16, 128), umma_idesc_bf16(128, 16, true, true),
-                          !(first && s == 0));
-            umma_commit(mbar);
+                          any || s != 0);
         }
         for (int L = 4; L >= 0; --L) {
             // D holds G_h(L+1) for the activations feeding W_(L+1); mask with H(L+1) > 0
-            if (!(ok = __syncthreads_and(mbar_wait(mbar, phase, err)))) break;
-            phase ^= 1u;
-            tc_fence_after();
-            tmem_row64(tmem, 0, g);
-            float h[64];
-            rc_load_row(smem + kSH + L * 16384, row, 64, h);  // H(L+1)
+            const uint32_t ga = kSGa + (L & 1) * 16384;
+            if (worker) {
+                rc_load_row<4>(smem + kSH + L * 16384, row, 64, c0, a);  // H(L+1)
 #pragma unroll
-            for (int k = 0; k < 64; ++k) g[k] = h[k] > 0.0f ? g[k] : 0.0f;
-            rc_store_row(smem + kSGa, row, 64, g);
-            publish_smem();
-            if (threadIdx.x == 0) {
-                const uint32_t a_in = L == 0 ? kSX : kSH + (L - 1) * 16384;  // input of W_L
+                for (int k = 0; k < 16; ++k) a[k] = positive_bf16x2(a[k]);
+                wait();
+                tmem_ld32(mine, d);
+                tmem_wait_ld();
+#pragma unroll
+                for (int k = 0; k < 16; ++k) a[k] &= pack_bf16x2(__uint_as_float(d[2 * k]), __uint_as_float(d[2 * k + 1]));
+                rc_store_row<4>(smem + ga, row, 64, c0, a);
+            }
+            if (!publish()) break;
+            if (issuer) {
+                const uint32_t a_in = L == 0 ? kSX + 24576 * b : kSH + (L - 1) * 16384;  // input of W_L
                 const int cin = mlp_in(L);
                 if (L > 0) {  // G_h(L) = Ga . W_L (W_L [64 out x 64 in] as MN-major B)
                     for (int s = 0; s < 4; ++s)
-                        umma_bf16(tmem, umma_desc(sbase + kSGa + s * 256, 128, 16 * 64),
+                        umma_bf16(tmem, umma_desc(sbase + ga + s * 256, 128, 16 * 64),
                                   umma_desc(sbase + kSW(L) + s * 2 * 16 * cin, 16 * cin, 128),
                                   umma_idesc_bf16(128, cin, false, true), s > 0);
+                    umma_commit(mbar);
                 }
                 for (int s = 0; s < 8; ++s)  // dW_L^T += A_in^T . Ga
                     umma_bf16(tmem + kDwCol(L), umma_desc(sbase + a_in + s * 2 * 16 * cin, 16 * cin, 128),
-                              umma_desc(sbase + kSGa + s * 2 * 16 * 64, 16 * 64, 128),
-                              umma_idesc_bf16(128, 64, true, true), !(first && s == 0));
-                umma_commit(mbar);
-            }
-            if (L == 0) {
-                if (!(ok = __syncthreads_and(mbar_wait(mbar, phase, err)))) break;
-                phase ^= 1u;
-                tc_fence_after();
+                              umma_desc(sbase + ga + s * 2 * 16 * 64, 16 * 64, 128), umma_idesc_bf16(128, 64, true, true),
+                              any || s != 0);
             }
         }
-        first = false;
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
+        if (!ok) break;
+        any = true;
     }
-    // flush the accumulated weight gradients (rows = input features, columns = outputs)
-    if (!first && ok) {
-        for (int L = 0; L < kMlpLayers; ++L) {
-            const int in = mlp_in(L), nout = L == 5 ? kMlpOut : 64;
-            float v[64];
-            if (L == 5)
-                tmem_ld16(tmem + lane_base + kDwCol(5), v);
-            else
-                tmem_row64(tmem, kDwCol(L), v);
-            if (row < in)
-                for (int o = 0; o < nout; ++o) atomicAdd(grad + mlp_offset(L) + o * in + row, v[o]);
+    cp_async_wait();
+    if (!ok) {  // a wait ran out: let what is in flight end, as far as it does
+        if (threadIdx.x == 0) mbar_wait(mbar, phase ^ 1u, err);
+    } else if (any) {  // the last tile's dW_0
+        if (issuer) umma_commit(mbar);
+        if (worker) wait();
+    }
+    // flush the accumulated weight gradients (rows = input features, columns = outputs), every CTA
+    // from another layer on
+    ok = __syncthreads_and(ok);
+    if (any && ok && worker) {
+        for (int i = 0; i < kMlpLayers; ++i) {
+            const int L = (i + (int)blockIdx.x) % kMlpLayers, in = mlp_in(L);
+            float* dst = grad + mlp_offset(L) + row;
+            if (L == 5) {
+                if (c0 == 0) {
+                    float v[16];
+                    tmem_ld16(mine + kDwCol(5), v);
+                    if (row < in)
+                        for (int o = 0; o < kMlpOut; ++o) atomicAdd(dst + o * in, v[o]);
+                }
+            } else {
+                uint32_t v[32];
+                tmem_ld32(mine + kDwCol(L), v);
+                tmem_wait_ld();
+                if (row < in) {
+#pragma unroll
+                    for (int o = 0; o < 32; ++o) atomicAdd(dst + (c0 + o) * in, __uint_as_float(v[o]));
+                }
+            }
         }
     }
     float tot = loss_acc;
@@ -495,11 +530,9 @@ __global__ __launch_bounds__(128) void k_mlp_train(const uint16_t* __restrict__ 
     if ((threadIdx.x & 31) == 0 && tot != 0.0f) atomicAdd(loss, tot / (3.0f * (float)n));
     tc_fence_before();
     __syncthreads();
-    if ((threadIdx.x >> 5) == 0) tmem_free(tmem, 512);
+    if (warp == 0) tmem_free(tmem, 512);
 }
 
-// One Adam step, then the inference copy: an exponential moving average of the weights with
-// decay `ema` (0: the weights themselves), kept in FP32 and BF16.
 __global__ void k_adam(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                        uint16_t* __restrict__ w16, float* __restrict__ e32, uint16_t* __restrict__ e16, int n, float lr,
                        float b1, float b2, float c1, float c2, float eps, float ema) {
@@ -701,7 +734,7 @@ std::string Mlp::train_step(const uint16_t* d_feat, const float* d_target, int n
     TRY(cudaMemsetAsync(grad_, 0, 4 * kMlpParams, s));
     TRY(cudaMemsetAsync(d_loss, 0, 4, s));
     const int tiles = (n + 127) / 128;
-    k_mlp_train<<<std::min(tiles, blocks_train_), 128, kTrainSmem, s>>>(w16_, d_feat, d_target, n, grad_, d_loss, d_err);
+    k_mlp_train<<<std::min(tiles, blocks_train_), kTrainThreads, kTrainSmem, s>>>(w16_, d_feat, d_target, n, grad_, d_loss, d_err);
     TRY(cudaGetLastError());
     return lr > 0 ? adam(lr, s) : std::string();
 }
