@@ -347,7 +347,8 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
 // costs one barrier; an epilogue works on two values at a time (conversion, ReLU, mask).  65,536
 // rows (four rounds of tiles over 152 SMs), us for a step and the parameters' readback: 88.6 with 128
 // threads that issued, waited and converted one by one; about 83 with the products taken off the
-// chain, 76 with two values at a time, 71.1 with every weight copy in flight at once.
+// chain, 76 with two values at a time, 71.1 with every weight copy in flight at once.  Four warps per 32
+// rows were slower (80 against 75, timed together).
 __global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* __restrict__ w16,
                                                                 const uint16_t* __restrict__ feat,
                                                                 const float* __restrict__ target, int n,
