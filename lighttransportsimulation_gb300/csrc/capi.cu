@@ -89,6 +89,7 @@ struct lts_ctx {
     std::unique_ptr<Mlp> mlp;
     int bvh_mode = -1;        // mode of the BVH currently held (-1: none)
     bool bvh_is_scene = false;
+    bool bvh_unchecked = false;  // built since the error word was last read
     std::unique_ptr<Tracer> tracer;
     lts_metrics metrics{};
 };
@@ -115,6 +116,12 @@ int check_device_error(lts_ctx* ctx) {
     uint32_t h = 0;
     CK(cudaMemcpyAsync(&h, ctx->d_error, 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    // a build that gave up has left no tree
+    if (ctx->bvh_unchecked && (h & (DEV_ERR_LOOKBACK_TIMEOUT | DEV_ERR_CAPACITY))) {
+        ctx->bvh_mode = -1;
+        ctx->bvh_is_scene = false;
+    }
+    ctx->bvh_unchecked = false;
     if (h) {
         CK(cudaMemsetAsync(ctx->d_error, 0, 4, ctx->stream));
         char hex[16];
@@ -143,6 +150,7 @@ int do_build(lts_ctx* ctx, const float* d_tri, int n, int mode, int code_limit) 
         return fail(ctx, e.find("memory") != std::string::npos ? LTS_ERR_OOM : LTS_ERR_CUDA, e);
     }
     ctx->bvh_mode = mode;
+    ctx->bvh_unchecked = true;
     return LTS_OK;
 }
 

@@ -43,10 +43,12 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
 __device__ int g_spin_limit = kSpinLimit;
 
 // One poll of a bounded wait: counts it and backs off, or, past the limit, sets
-// DEV_ERR_LOOKBACK_TIMEOUT and returns false so that the caller gives up.
-__device__ __forceinline__ bool spin_or_give_up(int& spins, uint32_t* err) {
+// DEV_ERR_LOOKBACK_TIMEOUT (and bit `pass` of the build's own *gave_up) and returns false so that
+// the caller gives up.
+__device__ __forceinline__ bool spin_or_give_up(int& spins, uint32_t* err, uint32_t* gave_up = nullptr, int pass = 0) {
     if (++spins > g_spin_limit) {
         atomicOr(err, DEV_ERR_LOOKBACK_TIMEOUT);
+        if (gave_up) atomicOr(gave_up, 1u << pass);
         return false;
     }
     __nanosleep(32);
@@ -261,12 +263,16 @@ __global__ void k_digit_prefix(const uint32_t* __restrict__ hist, uint32_t* __re
 
 // vin null: every value is its key's position (the identity ids of the first pass).  ITEMS keys per
 // thread; LOOKBACK predecessor tiles read per look-back round trip.
+// A look-back that runs out leaves digits counted too low: its pass writes some positions twice and
+// others not at all (all of them inside the arrays).  The keys are then no longer the ones that were
+// counted, and a pass over them could write past the arrays, so the passes after it and the tree do
+// nothing (*gave_up, bit p: pass p ran out).
 template <int ITEMS, int LOOKBACK, bool SCAN>
 __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                                                            uint32_t* __restrict__ kout, int32_t* __restrict__ vout,
                                                            int n, int shift, const uint32_t* __restrict__ prefix,
                                                            uint32_t* __restrict__ status, uint32_t* __restrict__ tile_counter,
-                                                           uint32_t* __restrict__ err) {
+                                                           uint32_t* gave_up, uint32_t* __restrict__ err) {
     constexpr int kTile = kSortThreads * ITEMS;
     __shared__ uint32_t s_keys[kTile];
     __shared__ int32_t s_vals[kTile];
@@ -277,10 +283,15 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
     __shared__ int s_tile;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = (int)atomicAdd(tile_counter, 1u);
+    if (threadIdx.x == 0) {
+        const uint32_t before = ld_relaxed(gave_up) & ((1u << (shift / 8)) - 1u);
+        const int t = (int)atomicAdd(tile_counter, 1u);
+        s_tile = before ? -1 : t;
+    }
     for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += kSortThreads) (&s_whist[0][0])[i] = 0;
     __syncthreads();
     const int tile = s_tile;
+    if (tile < 0) return;  // a pass before this one gave up
     const long base = (long)tile * kTile;
     const long wbase = base + (long)warp * 32 * ITEMS;
 
@@ -356,7 +367,7 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
             }
             if (done) break;
             k -= used;
-            if (used < LOOKBACK && !spin_or_give_up(spins, err)) break;
+            if (used < LOOKBACK && !spin_or_give_up(spins, err, gave_up, shift / 8)) break;
         }
         st_relaxed(st + dig, kFlagPrefix | (excl + tot));
     }
@@ -500,7 +511,8 @@ __device__ __forceinline__ int delta(const uint32_t* __restrict__ c, int n, int 
 //  * what is left of the block is its forest, the subtrees whose parents reach into another block:
 //    at most kForestCap - 1 of them (each side's deltas rise strictly outwards, and a delta takes
 //    54 values: 2..31 for distinct codes, 40 + 8..31 for equal ones), consecutive and covering the
-//    block.  The block writes them, in order, to device memory; the last block of a group of
+//    block.  The block writes them, in order, to device memory (a count beyond the capacity, which
+//    sorted codes cannot give, is cut and reported); the last block of a group of
 //    kTreeGroup to finish takes the group's forests as its items (subtrees instead of leaves) and
 //    climbs again, the last group of a group of groups likewise, up to the root.  No block waits:
 //    the others of a group just end.  (The ancestors of the block edges used to meet in a second
@@ -557,11 +569,11 @@ struct TreeShared {
 };
 
 // The climb over the block's `cnt` items (thread i < cnt holds item i: reference, box), the node
-// records, and the forest into `out` (entries in order, then their count).  Returns the count;
-// the whole tree (no forest) gives 0.  Every thread of the block calls it.
+// records, and the forest into `out` (entries in order, then their count; the whole tree gives 0).
+// Every thread of the block calls it.
 template <int kTreeBlock>
-__device__ int tree_climb(TreeShared<kTreeBlock>& sh, int cnt, int n, int ref, float* mn, float* mx, BvhNode* __restrict__ nodes,
-                          float* __restrict__ root_bounds, ForestEntry* __restrict__ out) {
+__device__ void tree_climb(TreeShared<kTreeBlock>& sh, int cnt, int n, int ref, float* mn, float* mx, BvhNode* __restrict__ nodes,
+                           float* __restrict__ root_bounds, ForestEntry* __restrict__ out, uint32_t* err) {
     const int i = threadIdx.x;
     auto have_of = [&](int slot) -> uint32_t* { return reinterpret_cast<uint32_t*>(&sh.slot[slot][4]) + 1; };
     sh.slot[i][4] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -651,9 +663,11 @@ __device__ int tree_climb(TreeShared<kTreeBlock>& sh, int cnt, int n, int ref, f
             out[at].b = b;
         }
     }
-    if (i == 0) out[kForestCap - 1].a.x = __int_as_float(total);
+    if (i == 0) {
+        if (total > kForestCap - 1) atomicOr(err, DEV_ERR_CAPACITY);
+        out[kForestCap - 1].a.x = __int_as_float(min(total, kForestCap - 1));
+    }
     __syncthreads();
-    return total;
 }
 
 template <int kTreeBlock>
@@ -661,7 +675,8 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
                                                      const int32_t* __restrict__ ids, const uint32_t* __restrict__ codes,
                                                      BvhNode* __restrict__ nodes, ForestEntry* __restrict__ forest,
                                                      uint32_t* __restrict__ group_done, int32_t* __restrict__ leaf_prim,
-                                                     float* __restrict__ root_bounds) {
+                                                     float* __restrict__ root_bounds, const uint32_t* __restrict__ gave_up,
+                                                     uint32_t* err) {
     __shared__ TreeShared<kTreeBlock> sh;
     const int b0 = blockIdx.x * kTreeBlock, cnt = min(kTreeBlock, n - b0);
     const int i = threadIdx.x, l = b0 + i;
@@ -674,6 +689,9 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
         sh.delta[cnt] = delta(codes, n, b0 + cnt - 1, b0 + cnt);
         sh.pos[cnt] = b0 + cnt;
     }
+    // the sort gave up: codes and ids are not a sorted order, whose properties all that follows needs
+    // (ids within the triangles, siblings that meet, forests that fit)
+    if (gave_up && __ldg(gave_up)) return;
     float mn[3], mx[3];
     if (i < cnt) {
         const int prim = (mode == BVH_MODE_REFERENCE) ? l : __ldg(ids + l);
@@ -683,7 +701,7 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
     }
     if (n == 1) return;
     long first = blockIdx.x;  // the first block of the forest this block has written
-    int roots = tree_climb(sh, cnt, n, ~l, mn, mx, nodes, root_bounds, forest + first * kForestCap);
+    tree_climb(sh, cnt, n, ~l, mn, mx, nodes, root_bounds, forest + first * kForestCap, err);
     long span = 1;            // blocks per forest of this level
     for (long count = gridDim.x; count > 1;) {
         // publish the forest; the last of its group goes on with the group's
@@ -737,7 +755,7 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
                 __syncthreads();
                 // chunk c's forest over list c: at most 127 entries a list, so the chunks up to c
                 // have read every list up to c
-                roots = tree_climb(sh, m, n, ref, mn, mx, nodes, root_bounds, forest + (first + c * step) * kForestCap);
+                tree_climb(sh, m, n, ref, mn, mx, nodes, root_bounds, forest + (first + c * step) * kForestCap, err);
             }
             if (chunks <= 1) break;
             nlists = chunks;
@@ -747,7 +765,6 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
         span *= kTreeGroup;
         count = groups;
     }
-    (void)roots;
 }
 
 inline int grid_for(long items, int per_block) { return (int)((items + per_block - 1) / per_block); }
@@ -788,9 +805,10 @@ constexpr int kStreamItems = 4;
 constexpr long sort_tile(long n) { return kSortThreads * (n <= kSortSmallMax ? kSortSmallItems : kSortItems); }
 constexpr long sort_tiles(long n) { return (n + sort_tile(n) - 1) / sort_tile(n); }
 
-// The words every build starts from zero, in one buffer: scene box (8), sort tile counters (8),
-// histograms (4 x 256), the tree's group counters, then the sort's look-back table.
-constexpr size_t kZeroHist = 16, kZeroGroups = kZeroHist + 4 * 256;
+// The words every build starts from zero, in one buffer: scene box (8), sort tile counters (4),
+// whether the sort gave up (4), histograms (4 x 256), the tree's group counters, then the sort's
+// look-back table.
+constexpr size_t kZeroGaveUp = 12, kZeroHist = 16, kZeroGroups = kZeroHist + 4 * 256;
 constexpr size_t zero_status(long n) { return kZeroGroups + ((size_t)tree_counters(n) + 7) / 8 * 8; }
 constexpr size_t zero_words(long n) { return zero_status(n) + 4 * 256 * (size_t)sort_tiles(n); }
 
@@ -802,6 +820,7 @@ cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, ui
                            int32_t* valt, uint32_t* zero, ForestEntry* forest, BvhNode* nodes, int32_t* leaf_prim,
                            float* root_bounds, uint32_t* err, int sms, cudaStream_t s, int* launches, Mark mark) {
     uint32_t* const groups = zero + kZeroGroups;
+    uint32_t* gave_up = nullptr;  // the one-block sort waits for nothing
     mark(0);
     if (n <= kSmallSort) {
         mark(1);
@@ -820,13 +839,14 @@ cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, ui
         mark(2);
         uint32_t* const status = zero + zero_status(n);
         const size_t tiles = (size_t)sort_tiles(n);
+        gave_up = zero + kZeroGaveUp;
         if (n > kSortSmallMax) k_digit_prefix<<<4, 256, 0, s>>>(hist, hist);
         uint32_t *kin = codes, *kout = kalt;
         int32_t *vin = ids, *vout = valt;
         for (int p = 0; p < 4; ++p) {
             auto k = n <= kSortSmallMax ? k_onesweep<kSortSmallItems, kSortSmallLookback, true> : k_onesweep<kSortItems, kSortLookback, false>;
             k<<<(int)tiles, kSortThreads, 0, s>>>(kin, (p == 0 && identity) ? nullptr : vin, kout, vout, n, 8 * p, hist + 256 * p,
-                                                  status + (size_t)p * 256 * tiles, zero + 8 + p, err);
+                                                  status + (size_t)p * 256 * tiles, zero + 8 + p, gave_up, err);
             std::swap(kin, kout);
             std::swap(vin, vout);
         }
@@ -835,7 +855,8 @@ cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, ui
     mark(3);
     mark(4);
     auto tree = tree_block(n) == 512 ? k_tree<512> : k_tree<256>;
-    tree<<<(int)tree_blocks(n), tree_block(n), 0, s>>>(tri, n, mode, ids, codes, nodes, forest, groups, leaf_prim, root_bounds);
+    tree<<<(int)tree_blocks(n), tree_block(n), 0, s>>>(tri, n, mode, ids, codes, nodes, forest, groups, leaf_prim, root_bounds,
+                                                                  gave_up, err);
     mark(5);
     return cudaGetLastError();
 }
