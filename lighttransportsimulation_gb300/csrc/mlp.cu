@@ -69,6 +69,7 @@ __global__ __launch_bounds__(128) void k_umma_probe(const uint16_t* __restrict__
         umma_commit(mbar);
     }
     const bool ok = mbar_wait(mbar, 0, err);
+    if (!ok && tid == 0) mbar_drain(mbar, 0, err);
     tc_fence_after();
     if (ok) {
         const int row = 32 * warp + lane;
@@ -222,13 +223,19 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
     uint32_t* tslot = (uint32_t*)(smem + kFwdBar + 16 * kFwdGroups);
     const uint32_t sbase = smem_u32(smem), buf = fwd_buf(g);
     const int ntiles = (n + 127) / 128, step = gridDim.x * kFwdGroups;
+    // A wait that runs out sets the error flag and is not repeated; the tile runs through, row 0 issues
+    // nothing more, and at the end it waits for what it has issued.
+    bool ok = true;
+    bool xpending = false, ppending = false;  // row 0's feature copy / product that nothing has waited for
+    uint32_t pphase = 0;                      // that product's phase
     // The features of tile t into the buffer, a warp its 32 rows: each access 8 rows x 64 bytes.
     // Returns this thread's feature row of the tile (-1: none).
     auto load_tile = [&](int t) -> long {
         const long i = (long)t * 128 + row;
         const bool valid = t < ntiles && i < n;
         if (MAP) {
-            if (row == 0 && t < ntiles) {
+            if (row == 0 && t < ntiles && ok) {
+                xpending = true;
                 mbar_expect(xbar, kFwdTileBytes);  // rows past n arrive as zeros
                 tma_load_2d(sbase + buf, &map_a, 0, t * 128, xbar);
                 tma_load_2d(sbase + buf + 16384, &map_b, 64, t * 128, xbar);
@@ -264,12 +271,17 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
     publish_smem();
     const uint32_t tmem = *tslot + kFwdTileCols * (uint32_t)g;
     const uint32_t mine = tmem + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16);  // warp w: lanes 32 (w % 4) ..
-    uint32_t phase = 0, xphase = 0;
-    bool ok = true;  // a wait that runs out sets the error flag and is not repeated; the tile runs through
+    uint32_t phase = 0, xphase = 0;  // xphase: row 0's, of the copy it waits for next
     auto product = [&](int L) {  // issue layer L's product and wait for it
-        if (row == 0) {
+        if (row == 0 && ok && L == 0 && MAP) {
+            ok = mbar_wait(xbar, xphase, err);
+            if (ok) {
+                xpending = false;
+                xphase ^= 1u;
+            }
+        }
+        if (row == 0 && ok) {
             if (L == 0 && MAP) {
-                if (ok) ok = mbar_wait(xbar, xphase, err);
                 const uint32_t idesc = umma_idesc_bf16(128, 64, false, false);
                 for (int s = 0; s < 6; ++s)
                     umma_bf16(tmem, s < 4 ? umma_desc_swizzled(sbase + buf + 32 * s, 128)
@@ -284,7 +296,13 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
             }
             umma_commit(mbar);
         }
-        if (ok) ok = mbar_wait(mbar, phase, err);
+        if (ok) {
+            ok = mbar_wait(mbar, phase, err);
+            if (!ok) {
+                ppending = row == 0;
+                pphase = phase;
+            }
+        }
         phase ^= 1u;
         __syncwarp();  // the lanes leave the wait one by one; the TMEM accesses are warp-wide
         tc_fence_after();
@@ -297,16 +315,9 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
             fence_async_smem();
         }
         tc_fence_before();
-        if (!wg_sync_and(bar_id, ok)) {  // a wait ran out: let what is in flight end, as far as it does
-            if (row == 0) {
-                mbar_wait(mbar, phase ^ 1u, err);
-                if (MAP) mbar_wait(xbar, xphase, err);
-            }
-            break;
-        }
+        if (!wg_sync_and(bar_id, ok)) break;
         tc_fence_after();
         product(0);
-        xphase ^= 1u;
         const long next = load_tile(tile + step);
         for (int L = 1; L < kMlpLayers; ++L) {
             uint32_t v[32], a[32];
@@ -329,6 +340,10 @@ __global__ __launch_bounds__(128 * kFwdGroups) void k_mlp_forward(const uint16_t
         if (r >= 0)
             for (int c = 0; c < kMlpOut; ++c) out[r * stride + c] = expf(z[c]);
         r = next;
+    }
+    if (row == 0) {
+        if (ppending) mbar_drain(mbar, pphase, err);
+        if (xpending) mbar_drain(xbar, xphase, err);
     }
     tc_fence_before();
     __syncthreads();
@@ -375,7 +390,7 @@ __global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* 
     };
     fetch(blockIdx.x, 0);
     load_weights(sbase, w16);
-    uint32_t phase = 0;
+    uint32_t phase = 0, commits = 0;  // commits: the issuer's
     bool any = false, ok = true;
     // Shared-memory operands to the tensor cores, TMEM reads done; false when a wait ran out in any thread.
     auto publish = [&]() {
@@ -393,11 +408,15 @@ __global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* 
     };
     publish();
     const uint32_t tmem = *tslot, mine = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + c0;
+    auto commit = [&]() {
+        umma_commit(mbar);
+        ++commits;
+    };
     // D = activations . W_L^T
     auto forward = [&](int L, int b) {
         if (!issuer) return;
         issue_fwd(tmem, sbase, L == 0 ? kSX + 24576 * b : kSH + (L - 1) * 16384, mlp_in(L), kSW(L), mlp_out(L), mlp_in(L));
-        umma_commit(mbar);
+        commit();
     };
     float loss_acc = 0.0f;
     const float inv_count = 1.0f / (3.0f * (float)n);
@@ -452,7 +471,7 @@ __global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* 
         if (issuer) {
             umma_bf16(tmem, umma_desc(sbase + kSGz, 128, 16 * 16), umma_desc(sbase + kSW(5), 16 * 64, 128),
                       umma_idesc_bf16(128, 64, false, true), false);
-            umma_commit(mbar);
+            commit();
             const uint32_t h5 = kSH + 4 * 16384;
             for (int s = 0; s < 8; ++s)
                 umma_bf16(tmem + kDwCol(5), umma_desc(sbase + h5 + s * 2 * 16 * 64, 16 * 64, 128),
@@ -482,7 +501,7 @@ __global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* 
                         umma_bf16(tmem, umma_desc(sbase + ga + s * 256, 128, 16 * 64),
                                   umma_desc(sbase + kSW(L) + s * 2 * 16 * cin, 16 * cin, 128),
                                   umma_idesc_bf16(128, cin, false, true), s > 0);
-                    umma_commit(mbar);
+                    commit();
                 }
                 for (int s = 0; s < 8; ++s)  // dW_L^T += A_in^T . Ga
                     umma_bf16(tmem + kDwCol(L), umma_desc(sbase + a_in + s * 2 * 16 * cin, 16 * cin, 128),
@@ -494,15 +513,19 @@ __global__ __launch_bounds__(kTrainThreads, 1) void k_mlp_train(const uint16_t* 
         any = true;
     }
     cp_async_wait();
-    if (!ok) {  // a wait ran out: let what is in flight end, as far as it does
-        if (threadIdx.x == 0) mbar_wait(mbar, phase ^ 1u, err);
-    } else if (any) {  // the last tile's dW_0
-        if (issuer) umma_commit(mbar);
+    if (ok && any) {  // the last tile's dW_0
+        if (issuer) commit();
         if (worker) wait();
+    }
+    ok = __syncthreads_and(ok);
+    if (!ok && issuer && commits > 0) {
+        // a wait ran out: let what is in flight end, the weight gradients behind the last commit too
+        mbar_drain(mbar, (commits - 1u) & 1u, err);
+        commit();
+        mbar_drain(mbar, (commits - 1u) & 1u, err);
     }
     // flush the accumulated weight gradients (rows = input features, columns = outputs), every CTA
     // from another layer on
-    ok = __syncthreads_and(ok);
     if (any && ok && worker) {
         for (int i = 0; i < kMlpLayers; ++i) {
             const int L = (i + (int)blockIdx.x) % kMlpLayers, in = mlp_in(L);

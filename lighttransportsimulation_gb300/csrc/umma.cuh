@@ -66,11 +66,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
 // "debug_spin_limit") to see a wait run out.
 __device__ int g_mbar_spin_limit = kSpinLimit;
 
-// Waits for phase `parity` of the mbarrier to complete, at most g_mbar_spin_limit polls; on
-// timeout sets DEV_ERR_MMA_TIMEOUT and returns false.
-__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t* err) {
+// Waits for phase `parity` of the mbarrier to complete, at most `limit` polls; on timeout sets
+// DEV_ERR_MMA_TIMEOUT and returns false.
+__device__ __forceinline__ bool mbar_wait_limit(uint64_t* mbar, uint32_t parity, uint32_t* err, int limit) {
     const uint32_t a = smem_u32(mbar);
-    const int limit = g_mbar_spin_limit;
     for (int i = 0; i < limit; ++i) {
         uint32_t done;
         asm volatile(
@@ -83,6 +82,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint3
     }
     atomicOr(err, DEV_ERR_MMA_TIMEOUT);
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t* err) {
+    return mbar_wait_limit(mbar, parity, err, g_mbar_spin_limit);
+}
+// After a wait that ran out: what was issued must end before the kernel frees its tensor memory and
+// returns.  At the full limit, whatever a test has set.
+__device__ __forceinline__ void mbar_drain(uint64_t* mbar, uint32_t parity, uint32_t* err) {
+    (void)mbar_wait_limit(mbar, parity, err, kSpinLimit);
 }
 
 // TMEM allocation by one whole warp; the column address lands in *dst (shared memory).
