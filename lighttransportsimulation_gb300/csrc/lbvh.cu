@@ -869,10 +869,19 @@ cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, ui
         if (e_ != cudaSuccess) return std::string(#call ": ") + cudaGetErrorString(e_); \
     } while (0)
 
-Lbvh::~Lbvh() {
+void Lbvh::release() {
     void* ptrs[] = {nodes, root_bounds, leaf_prim, codes, ids, codes_alt_, zero_};
-    for (void* p : ptrs)
-        if (p) dev_free(p);
+    for (void* p : ptrs) dev_free(p);
+    nodes = nullptr;
+    root_bounds = nullptr;
+    leaf_prim = ids = ids_alt_ = nullptr;
+    codes = codes_alt_ = zero_ = nullptr;
+    cap_ = 0;
+    bytes_ = 0;
+}
+
+Lbvh::~Lbvh() {
+    release();
     for (auto& e : ev_)
         if (e) cudaEventDestroy(e);
 }
@@ -881,11 +890,8 @@ std::string Lbvh::reserve(int nn) {
     if (!ev_[0])
         for (auto& e : ev_) LTS_TRY(cudaEventCreate(&e));
     if (nn <= cap_) return "";
-    void* ptrs[] = {nodes, root_bounds, leaf_prim, codes, ids, codes_alt_, zero_};
-    for (void* p : ptrs)
-        if (p) dev_free(p);
+    release();  // if an allocation below fails, the next build starts from nothing
     const size_t N = (size_t)nn;
-    bytes_ = 0;
     auto al = [&](void** p, size_t b) -> cudaError_t {
         bytes_ += b;
         return dev_alloc(p, b);

@@ -55,6 +55,7 @@ class Lbvh {
 
    private:
     std::string reserve(int n);
+    void release();
     int cap_ = 0;
     size_t bytes_ = 0;
     uint32_t *codes_alt_ = nullptr, *zero_ = nullptr;  // sort buffers, then the tree's forests; words zeroed per build
