@@ -1007,6 +1007,7 @@ std::string Tracer::prepare(const HostScene& sc, const Lbvh& bvh, const lts_rend
         film_ = nullptr;
         dev_free(rgb_);
         rgb_ = nullptr;
+        film_cap_ = 0;
         TRY(dev_alloc((void**)&film_, film_bytes));
         TRY(dev_alloc((void**)&rgb_, 12 * (size_t)sc.width * sc.height));
         film_cap_ = film_bytes;
@@ -1019,6 +1020,7 @@ std::string Tracer::prepare(const HostScene& sc, const Lbvh& bvh, const lts_rend
         if (splat_cap_ < sb) {
             dev_free(splat_);
             splat_ = nullptr;
+            splat_cap_ = 0;
             TRY(dev_alloc((void**)&splat_, sb));
             splat_cap_ = sb;
             TRY(cudaMemsetAsync(splat_, 0, sb, s));
@@ -1037,6 +1039,7 @@ std::string Tracer::prepare(const HostScene& sc, const Lbvh& bvh, const lts_rend
             dev_free(rec_sig_);
             rec_L_ = nullptr;
             rec_sig_ = nullptr;
+            rec_cap_ = 0;
             TRY(dev_alloc((void**)&rec_L_, 12 * (size_t)ns));
             TRY(dev_alloc((void**)&rec_sig_, 8 * (size_t)ns));
             rec_cap_ = (size_t)ns;

@@ -54,3 +54,31 @@ out["sorted"] = bool(np.array_equal(order, np.arange(50000)))
 ctx.close()
 """, 40)
     assert r["big"] == ERR_OOM and r["same"] and r["sorted"], r
+
+
+def test_renders_after_ones_that_did_not_fit(built_lib):
+    """A film (92 + 34 MB), the splats of a bidirectional render (47 MB beside a film of 63 + 24) and
+    per-sample records (98 + 66 MB) that do not fit into 120 MB: the small renders after them are those
+    before."""
+    r = child(r"""
+d = tempfile.mkdtemp()
+sc, sub = scenes.write_tri_light_box(d, level=1)
+ctx = lts.Context(0)
+def render(w, h, which, spp=1, record=False):
+    s = lts.Scene.parse(ctx, d, sc, sub, w, h)
+    return lts.PathTracingIntegrator(2, 3, s, integrator=which).render(spp, 3, record=record, film=not record)
+mega, bdpt = lts.INTEGRATOR_MEGAKERNEL, lts.INTEGRATOR_BDPT
+close = lambda a, b: bool(np.allclose(a, b, rtol=1e-5, atol=1e-6))  # the film's sums are atomic, in doubles
+a, b, c = render(64, 64, mega)["film"], render(64, 64, bdpt)["film"], render(64, 64, mega, record=True)["L"]
+out["film"] = code(lambda: render(2048, 1400, mega))
+out["a"] = close(render(64, 64, mega)["film"], a)
+out["splat"] = code(lambda: render(1400, 1400, bdpt))
+out["b"] = close(render(64, 64, bdpt)["film"], b)
+out["record"] = code(lambda: render(64, 64, mega, spp=2000, record=True))
+out["c"] = bool(np.array_equal(render(64, 64, mega, record=True)["L"], c))
+out = {k: (v if isinstance(v, bool) else [v[0], v[1] if isinstance(v[1], str) else ""]) for k, v in out.items()}
+ctx.close()
+""", 120)
+    for k in ("film", "splat", "record"):
+        assert r[k][0] != 0 and "out of memory" in r[k][1], r
+    assert r["a"] and r["b"] and r["c"], r
