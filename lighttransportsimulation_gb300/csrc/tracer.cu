@@ -1650,8 +1650,9 @@ std::string Tracer::render(const HostScene& sc, const Lbvh& bvh, const lts_rende
 }
 
 std::string Tracer::film_get(const HostScene& sc, float* rgb, double* sums, cudaStream_t s) {
-    if (!film_) return "nothing rendered";
     const int W = sc.width, H = sc.height;
+    // no film, or one that a scene of a smaller film has left
+    if (!film_ || film_cap_ < 32 * (size_t)W * H) return "nothing rendered";
     if (rgb) {
         k_resolve<<<(W * H + 255) / 256, 256, 0, s>>>(film_, rgb_, W, H, splat_spp_ > 0 ? splat_ : nullptr,
                                                       splat_spp_ > 0 ? 1.0 / splat_spp_ : 0.0, view_.filter);
