@@ -156,6 +156,7 @@ int do_build(lts_ctx* ctx, const float* d_tri, int n, int mode, int code_limit) 
 
 int dump_bvh(lts_ctx* ctx, lts_bvh_dump* d) {
     if (!ctx->bvh || ctx->bvh_mode < 0) return fail(ctx, LTS_ERR_STATE, "no BVH has been built");
+    CK(cudaSetDevice(ctx->device));
     int rc = check_device_error(ctx);
     if (rc) return rc;
     Lbvh& b = *ctx->bvh;
@@ -418,6 +419,7 @@ int lts_bvh_build_triangles(lts_ctx* ctx, const float* tri, int32_t n, int32_t m
 int lts_bvh_build_device_async(lts_ctx* ctx, const float* d_tri, int32_t n, int32_t mode, int32_t code_limit) {
     if (!ctx || !d_tri || n < 1) return fail(ctx, LTS_ERR_ARG, "bad triangle input");
     if (ctx->device == -1) return fail(ctx, LTS_ERR_STATE, "host-only context (device -1) cannot run kernels");
+    CK(cudaSetDevice(ctx->device));
     ctx->bvh_is_scene = false;
     return do_build(ctx, d_tri, n, mode, code_limit);
 }
@@ -490,6 +492,7 @@ int lts_render_async(lts_ctx* ctx, const lts_render_desc* desc) {
     if (!ctx || !desc) return fail(ctx, LTS_ERR_ARG, "null argument");
     if (ctx->device == -1) return fail(ctx, LTS_ERR_STATE, "host-only context (device -1) cannot run kernels");
     if (!ctx->loaded) return fail(ctx, LTS_ERR_STATE, "no scene loaded");
+    CK(cudaSetDevice(ctx->device));
     const int mode = desc->bvh_mode == LTS_BVH_REFERENCE ? LTS_BVH_REFERENCE : LTS_BVH_SORTED;
     if (!(ctx->bvh_is_scene && ctx->bvh_mode == mode)) {
         int rc = lts_bvh_build(ctx, mode, nullptr);
@@ -503,6 +506,7 @@ int lts_render_async(lts_ctx* ctx, const lts_render_desc* desc) {
 int lts_film_get(lts_ctx* ctx, float* film_rgb, double* film_sums) {
     if (!ctx) return LTS_ERR_ARG;
     if (!ctx->tracer) return fail(ctx, LTS_ERR_STATE, "nothing rendered");
+    CK(cudaSetDevice(ctx->device));
     int rc = check_device_error(ctx);
     if (rc) return rc;
     std::string e = ctx->tracer->film_get(ctx->scene, film_rgb, film_sums, ctx->stream);
@@ -540,6 +544,7 @@ int lts_write_image(const char* path, const float* rgb, int32_t w, int32_t h, in
 int lts_debug_umma_probe(lts_ctx* ctx, int32_t mode, int32_t swap, const uint16_t* a, const uint16_t* b, float* d) {
     if (!ctx || !a || !b || !d) return LTS_ERR_ARG;
     if (ctx->device < 0) return fail(ctx, LTS_ERR_STATE, "host-only context");
+    CK(cudaSetDevice(ctx->device));
     const std::string e = umma_probe(mode, swap, a, b, d, ctx->d_error, ctx->stream);
     if (!e.empty()) return fail(ctx, LTS_ERR_ARG, e);
     return check_device_error(ctx);
@@ -550,6 +555,7 @@ int mlp_ready(lts_ctx* ctx) {
     if (!ctx) return LTS_ERR_ARG;
     if (ctx->device < 0) return fail(ctx, LTS_ERR_STATE, "host-only context");
     if (!ctx->mlp || !ctx->mlp->ready()) return fail(ctx, LTS_ERR_STATE, "MLP not initialised (lts_mlp_init)");
+    CK(cudaSetDevice(ctx->device));
     return LTS_OK;
 }
 }  // namespace
@@ -557,6 +563,7 @@ int mlp_ready(lts_ctx* ctx) {
 int lts_mlp_init(lts_ctx* ctx, uint32_t seed) {
     if (!ctx) return LTS_ERR_ARG;
     if (ctx->device < 0) return fail(ctx, LTS_ERR_STATE, "host-only context");
+    CK(cudaSetDevice(ctx->device));
     if (!ctx->mlp) ctx->mlp.reset(new Mlp());
     const std::string e = ctx->mlp->init(seed, ctx->stream);
     return e.empty() ? LTS_OK : fail(ctx, LTS_ERR_DEVICE, e);
@@ -853,6 +860,7 @@ int lts_debug_trace_sample(lts_ctx* ctx, int64_t k) {
 int lts_debug_trace_get(lts_ctx* ctx, float* out) {
     if (!ctx || !out) return LTS_ERR_ARG;
     if (!ctx->tracer || !ctx->tracer->trace_) return fail(ctx, LTS_ERR_STATE, "no trace recorded");
+    CK(cudaSetDevice(ctx->device));
     CK(cudaMemcpy(out, ctx->tracer->trace_, 64 * 16 * 4, cudaMemcpyDeviceToHost));
     return LTS_OK;
 }
