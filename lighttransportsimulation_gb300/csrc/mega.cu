@@ -21,6 +21,7 @@
 
 #include "dev_common.cuh"
 #include "dev_math.cuh"
+#include "once_per_device.hpp"
 #include "tracer.cuh"
 #include "tracer_dev.cuh"
 #include "megakernel.cuh"
@@ -38,18 +39,19 @@ namespace {
 
 }  // namespace
 
-// This translation unit's copies of the procedural textures' tables (once per process).
+// This translation unit's copies of the procedural textures' tables on the current device.
 std::string mega_init() {
-    static bool consts = false;
-    if (!consts) {
+    static OncePerDevice once;
+    int dev = 0;
+    TRY(cudaGetDevice(&dev));
+    return once.run(dev, []() -> std::string {
         unsigned char p2[512];
         const float* mc = nullptr;
         texture_tables(p2, &mc);
         TRY(cudaMemcpyToSymbol(c_perm, p2, 512));
         TRY(cudaMemcpyToSymbol(c_marble, mc, 30 * sizeof(float)));
-        consts = true;
-    }
-    return "";
+        return "";
+    });
 }
 
 namespace {

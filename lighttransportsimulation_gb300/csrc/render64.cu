@@ -12,6 +12,7 @@
 
 #include "dev_common.cuh"
 #include "dev_math.cuh"
+#include "once_per_device.hpp"
 #include "tracer.cuh"
 #include "tracer_dev.cuh"
 #include "megakernel.cuh"
@@ -19,16 +20,18 @@
 namespace lts {
 
 std::string render64_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool record, cudaStream_t s) {
-    static bool consts = false;  // this translation unit's copies of the texture tables
-    if (!consts) {
+    static OncePerDevice once;  // this translation unit's copies of the texture tables
+    int tdev = 0;
+    cudaError_t te = cudaGetDevice(&tdev);
+    const std::string ts = te != cudaSuccess ? cudaGetErrorString(te) : once.run(tdev, []() -> std::string {
         unsigned char p2[512];
         const float* mc = nullptr;
         texture_tables(p2, &mc);
         cudaError_t e = cudaMemcpyToSymbol(c_perm, p2, 512);
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_marble, mc, 30 * sizeof(float));
-        if (e != cudaSuccess) return std::string("render64 tables: ") + cudaGetErrorString(e);
-        consts = true;
-    }
+        return e == cudaSuccess ? std::string() : std::string(cudaGetErrorString(e));
+    });
+    if (!ts.empty()) return "render64 tables: " + ts;
     SceneView v = sv;
     v.wnodes = nullptr;  // binary traversal in double
     v.wtris = nullptr;

@@ -13,6 +13,7 @@
 
 #include "dev_common.cuh"
 #include "dev_math.cuh"
+#include "once_per_device.hpp"
 #include "tracer.cuh"
 #include "tracer_dev.cuh"
 #include "mlp.cuh"
@@ -401,18 +402,19 @@ std::string upload(void*& slot, size_t& cap, const std::vector<T, A>& v, cudaStr
 
 float quake_host(float f) { return quake_rsqrt(f); }
 
-// The procedural textures' tables in this translation unit's device copies (once per process).
+// The procedural textures' tables in this translation unit's copies on the current device.
 std::string ensure_texture_tables() {
-    static bool consts = false;
-    if (!consts) {
+    static OncePerDevice once;
+    int dev = 0;
+    TRY(cudaGetDevice(&dev));
+    return once.run(dev, []() -> std::string {
         unsigned char p2[512];
         const float* mc = nullptr;
         texture_tables(p2, &mc);
         TRY(cudaMemcpyToSymbol(c_perm, p2, 512));
         TRY(cudaMemcpyToSymbol(c_marble, mc, 30 * sizeof(float)));
-        consts = true;
-    }
-    return "";
+        return "";
+    });
 }
 
 }  // namespace

@@ -139,7 +139,7 @@ size_t bdpt_sample_bytes(int max_bounce, int strategy);
 std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
                         bool matte_only, void* ws, long cap, uint32_t* d_count, cudaStream_t s);
 std::string mega_set_libm_double(int on);
-std::string mega_init();  // that translation unit's texture tables (once per process)
+std::string mega_init();  // that translation unit's texture tables on the current device
 constexpr int kBdptMaxBounce = 8;  // longest path of the bidirectional integrator
 
 // FP64 oracle renderer (render64.cu): the megakernel integrator in double on the binary LBVH.
