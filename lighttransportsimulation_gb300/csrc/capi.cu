@@ -154,6 +154,35 @@ int do_build(lts_ctx* ctx, const float* d_tri, int n, int mode, int code_limit) 
     return LTS_OK;
 }
 
+// The flattened tree without device memory for it: nodes in pieces of 16 MB, scattered by the host.
+int flatten_on_host(lts_ctx* ctx, const Lbvh& b, lts_bvh_dump* d) {
+    const int n = b.n;
+    constexpr int kPiece = 1 << 18;
+    std::vector<BvhNode> h((size_t)std::min(n - 1, kPiece));
+    if (d->node_bounds) CK(cudaMemcpyAsync(d->node_bounds, b.root_bounds, 24, cudaMemcpyDeviceToHost, ctx->stream));
+    for (int l = 0; l < n; ++l) {
+        if (d->node_left) d->node_left[n - 1 + l] = -1;
+        if (d->node_right) d->node_right[n - 1 + l] = -1;
+    }
+    auto flat = [n](int c) { return c < 0 ? (n - 1) + ~c : c; };
+    for (int first = 0; first < n - 1; first += kPiece) {
+        const int count = std::min(kPiece, n - 1 - first);
+        CK(cudaMemcpyAsync(h.data(), b.nodes + first, sizeof(BvhNode) * (size_t)count, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        for (int k = 0; k < count; ++k) {
+            const int lc = flat(h[(size_t)k].d.x), rc = flat(h[(size_t)k].d.y);
+            if (d->node_left) d->node_left[first + k] = lc;
+            if (d->node_right) d->node_right[first + k] = rc;
+            if (d->node_bounds) {
+                const float* f = reinterpret_cast<const float*>(&h[(size_t)k]);
+                memcpy(d->node_bounds + 6 * (size_t)lc, f, 24);
+                memcpy(d->node_bounds + 6 * (size_t)rc, f + 6, 24);
+            }
+        }
+    }
+    return LTS_OK;
+}
+
 int dump_bvh(lts_ctx* ctx, lts_bvh_dump* d) {
     if (!ctx->bvh || ctx->bvh_mode < 0) return fail(ctx, LTS_ERR_STATE, "no BVH has been built");
     CK(cudaSetDevice(ctx->device));
@@ -172,34 +201,43 @@ int dump_bvh(lts_ctx* ctx, lts_bvh_dump* d) {
     const size_t nodes = 2 * (size_t)n - 1;
     if (d->node_left || d->node_right || d->node_bounds) {
         // flattened on the device and copied straight into the caller's arrays; a workspace of up to
-        // kDumpKeep bytes stays with the context
+        // kDumpKeep bytes stays with the context.  32 bytes a node: where that much device memory cannot be
+        // had, the host flattens, as slow as its copies and scatter
         const size_t bytes = 8 * ((nodes + 1) / 2 * 2) + 24 * nodes;
         void* ws = ctx->dump_ws;
         if (ctx->dump_ws_cap < bytes) {
             dev_free(ctx->dump_ws);
             ctx->dump_ws = nullptr;
             ctx->dump_ws_cap = 0;
-            CK(dev_alloc(&ws, bytes));
-            if (bytes <= kDumpKeep) {
+            const cudaError_t ae = dev_alloc(&ws, bytes);
+            if (ae != cudaSuccess && ae != cudaErrorMemoryAllocation) return cuda_fail(ctx, ae, "tree workspace");
+            if (ae != cudaSuccess) {
+                cudaGetLastError();
+                ws = nullptr;
+            } else if (bytes <= kDumpKeep) {
                 ctx->dump_ws = ws;
                 ctx->dump_ws_cap = bytes;
             }
         }
-        int32_t* left = static_cast<int32_t*>(ws);
-        int32_t* right = left + (nodes + 1) / 2 * 2;
-        float* bounds = reinterpret_cast<float*>(right + (nodes + 1) / 2 * 2);
-        const std::string e = b.flatten(left, right, bounds, ctx->stream);
-        cudaError_t ce = e.empty() ? cudaSuccess : cudaErrorUnknown;
-        auto get = [&](void* to, const void* from, size_t bytes) {
-            if (to && ce == cudaSuccess) ce = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->stream);
-        };
-        get(d->node_left, left, 4 * nodes);
-        get(d->node_right, right, 4 * nodes);
-        get(d->node_bounds, bounds, 24 * nodes);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
-        if (ws != ctx->dump_ws) dev_free(ws);
-        if (!e.empty()) return fail(ctx, LTS_ERR_CUDA, e);
-        if (ce != cudaSuccess) return cuda_fail(ctx, ce, "copy the tree");
+        if (!ws) {
+            if (int r = flatten_on_host(ctx, b, d)) return r;
+        } else {
+            int32_t* left = static_cast<int32_t*>(ws);
+            int32_t* right = left + (nodes + 1) / 2 * 2;
+            float* bounds = reinterpret_cast<float*>(right + (nodes + 1) / 2 * 2);
+            const std::string e = b.flatten(left, right, bounds, ctx->stream);
+            cudaError_t ce = e.empty() ? cudaSuccess : cudaErrorUnknown;
+            auto get = [&](void* to, const void* from, size_t bytes) {
+                if (to && ce == cudaSuccess) ce = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+            };
+            get(d->node_left, left, 4 * nodes);
+            get(d->node_right, right, 4 * nodes);
+            get(d->node_bounds, bounds, 24 * nodes);
+            if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
+            if (ws != ctx->dump_ws) dev_free(ws);
+            if (!e.empty()) return fail(ctx, LTS_ERR_CUDA, e);
+            if (ce != cudaSuccess) return cuda_fail(ctx, ce, "copy the tree");
+        }
     }
     if (d->sorted_codes) CK(cudaMemcpyAsync(d->sorted_codes, b.codes, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
     if (d->sorted_ids) CK(cudaMemcpyAsync(d->sorted_ids, b.ids, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));

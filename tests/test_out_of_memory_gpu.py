@@ -82,3 +82,35 @@ ctx.close()
     for k in ("film", "splat", "record"):
         assert r[k][0] != 0 and "out of memory" in r[k][1], r
     assert r["a"] and r["b"] and r["c"], r
+
+
+def test_a_dump_without_memory_for_the_flattened_tree(built_lib):
+    """60,000 triangles: 4.9 MB of tree and sort buffers fit into 7 MB, the flattened tree's 3.8 MB beside them
+    do not.  The dump is the one of a build with room, whole or in parts."""
+    r = child(r"""
+n = 60000
+tris = scenes.random_triangles(n, seed=4)
+dev = torch.from_numpy(tris.reshape(-1).copy()).cuda()
+torch.cuda.synchronize()
+ctx = lts.Context(0)
+ctx.check(lib.lts_bvh_build_device_async(ctx.h, ctypes.c_void_p(dev.data_ptr()), n, lts.BVH_SORTED, -1))
+a, d = lts._dump_arrays(n)
+out["rc"] = lib.lts_bvh_dump_get(ctx.h, ctypes.byref(d))
+left = np.zeros(2 * n - 1, np.int32)
+part = lts.BvhDump(None, None, None, left.ctypes.data, None, None)
+out["part"] = lib.lts_bvh_dump_get(ctx.h, ctypes.byref(part))
+out["device_mb"] = ctx.metrics().device_bytes / 2**20
+from oracle import lbvh_np
+codes, ids = lbvh_np.stable_sort(*lbvh_np.morton_codes(tris, -1))
+l, r = lbvh_np.karras_topology(codes)
+out["order"] = bool(np.array_equal(a["sorted_codes"], codes) and np.array_equal(a["sorted_ids"], ids))
+out["tree"] = bool(np.array_equal(a["node_left"][: n - 1], l) and np.array_equal(a["node_right"][: n - 1], r)
+                   and np.all(a["node_left"][n - 1:] == -1) and np.all(a["node_right"][n - 1:] == -1)
+                   and np.array_equal(left, a["node_left"]))
+out["key"] = bool(np.array_equal(a["node_key"], np.concatenate([np.full(n - 1, -1), np.arange(n)]).astype(np.int32)))
+mn, mx = lbvh_np.tri_bounds(tris)
+lbvh_np.check_tree(a["node_left"], a["node_right"], a["node_bounds"], np.concatenate([mn, mx], 1)[ids])
+ctx.close()
+""", 7)
+    assert r["rc"] == 0 and r["part"] == 0 and r["device_mb"] < 7, r
+    assert r["order"] and r["tree"] and r["key"], r
