@@ -906,6 +906,7 @@ int lts_debug_trace_get(lts_ctx* ctx, float* out) {
 int lts_get_metrics(lts_ctx* ctx, lts_metrics* out) {
     if (!ctx || !out) return LTS_ERR_ARG;
     *out = ctx->metrics;
+    if (ctx->tracer) ctx->tracer->settle_gather(true);
     out->device_bytes = (int64_t)dev_bytes_in_use();
     out->kernel_launches = (ctx->bvh ? ctx->bvh->launches : 0) + (ctx->tracer ? ctx->tracer->last_launches : 0);
     out->render_launches = ctx->tracer ? ctx->tracer->last_launches : 0;

@@ -1113,6 +1113,7 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     last_launches = 1;
     last_iterations = 1;
     for (double& x : last_stage_ms) x = 0;
+    gather_timed_ = false;
     last_paths = (double)ns;
     return "";
 }
@@ -1320,6 +1321,7 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
     for (cudaEvent_t& e : wf_ev_)
         if (!e) TRY(cudaEventCreate(&e));
     for (double& x : last_stage_ms) x = 0;
+    gather_timed_ = false;
     // persistent trace grid: every SM filled with as many blocks as stay resident
     if (wf_trace_blocks_[0] == 0) {
         int dev = 0, sms = 0, per_w = 0, per_b = 0, per_i = 0;

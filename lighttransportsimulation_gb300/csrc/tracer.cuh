@@ -219,6 +219,8 @@ class Tracer {
     // (path rays, shadow rays, MIS rays).  Zero for the megakernel.
     double last_stage_ms[6] = {0, 0, 0, 0, 0, 0};
     double last_kind_work[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    // Adds the last render's film gather to last_stage_ms[5] (wait: first waits for it to end).
+    void settle_gather(bool wait);
 
     // Batch ray queries (lts_intersect, lts_intersect_arrays) over device arrays: d_tmax null, d_o
     // holds n x {o.xyz, tmax, d.xyz, 0}; else d_o, d_d n x 3 and d_tmax one value or n.  any = 0
@@ -314,7 +316,6 @@ class Tracer {
     HostWords* host_words_ = nullptr;
     std::string pinned(HostWords** w);
     bool gather_timed_ = false;  // wf_ev_[0] and [6] hold a film gather's time not yet in last_stage_ms[5]
-    void settle_gather(bool wait);
     // pools of up to this many paths are made whatever memory is free
     static constexpr long kPoolMin = 1l << 21;
     // the captured wavefront iteration (path rays in q_a, in q_b), kept between renders, and the
