@@ -291,7 +291,9 @@ __device__ __forceinline__ void load_ray(const RayBatch& b, int i, V3& o, V3& d,
 // k_intersect_wide, the 8-wide flat tree: persistent warps that fetch new rays for lanes whose ray has
 // finished, node visits and triangle tests apart, as the wavefront's trace kernel (1M scattered rays
 // against the 1.3M-triangle displaced sphere: 666 us; a ray per thread, a warp's rays in step,
-// 737).  k_intersect: any other tree, one ray per thread.
+// 737).  k_intersect: any other tree, one ray per thread; INST: the two-level tree, else the binary one,
+// each with its own steps only (any-hit queries of the binary tree in the common loop, whose lanes ended
+// up one by one in it: 302 us a call of 100 rays, 360 of 10,000; 91 and 141 in its own).
 template <bool ANY>
 __global__ __launch_bounds__(kThreads, kTraceMinBlocks) void k_intersect_wide(const SceneView sv, int nleaf, const RayBatch b,
                                                                               uint32_t n, uint32_t* fetch,
@@ -355,7 +357,7 @@ __global__ __launch_bounds__(kThreads, kTraceMinBlocks) void k_intersect_wide(co
         }
     }
 }
-template <bool ANY>
+template <bool ANY, bool INST>
 __global__ __launch_bounds__(kThreads) void k_intersect(const SceneView sv, int nleaf, const RayBatch b, int n,
                                                         int32_t* __restrict__ prim, float* __restrict__ tout, uint32_t* err) {
     __shared__ uint32_t s_stack[kStack * kThreads];
@@ -365,7 +367,20 @@ __global__ __launch_bounds__(kThreads) void k_intersect(const SceneView sv, int 
     real tmax, bu = 0, bv = 0, binv = 0;
     load_ray(b, i, o, d, tmax);
     Work wk{0u, 0u};
-    const int h = traverse<ANY, true>(sv, nleaf, make_trace_ray(o, d), tmax, bu, bv, binv, s_stack + threadIdx.x, err, wk);
+    int h;
+    if (INST) {
+        h = traverse<ANY, true>(sv, nleaf, make_trace_ray(o, d), tmax, bu, bv, binv, s_stack + threadIdx.x, err, wk);
+    } else {
+        Trav t;
+        if (trav_begin(ANY, t, sv, nleaf, o, d, tmax, wk))
+            while (!trav_step_binary(ANY, t, sv, s_stack + threadIdx.x, err, wk)) {
+            }
+        h = ANY ? (t.best == 1 ? 1 : -1) : hit_prim(t.best);
+        tmax = t.tmax;
+        bu = t.bu;
+        bv = t.bv;
+        binv = t.binv;
+    }
     if (!ANY && h >= 0) hit_exact(sv, h, o, d, tmax, bu, bv, binv);
     prim[i] = ANY ? (h > 0 ? 1 : 0) : h;
     if (tout) tout[i] = (!ANY && h >= 0) ? (float)tmax : INFINITY;
@@ -971,7 +986,9 @@ std::string Tracer::intersect(const Lbvh& bvh, const float* d_o, const float* d_
         k<<<grid, kThreads, 0, s>>>(sv, bvh.n, batch, (uint32_t)n, fetch, d_prim, d_t, d_err);
     } else {
         const unsigned grid = (unsigned)((n + kThreads - 1) / kThreads);
-        auto k = any ? k_intersect<true> : k_intersect<false>;
+        const bool inst = sv.ninst > 0;  // (the two-level tree is always 8-wide)
+        auto k = any ? (inst ? k_intersect<true, true> : k_intersect<true, false>)
+                     : (inst ? k_intersect<false, true> : k_intersect<false, false>);
         k<<<grid, kThreads, 0, s>>>(sv, bvh.n, batch, n, d_prim, d_t, d_err);
     }
     TRY(cudaGetLastError());
