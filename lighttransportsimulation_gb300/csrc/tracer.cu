@@ -1492,7 +1492,9 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
         if (graph) {
             // A pool that holds the whole batch drains after max_bounce + 1 iterations (every path
             // is at the same bounce; the last one only finalizes), so the host looks at the
-            // counts then; a smaller pool is refilled as paths end and is looked at in groups.
+            // counts then (18 iterations at most between looks); a smaller pool is refilled as paths end
+            // and is looked at in groups, of up to 16 iterations while as many are still to come at the
+            // rate so far (512 x 512 x 8 spp through 65,536 slots: 22.7 ms with groups of 4, 22.1 so).
             int par = 0, group = P >= ctot ? std::min(rp.max_bounce, 17) + 1 : 4;
             for (;;) {
                 for (int k = 0; k < group; ++k, par ^= 1) TRY(cudaGraphLaunch(wf_exec_[par], s));
@@ -1504,7 +1506,8 @@ std::string Tracer::run_wavefront(const std::vector<std::vector<WfView>>& batche
                                                     h_ctl->generated < h_ctl->ctot);
                 if (!left) break;
                 if (h_ctl->iters > 1000000) return "wavefront did not converge";
-                group = P >= ctot ? 8 : 4;
+                const double to_come = (double)(h_ctl->ctot - h_ctl->generated) * h_ctl->iters / std::max(1.0, (double)h_ctl->generated);
+                group = P >= ctot ? 8 : (int)std::max(4.0, std::min(16.0, to_come));
             }
             iters += (int)h_ctl->iters;
             last_cache_queries += (double)h_ctl->queries;
