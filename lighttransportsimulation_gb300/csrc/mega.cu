@@ -363,7 +363,8 @@ size_t bdpt_sample_bytes(int max_bounce, int strategy) {
 }
 
 std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
-                        bool matte_only, void* ws, long cap, uint32_t* d_count, cudaStream_t s) {
+                        bool matte_only, void* ws, long cap, uint32_t* d_count, cudaStream_t s, int* launches) {
+    *launches = 0;
     const int maxb = std::min(rp.max_bounce, kBdptMaxBounce);
     const BdptStrategies st = bdpt_strategies(maxb, strategy);
     const bool wide = sv.wnodes != nullptr && sv.ninst == 0;
@@ -399,6 +400,7 @@ std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, 
             kt<<<kBdptConnectBlocks * 4 * sms, kThreads, 0, s>>>(sv, rp, buf, st, first, strategy, splat);
         }
         k_bdpt_film<<<gs, kThreads, 0, s>>>(sv, rp, buf, st, n);
+        *launches += st.n > 0 ? 5 : 2;
         TRY(cudaGetLastError());
     }
     return "";

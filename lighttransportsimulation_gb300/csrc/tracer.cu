@@ -1120,14 +1120,15 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
         }
     }
     TRY(cudaEventRecord(ev0_, s));
+    int launches = 1;
     if (d.integrator == LTS_INTEGRATOR_FP64) e = render64_launch(sv, rp, bvh.n, d.record_samples != 0, s);
     else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, bdpt_ws_, bdpt_cap,
-                                                                   reinterpret_cast<uint32_t*>(counters_ + 13), s);
+                                                                   reinterpret_cast<uint32_t*>(counters_ + 13), s, &launches);
     else e = mega_launch(sv, rp, bvh.n, d.record_samples != 0, matte_only_, s);
     if (!e.empty()) return e;
     TRY(cudaEventRecord(ev1_, s));
     TRY(cudaGetLastError());
-    last_launches = 1;
+    last_launches = launches;
     last_iterations = 1;
     for (double& x : last_stage_ms) x = 0;
     gather_timed_ = false;
