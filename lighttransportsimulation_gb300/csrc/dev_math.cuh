@@ -52,10 +52,13 @@ __device__ __forceinline__ real xceil(real a) { return ceilf(a); }
 // the reference's host build gets from glibc (or from the double functions it calls on float
 // arguments); 0 (default) uses CUDA's float functions.  The flag is uniform over a launch.
 __constant__ int c_libm_double;
-__device__ __noinline__ float cos_via_double(float a) { return (float)cos((double)a); }
-__device__ __noinline__ float sin_via_double(float a) { return (float)sin((double)a); }
-__device__ __noinline__ float acos_via_double(float a) { return (float)acos((double)a); }
-__device__ __noinline__ float log2_via_double(float a) { return (float)log2((double)a); }
+#ifndef LTS_LIBM_CALL
+#define LTS_LIBM_CALL __noinline__  // a translation unit may choose __forceinline__
+#endif
+__device__ LTS_LIBM_CALL float cos_via_double(float a) { return (float)cos((double)a); }
+__device__ LTS_LIBM_CALL float sin_via_double(float a) { return (float)sin((double)a); }
+__device__ LTS_LIBM_CALL float acos_via_double(float a) { return (float)acos((double)a); }
+__device__ LTS_LIBM_CALL float log2_via_double(float a) { return (float)log2((double)a); }
 __device__ __forceinline__ real xcos(real a) { return c_libm_double ? cos_via_double(a) : cosf(a); }
 __device__ __forceinline__ real xsin(real a) { return c_libm_double ? sin_via_double(a) : sinf(a); }
 __device__ __forceinline__ real xacos(real a) { return c_libm_double ? acos_via_double(a) : acosf(a); }

@@ -308,28 +308,22 @@ std::string mega_set_libm_double(int on) {
 }
 
 // matte_only: every material is Lambertian / Oren-Nayar with constant textures.
-std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool record, bool matte_only,
-                        cudaStream_t s) {
-    const dim3 block(kBX, kBY);
-    dim3 grid((rp.x1 - rp.x0 + kBX - 1) / kBX, (rp.y1 - rp.y0 + kBY - 1) / kBY);
-    if (record) {  // per-sample radiance and event hashes: the reference-shaped kernel
-        k_pathtrace<true><<<grid, block, 0, s>>>(sv, rp, nleaf);
-    } else {
-        // sample slices until every SM's four tiles are filled kMegaWaves times over; blocks of
-        // fewer tiles when there are not four tiles for every SM (a thumbnail's few blocks
-        // would leave most SMs idle)
-        int dev = 0, sms = 0;
-        TRY(cudaGetDevice(&dev));
-        TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const long tiles = (long)grid.x * grid.y, want = (long)kMegaWaves * kMegaTiles * sms;
-        const long z = std::max(1L, std::min<long>({(long)rp.spp, (want + tiles - 1) / tiles, 65535L}));
-        const long per = std::max(1L, std::min<long>(kMegaTiles, tiles * z / sms));
-        const bool wide = sv.wnodes != nullptr && sv.ninst == 0;
-        auto k = !wide ? k_mega<LM_ALL, true, false> : matte_only ? k_mega<LM_MATTE, false, true> : k_mega<LM_ALL, true, true>;
-        TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kMegaWords * kMegaTiles));
-        k<<<dim3((unsigned)((tiles + per - 1) / per), 1, (unsigned)z), (unsigned)(kThreads * per), 4 * kMegaWords * per, s>>>(
-            sv, rp, nleaf, (int)grid.x, (int)tiles);
-    }
+std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool matte_only, cudaStream_t s) {
+    // sample slices until every SM's four tiles are filled kMegaWaves times over; blocks of fewer
+    // tiles when there are not four tiles for every SM (a thumbnail's few blocks would leave most SMs
+    // idle)
+    const dim3 grid((rp.x1 - rp.x0 + kBX - 1) / kBX, (rp.y1 - rp.y0 + kBY - 1) / kBY);
+    int dev = 0, sms = 0;
+    TRY(cudaGetDevice(&dev));
+    TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long tiles = (long)grid.x * grid.y, want = (long)kMegaWaves * kMegaTiles * sms;
+    const long z = std::max(1L, std::min<long>({(long)rp.spp, (want + tiles - 1) / tiles, 65535L}));
+    const long per = std::max(1L, std::min<long>(kMegaTiles, tiles * z / sms));
+    const bool wide = sv.wnodes != nullptr && sv.ninst == 0;
+    auto k = !wide ? k_mega<LM_ALL, true, false> : matte_only ? k_mega<LM_MATTE, false, true> : k_mega<LM_ALL, true, true>;
+    TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kMegaWords * kMegaTiles));
+    k<<<dim3((unsigned)((tiles + per - 1) / per), 1, (unsigned)z), (unsigned)(kThreads * per), 4 * kMegaWords * per, s>>>(
+        sv, rp, nleaf, (int)grid.x, (int)tiles);
     TRY(cudaGetLastError());
     return "";
 }

@@ -437,7 +437,8 @@ std::string ensure_texture_tables() {
 std::string set_libm_double(int on) {
     const int v = on ? 1 : 0;
     TRY(cudaMemcpyToSymbol(c_libm_double, &v, sizeof v));
-    return mega_set_libm_double(on);
+    const std::string e = mega_set_libm_double(on);
+    return e.empty() ? pathtrace_set_libm_double(on) : e;
 }
 
 std::string kat_launch(int fn, const float* d_in, int n, float* d_out, cudaStream_t s) {
@@ -584,6 +585,7 @@ std::string Tracer::upload_scene(const HostScene& sc, cudaStream_t s) {
     {
         std::string te = ensure_texture_tables();
         if (te.empty()) te = mega_init();
+        if (te.empty()) te = pathtrace_init();
         if (!te.empty()) return te;
     }
     if (!ev0_) {
@@ -1130,7 +1132,8 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     if (d.integrator == LTS_INTEGRATOR_FP64) e = render64_launch(sv, rp, bvh.n, d.record_samples != 0, s);
     else if (d.integrator == LTS_INTEGRATOR_BDPT) e = bdpt_launch(sv, rp, bvh.n, splat_, bdpt_strategy, matte_only_, bdpt_ws_, bdpt_cap,
                                                                    reinterpret_cast<uint32_t*>(counters_ + 13), s, &launches);
-    else e = mega_launch(sv, rp, bvh.n, d.record_samples != 0, matte_only_, s);
+    else if (d.record_samples) e = pathtrace_record_launch(sv, rp, bvh.n, s);
+    else e = mega_launch(sv, rp, bvh.n, matte_only_, s);
     if (!e.empty()) return e;
     TRY(cudaEventRecord(ev1_, s));
     TRY(cudaGetLastError());

@@ -131,8 +131,7 @@ std::string kat_launch(int fn, const float* d_in, int n, float* d_out, cudaStrea
 // The float one-launch integrators (mega.cu): the path-tracing megakernel and the bidirectional
 // integrator; set_libm_double of that translation unit.  matte_only: every material is Lambertian
 // or Oren-Nayar with constant textures.
-std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool record, bool matte_only,
-                        cudaStream_t s);
+std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool matte_only, cudaStream_t s);
 // The bidirectional integrator works on chunks of at most `cap` samples, whose vertices and
 // contributions lie in `ws` (bdpt_sample_bytes per sample); d_count: two words; *launches: kernels
 // launched.
@@ -140,6 +139,10 @@ size_t bdpt_sample_bytes(int max_bounce, int strategy);
 std::string bdpt_launch(const SceneView& sv, const RenderParams& rp, int nleaf, double* splat, int strategy,
                         bool matte_only, void* ws, long cap, uint32_t* d_count, cudaStream_t s, int* launches);
 std::string mega_set_libm_double(int on);
+// The path tracer's record mode and its translation unit's set-up (pathtrace.cu).
+std::string pathtrace_record_launch(const SceneView& sv, const RenderParams& rp, int nleaf, cudaStream_t s);
+std::string pathtrace_set_libm_double(int on);
+std::string pathtrace_init();
 std::string mega_init();  // that translation unit's texture tables on the current device
 constexpr int kBdptMaxBounce = 8;  // longest path of the bidirectional integrator
 
