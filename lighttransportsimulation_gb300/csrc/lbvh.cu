@@ -43,12 +43,12 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
 __device__ int g_spin_limit = kSpinLimit;
 
 // One poll of a bounded wait: counts it and backs off, or, past the limit, sets
-// DEV_ERR_LOOKBACK_TIMEOUT (and bit `pass` of the build's own *gave_up) and returns false so that
-// the caller gives up.
-__device__ __forceinline__ bool spin_or_give_up(int& spins, uint32_t* err, uint32_t* gave_up = nullptr, int pass = 0) {
+// DEV_ERR_LOOKBACK_TIMEOUT (and the build's own *gave_up) and returns false so that the caller
+// gives up.
+__device__ __forceinline__ bool spin_or_give_up(int& spins, uint32_t* err, uint32_t* gave_up = nullptr) {
     if (++spins > g_spin_limit) {
         atomicOr(err, DEV_ERR_LOOKBACK_TIMEOUT);
-        if (gave_up) atomicOr(gave_up, 1u << pass);
+        if (gave_up) atomicOr(gave_up, 1u);
         return false;
     }
     __nanosleep(32);
@@ -264,9 +264,9 @@ __global__ void k_digit_prefix(const uint32_t* __restrict__ hist, uint32_t* __re
 // vin null: every value is its key's position (the identity ids of the first pass).  ITEMS keys per
 // thread; LOOKBACK predecessor tiles read per look-back round trip.
 // A look-back that runs out leaves digits counted too low: its pass writes some positions twice and
-// others not at all (all of them inside the arrays).  The keys are then no longer the ones that were
-// counted, and a pass over them could write past the arrays, so the passes after it and the tree do
-// nothing (*gave_up, bit p: pass p ran out).
+// others not at all.  The keys are then no longer the ones that were counted, and the passes after it would
+// write past the arrays: every position is checked before its write.  *gave_up tells the tree.  (Asking it
+// at the start of every tile instead cost 2 us a pass.)
 template <int ITEMS, int LOOKBACK, bool SCAN>
 __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                                                            uint32_t* __restrict__ kout, int32_t* __restrict__ vout,
@@ -283,15 +283,10 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
     __shared__ int s_tile;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        const uint32_t before = ld_relaxed(gave_up) & ((1u << (shift / 8)) - 1u);
-        const int t = (int)atomicAdd(tile_counter, 1u);
-        s_tile = before ? -1 : t;
-    }
+    if (threadIdx.x == 0) s_tile = (int)atomicAdd(tile_counter, 1u);
     for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += kSortThreads) (&s_whist[0][0])[i] = 0;
     __syncthreads();
     const int tile = s_tile;
-    if (tile < 0) return;  // a pass before this one gave up
     const long base = (long)tile * kTile;
     const long wbase = base + (long)warp * 32 * ITEMS;
 
@@ -367,7 +362,7 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
             }
             if (done) break;
             k -= used;
-            if (used < LOOKBACK && !spin_or_give_up(spins, err, gave_up, shift / 8)) break;
+            if (used < LOOKBACK && !spin_or_give_up(spins, err, gave_up)) break;
         }
         st_relaxed(st + dig, kFlagPrefix | (excl + tot));
     }
@@ -389,8 +384,10 @@ __global__ __launch_bounds__(kSortThreads, LTS_SORT_MIN_BLOCKS) void k_onesweep(
         const uint32_t k = s_keys[j];
         const uint32_t d = (k >> shift) & 255u;
         const uint32_t dst = s_dst[d] + (uint32_t)j - s_tile_start[d];
-        kout[dst] = k;
-        vout[dst] = s_vals[j];
+        if (dst < (uint32_t)n) {
+            kout[dst] = k;
+            vout[dst] = s_vals[j];
+        }
     }
 }
 
@@ -689,12 +686,10 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
         sh.delta[cnt] = delta(codes, n, b0 + cnt - 1, b0 + cnt);
         sh.pos[cnt] = b0 + cnt;
     }
-    // the sort gave up: codes and ids are not a sorted order, whose properties all that follows needs
-    // (ids within the triangles, siblings that meet, forests that fit)
-    if (gave_up && __ldg(gave_up)) return;
     float mn[3], mx[3];
     if (i < cnt) {
-        const int prim = (mode == BVH_MODE_REFERENCE) ? l : __ldg(ids + l);
+        // (an id outside the triangles comes from a sort that gave up, below)
+        const int prim = (mode == BVH_MODE_REFERENCE) ? l : (int)min((uint32_t)__ldg(ids + l), (uint32_t)(n - 1));
         leaf_prim[l] = prim;
         gather_tri_bounds(tri, n, (reinterpret_cast<uintptr_t>(tri) & 15u) == 0, prim, mn, mx);
         if (n == 1) put_root(root_bounds, mn, mx);
@@ -709,7 +704,11 @@ __global__ __launch_bounds__(kTreeBlock, 2048 / kTreeBlock) void k_tree(const fl
         const int nlists0 = (int)min((long)kTreeGroup, count - group * kTreeGroup);
         if (i == 0) {
             __threadfence();
-            sh.last = (int)atomicAdd(group_done + group, 1u) == nlists0 - 1;
+            const bool last = (int)atomicAdd(group_done + group, 1u) == nlists0 - 1;
+            // The sort gave up: there is no tree.  A block's own climb stays within its items whatever their
+            // codes are (a subtree grows with every step, and its far ends are items), but what it left is
+            // no forest to go on with.
+            sh.last = last && !(gave_up && __ldg(gave_up));
             __threadfence();
         }
         __syncthreads();

@@ -1,7 +1,7 @@
 // The megakernel integrator's record mode (sm_103a): per-sample radiance and event hashes, one thread per
 // pixel (k_pathtrace, megakernel.cuh).  A translation unit of its own, compiled with the
 // double-precision math of libm_double in line: out of line, as the other kernels have it, this kernel's calls
-// cost it 5 % (box scene, 128 x 128, 4 spp recorded: 1.33 ms on the device in line, 1.40 out of line;
+// cost it 5 % (box scene, 128 x 128, 4 spp recorded: 1.34 ms on the device in line, 1.40 out of line;
 // k_mega the other way round, 4.74 out of line and 4.80 in line on the instanced stress scene).
 #define LTS_LIBM_CALL __forceinline__
 #include <cuda_runtime.h>
