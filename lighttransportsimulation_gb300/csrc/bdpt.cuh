@@ -19,7 +19,7 @@
 // caches.  Here a warp is at one strategy, and a kernel's body is one stage: the box lit by one
 // triangle, 256 x 256, 16 spp, 5 bounces, 81.2 -> 12.0 ms with the same contributions bit for bit
 // while the connection still traced its ray and weighted its result (10.5 of 32 lanes, waiting for
-// a warp's longest ray: 1.78 ms a chunk), 8.5 ms with the rays listed
+// a warp's longest ray: 1.78 ms a chunk), 8.6 ms with the rays listed
 // (0.41 ms a chunk connecting, 0.25 the rays, 0.31 the weights, beside 1.11 for the walks).
 //
 // The reference ships this integrator disabled and unfinished (intergrators/
@@ -56,12 +56,11 @@ enum : int { BV_CAMERA = 0, BV_LIGHT = 1, BV_SURFACE = 2 };
 
 struct BVert {
     int type;        // BV_*
-    int delta;       // surface vertex that sampled a specular lobe (0 for light and camera vertices)
     int light;       // light vertices and emitting surfaces: light index, else -1
     V3 p, n, perr;   // position, geometric normal (zero: not on a surface), position error bound
     V3 wo;           // surface: direction toward the vertex it was reached from
     Spec beta;       // throughput up to and including this vertex
-    real pdf_fwd, pdf_rev;  // area densities of sampling this vertex from either direction
+    real pdf_fwd;    // area density of a resampled light point (the walks' densities are in BdptBuf::pdf)
     Bsdf f;          // surface: its scattering functions
 };
 
@@ -296,13 +295,12 @@ __device__ __forceinline__ void bv_load(const BdptBuf& b, int slot, int k, BVert
 __device__ __forceinline__ BVert bv_camera(const BCam& cam) {
     BVert v;
     v.type = BV_CAMERA;
-    v.delta = 0;
     v.light = -1;
     v.p = cam.o;
     v.n = v3(0, 0, 0);
     v.perr = v3(0, 0, 0);
     v.beta = spec(1.0f);
-    v.pdf_fwd = v.pdf_rev = 0;
+    v.pdf_fwd = 0;
     v.f.lobe = LOBE_NONE;
     v.f.type = 0;
     return v;
@@ -331,7 +329,7 @@ constexpr int kBdptWalkThreads = 256;
 template <int LM, bool TEX, bool WIDE>
 __global__ __launch_bounds__(kBdptWalkThreads, LTS_BDPT_WALK_BLOCKS) void k_bdpt_walk(const SceneView sv, const RenderParams rp,
                                                                                       int nleaf, BdptBuf buf, long first, int n) {
-    __shared__ uint32_t s_stack[kStack * kBdptWalkThreads / 2 * 2];
+    __shared__ uint32_t s_stack[kStack * kBdptWalkThreads];
     uint32_t* stack = s_stack + (threadIdx.x / kThreads) * (kStack * kThreads) + threadIdx.x % kThreads;
     const int k = blockIdx.x * kBdptWalkThreads + threadIdx.x;
     const bool in = k < n;
@@ -580,8 +578,6 @@ __device__ __forceinline__ void bdpt_add_sample(const SceneView& sv, const Rende
         }
 }
 
-// only >= 0: the single strategy s = only / 100, t = only % 100, unweighted (each strategy alone
-// estimates its own paths; a debugging view of the estimator, as PBRT's visualizeStrategies).
 __device__ __forceinline__ void bdpt_add_splat(const SceneView& sv, real rx, real ry, Spec L, double* splat) {
     const int W = sv.width, H = sv.height;
     const int px0 = max((int)xceil(rx - 1.0f), 0), py0 = max((int)xceil(ry - 1.0f), 0);
@@ -599,6 +595,8 @@ __device__ __forceinline__ void bdpt_add_splat(const SceneView& sv, real rx, rea
         }
 }
 
+// only >= 0 (here and below): the single strategy s = only / 100, t = only % 100, unweighted (each strategy
+// alone estimates its own paths; a debugging view of the estimator, as PBRT's visualizeStrategies).
 // s = 1: the light point sampled from camera vertex pt of strategy (1, t), into qs; false: no light
 // reaches pt from it.
 template <int LM>

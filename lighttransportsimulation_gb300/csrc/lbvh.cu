@@ -3,10 +3,12 @@
 //                                                                 Geometry.cuh:647-655
 //   2 k_morton         centroid -> 30-bit Morton code + ids, and the 4x256 radix histograms
 //                                                                 BVH.cuh:101-116,134-137, Bound.cuh:169-175
-//   3 k_digit_prefix + 4 x k_onesweep   stable LSD radix sort of (code, id), 8-bit digits,
-//                      decoupled look-back (replaces thrust::stable_sort_by_key, BVH.cuh:140-146)
+//   3 4 x k_onesweep   stable LSD radix sort of (code, id), 8-bit digits, decoupled look-back, after
+//                      k_digit_prefix above 500,000 keys (replaces thrust::stable_sort_by_key,
+//                      BVH.cuh:140-146); up to 4,096 keys 1 to 3 are one block, k_small_sort
 //   4 k_tree           Karras topology and bottom-up AABBs in one climb
 //                                                                 BVH.cuh:173-262
+//   5 k_dump           the reference's flattened order            BVH.cuh:311-329
 // Output layout: one 64-byte node per interior node carrying both child boxes (see lbvh.cuh).
 #include <cuda/atomic>
 #include <cuda_runtime.h>
@@ -516,10 +518,14 @@ __device__ __forceinline__ int delta(const uint32_t* __restrict__ c, int n, int 
 //    kernel through arrival words in device memory, one dependent chain of exchanges per edge:
 //    24 us for 1,280 triangles, 47 for 200,000, 94 for 16M.)
 // Leaves (threads) per block: 512, or 256 above kTreeLarge leaves, where shorter longest climbs beat
-// the levels of merging they add (16M, sorted: 0.96 ms against 1.04; 1M: 0.097 against 0.094).
+// the levels of merging they add (16M, sorted: 0.96 ms against 1.04; 1M: 0.097 against 0.094; the line lies
+// between the two, its crossing is not measured).
 constexpr int kTreeLarge = 4000000;
 __host__ __device__ constexpr int tree_block(long n) { return n > kTreeLarge ? 256 : 512; }
-constexpr int kTreeGroup = 24;  // forests merged by one block: 24 x ~18 subtrees fill its threads
+// Forests merged by one block.  Random triangles leave 9.3 subtrees a block of 512 at the first level, 223 items
+// for the 512 threads, and longer forests above it; codes that close in on a block's edges leave up to 26, which
+// the merge then takes in chunks.
+constexpr int kTreeGroup = 24;
 constexpr int kForestCap = 128;  // entries of 32 bytes per block: up to 127 subtrees, the last word their count
 
 // One subtree of a forest: box, reference, last leaf (it begins after its predecessor's).
@@ -796,7 +802,8 @@ __global__ __launch_bounds__(kBlock) void k_dump(const BvhNode* __restrict__ nod
 // Sort tiles: kSortItems keys per thread once the tiles fill the SMs' resident blocks; smaller tiles
 // below that, whose passes are a tile's latency (a chain of ranking steps) and the look-back over
 // all tiles at once (400,000 keys, ms of the four passes: 15 keys and 4 tiles a round trip 0.055, 4
-// and 16 0.059, 8 and 16 0.051, 8 and 32 0.066, 10 and 16 0.051; at 700,000 15 keys are faster).
+// and 16 0.059, 8 and 16 0.051, 8 and 32 0.066, 10 and 16 0.051; at 700,000 15 keys are faster;
+// the line lies between the two, its crossing is not measured).
 constexpr int kSortSmallMax = 500000, kSortSmallItems = 8, kSortSmallLookback = 16, kSortLookback = 4;
 // Triangles per thread of the two streaming kernels before every SM has its eight blocks: each block
 // ends with atomics on the same words (400,000 triangles: Morton codes 12.2 us, 18.4 at one).
@@ -976,7 +983,7 @@ void Lbvh::stage_ms(float out[5]) const {
 // memory-pool callback, real-time render loops that forbid cudaMalloc/cudaFree (both can
 // synchronise the whole device), and plugins whose host application owns every device
 // allocation.  This variant keeps all of the build's scratch (the sort's ping-pong buffers and
-// look-back table, histograms, the tree's arrival words, the scene box and an error word) in
+// look-back table, histograms, the tree's forests and group counters, the scene box and an error word) in
 // one file-scope device array of fixed size, so a call allocates nothing; the caller supplies the
 // triangles and every output buffer.
 //

@@ -1,6 +1,6 @@
-// The one-launch integrators in float (sm_103a): the path-tracing megakernel (one thread per pixel
-// and slice of its samples, as the reference's PathTracingKernel, intergrators/
-// IntegratorKernels.cu:17-23) and the bidirectional integrator (bdpt.cuh).
+// The float integrators beside the wavefront (sm_103a): the path-tracing megakernel, one launch (one
+// thread per pixel and slice of its samples, as the reference's PathTracingKernel, intergrators/
+// IntegratorKernels.cu:17-23), and the bidirectional integrator, five launches a chunk (bdpt.cuh).
 //
 // Differences in mechanism, not in arithmetic:
 //  - scene tables are SoA arrays and materials/lights are `switch`-dispatched records, so the

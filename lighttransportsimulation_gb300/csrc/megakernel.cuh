@@ -1,8 +1,9 @@
 // Path-tracing megakernel: one thread per pixel, all samples and bounces, as the reference's
 // PathTracingKernel (intergrators/IntegratorKernels.cu:17-23) runs
 // PathTracingIntegrator::evaluate (intergrators/PathTracingIntegrator.cuh:26-109).  Compiled in
-// `real` = real by tracer.cu (the megakernel integrator) and in `real` = double by render64.cu
-// (the FP64 oracle renderer).
+// `real` = float by pathtrace.cu (the megakernel integrator's record mode) and in `real` = double by
+// render64.cu (the FP64 oracle renderer); mega.cu has the megakernel without record mode and takes the
+// film's sum from here.
 #pragma once
 
 #include "tracer_dev.cuh"

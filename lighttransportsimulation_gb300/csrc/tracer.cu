@@ -1,6 +1,6 @@
 // The renderer's host side and its set-up kernels (sm_103a): scene upload, traversal structures,
-// film resolve, ray queries and the wavefront path tracer (wavefront.cuh).  The one-launch
-// integrators are in mega.cu.
+// film resolve, ray queries and the wavefront path tracer (wavefront.cuh).  The megakernel and the
+// bidirectional integrator are in mega.cu, the megakernel's record mode in pathtrace.cu.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -1109,8 +1109,9 @@ std::string Tracer::render_async(const HostScene& sc, const Lbvh& bvh, const lts
     if (d.integrator == LTS_INTEGRATOR_WAVEFRONT) return render_wavefront(sc, bvh, d, s, d_err, rp, sv, ns);
     long bdpt_cap = 0;
     if (d.integrator == LTS_INTEGRATOR_BDPT) {
-        // one chunk's workspace, kept: 2^18 samples keep every SM busy over the chunk's launches
-        // (0.9 GB at five bounces); fewer when that much cannot be allocated
+        // one chunk's workspace, kept until the context ends: 2^18 samples keep every SM busy over the
+        // chunk's launches (0.9 GB at five bounces, 1.6 GB at eight, which is its limit); fewer when that much
+        // cannot be allocated
         const size_t per = bdpt_sample_bytes(d.max_bounce, bdpt_strategy);
         bdpt_cap = std::min<long>((ns + 31) / 32 * 32, 1l << 18);
         while (bdpt_ws_cap_ < per * bdpt_cap) {

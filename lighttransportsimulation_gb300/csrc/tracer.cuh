@@ -128,7 +128,7 @@ std::string set_libm_double(int on);
 // Known-answer check of single float device functions (lts_debug_kat): n records of 16 floats.
 std::string kat_launch(int fn, const float* d_in, int n, float* d_out, cudaStream_t s);
 
-// The float one-launch integrators (mega.cu): the path-tracing megakernel and the bidirectional
+// The float integrators of mega.cu: the path-tracing megakernel without record mode and the bidirectional
 // integrator; set_libm_double of that translation unit.  matte_only: every material is Lambertian
 // or Oren-Nayar with constant textures.
 std::string mega_launch(const SceneView& sv, const RenderParams& rp, int nleaf, bool matte_only, cudaStream_t s);

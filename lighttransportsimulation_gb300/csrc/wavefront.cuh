@@ -294,8 +294,8 @@ __device__ __forceinline__ void wf_ray_end(int kind, const Trav& t, const SceneV
 constexpr int kRefillIdle = LTS_REFILL_IDLE;
 // Resident blocks per SM the trace kernel is compiled for (caps its registers): 8 blocks = 32
 // warps at 64 registers without spills; the kernel waits on node and triangle loads, and the
-// extra warps hide them (stress scene: trace 420 ms per render at 8, 444 at 7, 484 at 6; 9 and
-// 10 spill).
+// extra warps hide them (stress scene, 256 spp, before a node was visited ahead: trace 420 ms per render
+// at 8, 444 at 7, 484 at 6; 9 and 10 spill.  400 at 8 now).
 #ifndef LTS_TRACE_MIN_BLOCKS
 #define LTS_TRACE_MIN_BLOCKS 8
 #endif
@@ -583,7 +583,8 @@ __device__ __forceinline__ void shade_one(const SceneView& sv, const RenderParam
 }
 
 // shade over one class's list (k_wf_classify), grid-stride: one launch per shade class present in
-// the scene, each compiled for its material kind (fewer registers, no spills, a smaller kernel).
+// the scene, each compiled for its material kind (a smaller kernel, and fewer spills at 96 registers: bytes
+// stored / loaded 36 / 108 glass, 62 / 176 mirror, 108 / 196 matte, 106 / 240 conductor, 380 / 472 every lobe).
 template <bool RECORD, int LM, bool TEX>
 __global__ __launch_bounds__(kShadeBlock, 1) void k_wf_shade(const SceneView sv, const RenderParams rp,
                                                                                  WfState st, int pool, int cls) {
@@ -698,8 +699,8 @@ __device__ __forceinline__ void finalize_one(const SceneView& sv, const RenderPa
     st.pend[p] = WF_FREE;
 }
 // Compiled for eight blocks per SM (64 registers): a path is a few dependent loads, and the rare
-// surface interaction of a MIS ray's light need not set everyone's occupancy (stress 1920x1080x64:
-// 12.9 ms per render, 16.5 at 79 registers, 13.3 at twelve blocks, 15.0 at sixteen).
+// surface interaction of a MIS ray's light need not set everyone's occupancy, at 32 / 40 bytes spilled (stress
+// 1920x1080x64: 12.9 ms per render, 16.5 at 79 registers, 13.3 at twelve blocks, 15.0 at sixteen).
 template <bool RECORD>
 __global__ __launch_bounds__(kWfBlock, 8) void k_wf_finalize(const SceneView sv, const RenderParams rp, WfState st,
                                                           const int32_t* __restrict__ q, const WfCtl* __restrict__ ctl) {
