@@ -775,7 +775,7 @@ int ray_queries(lts_ctx* ctx, const float* o, const float* d, const float* tmax,
     }
     if (n == 0) return LTS_OK;
     // rays, then results; up to kDumpKeep bytes stay with the context
-    const size_t N = (size_t)n, rays = d ? 24 * N + 4 * (one_tmax ? 4 : N) : 32 * N, bytes = rays + 8 * N;
+    const size_t N = (size_t)n, rays = d ? 24 * N + 4 * (one_tmax ? 4 : N) : 32 * N, bytes = rays + 8 * N + 4;
     unsigned char* ws = static_cast<unsigned char*>(ctx->ray_ws);
     if (ctx->ray_ws_cap < bytes) {
         dev_free(ctx->ray_ws);
@@ -792,12 +792,13 @@ int ray_queries(lts_ctx* ctx, const float* o, const float* d, const float* tmax,
     float* d_tmax = d ? d_d + 3 * N : nullptr;
     int32_t* d_prim = reinterpret_cast<int32_t*>(ws + rays);
     float* d_t = t ? reinterpret_cast<float*>(d_prim + N) : nullptr;
-    // a small batch goes up and comes back in one copy each (a single closest-hit query: 82 us with a copy
-    // per array, 61 so; the copies' fixed costs are its time)
+    // a small batch goes up in one copy and comes back in one, the device error word behind its results (a single
+    // closest-hit query: 82 us with a copy per array and the word read by itself, 62 so; the copies' fixed costs
+    // are its time)
     const bool small = N <= kSmallRays;
     const size_t nt = one_tmax ? 1 : N;
     float pack[7 * kSmallRays];
-    uint32_t both[2 * kSmallRays];
+    uint32_t back[2 * kSmallRays + 1];
     cudaError_t e;
     if (!d) {
         e = cudaMemcpyAsync(d_o, o, 32 * N, cudaMemcpyHostToDevice, ctx->stream);
@@ -812,13 +813,13 @@ int ray_queries(lts_ctx* ctx, const float* o, const float* d, const float* tmax,
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_tmax, tmax, 4 * nt, cudaMemcpyHostToDevice, ctx->stream);
     }
     std::string msg;
-    const uint32_t* host_err = nullptr;
     if (e == cudaSuccess)
-        msg = ctx->tracer->intersect(*ctx->bvh, d_o, d_d, d_tmax, one_tmax, n, any, d_prim, d_t, ctx->stream, ctx->d_error,
-                                     &host_err);
+        msg = ctx->tracer->intersect(*ctx->bvh, d_o, d_d, d_tmax, one_tmax, n, any, d_prim, d_t, ctx->stream, ctx->d_error);
+    const size_t words = t ? 2 * N : N;  // d_t follows d_prim
     if (e == cudaSuccess && msg.empty()) {
-        if (small && t) {  // d_t follows d_prim
-            e = cudaMemcpyAsync(both, d_prim, 8 * N, cudaMemcpyDeviceToHost, ctx->stream);
+        if (small) {
+            e = cudaMemcpyAsync(d_prim + words, ctx->d_error, 4, cudaMemcpyDeviceToDevice, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_prim, 4 * (words + 1), cudaMemcpyDeviceToHost, ctx->stream);
         } else {
             e = cudaMemcpyAsync(prim, d_prim, 4 * N, cudaMemcpyDeviceToHost, ctx->stream);
             if (e == cudaSuccess && t) e = cudaMemcpyAsync(t, d_t, 4 * N, cudaMemcpyDeviceToHost, ctx->stream);
@@ -829,11 +830,10 @@ int ray_queries(lts_ctx* ctx, const float* o, const float* d, const float* tmax,
     if (ws != ctx->ray_ws) dev_free(ws);
     if (!msg.empty()) return fail(ctx, LTS_ERR_CUDA, msg);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "ray query");
-    if (small && t) {
-        memcpy(prim, both, 4 * N);
-        memcpy(t, both + N, 4 * N);
-    }
-    return *host_err ? check_device_error(ctx) : LTS_OK;
+    if (!small) return check_device_error(ctx);
+    memcpy(prim, back, 4 * N);
+    if (t) memcpy(t, back + N, 4 * N);
+    return back[words] ? check_device_error(ctx) : LTS_OK;
 }
 }  // namespace
 

@@ -966,16 +966,12 @@ std::string Tracer::traversal_view(const Lbvh& bvh, cudaStream_t s, uint32_t* d_
 }
 
 std::string Tracer::intersect(const Lbvh& bvh, const float* d_o, const float* d_d, const float* d_tmax, bool one_tmax, int n,
-                              int any, int32_t* d_prim, float* d_t, cudaStream_t s, uint32_t* d_err,
-                              const uint32_t** host_err) {
+                              int any, int32_t* d_prim, float* d_t, cudaStream_t s, uint32_t* d_err) {
     if (bvh.n != view_.ntri) return "bad argument: BVH does not match the scene";
     SceneView sv;
     const std::string e = traversal_view(bvh, s, d_err, &sv);
     if (!e.empty()) return e;
     if (n <= 0) return "";
-    HostWords* w = nullptr;
-    const std::string pe = pinned(&w);
-    if (!pe.empty()) return pe;
     const RayBatch batch{d_o, d_d, d_tmax, one_tmax ? 0 : 1};
     if (sv.wnodes && sv.ninst == 0) {
         if (isect_grid_ == 0) {
@@ -998,8 +994,6 @@ std::string Tracer::intersect(const Lbvh& bvh, const float* d_o, const float* d_
         k<<<grid, kThreads, 0, s>>>(sv, bvh.n, batch, n, d_prim, d_t, d_err);
     }
     TRY(cudaGetLastError());
-    TRY(cudaMemcpyAsync(&w->err, d_err, 4, cudaMemcpyDeviceToHost, s));
-    *host_err = &w->err;
     return "";
 }
 

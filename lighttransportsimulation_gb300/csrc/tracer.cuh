@@ -228,10 +228,9 @@ class Tracer {
 
     // Batch ray queries (lts_intersect, lts_intersect_arrays) over device arrays: d_tmax null, d_o
     // holds n x {o.xyz, tmax, d.xyz, 0}; else d_o, d_d n x 3 and d_tmax one value or n.  any = 0
-    // closest hit -> prim (-1: none) and t; any = 1 -> prim 1 (occluded) or 0.  d_t may be null.  The
-    // device error word after the queries is *host_err once the stream has been waited for.
+    // closest hit -> prim (-1: none) and t; any = 1 -> prim 1 (occluded) or 0.  d_t may be null.
     std::string intersect(const Lbvh& bvh, const float* d_o, const float* d_d, const float* d_tmax, bool one_tmax, int n,
-                          int any, int32_t* d_prim, float* d_t, cudaStream_t s, uint32_t* d_err, const uint32_t** host_err);
+                          int any, int32_t* d_prim, float* d_t, cudaStream_t s, uint32_t* d_err);
 
     // n image-texture lookups (Mipmap::lookUp) of image `idx` at d_st[2n] into d_rgb[3n].
     std::string image_lookup(int idx, const float* d_st, int n, float* d_rgb, cudaStream_t s);
