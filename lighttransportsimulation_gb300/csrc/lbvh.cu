@@ -533,12 +533,12 @@ struct alignas(16) ForestEntry {
     float4 a;  // min.xyz, max.x
     float4 b;  // max.yz, reference bits, last leaf bits
 };
-__host__ __device__ constexpr long tree_blocks(long n) { return (n + tree_block(n) - 1) / tree_block(n); }
-constexpr size_t forest_bytes(long n) { return (size_t)tree_blocks(n) * kForestCap * sizeof(ForestEntry); }
+constexpr long tree_blocks(long n, int block) { return (n + block - 1) / block; }
+constexpr size_t forest_bytes(long n, int block) { return (size_t)tree_blocks(n, block) * kForestCap * sizeof(ForestEntry); }
 // Completion counters: one per group of every level.
-constexpr long tree_counters(long n) {
+constexpr long tree_counters(long n, int block) {
     long c = 0;
-    for (long m = tree_blocks(n); m > 1; m = (m + kTreeGroup - 1) / kTreeGroup) c += (m + kTreeGroup - 1) / kTreeGroup;
+    for (long m = tree_blocks(n, block); m > 1; m = (m + kTreeGroup - 1) / kTreeGroup) c += (m + kTreeGroup - 1) / kTreeGroup;
     return c;
 }
 
@@ -815,15 +815,16 @@ constexpr long sort_tiles(long n) { return (n + sort_tile(n) - 1) / sort_tile(n)
 // whether the sort gave up (4), histograms (4 x 256), the tree's group counters, then the sort's
 // look-back table.
 constexpr size_t kZeroGaveUp = 12, kZeroHist = 16, kZeroGroups = kZeroHist + 4 * 256;
-constexpr size_t zero_status(long n) { return kZeroGroups + ((size_t)tree_counters(n) + 7) / 8 * 8; }
+constexpr size_t zero_status(long n) { return kZeroGroups + ((size_t)tree_counters(n, tree_block(n)) + 7) / 8 * 8; }
 constexpr size_t zero_words(long n) { return zero_status(n) + 4 * 256 * (size_t)sort_tiles(n); }
 
 // The build's launches, shared by Lbvh and the allocation-free entry point.  kalt / valt: the sort's
-// second key and value buffers; `zero`: zero_words(n) words; `forest`: forest_bytes(n).  mark(k) is
-// called before stage k (bounds, Morton codes, sort, clear, tree) and after the last.
+// second key and value buffers; `zero`: zero_words(n) words; `block`: leaves per block of the tree,
+// tree_block(n) or 512; `forest`: forest_bytes(n, block).  mark(k) is called before stage k (bounds, Morton
+// codes, sort, clear, tree) and after the last.
 template <class Mark>
 cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, uint32_t* codes, int32_t* ids, uint32_t* kalt,
-                           int32_t* valt, uint32_t* zero, ForestEntry* forest, BvhNode* nodes, int32_t* leaf_prim,
+                           int32_t* valt, uint32_t* zero, int block, ForestEntry* forest, BvhNode* nodes, int32_t* leaf_prim,
                            float* root_bounds, uint32_t* err, int sms, cudaStream_t s, int* launches, Mark mark) {
     uint32_t* const groups = zero + kZeroGroups;
     uint32_t* gave_up = nullptr;  // the one-block sort waits for nothing
@@ -831,7 +832,7 @@ cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, ui
     if (n <= kSmallSort) {
         mark(1);
         mark(2);
-        k_small_sort<<<1, kSmallThreads, 0, s>>>(tri, n, code_limit, codes, ids, groups, (int)tree_counters(n));
+        k_small_sort<<<1, kSmallThreads, 0, s>>>(tri, n, code_limit, codes, ids, groups, (int)tree_counters(n, block));
         *launches = 2;
     } else {
         cudaError_t e = cudaMemsetAsync(zero, 0, 4 * zero_words(n), s);
@@ -860,8 +861,8 @@ cudaError_t build_launches(const float* tri, int n, int mode, int code_limit, ui
     }
     mark(3);
     mark(4);
-    auto tree = tree_block(n) == 512 ? k_tree<512> : k_tree<256>;
-    tree<<<(int)tree_blocks(n), tree_block(n), 0, s>>>(tri, n, mode, ids, codes, nodes, forest, groups, leaf_prim, root_bounds,
+    auto tree = block == 512 ? k_tree<512> : k_tree<256>;
+    tree<<<(int)tree_blocks(n, block), block, 0, s>>>(tri, n, mode, ids, codes, nodes, forest, groups, leaf_prim, root_bounds,
                                                                   gave_up, err);
     mark(5);
     return cudaGetLastError();
@@ -907,8 +908,21 @@ std::string Lbvh::reserve(int nn) {
     LTS_TRY(al((void**)&leaf_prim, 4 * N));
     LTS_TRY(al((void**)&codes, 4 * N));
     LTS_TRY(al((void**)&ids, 4 * N));
-    // the sort's ping-pong keys and ids, one allocation: after the sort it holds the tree's forests
-    LTS_TRY(al((void**)&codes_alt_, std::max({8 * N, forest_bytes(nn), forest_bytes(std::min(nn, kTreeLarge))})));
+    // the sort's ping-pong keys and ids, one allocation: after the sort it holds the tree's forests.  Those of
+    // blocks of 256 leaves need twice what the sort does (134 MB more at 16M); where that cannot be had, the
+    // tree is built by blocks of 512.
+    const size_t sort_bytes = std::max(8 * N, forest_bytes(nn, 512));
+    small_blocks_ = tree_block(nn) == 256;
+    if (small_blocks_) {
+        const cudaError_t e = al((void**)&codes_alt_, std::max(sort_bytes, forest_bytes(nn, 256)));
+        if (e != cudaSuccess) {
+            if (e != cudaErrorMemoryAllocation) LTS_TRY(e);
+            cudaGetLastError();
+            small_blocks_ = false;
+            bytes_ -= std::max(sort_bytes, forest_bytes(nn, 256));
+        }
+    }
+    if (!small_blocks_) LTS_TRY(al((void**)&codes_alt_, sort_bytes));
     ids_alt_ = reinterpret_cast<int32_t*>(codes_alt_ + N);
     // a smaller build may take smaller sort tiles, hence more of them than a larger one
     LTS_TRY(al((void**)&zero_, 4 * std::max(zero_words(nn), zero_words(std::min(nn, kSortSmallMax)))));
@@ -930,6 +944,7 @@ std::string Lbvh::build(const float* d_tri, int nn, int md, int code_limit, cuda
     LTS_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     cudaError_t me = cudaSuccess;
     LTS_TRY(build_launches(d_tri, nn, md, code_limit, codes, ids, codes_alt_, ids_alt_, zero_,
+                           small_blocks_ ? tree_block(nn) : 512,
                            reinterpret_cast<ForestEntry*>(codes_alt_), nodes, leaf_prim, root_bounds, d_error, sms, s, &launches,
                            [&](int k) {
                                const cudaError_t e = cudaEventRecord(ev_[k], s);
@@ -1005,7 +1020,7 @@ constexpr int kNoAllocMaxPrims = 1 << 18;
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kOffCodes = 0;
 constexpr size_t kOffIds = kOffCodes + 4ull * kNoAllocMaxPrims;
-static_assert(kOffIds + 4ull * kNoAllocMaxPrims >= forest_bytes(kNoAllocMaxPrims), "the tree's forests lie in both sort buffers");
+static_assert(tree_block(kNoAllocMaxPrims) == 512 && kOffIds + 4ull * kNoAllocMaxPrims >= forest_bytes(kNoAllocMaxPrims, 512), "the tree's forests lie in both sort buffers");
 constexpr size_t kOffZero = align256(kOffIds + 4ull * kNoAllocMaxPrims);
 constexpr size_t kOffError = kOffZero + align256(4 * zero_words(kNoAllocMaxPrims));
 constexpr size_t kNoAllocBytes = kOffError + 256;
@@ -1057,7 +1072,7 @@ extern "C" int lts_bvh_build_noalloc(const float* d_tri, int32_t n, int32_t mode
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return LTS_ERR_CUDA;
     const bool waits = n > kSmallSort;  // the sort's look-back: the only wait that can run out
     if (waits && cudaMemsetAsync(err, 0, 4, s) != cudaSuccess) return LTS_ERR_CUDA;
-    if (build_launches(d_tri, n, mode, code_limit, d_codes, d_ids, codes_alt, ids_alt, zero,
+    if (build_launches(d_tri, n, mode, code_limit, d_codes, d_ids, codes_alt, ids_alt, zero, 512,
                        reinterpret_cast<ForestEntry*>(codes_alt), static_cast<BvhNode*>(d_nodes), d_leaf_prim, d_root_bounds, err,
                        sms, s, &launches, [](int) {}) != cudaSuccess)
         return LTS_ERR_CUDA;

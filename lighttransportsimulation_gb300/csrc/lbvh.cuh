@@ -57,6 +57,7 @@ class Lbvh {
     std::string reserve(int n);
     void release();
     int cap_ = 0;
+    bool small_blocks_ = false;  // the buffers hold the forests of the large trees' blocks of 256 leaves
     size_t bytes_ = 0;
     uint32_t *codes_alt_ = nullptr, *zero_ = nullptr;  // sort buffers, then the tree's forests; words zeroed per build
     int32_t* ids_alt_ = nullptr;  // second half of codes_alt_'s allocation

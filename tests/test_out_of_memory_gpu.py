@@ -114,3 +114,25 @@ ctx.close()
 """, 7)
     assert r["rc"] == 0 and r["part"] == 0 and r["device_mb"] < 7, r
     assert r["order"] and r["tree"] and r["key"], r
+
+
+def test_a_large_tree_without_memory_for_its_small_blocks(built_lib):
+    """4,200,000 triangles: 391 MB with the forests of blocks of 256 leaves, 357 MB with those of 512, which is
+    what 360 MB (377 million bytes) hold.  Both blocks build the same tree."""
+    body = r"""
+import hashlib
+n = 4200000
+g = torch.Generator(device="cuda").manual_seed(3)
+x = (torch.rand((n, 1, 3), generator=g, device="cuda") + torch.randn((n, 3, 3), generator=g, device="cuda") * 1e-3).reshape(-1)
+torch.cuda.synchronize()
+ctx = lts.Context(0)
+ctx.check(lib.lts_bvh_build_device_async(ctx.h, ctypes.c_void_p(x.data_ptr()), n, lts.BVH_SORTED, -1))
+out["mb"] = ctx.metrics().device_bytes / 1e6
+a, d = lts._dump_arrays(n)
+ctx.check(lib.lts_bvh_dump_get(ctx.h, ctypes.byref(d)))
+out["tree"] = hashlib.sha256(b"".join(a[k].tobytes() for k in sorted(a))).hexdigest()
+ctx.close()
+"""
+    small, large = child(body, 360), child(body, 4096)
+    assert small["mb"] < 377 < large["mb"], (small, large)
+    assert small["tree"] == large["tree"]
