@@ -630,19 +630,18 @@ std::string umma_probe(int mode, int swap, const uint16_t* a, const uint16_t* b,
 }
 
 
-Mlp::~Mlp() {
-    dev_free(w32_);
-    dev_free(grad_);
-    dev_free(m_);
-    dev_free(v_);
-    dev_free(w16_);
-    dev_free(e32_);
-    dev_free(e16_);
-    dev_free(loss_);
+void Mlp::release() {
+    for (void* p : {(void*)w32_, (void*)grad_, (void*)m_, (void*)v_, (void*)w16_, (void*)e32_, (void*)e16_, (void*)loss_}) dev_free(p);
+    w32_ = grad_ = m_ = v_ = e32_ = loss_ = nullptr;
+    w16_ = e16_ = nullptr;
+    allocated_ = false;
 }
 
+Mlp::~Mlp() { release(); }
+
 std::string Mlp::init(uint32_t seed, cudaStream_t s) {
-    if (!w32_) {
+    if (!allocated_) {
+        release();  // what an init that failed part way has left
         TRY(dev_alloc((void**)&w32_, 4 * kMlpParams));
         TRY(dev_alloc((void**)&grad_, 4 * kMlpParams));
         TRY(dev_alloc((void**)&m_, 4 * kMlpParams));
@@ -659,6 +658,7 @@ std::string Mlp::init(uint32_t seed, cudaStream_t s) {
         TRY(cudaFuncSetAttribute(k_mlp_forward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
         blocks_train_ = sms;
         blocks_fwd_ = sms;  // one CTA of kFwdGroups tiles per SM
+        allocated_ = true;
     }
     // He-uniform weights, xorshift32 stream from the seed; W5 rows 3..15 zero
     std::vector<float> w(kMlpParams, 0.0f);
@@ -685,7 +685,7 @@ std::string Mlp::sync_bf16(cudaStream_t s) {
 }
 
 std::string Mlp::set_params(const float* host, cudaStream_t s) {
-    if (!w32_) return "MLP not initialised";
+    if (!allocated_) return "MLP not initialised";
     TRY(cudaMemcpyAsync(w32_, host, 4 * kMlpParams, cudaMemcpyHostToDevice, s));
     TRY(cudaMemsetAsync(grad_, 0, 4 * kMlpParams, s));
     TRY(cudaMemsetAsync(m_, 0, 4 * kMlpParams, s));
@@ -698,14 +698,14 @@ std::string Mlp::set_params(const float* host, cudaStream_t s) {
 }
 
 std::string Mlp::get_params(float* host, cudaStream_t s) {
-    if (!w32_) return "MLP not initialised";
+    if (!allocated_) return "MLP not initialised";
     TRY(cudaMemcpyAsync(host, w32_, 4 * kMlpParams, cudaMemcpyDeviceToHost, s));
     TRY(cudaStreamSynchronize(s));
     return "";
 }
 
 std::string Mlp::get_grad(float* host, cudaStream_t s) {
-    if (!w32_) return "MLP not initialised";
+    if (!allocated_) return "MLP not initialised";
     TRY(cudaMemcpyAsync(host, grad_, 4 * kMlpParams, cudaMemcpyDeviceToHost, s));
     TRY(cudaStreamSynchronize(s));
     return "";
@@ -737,7 +737,7 @@ bool feature_map(const uint16_t* d_feat, int n, int cols, CUtensorMapSwizzle swi
 
 std::string Mlp::forward(const uint16_t* d_feat, int n, float* d_out, uint32_t* d_err, cudaStream_t s,
                          const int32_t* d_rows, int out_stride, const uint32_t* d_n) {
-    if (!w32_) return "MLP not initialised";
+    if (!allocated_) return "MLP not initialised";
     if (n <= 0) return "";
     const int tiles = (n + 127) / 128;
     // features in row order come through tensor maps of this call's buffer (96 columns as 64 + 32)
@@ -753,7 +753,7 @@ std::string Mlp::forward(const uint16_t* d_feat, int n, float* d_out, uint32_t* 
 
 std::string Mlp::train_step(const uint16_t* d_feat, const float* d_target, int n, float lr, float* d_loss,
                             uint32_t* d_err, cudaStream_t s) {
-    if (!w32_) return "MLP not initialised";
+    if (!allocated_) return "MLP not initialised";
     if (n <= 0) return "";
     TRY(cudaMemsetAsync(grad_, 0, 4 * kMlpParams, s));
     TRY(cudaMemsetAsync(d_loss, 0, 4, s));
@@ -764,7 +764,7 @@ std::string Mlp::train_step(const uint16_t* d_feat, const float* d_target, int n
 }
 
 std::string Mlp::adam(float lr, cudaStream_t s) {
-    if (!w32_) return "MLP not initialised";
+    if (!allocated_) return "MLP not initialised";
     ++steps;
     const float b1 = 0.9f, b2 = 0.99f;
     const float c1 = 1.0f - std::pow(b1, (float)steps), c2 = 1.0f - std::pow(b2, (float)steps);

@@ -59,7 +59,7 @@ class Mlp {
     // One Adam step with the gradient buffer (zeroes it).
     std::string adam(float lr, cudaStream_t s);
 
-    bool ready() const { return w32_ != nullptr; }
+    bool ready() const { return allocated_; }
     float* scratch_loss() const { return loss_; }  // one device float for callers that drop the loss
     int steps = 0;
 
@@ -69,6 +69,8 @@ class Mlp {
     float* e32_ = nullptr;  // weight average (inference), FP32 and BF16
     uint16_t* e16_ = nullptr;
     int blocks_train_ = 0, blocks_fwd_ = 0;
+    bool allocated_ = false;  // every buffer above
+    void release();
     std::string sync_bf16(cudaStream_t s);
 };
 

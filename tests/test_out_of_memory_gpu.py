@@ -136,3 +136,26 @@ ctx.close()
     small, large = child(body, 360), child(body, 4096)
     assert small["mb"] < 377 < large["mb"], (small, large)
     assert small["tree"] == large["tree"]
+
+
+def test_a_network_that_did_not_fit(built_lib):
+    """A tree of 8,000 triangles leaves a third of 1 MB, the network needs half of it: its calls are then refused
+    as they are without one, and a context with room has one."""
+    r = child(r"""
+x = torch.from_numpy(scenes.random_triangles(8000, seed=1).reshape(-1).copy()).cuda()
+f, o = torch.zeros((64, 96), dtype=torch.bfloat16, device="cuda"), torch.zeros((64, 3), device="cuda")
+torch.cuda.synchronize()
+ctx = lts.Context(0)
+ctx.check(lib.lts_bvh_build_device_async(ctx.h, ctypes.c_void_p(x.data_ptr()), 8000, lts.BVH_SORTED, -1))
+call = lambda c: lib.lts_mlp_forward_device_async(c.h, ctypes.c_void_p(f.data_ptr()), 64, ctypes.c_void_p(o.data_ptr()))
+out["init"] = [lib.lts_mlp_init(ctx.h, 1), lib.lts_mlp_init(ctx.h, 1)]
+out["call"] = call(ctx)
+ctx.close()
+ctx = lts.Context(0)
+out["again"] = [lib.lts_mlp_init(ctx.h, 1), call(ctx)]
+torch.cuda.synchronize()
+out["ones"] = bool((o == 1).all())  # every activation of zero features is 0, and exp(0) is 1
+ctx.close()
+""", 1)
+    assert r["init"][0] != 0 and r["init"][1] != 0 and r["call"] == 7, r  # LTS_ERR_STATE
+    assert r["again"] == [0, 0] and r["ones"], r
